@@ -30,7 +30,10 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .plan import AttentionPlan, GemmPlan, SoftmaxPlan, _host_i64
+from . import _ops
+from .plan import GemmPlan, _host_i64
+
+_ops.setup(_host_i64, L.BlkError)
 
 _CACHE: "OrderedDict[tuple, object]" = OrderedDict()
 _CACHE_MAX = 32
@@ -76,6 +79,7 @@ def _cached(key, build):
 
 def clear_plan_cache() -> None:
     """Forgets every cached plan and list (plans still referenced elsewhere stay usable)."""
+    _ops.clear()
     _CACHE.clear()
     _LISTS.clear()
 
@@ -84,89 +88,11 @@ def check_plans() -> None:
     """Synchronises the current stream of every cached plan's device and raises ``BlkError``
     (``BLK_ERR_TIMEOUT``) if a kernel of one of them gave up a bounded device-side wait since the last check --
     the result of that call is then incomplete.  ``BLK_CHECK=1`` in the environment does this after every run."""
+    _ops.check()
     for plan in list(_CACHE.values()):
         inner = getattr(plan, "plan", plan)   # a host pipe wraps its plan
         if getattr(inner, "device", None) is not None:
             inner.check()
-
-
-def _check_operand(name: str, t: torch.Tensor) -> None:
-    # the two TORCH_CHECKs of upstream csrc/sparseBlockedAttention.h:6-8
-    if not isinstance(t, torch.Tensor) or not t.is_cuda:
-        raise RuntimeError(f"{name} must be CUDA Tensor")
-    if not t.is_contiguous():
-        raise RuntimeError(f"{name} must be contiguous Tensor")
-
-
-def _lists_from_offsets(a1, a2, ao):
-    a1, a2, ao = _host_i64(a1), _host_i64(a2), _host_i64(ao)
-    S = len(a1) - 1
-    M = np.empty(S, np.int64); N = np.empty(S, np.int64); K = np.empty(S, np.int64)
-    L.check(L.lib.blk_lists_from_offsets(L.i64(a1), L.i64(a2), L.i64(ao), S, L.i64(M), L.i64(N), L.i64(K)))
-    return M, N, K
-
-
-def _gemm_backward(ctx_meta, mat1, mat2, grad_out, scale):
-    """The two launches of upstream sparseBlockedGEMM::backward (csrc/sparseBlockedAttention.cpp:52-72):
-    mat1Grad = blockedGEMM(outGrad, mat2; offsets (out, mat2, mat1); lists (M, K, N); false, !transpose2) and
-    mat2Grad = blockedGEMM(outGrad, mat1; offsets (out, mat1, mat2); lists (N, K, M); true, !transpose1)."""
-    M, N, K, a1, a2, ao, ta, tb, H = ctx_meta
-    g = grad_out.contiguous()
-    m1 = mat1.to(g.dtype)
-    m2 = mat2.to(g.dtype)
-    dev = g.device
-    k1 = ("gemm_bwd1", M.tobytes(), N.tobytes(), K.tobytes(), a1.tobytes(), a2.tobytes(), ao.tobytes(), tb, H, g.dtype, str(dev))
-    p1 = _cached(k1, lambda: GemmPlan(M, K, N, H, g.dtype, g.dtype, False, not tb, False, accum=(ao, a2, a1), device=dev))
-    k2 = ("gemm_bwd2", M.tobytes(), N.tobytes(), K.tobytes(), a1.tobytes(), a2.tobytes(), ao.tobytes(), ta, H, g.dtype, str(dev))
-    p2 = _cached(k2, lambda: GemmPlan(N, K, M, H, g.dtype, g.dtype, True, not ta, False, accum=(ao, a1, a2), device=dev))
-    return p1.run(g, m2, scale=scale), p2.run(g, m1, scale=scale)
-
-
-class _BlockGEMMFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, mat1, mat2, plan, scale, softmax):
-        out = plan.run(mat1, mat2, scale=scale)
-        a1, a2, ao = plan.offsets
-        ctx.meta = (plan.M, plan.N, plan.K, a1, a2, ao, plan.ta, plan.tb, plan.H)
-        ctx.scale, ctx.softmax = scale, softmax
-        ctx.lead = (mat1.shape, mat2.shape)
-        ctx.save_for_backward(mat1, mat2, out if softmax else None)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        mat1, mat2, probs = ctx.saved_tensors
-        M, N, K, a1, a2, ao, ta, tb, H = ctx.meta
-        g = grad_out.contiguous()
-        if ctx.softmax:
-            # d(scores * scale) from d(probabilities), then the GEMM backward carries the scale
-            key = ("smx_bwd_of_gemm", M.tobytes(), N.tobytes(), ao.tobytes(), H, g.dtype, str(g.device))
-            sp = _cached(key, lambda: SoftmaxPlan(M, N, H, g.dtype, accum=ao, device=g.device))
-            g = sp.run_backward(probs.to(g.dtype), g)
-        g1, g2 = _gemm_backward(ctx.meta, mat1, mat2, g, ctx.scale)
-        return g1.reshape(ctx.lead[0]).to(mat1.dtype), g2.reshape(ctx.lead[1]).to(mat2.dtype), None, None, None
-
-
-class _BlockSoftmaxFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, src, plan, scale):
-        out = plan.run(src, scale=scale)
-        ctx.plan, ctx.scale = plan, scale
-        ctx.lead = src.shape
-        ctx.save_for_backward(out)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        (out,) = ctx.saved_tensors
-        g = grad_out.contiguous()
-        plan = ctx.plan
-        if g.dtype != plan.dtype:  # upstream converts the saved result to the gradient's dtype
-            key = ("smx_bwd_cast", plan.rows.tobytes(), plan.cols.tobytes(), plan.offsets.tobytes(), plan.H, g.dtype,
-                   str(g.device))
-            plan = _cached(key, lambda: SoftmaxPlan(ctx.plan.rows, ctx.plan.cols, ctx.plan.H, g.dtype,
-                                                    accum=ctx.plan.offsets, device=g.device))
-        return plan.run_backward(out.to(g.dtype), g, scale=ctx.scale).reshape(ctx.lead), None, None
 
 
 def blockGEMM(mat1: torch.Tensor, mat2: torch.Tensor,
@@ -186,39 +112,8 @@ def blockGEMM(mat1: torch.Tensor, mat2: torch.Tensor,
     ``transpose1``: mat1_s is stored (k, m); ``transpose2``: mat2_s is stored
     (k, n).  Any leading shape of mat1 flattens to H.
     """
-    _check_operand("mat1", mat1)
-    _check_operand("mat2", mat2)
-    have_acc = mat1Accum is not None and mat2Accum is not None and outAccum is not None
-    have_lists = MList is not None and NList is not None and KList is not None
-    if not (have_acc or have_lists):
-        raise RuntimeError("blockGEMM needs either mat1Accum/mat2Accum/outAccum or MList/NList/KList")
-    if mat1.dtype != mat2.dtype:
-        raise RuntimeError("mat1 and mat2 must have the same dtype")
-    odt = out_dtype if out_dtype is not None else mat1.dtype
-    key = ("gemm", _key_of(mat1Accum) if have_acc else None, _key_of(mat2Accum) if have_acc else None,
-           _key_of(outAccum) if have_acc else None, _key_of(MList) if have_lists else None,
-           _key_of(NList) if have_lists else None, _key_of(KList) if have_lists else None,
-           mat1.numel(), mat1.dtype, odt, bool(transpose1), bool(transpose2), bool(softmax), str(mat1.device))
-
-    def build():
-        if have_lists:
-            M, N, K = _host_i64(MList), _host_i64(NList), _host_i64(KList)
-        else:
-            M, N, K = _lists_from_offsets(mat1Accum, mat2Accum, outAccum)
-        accum = (mat1Accum, mat2Accum, outAccum) if have_acc else None
-        Dm1 = int(_host_i64(mat1Accum)[-1]) if have_acc else int((M * K).sum())
-        if Dm1 <= 0 or mat1.numel() % Dm1:
-            raise RuntimeError(f"mat1 has {mat1.numel()} elements, not a multiple of the packed extent {Dm1}")
-        H = mat1.numel() // Dm1
-        return GemmPlan(M, N, K, H, mat1.dtype, odt, bool(transpose1), bool(transpose2), bool(softmax),
-                        accum=accum, device=mat1.device)
-
-    plan = _cached(key, build)
-    if mat1.shape[-1] != plan.Dm1 and mat1.numel() != plan.H * plan.Dm1:
-        raise RuntimeError(f"mat1.size(-1) = {mat1.shape[-1]} does not match mat1Accum[-1] = {plan.Dm1}")
-    if torch.is_grad_enabled() and (mat1.requires_grad or mat2.requires_grad):
-        return _BlockGEMMFn.apply(mat1, mat2, plan, scale, bool(softmax))
-    return plan.run(mat1, mat2, scale=scale)
+    return _ops.gemm(mat1, mat2, mat1Accum, mat2Accum, outAccum, MList, NList, KList, transpose1, transpose2, scale,
+                     out_dtype, softmax)
 
 
 def blockSoftmax(src: torch.Tensor, rowList: torch.Tensor, colList: torch.Tensor,
@@ -230,22 +125,7 @@ def blockSoftmax(src: torch.Tensor, rowList: torch.Tensor, colList: torch.Tensor
     (rows_1, rows_2, ...)``, ``colList = (cols_1, ...)``; ``srcAccum = (0,
     rows_1*cols_1, ...)`` is optional.  ``out=src`` runs in place.
     """
-    _check_operand("src", src)
-    if rowList is None or colList is None:
-        raise RuntimeError("blockSoftmax needs rowList and colList")
-    key = ("smx", _key_of(rowList), _key_of(colList), _key_of(srcAccum), src.numel(), src.dtype, str(src.device))
-
-    def build():
-        rows, cols = _host_i64(rowList), _host_i64(colList)
-        D = int(_host_i64(srcAccum)[-1]) if srcAccum is not None else int((rows * cols).sum())
-        if D <= 0 or src.numel() % D:
-            raise RuntimeError(f"src has {src.numel()} elements, not a multiple of the packed extent {D}")
-        return SoftmaxPlan(rows, cols, src.numel() // D, src.dtype, accum=srcAccum, device=src.device)
-
-    plan = _cached(key, build)
-    if out is None and torch.is_grad_enabled() and src.requires_grad:
-        return _BlockSoftmaxFn.apply(src, plan, scale)
-    return plan.run(src, out=out, scale=scale)
+    return _ops.softmax(src, rowList, colList, srcAccum, scale, out)
 
 
 def blockAttnScores(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, scale: float = 1.0,
@@ -253,38 +133,7 @@ def blockAttnScores(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, scale
     """``softmax_rows(scale * Q_s K_s^T)`` for every segment in one pass: the
     fused form of ``blockSoftmax(blockGEMM(q, k, ...), MList, NList)``; the raw
     scores are never written to memory."""
-    return blockGEMM(q, k, None, None, None, MList, NList, KList, False, False,
-                     scale=scale, out_dtype=out_dtype, softmax=True)
-
-
-class _BlockAttentionFn(torch.autograd.Function):
-    """Fused forward.  The backward recomputes the probabilities with the fused scores operator and runs the softmax
-    backward kernel and four blocked products (the same kernels the two-operator path differentiates with), so the
-    probabilities exist in memory only during the backward pass.  Gradients have the layouts of q, k and v."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, plan, scale):
-        ctx.plan, ctx.scale = plan, scale
-        ctx.save_for_backward(q, k, v)
-        return plan.run(q, k, v, scale=scale)
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        q, k, v = ctx.saved_tensors
-        plan, scale = ctx.plan, ctx.scale
-        m, n = plan.M, plan.N
-        dl = np.full_like(m, plan.d)
-        with torch.no_grad():
-            go = grad_out.contiguous().reshape(q.shape).to(q.dtype)
-            p = blockGEMM(q, k, None, None, None, m, n, dl, False, False, scale=scale, softmax=True)   # (m, n)
-            dv = blockGEMM(p, go, None, None, None, n, dl, m, True, True)           # P^T dO: (n, d)
-            dp = blockGEMM(go, v, None, None, None, m, n, dl, False, False)         # dO V^T: (m, n)
-            key = ("attn_bwd_smx", m.tobytes(), n.tobytes(), plan.H, q.dtype, str(q.device))
-            sp = _cached(key, lambda: SoftmaxPlan(m, n, plan.H, q.dtype, device=q.device))
-            ds = sp.run_backward(p, dp)                                              # d(scale * scores)
-            dq = blockGEMM(ds, k, None, None, None, m, dl, n, False, True, scale=scale)   # dS K: (m, d)
-            dk = blockGEMM(ds, q, None, None, None, n, dl, m, True, True, scale=scale)    # dS^T Q: (n, d)
-        return dq.reshape(q.shape), dk.reshape(k.shape), dv.reshape(v.shape), None, None
+    return _ops.gemm(q, k, None, None, None, MList, NList, KList, False, False, scale, out_dtype, True)
 
 
 def blockAttention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, MList, NList, scale: float = 1.0,
@@ -295,36 +144,7 @@ def blockAttention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, MList, NLi
     ``d = 64``, the tcgen05 attention kernel otherwise); any other batch is the composition
     ``blockGEMM(blockAttnScores(q, k), v, transpose2=True)`` of the two operators.  Carries autograd history: the
     backward pass recomputes the probabilities with the two-operator path."""
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _check_operand(name, t)
-    M, N = _host_i64(MList), _host_i64(NList)
-    rows_q, rows_kv = int(M.sum()), int(N.sum())
-    if rows_q <= 0 or rows_kv <= 0:
-        raise RuntimeError("blockAttention needs at least one query row and one key row")
-    if d is None:
-        # a (H, sum m_s * d) tensor tells d by its last extent; a flat one cannot (d and H only appear as a product)
-        if q.dim() >= 2 and q.shape[-1] % rows_q == 0:
-            d = int(q.shape[-1]) // rows_q
-        else:
-            raise RuntimeError("give the head dimension d (a flat tensor cannot tell it apart from the number of heads)")
-    if q.numel() % (rows_q * d) or k.numel() != (q.numel() // (rows_q * d)) * rows_kv * d or v.numel() != k.numel():
-        raise RuntimeError("q / k / v do not match the packed extents of the lists")
-    H = q.numel() // (rows_q * d)
-    fused = (d in (64, 128) and q.dtype in (torch.float16, torch.bfloat16) and k.dtype == q.dtype and v.dtype == q.dtype
-             and int(N[M > 0].min() if (M > 0).any() else 1) >= 1)
-    if fused:
-        key = ("attn", M.tobytes(), N.tobytes(), H, d, q.dtype, str(q.device))
-        try:
-            plan = _cached(key, lambda: AttentionPlan(M, N, H, q.dtype, device=q.device, d=d))
-            if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
-                return _BlockAttentionFn.apply(q, k, v, plan, scale)
-            return plan.run(q, k, v, scale=scale)
-        except L.BlkError as e:
-            if e.code != L.BLK_ERR_UNSUPPORTED:
-                raise
-    dl = np.full_like(M, d)
-    p = blockGEMM(q, k, None, None, None, M, N, dl, False, False, scale=scale, softmax=True)
-    return blockGEMM(p, v, None, None, None, M, dl, N, False, True)
+    return _ops.attention(q, k, v, MList, NList, scale, d)
 
 
 def blockAttentionTokenMajor(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, nList, scale: float = 1.0) -> torch.Tensor:
@@ -332,15 +152,7 @@ def blockAttentionTokenMajor(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     ``q, k, v -> (sum n_s, H, d)`` (the nodes of all graphs in batch order), ``d`` 64 or 128, result of the same
     shape: ``out[rows of s] = softmax(scale * Q_s K_s^T) V_s`` per graph and head.  One kernel, no permuted copies,
     no probabilities in memory; graphs of any size, 16-bit inputs.  Forward only."""
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _check_operand(name, t)
-    if q.dim() != 3 or q.shape != k.shape or q.shape != v.shape or q.shape[2] not in (64, 128):
-        raise RuntimeError("q, k and v must all have shape (sum n, H, d), d 64 or 128")
-    n = _host_i64(nList)
-    H, d = int(q.shape[1]), int(q.shape[2])
-    key = ("attn", n.tobytes(), n.tobytes(), H, d, q.dtype, str(q.device))
-    plan = _cached(key, lambda: AttentionPlan(n, n, H, q.dtype, device=q.device, d=d))
-    return plan.run_token_major(q, k, v, scale=scale)
+    return _ops.attention_token_major(q, k, v, nList, scale)
 
 
 def blockAttnScoresTokenMajor(q: torch.Tensor, k: torch.Tensor, nList, scale: float = 1.0,
@@ -351,17 +163,7 @@ def blockAttnScoresTokenMajor(q: torch.Tensor, k: torch.Tensor, nList, scale: fl
     ``blockAttnScores``.  Needs 16-bit inputs and ``d`` a multiple of 8 (16-byte rows for the tensor maps); with ``d = 32`` a batch
     with hundreds of segments of at most 64 tokens is refused (those run on a kernel that reads packed strips only).
     Forward only."""
-    _check_operand("q", q)
-    _check_operand("k", k)
-    if q.dim() != 3 or q.shape != k.shape:
-        raise RuntimeError("q and k must both have shape (sum n, H, d)")
-    n = _host_i64(nList)
-    H, d = int(q.shape[1]), int(q.shape[2])
-    odt = out_dtype if out_dtype is not None else q.dtype
-    key = ("tokmajor", n.tobytes(), H, d, q.dtype, odt, bool(softmax), str(q.device))
-    plan = _cached(key, lambda: GemmPlan(n, n, np.full_like(n, d), H, q.dtype, odt, False, False, bool(softmax),
-                                         device=q.device))
-    return plan.run_token_major(q, k, scale=scale)
+    return _ops.scores_token_major(q, k, nList, scale, out_dtype, softmax)
 
 
 class _HostPipe:
@@ -411,7 +213,7 @@ def blockAttnScoresHost(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, s
         out = torch.empty((H, Dout), dtype=odt).pin_memory()
     elif out.is_cuda or not out.is_contiguous() or out.dtype != odt or out.numel() != H * Dout:
         raise RuntimeError("out must be a contiguous host tensor of the output dtype with H*Dout elements")
-    key = ("hostpipe", M.tobytes(), N.tobytes(), K.tobytes(), H, groups, q.dtype, odt, bool(softmax), str(dev))
+    key = ("hostpipe", _key_of(MList), _key_of(NList), _key_of(KList), H, groups, q.dtype, odt, bool(softmax), str(dev))
     pipe = _cached(key, lambda: _HostPipe(M, N, K, H, groups, q.dtype, odt, bool(softmax), dev))
     Hg = pipe.Hg
     qv, kv, ov = q.reshape(H, Dm1), k.reshape(H, Dm2), out.reshape(H, Dout)

@@ -1,9 +1,10 @@
 """Builds ``blockedattention_b200/lib/libblkattn.so`` for sm_100a with nvcc.
 
 The library is built in-tree (no JIT cache) so that it travels with the source
-tree.  ``build()`` also compiles the torch-extension module ``blockAttention/_C``
-(``csrc/sparseBlockedAttention.cpp``: the upstream extension's two operators as
-a shim over the library) with g++ against the installed torch.  ``python blockedattention_b200/build.py`` rebuilds what is out of date (run it
+tree.  ``build_extension()`` compiles two torch modules with g++ against the installed torch:
+``blockedattention_b200/_ops`` (``csrc/blk_torch.cpp``: the host path of the Python operators) and
+``blockAttention/_C`` (``csrc/sparseBlockedAttention.cpp``: the upstream extension's two operators as
+a shim over the library).  ``python blockedattention_b200/build.py`` rebuilds what is out of date (run it
 as a script: importing the package first would load the old library);
 ``--force`` rebuilds everything; ``--verbose`` adds ``-Xptxas -v``.
 """
@@ -77,41 +78,53 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
-def build_extension(force: bool = False, verbose: bool = False) -> str:
-    """``blockAttention/_C<ext suffix>``: the pybind/torch module with upstream's operator names, linked against
-    libtorch and ``libblkattn.so`` only (no kernels of its own, so g++ compiles it)."""
+def _torch_module(target: str, src: str, name: str, rpath: str, extra_deps, force: bool, verbose: bool) -> str:
+    """A Python module compiled by g++ against the installed torch and linked to libblkattn (it has no kernels)."""
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension as ce
 
-    src = os.path.join(CSRC, "sparseBlockedAttention.cpp")
-    deps = [src, os.path.join(CSRC, "sparseBlockedAttention.h"), os.path.join(ROOT, "include", "blkattn.h")]
-    outdir = os.path.join(ROOT, "blockAttention")
-    target = os.path.join(outdir, "_C" + sysconfig.get_config_var("EXT_SUFFIX"))
-    obj = os.path.join(OBJ, "sparseBlockedAttention.cpp.o")
+    deps = [src, os.path.join(ROOT, "include", "blkattn.h"), *extra_deps]
+    obj = os.path.join(OBJ, os.path.basename(src) + ".o")
     if not force and not _stale(target, deps + [LIB]):
         return target
     os.makedirs(OBJ, exist_ok=True)
-    incs = ce.include_paths("cuda") + [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"), CSRC]
-    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-DTORCH_EXTENSION_NAME=_C",
-           "-DTORCH_API_INCLUDE_EXTENSION_H", *[f"-I{p}" for p in incs], "-c", src, "-o", obj]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or r.returncode:
-        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-    if r.returncode:
-        raise RuntimeError("g++ failed on sparseBlockedAttention.cpp")
+    if force or _stale(obj, deps):
+        incs = ce.include_paths("cuda") + [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"), CSRC]
+        abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+        cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", f"-DTORCH_EXTENSION_NAME={name}",
+               "-DTORCH_API_INCLUDE_EXTENSION_H", *[f"-I{p}" for p in incs], "-c", src, "-o", obj]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or r.returncode:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode:
+            raise RuntimeError(f"g++ failed on {os.path.basename(src)}")
     libdirs = ce.library_paths("cuda")
-    link = ["g++", "-shared", "-o", target, obj, f"-L{LIBDIR}", "-lblkattn",
-            "-Wl,-rpath,$ORIGIN/../blockedattention_b200/lib", *[f"-L{p}" for p in libdirs],
-            *[f"-Wl,-rpath,{p}" for p in libdirs], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
-            "-ltorch_python", "-lcudart"]
+    link = ["g++", "-shared", "-o", target, obj, f"-L{LIBDIR}", "-lblkattn", f"-Wl,-rpath,{rpath}",
+            *[f"-L{p}" for p in libdirs], *[f"-Wl,-rpath,{p}" for p in libdirs], "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcudart"]
     r = subprocess.run(link, capture_output=True, text=True)
     if r.returncode:
         sys.stderr.write(" ".join(link) + "\n" + r.stdout + r.stderr)
-        raise RuntimeError("link of blockAttention/_C failed")
+        raise RuntimeError(f"link of {os.path.basename(target)} failed")
     return target
+
+
+def build_extension(force: bool = False, verbose: bool = False) -> str:
+    """The two torch modules: ``blockAttention/_C<ext suffix>`` (upstream's operator names, pybind11) and
+    ``blockedattention_b200/_ops<ext suffix>`` (the host path of the Python operators)."""
+    import sysconfig
+
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    with ThreadPoolExecutor(max_workers=2) as ex:
+        ops = ex.submit(_torch_module, os.path.join(PKG, "_ops" + suffix), os.path.join(CSRC, "blk_torch.cpp"), "_ops",
+                        "$ORIGIN/lib", [], force, verbose)
+        shim = ex.submit(_torch_module, os.path.join(ROOT, "blockAttention", "_C" + suffix),
+                         os.path.join(CSRC, "sparseBlockedAttention.cpp"), "_C", "$ORIGIN/../blockedattention_b200/lib",
+                         [os.path.join(CSRC, "sparseBlockedAttention.h")], force, verbose)
+        ops.result()
+        return shim.result()
 
 
 def main(argv=None) -> int:

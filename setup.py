@@ -32,6 +32,6 @@ setup(
     python_requires=">=3.9",
     install_requires=[],
     packages=["blockedattention_b200", "blockedAttention", "blockAttention"],
-    package_data={"blockedattention_b200": ["lib/libblkattn.so"], "blockAttention": ["_C*.so"]},
+    package_data={"blockedattention_b200": ["lib/libblkattn.so", "_ops*.so"], "blockAttention": ["_C*.so"]},
     cmdclass={"build_py": BuildWithLibrary},
 )

@@ -58,6 +58,13 @@ struct DeviceScope {
     int target = -1;
 };
 
+// SMs of the plan's device (the schedule's own default without one).
+void find_sms(blk_plan* p) {
+    int sms = 0;
+    if (p->device >= 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device) == cudaSuccess && sms > 0)
+        p->num_sms = sms;
+}
+
 // All device tables of a plan live in one allocation, filled by one copy: the tables are laid out in a host
 // staging block (kept per thread and reused, so a new plan touches no fresh pages) at 256-byte aligned offsets,
 // followed by the status / counter words, and the block goes up with a single cudaMemcpy.
@@ -67,11 +74,6 @@ int upload_plan(blk_plan* p) {
     if (!scope.ok) {
         blk_set_error("cannot select CUDA device " + std::to_string(p->device));
         return BLK_ERR_CUDA;
-    }
-    {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device) == cudaSuccess && sms > 0)
-            p->num_sms = sms;
     }
     struct Piece { const void* src; size_t bytes; void** dst; size_t off; };
     std::vector<Piece> pieces;
@@ -94,7 +96,7 @@ int upload_plan(blk_plan* p) {
     for (int b = 0; b < BLK_SMALL_BUCKETS; ++b) add_vec(p->small_items[b], &p->d_small_items[b]);
     add_vec(p->umma_items, &p->d_umma_items);
     add_vec(p->pv_items, &p->d_pv_items);
-    add_vec(p->flash_items, &p->d_flash_items);
+    add_vec(p->flash_pairs, &p->d_flash_pairs);
     add_vec(p->packs, &p->d_packs);
     add_vec(p->pack_blocks, &p->d_pack_blocks);
     add_vec(p->smx_chunks, &p->d_smx_chunks);
@@ -177,6 +179,7 @@ extern "C" int blk_gemm_plan_create(blk_plan_t** plan, const int64_t* M, const i
     p->tb = transpose2 ? 1 : 0;
     p->epi = epilogue;
     p->device = device;
+    find_sms(p);
     p->M.assign(M, M + S);
     p->N.assign(N, N + S);
     p->K.assign(K, K + S);
@@ -233,6 +236,7 @@ extern "C" int blk_softmax_plan_create(blk_plan_t** plan, const int64_t* rows, c
     p->H = H;
     p->dtype_in = p->dtype_out = dtype;
     p->device = device;
+    find_sms(p);
     p->M.assign(rows, rows + S);
     p->N.assign(cols, cols + S);
     p->a1.resize(S + 1);
@@ -399,6 +403,29 @@ static int build_flash_items(blk_plan* p, bool skip_small) {
     }
     std::stable_sort(p->flash_items.begin(), p->flash_items.end(),
                      [](const BlkFlashItem& a, const BlkFlashItem& b) { return a.N > b.N; });
+    // Pairs: neighbouring blocks of a segment (the stable sort keeps a segment's blocks in order and segments of one
+    // length apart), then what is left of the odd ones, two at a time (their key sweeps are of similar length, since
+    // the list is sorted).  A batch with no more blocks than SMs is better spread than paired.
+    auto block = [](const BlkFlashItem& a) { return BlkFlashPair::Block{a.rowQ, a.rowKV, a.M, a.N}; };
+    const std::vector<BlkFlashItem>& items = p->flash_items;
+    const bool spread = (int64_t)items.size() * p->H <= p->num_sms;
+    p->flash_pairs.clear();
+    p->flash_pairs.reserve(items.size() / 2 + 1);
+    int64_t open = -1;  // a pair that still lacks its second block
+    for (size_t i = 0; i < items.size(); ++i) {
+        BlkFlashPair pr{};
+        pr.block[0] = block(items[i]);
+        if (!spread && i + 1 < items.size() && items[i + 1].rowKV == items[i].rowKV && items[i + 1].rowQ == items[i].rowQ + BLK_FLASH_BM) {
+            pr.block[1] = block(items[++i]);
+        } else if (!spread && open >= 0) {
+            p->flash_pairs[(size_t)open].block[1] = pr.block[0];
+            open = -1;
+            continue;
+        } else if (!spread) {
+            open = (int64_t)p->flash_pairs.size();
+        }
+        p->flash_pairs.push_back(pr);
+    }
     return BLK_OK;
 }
 
@@ -450,6 +477,7 @@ static int attention_plan_impl(blk_plan_t** plan, const int64_t* M, const int64_
     p->ta = p->tb = 0;
     p->epi = BLK_EPI_SOFTMAX;
     p->device = device;
+    find_sms(p);
     p->M.assign(M, M + S);
     p->N.assign(N, N + S);
     p->K.assign((size_t)S, head_dim);
@@ -564,8 +592,8 @@ static int attention_run_impl(const blk_plan* p, const void* q, const void* k, c
         const bool strips = row_stride == 0;
         BlkFlashParams fp{};
         fp.out = out;
-        fp.items = p->d_flash_items;
-        fp.num_items = (int)p->flash_items.size();
+        fp.pairs = p->d_flash_pairs;
+        fp.num_pairs = (int)p->flash_pairs.size();
         fp.H = (int)p->H;
         fp.D = (int)d;
         fp.bf16 = p->dtype_in == BLK_BF16;

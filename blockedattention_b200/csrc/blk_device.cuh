@@ -84,6 +84,24 @@ __device__ __forceinline__ float blk_exp2(float x) {
     return y;
 }
 
+// Two fp32 operations in one instruction (packed forms of sm_100): a * b + c and a + b, element by element.
+__device__ __forceinline__ float2 blk_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+        " fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 blk_add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 d, a, b;\n"
+        " mov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
 // max(a, b, c) in one instruction (three-input maximum of sm_100).
 __device__ __forceinline__ float blk_max3(float a, float b, float c) {
     float y;

@@ -223,7 +223,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             // the operand tiles of chunk ch of an item
             auto load_chunk = [&](const Work& k, int ch) {
                 for (int kb = 0; kb < k.nkb; ++kb) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, 1, lim)) { ok = false; return; }
+                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 1, lim)) { ok = false; return; }
                     const uint32_t sA = smem_u32 + stage * UM_STAGE_BYTES, sB = sA + UM_A_BYTES;
                     mbar_expect_tx(full_bar(stage), UM_STAGE_BYTES);
                     // coordinates (k, row, head), or (k, head, row) for a token-major operand
@@ -261,13 +261,13 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             // the products of chunk ch of an item into the next accumulator
             auto mma_chunk = [&](const Work& k, int ch) {
                 const int buf = slot & 1;
-                if (!mbar_wait(tempty_bar(buf), ((slot >> 1) & 1u) ^ 1u, abort_flag, p.status, 2, lim)) { ok = false; return; }
+                if (!mbar_wait(tempty_bar(buf), ((slot >> 1) & 1u) ^ 1u, abort_flag, 2, lim)) { ok = false; return; }
                 tc_fence_after();
                 const int ncols = min(k.it.N - ch * UM_BN, UM_BN);
                 const uint32_t idesc = instr_desc(p.bf16, (ncols + 15) & ~15, p.epi == BLK_EPI_SOFTMAX && p.scale < 0.f);
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * UM_BN);
                 for (int kb = 0; kb < k.nkb; ++kb) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, p.status, 3, lim)) { ok = false; return; }
+                    if (!mbar_wait(full_bar(stage), phase, abort_flag, 3, lim)) { ok = false; return; }
                     tc_fence_after();
                     const uint32_t sA = smem_u32 + stage * UM_STAGE_BYTES, sB = sA + UM_A_BYTES;
                     // steps of 16 along k in this block: all four, or as many as reach the end of a short last block
@@ -307,7 +307,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             const uint32_t strip = blk_smem_u32(strips + (sq * 2 + sb) * UM_STRIP_BYTES);
             const uint32_t filled_bar = bar0 + 8u * (20 + sq * 2 + sb), drained_bar = bar0 + 8u * (28 + sq * 2 + sb);
             const volatile UmPiece* desc = pieces_desc + sq * 2 + sb;
-            if (!mbar_wait(filled_bar, use & 1u, abort_flag, p.status, 10, lim)) break;
+            if (!mbar_wait(filled_bar, use & 1u, abort_flag, 10, lim)) break;
             if (desc->stop) break;
             const int64_t g0 = desc->g0;
             const int N = desc->N, pcols = desc->pcols, rows = desc->rows;
@@ -441,7 +441,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
         auto pair_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(stat_bar);
-            const bool good = mbar_wait(stat_bar, stat_phase, abort_flag, p.status, 8, lim);
+            const bool good = mbar_wait(stat_bar, stat_phase, abort_flag, 8, lim);
             stat_phase ^= 1u;
             __syncwarp();
             return good;
@@ -469,7 +469,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             const uint32_t srow = strip + (uint32_t)lane * (UM_STRIP_PITCHW * 4) + (uint32_t)h * (SH * ES);  // word 32 h of my row
             const int mycols = min(SH, pcols - h * SH);              // columns of the piece this warp converts (<= 0: none)
             // the strip's previous piece (two pieces ago) has been written out
-            if (!mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, p.status, 8, lim)) return false;
+            if (!mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, 8, lim)) return false;
             if (mycols <= 0) {
                 loaded();
             } else if constexpr (OUT32) {
@@ -550,7 +550,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
         auto first_sweep_chunk = [&](int N, int ch) {
             uint32_t r[32];
             const int buf = slot & 1;
-            if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, p.status, 6, lim)) { ok = false; return; }
+            if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 6, lim)) { ok = false; return; }
             tc_fence_after();
             const int ncols = min(N - ch * UM_BN, UM_BN);
             for (int b0 = h * SH; b0 < ncols; b0 += PC) {
@@ -616,7 +616,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             if (!softmax) {
                 for (int ch = wk.it.ch0; ok && ch < wk.it.ch0 + wk.nchunks; ++ch, ++slot) {
                     const int buf = slot & 1;
-                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, p.status, 4, lim)) { ok = false; break; }
+                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 4, lim)) { ok = false; break; }
                     tc_fence_after();
                     const int ncols = min(N - ch * UM_BN, UM_BN);
                     auto release = [&]() {
@@ -632,7 +632,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                 // whole row resident: chunk k of the row sits in accumulator (slot + k) & 1
                 volatile float* xm = xch + (seq++ & 1) * (2 * UM_SPLIT * 128);  // [part][row] maxima, then [UM_SPLIT + part][row] sums
                 for (int ch = 0; ok && ch < wk.nchunks; ++ch)
-                    if (!mbar_wait(tfull_bar((slot + ch) & 1), ((slot + ch) >> 1) & 1u, abort_flag, p.status, 5, lim)) ok = false;
+                    if (!mbar_wait(tfull_bar((slot + ch) & 1), ((slot + ch) >> 1) & 1u, abort_flag, 5, lim)) ok = false;
                 if (!ok) break;
                 tc_fence_after();
                 auto tcol = [&](int c) {  // tensor-memory column of row column c
@@ -711,7 +711,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                 if (pair) { mx1 = -INFINITY; sum1 = 0.f; }
                 for (int ch = 0; ok && ch < wk.nchunks; ++ch) {
                     const int buf = slot & 1;
-                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, p.status, 7, lim)) { ok = false; break; }
+                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 7, lim)) { ok = false; break; }
                     tc_fence_after();
                     const int ncols = min(N - ch * UM_BN, UM_BN);
                     auto release = [&]() {
@@ -734,7 +734,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
         for (int t = 0; t < 2; ++t) {
             const int sb = (int)(pieces & 1u);
             const uint32_t filled_bar = bar0 + 8u * (20 + q * 2 + sb), drained_bar = bar0 + 8u * (28 + q * 2 + sb);
-            if (ok && !mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, p.status, 8, lim)) ok = false;
+            if (ok && !mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, 8, lim)) ok = false;
             if (h == 0 && lane == 0) (pieces_desc + q * 2 + sb)->stop = 1;
             __syncwarp();
             if (lane == 0) mbar_arrive(filled_bar);
@@ -745,11 +745,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag) {
-        // a role gave up: let copies that may still be in flight land before the CTA's memory is released
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-        __syncthreads();
-    }
+    wait_report(abort_flag, p.status);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512));

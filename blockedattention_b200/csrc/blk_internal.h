@@ -132,6 +132,14 @@ struct BlkFlashItem {
     int32_t N;      // key / value rows of the segment
 };
 static_assert(sizeof(BlkFlashItem) == 16, "BlkFlashItem layout");
+// What a CTA of that kernel works on at a time: one or two such blocks of one head (M = 0: no second block).  Two blocks
+// of one segment have the same rowKV and share its key and value tiles.
+struct BlkFlashPair {
+    struct Block {
+        int32_t rowQ, rowKV, M, N;
+    } block[2];
+};
+static_assert(sizeof(BlkFlashPair) == 32, "BlkFlashPair layout");
 
 // ---- kernel geometry constants the scheduler must agree with ----------------
 constexpr int BLK_TILE_BM = 64;
@@ -184,7 +192,8 @@ struct blk_plan {
                                             // 2 every segment on the tcgen05 attention kernel
     int head_dim = 64;                      // attention plans: columns of q, k, v and result rows
     std::vector<BlkFlashItem> flash_items;
-    BlkFlashItem* d_flash_items = nullptr;
+    std::vector<BlkFlashPair> flash_pairs;  // the same blocks as the kernel takes them
+    BlkFlashPair* d_flash_pairs = nullptr;
     std::vector<BlkPack> packs;
     std::vector<BlkPackBlock> pack_blocks;
     BlkPack* d_packs = nullptr;

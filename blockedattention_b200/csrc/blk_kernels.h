@@ -111,8 +111,9 @@ struct BlkPackParams {
 
 struct BlkFlashParams {
     void* out;
-    const BlkFlashItem* items;
-    int num_items;
+    float* lse;                 // [head][query row] base-2 logarithm of the row sums (reference included); null: not wanted
+    const BlkFlashPair* pairs;
+    int num_pairs;
     int H;
     int D;  // head dimension: 64 or 128
     int bf16;

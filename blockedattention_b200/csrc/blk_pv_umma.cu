@@ -156,7 +156,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
             for (uint32_t w = blockIdx.x; ok && pv_work(p, w, wk); w += gridDim.x) {
                 for (int j = 0; j < wk.T; ++j, ++g) {
                     const int vs = (int)(g % VS);
-                    if (!mbar_wait(v_empty(vs), ((g / VS) & 1u) ^ 1u, abort_flag, p.status, 41)) { ok = false; break; }
+                    if (!mbar_wait(v_empty(vs), ((g / VS) & 1u) ^ 1u, abort_flag, 41)) { ok = false; break; }
                     mbar_expect_tx(v_full(vs), L::OPER_BYTES);
                     const int row = wk.it.rowB + j * PV_BK;
 #pragma unroll
@@ -174,11 +174,11 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && pv_work(p, w, wk); w += gridDim.x, ++itc) {
                 const int ob = (int)(itc & 1u);
-                if (!mbar_wait(o_free(ob), ((itc >> 1) & 1u) ^ 1u, abort_flag, p.status, 42)) break;
+                if (!mbar_wait(o_free(ob), ((itc >> 1) & 1u) ^ 1u, abort_flag, 42)) break;
                 for (int j = 0; j < wk.T; ++j, ++g) {
                     const int vs = (int)(g % VS), buf = (int)(g % PV_PBUFS);
-                    if (!mbar_wait(p_full(buf), (g / PV_PBUFS) & 1u, abort_flag, p.status, 43)) { ok = false; break; }
-                    if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, p.status, 44)) { ok = false; break; }
+                    if (!mbar_wait(p_full(buf), (g / PV_PBUFS) & 1u, abort_flag, 43)) { ok = false; break; }
+                    if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, 44)) { ok = false; break; }
                     tc_fence_after();
                     const int ncols = min(wk.it.K - j * PV_BK, PV_BK);
                     const int ksteps = (ncols + 15) >> 4;
@@ -255,7 +255,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
                         else if (2 * i + 1 >= nv) pk[i] &= 0xffffu;
                     }
                 }
-                if (!mbar_wait(p_free(buf), ((g / PV_PBUFS) & 1u) ^ 1u, abort_flag, p.status, 45)) { ok = false; break; }
+                if (!mbar_wait(p_free(buf), ((g / PV_PBUFS) & 1u) ^ 1u, abort_flag, 45)) { ok = false; break; }
                 tc_fence_after();
                 // this row's elements [64 h, 64 h + 64) of the tile: columns [32 h, 32 h + 32) of the buffer (only the
                 // columns the products of this tile read)
@@ -265,7 +265,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
                 }
                 if (ncols & 15) {
                     // last tile of the row: clear the value rows between its end and the next multiple of 16
-                    if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, p.status, 46)) { ok = false; break; }
+                    if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, 46)) { ok = false; break; }
                     const int nz = (16 - (ncols & 15)) * L::NB * 8;  // 16-byte pieces to clear
                     const int t = lw * 32 + lane;
                     if (t < nz) {
@@ -289,7 +289,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
         uint32_t r[32];
         for (uint32_t w = blockIdx.x; pv_work(p, w, wk); w += gridDim.x, ++itc) {
             const int ob = (int)(itc & 1u);
-            if (!mbar_wait(o_ready(ob), (itc >> 1) & 1u, abort_flag, p.status, 47)) break;
+            if (!mbar_wait(o_ready(ob), (itc >> 1) & 1u, abort_flag, 47)) break;
             tc_fence_after();
             // a thread stores its row, 64 bytes at a time
             uint16_t* orow = reinterpret_cast<uint16_t*>(p.C) + (int64_t)wk.head * p.Dout + wk.it.offC + (int64_t)row * D;
@@ -314,11 +314,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
     // ---------------- teardown ----------------
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag) {
-        // a role gave up: let copies that may still be in flight land before the CTA's memory is released
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-        __syncthreads();
-    }
+    wait_report(abort_flag, p.status);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512));

@@ -19,15 +19,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred q;\n mbarrier.test_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // One suspended wait: the thread sleeps in hardware until the phase completes or about two microseconds pass,
 // whichever comes first, so a waiting role costs no issue slots.
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -39,18 +30,29 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait.  Returns false when another role has already given up or when the bound is hit
-// (then the status word and the CTA's abort flag are set).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                          int code, uint32_t limit = BLK_UMMA_SPIN_LIMIT) {
-    if (mbar_test(bar, parity)) return true;
-    for (uint32_t i = 0; i < limit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if ((i & 7u) == 7u && *abort_flag) return false;
+// Bounded wait.  Returns false when another role has already given up or when the bound is hit (the CTA's abort flag is
+// then the code; wait_report passes it on to the plan's status word when the roles have left their loops).  Kept to a few
+// instructions: the roles of these kernels run different code side by side and every wait is expanded where it stands.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code,
+                                          uint32_t limit = BLK_UMMA_SPIN_LIMIT) {
+#pragma unroll 1
+    for (uint32_t i = 0; !mbar_try(bar, parity); ++i) {
+        if (*abort_flag) return false;
+        if (i >= limit) {
+            *abort_flag = code;
+            return false;
+        }
     }
-    *abort_flag = 1;
-    atomicCAS(status, 0, code);
-    return false;
+    return true;
+}
+// After the CTA's roles have met again: a role gave up.  Copies that may still be in flight land before the CTA's memory
+// is released.
+__device__ __forceinline__ void wait_report(volatile int* abort_flag, int* status) {
+    if (*abort_flag) {
+        if (threadIdx.x == 0) atomicCAS(status, 0, *abort_flag);
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
     asm volatile(
@@ -141,6 +143,17 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, 
         : "memory");
 }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// The wait, tied to the registers of an earlier tc_ld32_nowait: nothing that uses them can be scheduled before it.
+__device__ __forceinline__ void tc_ld_wait(uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                   "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                   "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
 __device__ __forceinline__ void tc_sts_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -149,6 +162,15 @@ __device__ __forceinline__ void tc_sts_v4(uint32_t addr, uint32_t a, uint32_t b,
 __device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t addr, uint32_t lbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+// True in one lane of a converged warp.  Issue groups of tcgen05.mma / commit under `if (elect_one())` in code that the
+// whole warp runs: the compiler knows that form, keeps descriptors in uniform registers and spends four instructions per
+// tcgen05.mma instead of nine in a branch on the lane number.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}\n" : "=r"(e));
+    return e != 0;
 }
 
 }  // namespace

@@ -43,6 +43,9 @@ SIGNATURES = {
                                                 C.c_int]),
     "blk_attention_run": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_float, _vp]),
     "blk_attention_run_strided": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_int64, C.c_int64, C.c_float, _vp]),
+    "blk_attention_run_lse": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp]),
+    "blk_attention_prepare_backward": (C.c_int, [_vp]),
+    "blk_attention_backward_run": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp]),
     "blk_softmax_plan_create": (C.c_int, [C.POINTER(_vp), _i64p, _i64p, _i64p, C.c_int64, C.c_int64, C.c_int,
                                           C.c_int]),
     "blk_softmax_run": (C.c_int, [_vp, _vp, _vp, C.c_float, _vp]),

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 
@@ -264,6 +265,7 @@ extern "C" void blk_plan_destroy(blk_plan_t* p) {
     if (p->device >= 0) {
         DeviceScope scope(p->device);
         cudaFree(p->d_pool);  // every table and the status words are pieces of this one allocation
+        cudaFree(p->d_bwd_pool);
     }
     delete p;
 }
@@ -548,12 +550,12 @@ extern "C" int blk_attention_plan_create_dim(blk_plan_t** plan, const int64_t* M
 }
 
 // Shared body of blk_attention_run (strides 0: packed head-major strips) and blk_attention_run_strided.
-static int attention_run_impl(const blk_plan* p, const void* q, const void* k, const void* v, void* out,
+static int attention_run_impl(const blk_plan* p, const void* q, const void* k, const void* v, void* out, float* lse,
                               int64_t row_stride, int64_t head_stride, float scale, void* cuda_stream);
 
 extern "C" int blk_attention_run(const blk_plan_t* p, const void* q, const void* k, const void* v, void* out,
                                  float scale, void* cuda_stream) {
-    return attention_run_impl(p, q, k, v, out, 0, 0, scale, cuda_stream);
+    return attention_run_impl(p, q, k, v, out, nullptr, 0, 0, scale, cuda_stream);
 }
 
 extern "C" int blk_attention_run_strided(const blk_plan_t* p, const void* q, const void* k, const void* v, void* out,
@@ -563,10 +565,15 @@ extern "C" int blk_attention_run_strided(const blk_plan_t* p, const void* q, con
                       "the head dimension");
         return BLK_ERR_INVALID;
     }
-    return attention_run_impl(p, q, k, v, out, row_stride, head_stride, scale, cuda_stream);
+    return attention_run_impl(p, q, k, v, out, nullptr, row_stride, head_stride, scale, cuda_stream);
 }
 
-static int attention_run_impl(const blk_plan* p, const void* q, const void* k, const void* v, void* out,
+extern "C" int blk_attention_run_lse(const blk_plan_t* p, const void* q, const void* k, const void* v, void* out, float* lse,
+                                     float scale, void* cuda_stream) {
+    return attention_run_impl(p, q, k, v, out, lse, 0, 0, scale, cuda_stream);
+}
+
+static int attention_run_impl(const blk_plan* p, const void* q, const void* k, const void* v, void* out, float* lse,
                               int64_t row_stride, int64_t head_stride, float scale, void* cuda_stream) {
     BlkRange range("blk_attention_run");
     if (!p || p->kind != 0 || !p->attn) {
@@ -592,6 +599,7 @@ static int attention_run_impl(const blk_plan* p, const void* q, const void* k, c
         const bool strips = row_stride == 0;
         BlkFlashParams fp{};
         fp.out = out;
+        fp.lse = lse;
         fp.pairs = p->d_flash_pairs;
         fp.num_pairs = (int)p->flash_pairs.size();
         fp.H = (int)p->H;
@@ -629,6 +637,131 @@ static int attention_run_impl(const blk_plan* p, const void* q, const void* k, c
     pp.out_head_stride = packed ? p->Dm1 : head_stride;
     cudaError_t e = blk_launch_scores_pipe(pp, p->dtype_in, p->num_sms, reinterpret_cast<cudaStream_t>(cuda_stream));
     if (e != cudaSuccess) return cuda_fail("attention launch", e);
+    return BLK_OK;
+}
+
+// The work items of the backward kernels and their upload, once per plan.
+extern "C" int blk_attention_prepare_backward(blk_plan_t* p) {
+    BlkRange range("blk_attention_prepare_backward");
+    if (!p || p->kind != 0 || !p->attn) {
+        blk_set_error("blk_attention_prepare_backward: not an attention plan");
+        return BLK_ERR_INVALID;
+    }
+    static std::mutex mu;
+    std::lock_guard<std::mutex> g(mu);
+    if (p->bwd_ready) return BLK_OK;
+    const int64_t d = p->head_dim;
+    std::vector<BlkFlashItem> lists[blk_plan::BWD_LISTS];
+    for (int64_t s = 0; s < p->S; ++s) {
+        const int64_t M = p->M[s], N = p->N[s];
+        if (M == 0 || N == 0) continue;
+        const int32_t rowQ = (int32_t)(p->a1[s] / d), rowKV = (int32_t)(p->a2[s] / d);
+        if (M <= 64 && N <= 64) {
+            lists[M <= 32 && N <= 32 ? blk_plan::BWD_SMALL_32 : blk_plan::BWD_SMALL_64].push_back(
+                BlkFlashItem{rowQ, rowKV, (int32_t)M, (int32_t)N});
+            continue;
+        }
+        for (int64_t t = 0; t < M; t += 128)
+            lists[blk_plan::BWD_QUERIES].push_back(BlkFlashItem{(int32_t)(rowQ + t), rowKV, (int32_t)(M - t), (int32_t)N});
+        for (int64_t t = 0; t < N; t += 128)
+            lists[blk_plan::BWD_KEYS].push_back(BlkFlashItem{(int32_t)(rowKV + t), rowQ, (int32_t)(N - t), (int32_t)M});
+    }
+    std::vector<BlkFlashItem> all;
+    size_t at[blk_plan::BWD_LISTS];
+    for (int i = 0; i < blk_plan::BWD_LISTS; ++i) {
+        if (i == blk_plan::BWD_QUERIES || i == blk_plan::BWD_KEYS)  // persistent CTAs: longest sweeps first
+            std::stable_sort(lists[i].begin(), lists[i].end(), [](const BlkFlashItem& a, const BlkFlashItem& b) { return a.N > b.N; });
+        if ((int64_t)lists[i].size() * p->H >= ((int64_t)1 << 31)) {
+            blk_set_error("attention plan: more than 2^31 work items");
+            return BLK_ERR_UNSUPPORTED;
+        }
+        at[i] = all.size();
+        p->bwd_count[i] = (int)lists[i].size();
+        all.insert(all.end(), lists[i].begin(), lists[i].end());
+    }
+    if (p->device >= 0 && !all.empty()) {
+        DeviceScope scope(p->device);
+        if (!scope.ok) {
+            blk_set_error("cannot select CUDA device " + std::to_string(p->device));
+            return BLK_ERR_CUDA;
+        }
+        cudaError_t e = cudaMalloc(&p->d_bwd_pool, all.size() * sizeof(BlkFlashItem));
+        if (e != cudaSuccess) return cuda_fail("allocate backward tables", e);
+        e = cudaMemcpy(p->d_bwd_pool, all.data(), all.size() * sizeof(BlkFlashItem), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail("upload backward tables", e);
+        for (int i = 0; i < blk_plan::BWD_LISTS; ++i) p->d_bwd[i] = static_cast<BlkFlashItem*>(p->d_bwd_pool) + at[i];
+    }
+    p->bwd_ready = 1;
+    return BLK_OK;
+}
+
+extern "C" int blk_attention_backward_run(const blk_plan_t* p, const void* q, const void* k, const void* v, const void* out,
+                                          const float* lse, const void* grad_out, float* row_work, void* dq, void* dk, void* dv,
+                                          float scale, void* cuda_stream) {
+    BlkRange range("blk_attention_backward_run");
+    if (!p || p->kind != 0 || !p->attn || !p->bwd_ready || p->device < 0) {
+        blk_set_error("blk_attention_backward_run: not an attention plan prepared for the backward pass on a device");
+        return BLK_ERR_INVALID;
+    }
+    if (p->H == 0) return BLK_OK;
+    const int64_t d = p->head_dim;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
+    for (const void* t : {q, k, v, out, grad_out, (const void*)dq, (const void*)dk, (const void*)dv})
+        if (!t || !aligned16(t)) {
+            blk_set_error("blk_attention_backward_run: buffers must be 16-byte aligned, none null");
+            return t ? BLK_ERR_UNALIGNED : BLK_ERR_INVALID;
+        }
+    if (scale == 0.f) scale = 1.17549435e-38f;  // as in the forward run
+    const int64_t rows_q = p->a1[p->S] / d, rows_kv = p->a2[p->S] / d;
+    cudaError_t e;
+    // keys that no query looks at have zero gradients; no work item covers them
+    for (int64_t s = 0; s < p->S; ++s)
+        if (p->M[s] == 0 && p->N[s] > 0)
+            for (void* t : {dk, dv}) {
+                e = cudaMemset2DAsync(static_cast<unsigned char*>(t) + p->a2[s] * 2, (size_t)(rows_kv * d * 2), 0,
+                                      (size_t)(p->N[s] * d * 2), (size_t)p->H, st);
+                if (e != cudaSuccess) return cuda_fail("attention backward: clear", e);
+            }
+    for (int i : {blk_plan::BWD_SMALL_64, blk_plan::BWD_SMALL_32}) {
+        if (p->bwd_count[i] == 0) continue;
+        auto in = [](const void* t) { return reinterpret_cast<const uint16_t*>(t); };
+        auto res = [](void* t) { return reinterpret_cast<uint16_t*>(t); };
+        const BlkAttnBwdSmallParams sp{in(q), in(k), in(v), in(grad_out), res(dq), res(dk), res(dv), p->d_bwd[i], p->bwd_count[i],
+                                       (int)p->H, rows_q, rows_kv, scale};
+        e = blk_launch_attn_bwd_small(sp, (int)d, i == blk_plan::BWD_SMALL_32 ? 32 : 64, p->dtype_in == BLK_BF16, st);
+        if (e != cudaSuccess) return cuda_fail("attention backward launch (small segments)", e);
+    }
+    if (p->bwd_count[blk_plan::BWD_QUERIES] == 0) return BLK_OK;
+    if (!lse || !row_work) {
+        blk_set_error("blk_attention_backward_run: null buffer");
+        return BLK_ERR_INVALID;
+    }
+    const BlkOperandLayout layQ{rows_q, d, rows_q * d}, layK{rows_kv, d, rows_kv * d};
+    BlkFlashBwdParams bp{};
+    bp.H = (int)p->H;
+    bp.D = (int)d;
+    bp.bf16 = p->dtype_in == BLK_BF16;
+    bp.scale = scale;
+    bp.status = p->d_status;
+    bp.o = out;
+    bp.lse = lse;
+    bp.delta = row_work;
+    bp.rows_q = rows_q;
+    bp.items = p->d_bwd[blk_plan::BWD_QUERIES];
+    bp.num_items = p->bwd_count[blk_plan::BWD_QUERIES];
+    bp.rows_r = rows_q;
+    bp.out1 = dq;
+    const void* queries[4] = {q, grad_out, k, v};
+    e = blk_launch_attn_bwd_umma(bp, 0, queries, layQ, layK, p->num_sms, st);
+    if (e != cudaSuccess) return cuda_fail("attention backward launch (queries)", e);
+    bp.items = p->d_bwd[blk_plan::BWD_KEYS];
+    bp.num_items = p->bwd_count[blk_plan::BWD_KEYS];
+    bp.rows_r = rows_kv;
+    bp.out0 = dv;
+    bp.out1 = dk;
+    const void* keys[4] = {k, v, q, grad_out};
+    e = blk_launch_attn_bwd_umma(bp, 1, keys, layK, layQ, p->num_sms, st);
+    if (e != cudaSuccess) return cuda_fail("attention backward launch (keys)", e);
     return BLK_OK;
 }
 

@@ -194,6 +194,14 @@ struct blk_plan {
     std::vector<BlkFlashItem> flash_items;
     std::vector<BlkFlashPair> flash_pairs;  // the same blocks as the kernel takes them
     BlkFlashPair* d_flash_pairs = nullptr;
+    // Backward pass, made by blk_attention_prepare_backward: work items of the tcgen05 kernels (BlkFlashItem: first
+    // resident row, first passing row, resident rows from there on, passing rows) for the segments beyond 64 x 64, and the
+    // others whole, by size.
+    enum { BWD_QUERIES, BWD_KEYS, BWD_SMALL_32, BWD_SMALL_64, BWD_LISTS };
+    int bwd_count[BWD_LISTS] = {0, 0, 0, 0};
+    BlkFlashItem* d_bwd[BWD_LISTS] = {nullptr, nullptr, nullptr, nullptr};
+    void* d_bwd_pool = nullptr;
+    int bwd_ready = 0;
     std::vector<BlkPack> packs;
     std::vector<BlkPackBlock> pack_blocks;
     BlkPack* d_packs = nullptr;

@@ -124,6 +124,37 @@ struct BlkFlashParams {
     int64_t out_row_stride, out_head_stride;    // elements; result row r of head h at out[h * head_stride + r * row_stride]
 };
 
+// One launch of the backward of the attention kernel (see blk_attn_bwd_umma.cu).  items: first resident row, first
+// passing row, resident rows from there on, passing rows.
+struct BlkFlashBwdParams {
+    const BlkFlashItem* items;
+    int num_items;
+    int H;
+    int D;
+    int bf16;
+    float scale;
+    int* status;
+    const void* o;     // forward result (query launch)
+    const float* lse;  // [head][query row] as the forward kernel leaves it
+    float* delta;      // [head][query row] rowsum(dO O): written by the query launch, read by the key launch
+    void* out0;        // dV (key launch)
+    void* out1;        // dQ or dK
+    int64_t rows_q;    // query rows per head
+    int64_t rows_r;    // rows per head of the resident operands
+    int head_firstR, head_firstT;  // coordinate order of the tensor maps (filled by the launcher)
+};
+
+// The backward of segments of at most 64 x 64 (blk_attn_bwd_small.cu); packed head-major strips.
+struct BlkAttnBwdSmallParams {
+    const uint16_t *q, *k, *v, *g;  // g: gradient of the result
+    uint16_t *dq, *dk, *dv;
+    const BlkFlashItem* items;      // rowQ, rowKV, M, N of a segment
+    int num_items;
+    int H;
+    int64_t rows_q, rows_kv;        // rows per head
+    float scale;
+};
+
 struct BlkSmxParams {
     const void* src;
     void* dst;
@@ -178,5 +209,10 @@ cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p, const BlkUmmaOperand& A
 cudaError_t blk_launch_pv_umma(const BlkPvParams& p, const void* V, int sms, cudaStream_t st);
 cudaError_t blk_launch_attn_umma(const BlkFlashParams& p, const void* q, const void* k, const void* v, int sms,
                                  cudaStream_t st);
+// keys = 0: tensors Q, dO (resident), K, V (passing); keys = 1: K, V (resident), Q, dO (passing).
+cudaError_t blk_launch_attn_bwd_umma(const BlkFlashBwdParams& p, int keys, const void* const* tensors,
+                                     const BlkOperandLayout& layR, const BlkOperandLayout& layT, int sms, cudaStream_t st);
+// rows: 32 or 64, the most a segment of the list has of either kind.
+cudaError_t blk_launch_attn_bwd_small(const BlkAttnBwdSmallParams& p, int D, int rows, int bf16, cudaStream_t st);
 cudaError_t blk_launch_scores_pipe(const BlkPackParams& p, int dtype_in, int sms, cudaStream_t st);
 cudaError_t blk_launch_softmax(const BlkSmxParams& p, int dtype, cudaStream_t st);

@@ -225,7 +225,7 @@ struct Plan {
     bool ta = false, tb = false, softmax = false, compose = false;
     c10::Device device = c10::Device(c10::kCUDA, 0);
     // plans of the backward pass and of compositions, made when first needed; index: purpose, type
-    std::shared_ptr<Plan> derived[6][3];
+    std::shared_ptr<Plan> derived[5][3];
     ~Plan() {
         if (h) blk_plan_destroy(h);
     }
@@ -236,7 +236,7 @@ struct Plan {
 };
 typedef std::shared_ptr<Plan> PlanP;
 
-enum Purpose { FOR_GRAD1 = 0, FOR_GRAD2, FOR_SOFTMAX, FOR_SCORES, FOR_VALUES, FOR_PRODUCT };
+enum Purpose { FOR_GRAD1 = 0, FOR_GRAD2, FOR_SOFTMAX, FOR_SCORES, FOR_PRODUCT };
 
 struct PlanKey {
     int op, dt, odt, flags, device, d;
@@ -382,7 +382,8 @@ Tensor run_softmax_backward(const Plan& p, const Tensor& result, const Tensor& g
     return out;
 }
 
-Tensor run_attention(const Plan& p, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool tokens) {
+Tensor run_attention(const Plan& p, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool tokens,
+                     Tensor* lse = nullptr) {
     c10::cuda::CUDAGuard guard(p.device);
     const Tensor a = aligned(q), b = aligned(k), c = aligned(v);
     cudaStream_t st = stream_of(p.device);
@@ -393,7 +394,9 @@ Tensor run_attention(const Plan& p, const Tensor& q, const Tensor& k, const Tens
         ok(blk_attention_run_strided(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr(), p.H * p.d, p.d, (float)scale, st));
     } else {
         out = empty2(p.H, p.rows_q * p.d, p.dt, p.device);
-        ok(blk_attention_run(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr(), (float)scale, st));
+        if (lse) *lse = empty2(p.H, p.rows_q, at::kFloat, p.device);
+        ok(blk_attention_run_lse(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr(),
+                                 lse ? static_cast<float*>(lse->data_ptr()) : nullptr, (float)scale, st));
     }
     after_run(p, st);
     return out;
@@ -508,10 +511,9 @@ Tensor gemm_op(const PlanP& p, const Tensor& mat1, const Tensor& mat2, double sc
     return out;
 }
 
-// The backward recomputes the probabilities with the fused scores operator and runs the softmax backward kernel and
-// four blocked products; the probabilities exist in memory only during the backward pass.
+// The backward kernels recompute the probabilities: segments beyond 64 x 64 from the saved row logarithms.
 struct BlockAttentionBackward : public Node {
-    SavedVariable q_, k_, v_;
+    SavedVariable q_, k_, v_, out_, lse_;
     PlanP plan;
     double scale = 1.0;
     std::string name() const override { return "BlockAttentionBackward"; }
@@ -519,31 +521,29 @@ struct BlockAttentionBackward : public Node {
         q_.reset_data();
         k_.reset_data();
         v_.reset_data();
-    }
-    PlanP product(Purpose what, const std::vector<int64_t>& M, const std::vector<int64_t>& N, const std::vector<int64_t>& K, bool ta,
-                  bool tb, bool softmax) {
-        return derived(plan, what, plan->dt, [&]() {
-            return make_gemm(M.data(), N.data(), K.data(), plan->S, nullptr, nullptr, nullptr, plan->H, plan->dt, plan->dt, ta, tb,
-                             softmax, plan->device);
-        });
+        out_.reset_data();
+        lse_.reset_data();
     }
     variable_list apply(variable_list&& grads) override {
         variable_list res(3);
         if (!grads[0].defined()) return res;
-        const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack();
+        const Plan& p = *plan;
+        const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), out = out_.unpack(shared_from_this()), lse = lse_.unpack();
         const Tensor go = to_type(grads[0].contiguous(), q.scalar_type());
-        const auto &M = plan->M, &N = plan->N, &D = plan->K;
-        const Tensor p = run_gemm(*product(FOR_SCORES, M, N, D, false, false, true), q, k, scale);                    // (m, n)
-        if (task_should_compute_output(2))
-            res[2] = run_gemm(*product(FOR_VALUES, N, D, M, true, true, false), p, go, 1.0).reshape(v.sizes());       // P^T dO
-        const Tensor dp = run_gemm(*product(FOR_PRODUCT, M, N, D, false, false, false), go, v, 1.0);                  // dO V^T
-        PlanP sp = derived(plan, FOR_SOFTMAX, plan->dt,
-                           [&]() { return make_softmax(M, N, nullptr, plan->H, plan->dt, plan->device); });
-        const Tensor ds = run_softmax_backward(*sp, p, dp, 1.0);                                                      // d(scale S)
-        if (task_should_compute_output(0))
-            res[0] = run_gemm(*product(FOR_GRAD1, M, D, N, false, true, false), ds, k, scale).reshape(q.sizes());     // dS K
-        if (task_should_compute_output(1))
-            res[1] = run_gemm(*product(FOR_VALUES, N, D, M, true, true, false), ds, q, scale).reshape(k.sizes());     // dS^T Q
+        TORCH_CHECK(go.numel() == q.numel(), "the gradient does not match the attention result");
+        c10::cuda::CUDAGuard guard(p.device);
+        const Tensor a = aligned(q), b = aligned(k), c = aligned(v), g = aligned(go);
+        const int64_t nq = p.rows_q * p.d, nkv = p.rows_kv * p.d;
+        Tensor work = empty2(p.H, p.rows_q, at::kFloat, p.device);
+        Tensor dq = empty2(p.H, nq, p.dt, p.device), dk = empty2(p.H, nkv, p.dt, p.device), dv = empty2(p.H, nkv, p.dt, p.device);
+        cudaStream_t st = stream_of(p.device);
+        ok(blk_attention_backward_run(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr(),
+                                      static_cast<const float*>(lse.data_ptr()), g.data_ptr(), static_cast<float*>(work.data_ptr()),
+                                      dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (float)scale, st));
+        after_run(p, st);
+        res[0] = dq.reshape(q.sizes());
+        res[1] = dk.reshape(k.sizes());
+        res[2] = dv.reshape(v.sizes());
         return res;
     }
 };
@@ -558,8 +558,12 @@ Tensor attention_op(const PlanP& p, const Tensor& q, const Tensor& k, const Tens
     node->q_ = SavedVariable(q, false);
     node->k_ = SavedVariable(k, false);
     node->v_ = SavedVariable(v, false);
-    Tensor out = run_attention(*p, q.detach(), k.detach(), v.detach(), scale, false);
+    ok(blk_attention_prepare_backward(p->h));
+    Tensor lse;
+    Tensor out = run_attention(*p, q.detach(), k.detach(), v.detach(), scale, false, &lse);
     torch::autograd::set_history(out, node);
+    node->out_ = SavedVariable(out, true);
+    node->lse_ = SavedVariable(lse, false);
     return out;
 }
 

@@ -173,6 +173,24 @@ BLK_API int blk_attention_run(const blk_plan_t* plan, const void* q, const void*
 BLK_API int blk_attention_run_strided(const blk_plan_t* plan, const void* q, const void* k, const void* v, void* out,
                               int64_t row_stride, int64_t head_stride, float scale, void* cuda_stream);
 
+/* blk_attention_run that also leaves, for every query row of the segments on
+ * the tcgen05 kernel, the base-2 logarithm of its softmax denominator (row
+ * maximum included) in lse (dev, H x sum M_s floats, or NULL): what the
+ * backward pass recomputes the probabilities from. */
+BLK_API int blk_attention_run_lse(const blk_plan_t* plan, const void* q, const void* k, const void* v, void* out,
+                                  float* lse, float scale, void* cuda_stream);
+/* Builds and uploads what blk_attention_backward_run needs, once per plan
+ * (allocates; may be called again at no cost). */
+BLK_API int blk_attention_prepare_backward(blk_plan_t* plan);
+/* Gradients of out = softmax(scale q k^T) v: dq (H, sum M_s * d), dk and dv
+ * (H, sum N_s * d), from the forward operands, its result, its lse and
+ * grad_out.  P is recomputed tile by tile and never stored; row_work: H x sum
+ * M_s floats of workspace.  Replaces, for this use, the operator-by-operator
+ * backward of upstream csrc/sparseBlockedAttention.cpp:52-72,103-114. */
+BLK_API int blk_attention_backward_run(const blk_plan_t* plan, const void* q, const void* k, const void* v,
+                                       const void* out, const float* lse, const void* grad_out, float* row_work,
+                                       void* dq, void* dk, void* dv, float scale, void* cuda_stream);
+
 /* ---- varlen row softmax ---------------------------------------------------- */
 
 /* Replaces the per-row host table at upstream csrc/cuda/spBlkSoftmax.cu:358-373

@@ -1,0 +1,54 @@
+"""GPU: the backward kernels of the fused attention (16-row blocks up to 64 x 64, tcgen05 beyond) at the edges of their
+tiles -- 16-row MMA steps, 32 / 64-row segments, 64-row passing tiles, 128-row resident blocks -- against torch autograd
+of the per-segment formula in float64."""
+import numpy as np
+import pytest
+import torch
+
+from blockedattention_b200 import blockAttention, check_plans
+
+pytestmark = pytest.mark.gpu
+F16, BF16 = torch.float16, torch.bfloat16
+
+SMALL_M = [1, 2, 15, 16, 17, 31, 32, 33, 48, 64, 64, 1]
+SMALL_N = [1, 3, 16, 15, 32, 17, 31, 64, 20, 64, 1, 64]
+LARGE_M = [1, 127, 128, 129, 5, 300, 0, 257, 16, 200, 65]
+LARGE_N = [100, 128, 127, 129, 300, 70, 30, 65, 256, 385, 1]
+
+
+def reference(q, k, v, go, m, n, d, scale):
+    H = q.shape[0]
+    qr, kr, vr = (t.double().requires_grad_(True) for t in (q, k, v))
+    outs, oq, ok = [], 0, 0
+    for ms, ns in zip(m, n):
+        Q, K, V = (t[:, o * d:(o + r) * d].reshape(H, r, d) for t, o, r in ((qr, oq, ms), (kr, ok, ns), (vr, ok, ns)))
+        outs.append((torch.softmax(scale * Q @ K.transpose(1, 2), -1) @ V).reshape(H, ms * d))
+        oq += ms
+        ok += ns
+    out = torch.cat(outs, 1)
+    out.backward(go.double())
+    return out.detach(), qr.grad, kr.grad, vr.grad
+
+
+@pytest.mark.parametrize("dtype", [F16, BF16])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("m,n,scale", [(SMALL_M, SMALL_N, 0.1), (SMALL_M, SMALL_N, -0.07), (LARGE_M, LARGE_N, 0.1),
+                                       (LARGE_M, LARGE_N, -0.07), ([150, 7, 64, 700, 30], [90, 7, 65, 1500, 60], 0.1)])
+def test_attention_backward_edges(cuda_device, dtype, d, m, n, scale):
+    H = 3
+    g = torch.Generator(device=cuda_device).manual_seed(d + len(m))
+
+    def made(rows):
+        return torch.randn((H, rows * d), generator=g, device=cuda_device).to(dtype)
+
+    q, k, v, go = made(sum(m)), made(sum(n)), made(sum(n)), made(sum(m))
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out = blockAttention(*leaves, np.array(m), np.array(n), scale=scale, d=d)
+    got = (out.detach(),) + torch.autograd.grad(out, leaves, go)
+    check_plans()
+    tol = 1e-2 if dtype == BF16 else 2e-3
+    for name, a, b in zip(("out", "dq", "dk", "dv"), got, reference(q, k, v, go, m, n, d, scale)):
+        assert torch.isfinite(a.float()).all(), name
+        rel = float((a.double() - b).norm() / b.norm())
+        worst = float((a.double() - b).abs().max() / b.abs().max())
+        assert rel <= tol and worst <= tol, f"{name}: rel {rel}, max {worst}"

@@ -1,53 +1,44 @@
 // Large-segment kernel of the varlen blocked GEMM on the 5th-generation tensor
 // cores: TMA-fed tcgen05.mma with the accumulator in tensor memory.
 //
-// A persistent CTA (one per SM; 22 warps for the two-sweep fused softmax, 14 otherwise) walks a static list of work
-// items, an item being a 128-row block of one segment of one head (or one 256-column chunk of it).  Roles:
-//   warp 0   producer: one lane issues 3-D tiled TMA loads (k, row, head) of a
-//            128 x 64 tile of the first operand and a 256 x 64 tile of the
-//            second into a 3-stage ring of 128-byte-swizzled shared memory;
-//   warp 1   MMA: allocates the 512 tensor-memory columns, and one lane issues
-//            tcgen05.mma (M = 128, N up to 256, K = 16 per instruction) into
-//            one of two 256-column accumulators; tcgen05.commit hands shared
-//            memory stages back to the producer and accumulators to the epilogue;
-//   next 16 or 8 warps  epilogue arithmetic: a warp may read the 32 accumulator lanes (= rows)
-//            of its quarter; the four or two warps of a quarter (SPLIT) each take an equal share of every
-//            staged piece's columns and exchange partial row statistics through
-//            shared memory.  A thread reads its row 32 columns at a time
-//            (tcgen05.ld), applies the epilogue and writes the packed words into
-//            one of the quarter's two strips (32 rows x 128 16-bit or 64 fp32 columns each, used
-//            alternately), at the position the row has in global memory modulo
-//            one 32-bit word;
-//   last 4 warps  stores: one warp per quarter.  It waits for a strip to
-//            be filled, writes its 32 rows to global memory -- a row piece is 256
-//            contiguous bytes stored as two fully coalesced 128-byte word stores;
-//            an odd first or last element goes out as a 16-bit store -- and hands
-//            the strip back.  Keeping the stores in warps of their own matters:
-//            a warp that alternates between exponentials and stores leaves the
-//            special-function unit idle whenever the memory system pushes back
-//            on its stores, and all warps of a CTA reach that point together;
-//            with separate warps the exponentials of one piece run while the
-//            previous piece drains.  Wide contiguous row pieces matter as well:
-//            the same data written as 128-byte pieces with element-wise ragged
-//            edges runs at little more than half the rate.
+// A persistent CTA (one per SM) walks a static list of work items, an item being a 128-row block of one segment of one head
+// (or one 256-column chunk of it).  An item's columns are taken in chunks: 128 wide, or 256 wide in the variant for plain
+// scores of long contractions (WIDE), which want the widest instruction.  Roles:
+//   warp 0     producer: one lane issues 3-D tiled TMA loads (k, row, head) of a 128 x 64 tile of the first operand and a
+//              chunk x 64 tile of the second into a ring of 128-byte-swizzled stages;
+//   warp 1     MMA: one lane issues tcgen05.mma (M = 128, K = 16 per instruction) into the next of four 128-column (two
+//              256-column) accumulators;
+//   last warp  planner: one lane reads the work items ahead of everybody and hands them out through a ring in shared
+//              memory (a role that fetched its own would wait for that load at every item);
+//   the others groups of four epilogue warps, four groups (two when WIDE); a warp owns 32 rows (the accumulator lanes it may
+//              read), a thread one row.  Plain scores: groups take chunks in turn.  Softmax: two groups share an item, its
+//              chunks in turn, and meet once to combine the row statistics; the other two have the next item.  So some
+//              groups take exponentials while others store or wait for products: with all warps on one item, in step
+//              through maximum, exponentials and stores, the special-function unit was busy a quarter of the time.
+// A thread reads its row 32 columns at a time (tcgen05.ld), applies the epilogue and writes packed words into its warp's
+// strip (32 rows x 128 16-bit or 64 fp32 columns) at the position the row has in global memory modulo one 32-bit word; then
+// the warp writes the strip out as row pieces of 256 contiguous bytes, two fully coalesced 128-byte word stores each, with
+// odd first and last elements as 16-bit stores.  Wide contiguous row pieces matter: the same data written as 128-byte pieces
+// with element-wise ragged edges runs at little more than half the rate.
 //
-// Epilogues.  Scores: scale and round.  Softmax with N <= 512: both
-// accumulators hold the whole row; pass 1 takes the row maximum, pass 2 writes
-// exp2 back into tensor memory while summing, pass 3 normalises and stores, so
-// the exponential is evaluated once per element and the scores never leave the
-// SM.  Softmax with N > 512: the products are computed twice -- a first sweep
-// over the 256-column chunks keeps only a running (max, sum) per row, a second
-// sweep recomputes each chunk and stores normalised probabilities; when the CTA's next item is of the same kind and
-// length, its first sweep is interleaved chunk by chunk with this item's second.
+// Epilogues.  Scores: scale and round.  Softmax with N <= 512: the whole row stays in tensor memory; pass 1 takes the
+// exponentials against a running reference (the first piece's maximum; moved, with what was written rescaled, only when a
+// piece exceeds it by 2^32) and writes them back as fp32 while summing, pass 2 normalises and stores, so the exponential is
+// evaluated once per element and the scores never leave the SM.  Softmax with N > 512: the products are computed twice -- a
+// first sweep keeps only (reference, sum) per row, a second recomputes each chunk and stores normalised probabilities; the
+// second sweep of an item alternates chunk by chunk with the first sweep of the next, which the other two groups do.
 //
-// Rows of the operand views past the end of a segment belong to its neighbour
-// (or are zero-filled past the end of the buffer); they only reach accumulator
-// rows/columns the epilogue never stores, and columns >= N are masked before
-// any row reduction.
+// Measured against one item at a time with 8 arithmetic and 4 store warps: scores + softmax of 1024 segments of 64..512 rows,
+// 16 heads, K = 128: 2054 -> 1532 us; 2048 products of at most 256 x 256, fp32 out: 56.6 -> 54.3 us; 64 products of
+// 1024..2048 rows and columns, K 1024..4096: 850 -> 729 us (1.04 PFLOP/s).  Without its stores the first takes 1230 us: what
+// is left is the latency of a chunk through loads, products and registers, then the write rate of misaligned rows.
 //
-// Every wait on an mbarrier is bounded: when the bound is hit the kernel
-// records a status code, all roles leave their loops, tensor memory is
-// released and the kernel returns.
+// Rows of the operand views past the end of a segment belong to its neighbour (or are zero-filled past the end of the
+// buffer); they only reach accumulator rows/columns the epilogue never stores, and columns >= N are masked before any row
+// reduction.  A warp none of whose rows exist only hands its accumulators back.
+//
+// Every wait on an mbarrier is bounded: when the bound is hit the kernel records a status code, all roles leave their
+// loops, tensor memory is released and the kernel returns.
 //
 // Replaces upstream sparseBlockedHGEMM_half / _bf16 with the 128 x 128 x 16
 // WMMA tile (csrc/cuda/spBlkGEMM.cu:424-817, :866-868) and, fused, the softmax
@@ -63,50 +54,46 @@
 namespace {
 
 constexpr int UM_BM = BLK_UMMA_BM;      // 128 rows per work item
-constexpr int UM_BN = 256;              // columns per accumulator
 constexpr int UM_BK = 64;               // k elements per shared-memory stage (one 128-byte swizzle row)
-constexpr int UM_STAGES = 3;
 constexpr int UM_A_BYTES = UM_BM * UM_BK * 2;  // 16 KB
-constexpr int UM_B_BYTES = UM_BN * UM_BK * 2;  // 32 KB
-constexpr int UM_STAGE_BYTES = UM_A_BYTES + UM_B_BYTES;
-// Arithmetic warps per accumulator-lane quarter (SPLIT, a template parameter of the kernel): four for the fused
-// softmax over rows too long for tensor memory (each converts 32 of every 128 columns: with two warps per scheduler
-// partition the special-function unit idles half the time in the two-sweep scheme), two otherwise -- rows that stay
-// resident, scores only (both a few per cent faster with fewer, fatter warps) and fp32 results (a staged piece is 64
-// columns there, and a warp's share must be whole 32-column loads).
-constexpr int UM_SPLIT_MAX = 4;
-constexpr int UM_STORE_WARPS = 4;                     // one per quarter
-constexpr int um_threads(int split) { return 64 + 32 * (4 * split + UM_STORE_WARPS); }
-constexpr int UM_PIECE = 32;                          // columns per tcgen05.ld
 constexpr int UM_PW = 64;                             // 32-bit words of a staged row piece (128 x 16-bit, 64 x fp32)
 // Strip row pitch in words: odd, so that the 32 row-owning lanes of a store (same word, consecutive rows) hit 32
 // different banks; a row holds UM_PW words plus the half word an odd first element pushes past the end.
-constexpr int UM_STRIP_PITCHW = UM_PW + 5;
-constexpr int UM_STRIP_BYTES = 32 * UM_STRIP_PITCHW * 4;  // one strip; a quarter has two
-// What the arithmetic warps tell the store warp about the piece in a strip.
-struct UmPiece {
-    int64_t g0;   // element index in the output of the piece's first element in the quarter's first row
-    int32_t N;    // row pitch of the output block
-    int32_t pcols;  // columns of the piece
-    int32_t rows;   // rows of the quarter inside the block (0..32)
-    int32_t halves; // a row may start or end on half a word
-    int32_t stop;   // no more pieces: the store warp leaves
-    int32_t pad;
-};
-static_assert(sizeof(UmPiece) == 32, "UmPiece layout");
-constexpr int PCOLS16 = UM_PW * 2;                    // columns of a whole 16-bit piece
-constexpr int UM_XCH_BYTES = 2 * 2 * UM_SPLIT_MAX * 128 * 4;  // row statistics exchanged between the two halves, double-buffered
-constexpr int UM_SMEM_BYTES = UM_STAGES * UM_STAGE_BYTES + 8 * UM_STRIP_BYTES + UM_XCH_BYTES + 8 * 32 + 512;
-static_assert(UM_SMEM_BYTES <= 227 * 1024, "shared memory budget");
-static_assert(UM_STAGES <= 4, "barrier slots");
+constexpr int UM_STRIP_PITCHW = UM_PW + 1;
+constexpr int UM_STRIP_BYTES = 32 * UM_STRIP_PITCHW * 4;  // one per warp of the groups
+constexpr float UM_LAZY = 32.f;                       // exponent slack before a softmax reference moves
+constexpr uint32_t UM_ITEMS = 8;                      // ring of item records
 
-struct Work {
-    BlkUmmaItem it;
-    int head;
-    int nchunks;
-    int sweeps;
-    int nkb;     // k-blocks of UM_BK; the last may be short (the tensor map fills what lies past K with zeros)
+template <bool WIDE>
+struct UL {
+    static constexpr int GROUPS = WIDE ? 2 : 4;       // of four epilogue warps
+    static constexpr int THREADS = 96 + 128 * GROUPS;
+    static constexpr int BN = WIDE ? 256 : 128;       // columns of a chunk = of an accumulator
+    static constexpr uint32_t NBUF = 512 / BN;
+    static constexpr int STAGES = 3;
+    static constexpr int STAGE_BYTES = UM_A_BYTES + BN * UM_BK * 2;
+    static constexpr int STRIP_OFF = STAGES * STAGE_BYTES;
+    static constexpr int BAR_OFF = STRIP_OFF + 4 * GROUPS * UM_STRIP_BYTES;
+    static constexpr int SMEM_BYTES = BAR_OFF + 448 + (int)UM_ITEMS * 64;
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
+
+struct UmYes { static constexpr bool value = true; };
+struct UmNo { static constexpr bool value = false; };
+
+// A work item as the roles see it, in shared memory.
+struct __align__(16) Work {
+    int64_t cbase;   // element of the output where the item's rows start (head, segment and row block included)
+    int32_t rows, N; // rows of the block | first quarter that holds them << 8; columns of the segment
+    int32_t ch0, nchunks;  // chunks [ch0, ch0 + nchunks)
+    int32_t sweeps;
+    int32_t pair;    // chunks of the next item's first sweep, which alternates with this one's second (0: it does not)
+    int32_t rowA, rowB, K, views;
+    int32_t head;
+    int32_t valid;   // 0: nothing follows
+    int32_t next_rows, next_N;  // of the item this one pairs with
+};
+static_assert(sizeof(Work) == 64, "Work is written as four 16-byte vectors");
 
 // The tensor maps of the operands' views (BlkUmmaView), passed as one kernel parameter.
 struct UmMaps {
@@ -114,32 +101,68 @@ struct UmMaps {
     CUtensorMap b[BLK_UMMA_VIEWS];
 };
 
-// Work w of a CTA's walk (w = blockIdx.x + k gridDim.x in round k).  Odd rounds run through the CTAs backwards, so
-// that with the items sorted by cost no CTA always gets the heaviest of a round.  Only the last round can point past
-// the end, so a CTA that gets nothing there has nothing left either.
-__device__ __forceinline__ bool next_work(const BlkUmmaParams& p, uint32_t w, Work& wk) {
-    const uint32_t total = (uint32_t)p.num_items * (uint32_t)p.H;
-    const uint32_t round = w / gridDim.x;
-    if (round & 1u) w = round * gridDim.x + (gridDim.x - 1u - (w - round * gridDim.x));
-    if (w >= total) return false;
+// Item n of a CTA's walk, from global memory.  Odd rounds run through the CTAs backwards, so that with the items sorted by
+// cost no CTA always gets the heaviest of a round.  Only the last round can point past the end, so a CTA that gets nothing
+// there has nothing left either.
+__device__ __forceinline__ bool fetch_item(const BlkUmmaParams& p, uint32_t n, BlkUmmaItem& it, int& head) {
+    const uint32_t w = n * gridDim.x + ((n & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
+    if (w >= (uint32_t)p.num_items * (uint32_t)p.H) return false;
     const uint32_t item = w / (uint32_t)p.H;
-    wk.head = (int)(w - item * (uint32_t)p.H);
-    wk.it = p.items[item];
-    wk.nchunks = wk.it.nch ? wk.it.nch : (wk.it.N + UM_BN - 1) / UM_BN;  // chunks [it.ch0, it.ch0 + nchunks)
-    wk.nkb = (wk.it.K + UM_BK - 1) / UM_BK;
-    wk.sweeps = (p.epi == BLK_EPI_SOFTMAX && wk.nchunks > 2) ? 2 : 1;
+    head = (int)(w - item * (uint32_t)p.H);
+    const int4* src = reinterpret_cast<const int4*>(p.items + item);
+    int4* dst = reinterpret_cast<int4*>(&it);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
     return true;
 }
+// Rows of an item's block.  A block that fills less than four quarters of the accumulator lanes is put into other
+// quarters from item to item (its operand rows are loaded that much earlier): a quarter is one scheduler's warps.
+__device__ __forceinline__ int item_rows(const BlkUmmaItem& it, uint32_t n) {
+    const int rows = min(it.M - it.tm * UM_BM, UM_BM);
+    const uint32_t slack = 4u - (uint32_t)((rows + 31) >> 5);
+    return rows | (int)((n % (slack + 1u)) << 8);
+}
+template <bool SOFT, bool WIDE>
+__device__ __forceinline__ void publish(const BlkUmmaParams& p, Work* dst, const BlkUmmaItem& it, int head, uint32_t n,
+                                        bool valid, const BlkUmmaItem& nx, bool nx_valid) {
+    constexpr int BN = UL<WIDE>::BN;
+    Work w{};
+    if (valid) {
+        w.rows = item_rows(it, n);
+        w.cbase = (int64_t)head * p.Dout + it.offC + (int64_t)it.tm * UM_BM * it.N;
+        w.N = it.N;
+        w.ch0 = it.ch0 * (256 / BN);  // (the plan counts chunks of 256 columns)
+        w.nchunks = (it.N + BN - 1) / BN - w.ch0;
+        if (it.nch) w.nchunks = min(w.nchunks, it.nch * (256 / BN));
+        w.sweeps = SOFT && it.N > 512 ? 2 : 1;
+        w.pair = w.sweeps == 2 && nx_valid && nx.N > 512 ? (nx.N + BN - 1) / BN : 0;
+        w.rowA = it.rowA - 32 * (w.rows >> 8);
+        w.rowB = it.rowB;
+        w.K = it.K;
+        w.views = it.views;
+        w.head = head;
+        w.valid = 1;
+        w.next_rows = item_rows(nx, n + 1u);
+        w.next_N = nx.N;
+    }
+    *dst = w;
+}
 
-// Two consecutive items of a CTA's walk pair up when both take the two-sweep softmax over the same number of chunks:
-// then the first sweep of the later one (special-function bound, stores nothing) is interleaved chunk by chunk with the
-// second sweep of the earlier one (bound by the stores).  nx receives the later item.
-__device__ __forceinline__ bool pairs_with_next(const BlkUmmaParams& p, uint32_t w, const Work& wk, Work& nx) {
-#ifdef UM_NO_PAIRING
-    return false;
-#else
-    return wk.sweeps == 2 && next_work(p, w + gridDim.x, nx) && nx.sweeps == 2 && nx.nchunks == wk.nchunks;
-#endif
+// The chunks of item n in the order in which they are loaded, multiplied and consumed: its first sweep (unless that ran
+// alongside the item before), then the storing chunks, each followed by a first-sweep chunk of the next item when the two
+// pair up.  f(next, ch, first): chunk ch of this item or the next, in its first sweep or storing; false stops.
+template <typename F>
+__device__ __forceinline__ void chunk_order(int ch0, int nchunks, int sweeps, int pair, bool pre, F f) {
+    const int first = sweeps == 2 && !pre ? nchunks : 0;
+    const int rest = pair ? 2 * max(nchunks, pair) : nchunks;
+#pragma unroll 1
+    for (int i = 0; i < first + rest; ++i) {
+        const int t = i - first;
+        const bool nx = pair && t >= 0 && (t & 1);
+        const int ch = t < 0 ? i : pair ? t >> 1 : t;
+        if (t >= 0 && ch >= (nx ? pair : nchunks)) continue;  // the other item has more chunks
+        if (!f(nx, t < 0 || nx ? ch : ch0 + ch, t < 0 || nx)) return;
+    }
 }
 
 // Predicated global stores as single instructions (no branch around them).
@@ -158,48 +181,122 @@ __device__ __forceinline__ uint32_t lds_b32(uint32_t addr) {
     return v;
 }
 
-template <typename Tag, bool OUT32, int SPLIT>
-__global__ void __launch_bounds__(um_threads(SPLIT), 1)
+// A warp writes the piece in its strip to the output: element g0 is the first of its first row, row k starts N elements
+// further each; `rows` rows of pcols columns exist.  halves: some row starts or ends on half a word.
+template <bool OUT32>
+__device__ __forceinline__ void store_strip(uint32_t strip, void* out, int64_t g0, int N, int pcols, int rows, bool halves,
+                                            int lane) {
+    constexpr int BATCH = 8;  // rows whose words are in registers at a time
+    // lane l carries words l and l + 32 of a row: two stores of 128 contiguous bytes per row
+    const uint32_t rbase = strip + 4u * lane;
+    uint32_t v[BATCH][2];
+    auto fetch = [&](int kb) {
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
+    };
+    if (rows == 32 && pcols == (OUT32 ? UM_PW : 2 * UM_PW)) {
+        // A whole piece (the common case), with as few instructions per row as it takes.  Row k starts at element g0 + k N:
+        // of 16-bit elements, at word (t >> 1) past the word of g0 with t = (g0 & 1) + k N, on its odd half when t is odd.
+        // Words 1..63 of the row are whole; word 0 is whole when the row starts on an even element (its upper half goes out
+        // below otherwise, and so does the lower half of word 64).
+        uint32_t* const w0 = static_cast<uint32_t*>(out) + (OUT32 ? g0 : g0 >> 1) + lane;
+        uint32_t t = OUT32 ? 0u : (uint32_t)(g0 & 1);
+#pragma unroll 1
+        for (int kb = 0; kb < 32; kb += BATCH) {
+            fetch(kb);
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                uint32_t* wp = w0 + (OUT32 ? t : t >> 1);
+                if (OUT32) asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp), "r"(v[k][0]) : "memory");
+                else stg_b32_if(wp, v[k][0], lane >= (int)(t & 1u));
+                asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp + 32), "r"(v[k][1]) : "memory");
+                t += (uint32_t)N;
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int kb = 0; kb < rows; kb += BATCH) {
+            fetch(kb);
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) {
+                const int64_t gr = g0 + (int64_t)(kb + k) * N;
+                const int pr = OUT32 ? 0 : (int)(gr & 1);
+                // whole words of the piece: [pr, (pr + pcols) / 2) for 16-bit elements, [0, pcols) for fp32
+                const int wl = kb + k < rows ? (OUT32 ? pcols : (pr + pcols) >> 1) : 0;
+                uint32_t* wp = static_cast<uint32_t*>(out) + (OUT32 ? gr : gr >> 1) + lane;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) stg_b32_if(wp + 32 * i, v[k][i], lane + 32 * i >= pr && lane + 32 * i < wl);
+            }
+        }
+    }
+    if (!OUT32 && halves) {
+        // half words at the ends: lane k the odd first element of row k, then the last element of row k when the
+        // piece ends on half a word
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const bool tail = t != 0;
+            const int64_t gr = g0 + (int64_t)lane * N;
+            const int pr = (int)(gr & 1);
+            const int endh = pr + pcols;                 // half words [pr, endh) of the row's words are the piece
+            const int wi = tail ? (endh >> 1) : 0;       // word that is only half inside the piece
+            const bool need = lane < rows && (tail ? (endh & 1) != 0 : pr != 0);
+            const uint32_t word = lds_b32(strip + (uint32_t)lane * (UM_STRIP_PITCHW * 4) + 4u * (need ? wi : 0));
+            unsigned char* dst = static_cast<unsigned char*>(out) + (gr - pr) * 2 + 4 * (int64_t)wi + (tail ? 0 : 2);
+            stg_b16_if(dst, tail ? (word & 0xffffu) : (word >> 16), need);
+        }
+    }
+}
+
+template <typename Tag, bool OUT32, bool SOFT, bool WIDE>
+__global__ void __launch_bounds__(UL<WIDE>::THREADS, 1)
 blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps) {
+    static_assert(!(SOFT && WIDE), "the fused softmax keeps up to four 128-column chunks of a row");
+    using L = UL<WIDE>;
+    constexpr int BN = L::BN;
+    constexpr uint32_t GROUPS = L::GROUPS;
+    constexpr uint32_t NBUF = L::NBUF;
     extern __shared__ __align__(1024) unsigned char um_smem_raw[];  // the swizzled tiles need a 1024-byte aligned base
     unsigned char* smem = um_smem_raw;
     if (blk_smem_u32(smem) & 1023u) {  // cannot happen with the alignment above; checked because the swizzle relies on it
         if (threadIdx.x == 0) atomicCAS(p.status, 0, 9);
         return;
     }
-    constexpr int UM_SPLIT = SPLIT;
-    static_assert(!OUT32 || SPLIT == 2, "fp32 results: two arithmetic warps per quarter");
-    constexpr int UM_EPI_WARPS = 4 * UM_SPLIT;
-    unsigned char* strips = smem + UM_STAGES * UM_STAGE_BYTES;
-    float* xch = reinterpret_cast<float*>(strips + 8 * UM_STRIP_BYTES);
-    UmPiece* pieces_desc = reinterpret_cast<UmPiece*>(strips + 8 * UM_STRIP_BYTES + UM_XCH_BYTES);  // [quarter][strip]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(strips + 8 * UM_STRIP_BYTES + UM_XCH_BYTES + 8 * 32);
-    // bars[0..3] full (UM_STAGES used), [4..7] empty, [8..9] tmem_full, [10..11] tmem_empty; per quarter q:
-    // [16+q] rendezvous for the row statistics; per quarter and strip: [20 + 2q + b] strip filled, [28 + 2q + b] strip drained
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 13);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+    // [0..] stage full, [4..] stage empty, [8..] accumulator free, [12 + 4 g + i] chunk i mod 4 of group g ready,
+    // [28..] item record written, [36..] read by all, [44 + 4 (g / 2) + q] rendezvous of quarter q's warps of two groups
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 52);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 53);
+    Work* const ring = reinterpret_cast<Work*>(bars + 56);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_u32 = blk_smem_u32(smem);
     const uint32_t bar0 = blk_smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (4 + s); };
-    auto tfull_bar = [&](int b) { return bar0 + 8u * (8 + b); };
-    auto tempty_bar = [&](int b) { return bar0 + 8u * (10 + b); };
+    auto tempty_bar = [&](uint32_t b) { return bar0 + 8u * (8u + b); };
+    auto ready_bar = [&](uint32_t g, uint32_t k) { return bar0 + 8u * (12u + 4u * g + (k & 3u)); };
+    auto item_full = [&](uint32_t n) { return bar0 + 8u * (28u + n % UM_ITEMS); };
+    auto item_empty = [&](uint32_t n) { return bar0 + 8u * (36u + n % UM_ITEMS); };
+    // the group that takes a chunk: scores in turn (by slot); softmax two groups per item, in turn within it
+    auto group_of = [&](uint32_t slot, uint32_t n, int ch) {
+        return SOFT ? 2u * (n & 1u) + (((uint32_t)ch + (n >> 1)) & 1u) : slot % GROUPS;
+    };
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < UM_STAGES; ++s) {
+        for (int s = 0; s < 4; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
+            mbar_init(tempty_bar(s), 4);  // the warps of the group that consumed the chunk
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(tfull_bar(b), 1);
-            mbar_init(tempty_bar(b), UM_EPI_WARPS);
+        for (uint32_t i = 0; i < 16; ++i) mbar_init(ready_bar(i >> 2, i), 1);
+        for (uint32_t i = 0; i < 8; ++i) mbar_init(bar0 + 8u * (44u + i), 2);
+        for (uint32_t i = 0; i < UM_ITEMS; ++i) {
+            mbar_init(item_full(i), 1);
+            mbar_init(item_empty(i), 2 + 4 * GROUPS);  // producer, MMA, the groups
         }
         *abort_flag = 0;
-        for (int i = 0; i < 4; ++i) mbar_init(bar0 + 8u * (16 + i), UM_SPLIT);   // one arrival per arithmetic warp of the quarter
-        for (int i = 0; i < 8; ++i) mbar_init(bar0 + 8u * (20 + i), UM_SPLIT);   // strip filled: the quarter's arithmetic warps
-        for (int i = 0; i < 8; ++i) mbar_init(bar0 + 8u * (28 + i), 1);          // strip drained: its store warp
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {
@@ -212,533 +309,387 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t lim = p.spin_limit ? p.spin_limit : BLK_UMMA_SPIN_LIMIT;
+    auto item_wait = [&](uint32_t n) { return mbar_wait(item_full(n), (n / UM_ITEMS) & 1u, abort_flag, 11, lim); };
 
     if (warp == 0) {
-        // ---------------- producer ----------------
-        if (lane == 0 && !p.stall) {
+        // ---------------- producer (one lane) ----------------
+        if (elect_one() && !p.stall) {
             int stage = 0;
             uint32_t phase = 0;
-            Work wk;
-            bool ok = true;
-            // the operand tiles of chunk ch of an item
-            auto load_chunk = [&](const Work& k, int ch) {
-                for (int kb = 0; kb < k.nkb; ++kb) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 1, lim)) { ok = false; return; }
-                    const uint32_t sA = smem_u32 + stage * UM_STAGE_BYTES, sB = sA + UM_A_BYTES;
-                    mbar_expect_tx(full_bar(stage), UM_STAGE_BYTES);
+            bool ok = true, pre = false;
+#pragma unroll 1
+            for (uint32_t n = 0; ok; ++n) {
+                if (!item_wait(n)) break;
+                const Work& wk = ring[n % UM_ITEMS];
+                if (!wk.valid) break;
+                const int pair = wk.pair;
+                if (pair && !item_wait(n + 1u)) break;
+                chunk_order(wk.ch0, wk.nchunks, wk.sweeps, pair, pre, [&](bool next, int ch, bool) -> bool {
+                    const Work& k = ring[(next ? n + 1u : n) % UM_ITEMS];
                     // coordinates (k, row, head), or (k, head, row) for a token-major operand
-                    const int rA = k.it.rowA, rB = k.it.rowB + ch * UM_BN;
-                    tma_load_3d(sA, &maps.a[k.it.views & 255], full_bar(stage), kb * UM_BK, p.head_firstA ? k.head : rA,
-                                p.head_firstA ? rA : k.head);
-                    tma_load_3d(sB, &maps.b[k.it.views >> 8], full_bar(stage), kb * UM_BK, p.head_firstB ? k.head : rB,
-                                p.head_firstB ? rB : k.head);
-                    if (++stage == UM_STAGES) { stage = 0; phase ^= 1u; }
-                }
-            };
-            // the order of the chunks is that of the arithmetic warps (see there): first sweep (unless it ran alongside
-            // the previous item), then the storing chunks, each followed by a first-sweep chunk of the next item when
-            // the two items pair up
-            Work nx;
-            bool pre = false;
-            for (uint32_t w = blockIdx.x; ok && next_work(p, w, wk); w += gridDim.x) {
-                const bool pair = pairs_with_next(p, w, wk, nx);
-                if (wk.sweeps == 2 && !pre)
-                    for (int ch = 0; ok && ch < wk.nchunks; ++ch) load_chunk(wk, ch);
-                for (int ch = wk.it.ch0; ok && ch < wk.it.ch0 + wk.nchunks; ++ch) {
-                    load_chunk(wk, ch);
-                    if (ok && pair) load_chunk(nx, ch);
-                }
-                pre = pair;
+                    const int rA = k.rowA, rB = k.rowB + ch * BN, hd = k.head, K = k.K;
+                    const CUtensorMap *mapA = &maps.a[k.views & 255], *mapB = &maps.b[k.views >> 8];
+#pragma unroll 1
+                    for (int kk = 0; kk < K; kk += UM_BK) {
+                        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 1, lim)) { ok = false; return false; }
+                        const uint32_t sA = smem_u32 + stage * L::STAGE_BYTES, sB = sA + UM_A_BYTES;
+                        mbar_expect_tx(full_bar(stage), L::STAGE_BYTES);
+                        tma_load_3d(sA, mapA, full_bar(stage), kk, p.head_firstA ? hd : rA, p.head_firstA ? rA : hd);
+                        tma_load_3d(sB, mapB, full_bar(stage), kk, p.head_firstB ? hd : rB, p.head_firstB ? rB : hd);
+                        if (++stage == L::STAGES) { stage = 0; phase ^= 1u; }
+                    }
+                    return true;
+                });
+                pre = pair != 0;
+                mbar_arrive(item_empty(n));
+            }
+        }
+    } else if (warp == 2 + 4 * (int)GROUPS) {
+        // ---------------- planner (one lane): the records of the items ----------------
+        if (elect_one() && !p.stall) {
+            BlkUmmaItem it{}, nx{};  // records n and n + 1
+            int head = 0, nhead = 0;
+            bool have = fetch_item(p, 0, it, head), nhave = have && fetch_item(p, 1, nx, nhead);
+#pragma unroll 1
+            for (uint32_t n = 0;; ++n) {
+                if (!mbar_wait(item_empty(n), ((n / UM_ITEMS) & 1u) ^ 1u, abort_flag, 12, lim)) break;
+                publish<SOFT, WIDE>(p, ring + n % UM_ITEMS, it, head, n, have, nx, nhave);
+                mbar_arrive(item_full(n));  // release: the record is visible to whoever sees the phase end
+                if (!have) break;
+                it = nx;
+                head = nhead;
+                have = nhave;
+                if (nhave) nhave = fetch_item(p, n + 2u, nx, nhead);
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        // ---------------- MMA issue (one lane) ----------------
+        if (elect_one()) {
             int stage = 0;
-            uint32_t phase = 0, slot = 0;
-            Work wk;
-            bool ok = true;
-            // the products of chunk ch of an item into the next accumulator
-            auto mma_chunk = [&](const Work& k, int ch) {
-                const int buf = slot & 1;
-                if (!mbar_wait(tempty_bar(buf), ((slot >> 1) & 1u) ^ 1u, abort_flag, 2, lim)) { ok = false; return; }
-                tc_fence_after();
-                const int ncols = min(k.it.N - ch * UM_BN, UM_BN);
-                const uint32_t idesc = instr_desc(p.bf16, (ncols + 15) & ~15, p.epi == BLK_EPI_SOFTMAX && p.scale < 0.f);
-                const uint32_t d_tmem = tmem_base + (uint32_t)(buf * UM_BN);
-                for (int kb = 0; kb < k.nkb; ++kb) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, 3, lim)) { ok = false; return; }
-                    tc_fence_after();
-                    const uint32_t sA = smem_u32 + stage * UM_STAGE_BYTES, sB = sA + UM_A_BYTES;
-                    // steps of 16 along k in this block: all four, or as many as reach the end of a short last block
-                    const int ksteps = min(UM_BK / 16, (k.it.K - kb * UM_BK + 15) / 16);
+            uint32_t phase = 0, slot = 0, counts = 0;  // chunks so far; of the groups, modulo 4, a byte each
+            bool ok = true, pre = false;
+            const uint32_t idesc0 = instr_desc(p.bf16, 0, SOFT && p.scale < 0.f);
+#pragma unroll 1
+            for (uint32_t n = 0; ok; ++n) {
+                if (!item_wait(n)) break;
+                const Work& wk = ring[n % UM_ITEMS];
+                const int ch0 = wk.ch0, nchunks = wk.nchunks, sweeps = wk.sweeps, pair = wk.pair, N = wk.N, K = wk.K;
+                if (!wk.valid) break;
+                int N2 = 0, K2 = 0;
+                if (pair) {
+                    if (!item_wait(n + 1u)) break;
+                    N2 = ring[(n + 1u) % UM_ITEMS].N;
+                    K2 = ring[(n + 1u) % UM_ITEMS].K;
+                }
+                mbar_arrive(item_empty(n));
+                chunk_order(ch0, nchunks, sweeps, pair, pre, [&](bool next, int ch, bool) -> bool {
+                    // the chunk's products into the next accumulator
+                    const uint32_t buf = slot % NBUF, grp = group_of(slot, next ? n + 1u : n, ch);
+                    const uint32_t ready = ready_bar(grp, counts >> (8u * grp));
+                    const int ncols = min((next ? N2 : N) - ch * BN, BN);
+                    const uint32_t idesc = idesc0 | ((uint32_t)((ncols + 15) >> 4) << 18);  // columns in units of 16
+                    const uint32_t d_tmem = tmem_base + buf * (uint32_t)BN;
+                    if (!mbar_wait(tempty_bar(buf), ((slot / NBUF) & 1u) ^ 1u, abort_flag, 2, lim)) { ok = false; return false; }
+#pragma unroll 1
+                    for (int krem = next ? K2 : K, kb = 0; krem > 0; krem -= UM_BK, ++kb) {
+                        const uint32_t sA = smem_u32 + stage * L::STAGE_BYTES;
+                        const uint64_t da = smem_desc_sw128(sA), db = smem_desc_sw128(sA + UM_A_BYTES);
+                        if (!mbar_wait(full_bar(stage), phase, abort_flag, 3, lim)) { ok = false; return false; }
+                        tc_fence_after();
+                        // steps of 16 along k in this block: all four, or as many as reach the end of a short last block
+                        // (the tensor map fills what lies past K with zeros)
+                        if (krem > UM_BK - 16) {
 #pragma unroll
-                    for (int j = 0; j < UM_BK / 16; ++j)
-                        if (j < ksteps)
-                            tc_mma_f16(d_tmem, smem_desc_sw128(sA + 32 * j), smem_desc_sw128(sB + 32 * j), idesc, (kb | j) != 0);
-                    tc_commit(empty_bar(stage));  // stage reusable once these products have read it
-                    if (++stage == UM_STAGES) { stage = 0; phase ^= 1u; }
-                }
-                tc_commit(tfull_bar(buf));
-                ++slot;
-            };
-            Work nx;
-            bool pre = false;
-            for (uint32_t w = blockIdx.x; ok && next_work(p, w, wk); w += gridDim.x) {
-                const bool pair = pairs_with_next(p, w, wk, nx);
-                if (wk.sweeps == 2 && !pre)
-                    for (int ch = 0; ok && ch < wk.nchunks; ++ch) mma_chunk(wk, ch);
-                for (int ch = wk.it.ch0; ok && ch < wk.it.ch0 + wk.nchunks; ++ch) {
-                    mma_chunk(wk, ch);
-                    if (ok && pair) mma_chunk(nx, ch);
-                }
-                pre = pair;
+                            for (int j = 0; j < UM_BK / 16; ++j)
+                                tc_mma_f16(d_tmem, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, j ? 1u : (uint32_t)kb);
+                        } else {
+#pragma unroll 1
+                            for (int j = 0; 16 * j < krem; ++j)
+                                tc_mma_f16(d_tmem, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, (uint32_t)(kb | j));
+                        }
+                        tc_commit(empty_bar(stage));  // stage reusable once these products have read it
+                        if (++stage == L::STAGES) { stage = 0; phase ^= 1u; }
+                    }
+                    tc_commit(ready);
+                    ++slot;
+                    counts = (counts + (1u << (8u * grp))) & 0x03030303u;
+                    return true;
+                });
+                pre = pair != 0;
             }
-        }
-    } else if (warp >= 2 + UM_EPI_WARPS) {
-        // ---------------- stores: the last four warps, one per quarter ----------------
-        const int sq = warp & 3;
-        unsigned char* const C = reinterpret_cast<unsigned char*>(p.C);
-        constexpr int ES = OUT32 ? 4 : 2;
-        for (uint32_t n = 0;; ++n) {
-            // the quarter's pieces in order, piece m from strip m & 1
-            const int sb = (int)(n & 1u);
-            const uint32_t use = n >> 1;   // how often the strip has been used before
-            const uint32_t strip = blk_smem_u32(strips + (sq * 2 + sb) * UM_STRIP_BYTES);
-            const uint32_t filled_bar = bar0 + 8u * (20 + sq * 2 + sb), drained_bar = bar0 + 8u * (28 + sq * 2 + sb);
-            const volatile UmPiece* desc = pieces_desc + sq * 2 + sb;
-            if (!mbar_wait(filled_bar, use & 1u, abort_flag, 10, lim)) break;
-            if (desc->stop) break;
-            const int64_t g0 = desc->g0;
-            const int N = desc->N, pcols = desc->pcols, rows = desc->rows;
-            const bool halves = desc->halves != 0;
-            // lane l carries words l and l + 32 of a row: two stores of 128 contiguous bytes per row, four rows a batch
-            const uint32_t rbase = strip + 4u * lane;
-            if (!OUT32 && pcols == PCOLS16 && rows == 32) {
-                // A whole piece (the common case), with as few instructions per row as it takes: the store warps share
-                // their scheduler's issue slots with the arithmetic warps, and a row costing twenty instructions here
-                // made the second sweep issue bound.  Row k starts at element g0 + k N: at word (t >> 1) past the word
-                // of g0 with t = (g0 & 1) + k N, on its odd half when t is odd.  Words 1..63 of the row are whole; word 0
-                // is whole when the row starts on an even element (its upper half goes out below otherwise), and so does
-                // the lower half of word 64.
-                uint32_t* const w0 = reinterpret_cast<uint32_t*>(C) + (g0 >> 1) + lane;
-                uint32_t t = (uint32_t)(g0 & 1);
-#pragma unroll 2
-                for (int kb = 0; kb < 32; kb += 4) {
-                    uint32_t v[4][2];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        uint32_t* wp = w0 + (t >> 1);
-                        stg_b32_if(wp, v[k][0], lane >= (int)(t & 1u));
-                        asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp + 32), "r"(v[k][1]) : "memory");
-                        t += (uint32_t)N;
-                    }
-                }
-            } else if (OUT32 && pcols == UM_PW && rows == 32) {
-                // the same for a whole piece of fp32 results: row k is the 64 words from word g0 + k N on
-                uint32_t* wp = reinterpret_cast<uint32_t*>(C) + g0 + lane;
-#pragma unroll 2
-                for (int kb = 0; kb < 32; kb += 4) {
-                    uint32_t v[4][2];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp), "r"(v[k][0]) : "memory");
-                        asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp + 32), "r"(v[k][1]) : "memory");
-                        wp += N;
-                    }
-                }
-            } else if constexpr (OUT32) {
-                // a partial piece of fp32 results (fewer rows or columns): the same walk with the bounds as predicates
-                uint32_t* wp = reinterpret_cast<uint32_t*>(C) + g0 + lane;
-#pragma unroll 2
-                for (int kb = 0; kb < 32; kb += 4) {
-                    if (kb >= rows) break;
-                    uint32_t v[4][2];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const bool row_ok = kb + k < rows;
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) stg_b32_if(wp + 32 * i, v[k][i], row_ok && lane + 32 * i < pcols);
-                        wp += N;
-                    }
-                }
-            } else
-#pragma unroll 2
-            for (int kb = 0; kb < 32; kb += 4) {
-                if (kb >= rows) break;
-                uint32_t v[4][2];
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int64_t gr = g0 + (int64_t)(kb + k) * N;
-                    const int pr = OUT32 ? 0 : (int)(gr & 1);
-                    const bool row_ok = kb + k < rows;
-                    // whole words of the piece: [pr, (pr + pcols) / 2) for 16-bit elements, [0, pcols) for fp32
-                    const int wl = OUT32 ? pcols : ((pr + pcols) >> 1);
-                    uint32_t* wp = reinterpret_cast<uint32_t*>(C + (gr - pr) * ES);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int wi = lane + 32 * i;
-                        stg_b32_if(wp + wi, v[k][i], row_ok && wi >= pr && wi < wl);
-                    }
-                }
-            }
-            if (!OUT32 && halves) {
-                // half words at the ends: lane k the odd first element of row k, then the last element of row k when the
-                // piece ends on half a word
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const bool tail = t != 0;
-                    const int64_t gr = g0 + (int64_t)lane * N;
-                    const int pr = (int)(gr & 1);
-                    const int endh = pr + pcols;                 // half words [pr, endh) of the row's words are the piece
-                    const int wi = tail ? (endh >> 1) : 0;       // word that is only half inside the piece
-                    const bool need = lane < rows && (tail ? (endh & 1) != 0 : pr != 0);
-                    const uint32_t word = lds_b32(strip + (uint32_t)lane * (UM_STRIP_PITCHW * 4) + 4u * (need ? wi : 0));
-                    unsigned char* dst = C + (gr - pr) * 2 + 4 * (int64_t)wi + (tail ? 0 : 2);
-                    stg_b16_if(dst, tail ? (word & 0xffffu) : (word >> 16), need);
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(drained_bar);
         }
     } else {
-        // ---------------- epilogue arithmetic: warps 2 .. 2 + 4 SPLIT - 1 ----------------
-        // lane quarter q = warp % 4 (the 32 accumulator lanes a warp may read); the SPLIT warps of a quarter split the
-        // columns (share h: the columns c of a chunk with (c mod PC) / SH == h) and exchange their partial row
-        // statistics.
-        const int q = warp & 3, h = (warp - 2) >> 2;  // h in [0, UM_SPLIT)
+        // ---------------- epilogue: groups of four warps ----------------
+        const int q = warp & 3;
+        const uint32_t grp = (uint32_t)(warp - 2) >> 2;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-        const int myrow = q * 32 + lane;
-        uint32_t slot = 0, seq = 0;
-        Work wk;
-        bool ok = true;
-        const bool softmax = p.epi == BLK_EPI_SOFTMAX;
-        const float sl = softmax ? fabsf(p.scale) * BLK_LOG2E : p.scale;  // a negative softmax scale is applied by
-                                                                          // the MMA (negated A), see instr_desc
-        constexpr int ES = OUT32 ? 4 : 2;
-        constexpr int PC = UM_PW * 4 / ES;   // columns of a staged row piece: 128 x 16-bit or 64 x fp32
-        constexpr int SH = PC / UM_SPLIT;    // columns of a piece this warp converts (32 words)
-        // Rendezvous of the two warps of a quarter: an mbarrier that one lane of each warp arrives on, waited for like
-        // every other barrier (suspended, bounded), so that a warp whose partner gave up cannot wait for ever.
-        const uint32_t stat_bar = bar0 + 8u * (16 + q);
-        uint32_t stat_phase = 0;
-        auto pair_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(stat_bar);
-            const bool good = mbar_wait(stat_bar, stat_phase, abort_flag, 8, lim);
-            stat_phase ^= 1u;
-            __syncwarp();
+        const uint32_t strip = smem_u32 + L::STRIP_OFF + (uint32_t)(warp - 2) * UM_STRIP_BYTES;
+        const uint32_t srow = strip + (uint32_t)lane * (UM_STRIP_PITCHW * 4);
+        const float sl = SOFT ? fabsf(p.scale) * BLK_LOG2E : p.scale;  // a negative softmax scale is applied by the MMA (negated A)
+        const float2 sl2 = make_float2(sl, sl);
+        constexpr int PC = OUT32 ? UM_PW : 2 * UM_PW;  // columns of a staged piece
+        uint32_t slot = 0, mychunks = 0, meetings = 0;
+        bool ok = true, pre = false;
+
+        auto chunk_wait = [&]() -> bool {
+            const bool good = mbar_wait(ready_bar(grp, mychunks), (mychunks >> 2) & 1u, abort_flag, 4, lim);
+            ++mychunks;
+            tc_fence_after();
             return good;
         };
-        uint32_t pieces = 0;  // pieces staged so far by this quarter: piece n goes into strip n & 1
-
-        // Stage the piece of up to PC columns starting at column c0 of the 32 rows of this quarter for its store warp.
-        // tcol(c) gives the tensor-memory column of row column c; pack(r, w) turns 32 raw accumulator words into
-        // output words (32 fp32 words, or 16 words of 16-bit pairs); loaded() runs right after this warp's last
-        // tensor-memory load of the piece, where the caller hands the accumulator back to the MMA role.  This warp
-        // converts columns [c0 + h SH, c0 + (h + 1) SH) of its lane's row and writes the words into the row of the
-        // strip, at the word the element has in global memory: strip word j of a row holds the output's 32-bit word
-        // (first word of the piece) + j.  A 16-bit piece that starts on an odd element is shifted by half a word with
-        // a funnel shift through the previous pair; its first and last half words are written as 16-bit stores, since
-        // the other half of those words belongs to the other warp.
-        auto store_piece = [&](int c0, int pcols, auto tcol, auto pack, int64_t cbase, int M, int N, bool anyodd,
-                               auto loaded) -> bool {
-            uint32_t r[32];
-            const int sb = (int)(pieces & 1u);
-            const uint32_t strip = blk_smem_u32(strips + (q * 2 + sb) * UM_STRIP_BYTES);
-            const uint32_t filled_bar = bar0 + 8u * (20 + q * 2 + sb), drained_bar = bar0 + 8u * (28 + q * 2 + sb);
-            const int64_t g = cbase + (int64_t)myrow * N + c0;       // element index of this lane's piece in the output
-            const uint32_t par = OUT32 ? 0u : (uint32_t)(g & 1);
-            [[maybe_unused]] const uint32_t par16 = par * 16u;
-            const uint32_t srow = strip + (uint32_t)lane * (UM_STRIP_PITCHW * 4) + (uint32_t)h * (SH * ES);  // word 32 h of my row
-            const int mycols = min(SH, pcols - h * SH);              // columns of the piece this warp converts (<= 0: none)
-            // the strip's previous piece (two pieces ago) has been written out
-            if (!mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, 8, lim)) return false;
-            if (mycols <= 0) {
-                loaded();
-            } else if constexpr (OUT32) {
-                uint32_t w[32];
-                tc_ld32(lane_addr + tcol(c0 + h * SH), r);
-                loaded();
-                pack(r, w);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) blk_sts_b32(srow + 4 * i, w[i]);
-            } else {
-                uint32_t w[16];
-                uint32_t prev = 0;
-                const int nu = (mycols + UM_PIECE - 1) / UM_PIECE;
-                for (int u = 0; u < nu; ++u) {
-                    tc_ld32(lane_addr + tcol(c0 + h * SH + u * UM_PIECE), r);
-                    if (u == nu - 1) loaded();
-                    pack(r, w);
-                    const uint32_t a = srow + 64 * u;
-                    if (!anyodd) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) blk_sts_b32(a + 4 * i, w[i]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const uint32_t v = __funnelshift_l(prev, w[i], par16);
-                            if (u == 0 && i == 0) {
-                                // the low half of my first word is the other warp's last element when the piece is odd
-                                if (par) blk_sts_b16(a + 2, v >> 16);
-                                else blk_sts_b32(a, v);
-                            } else {
-                                blk_sts_b32(a + 4 * i, v);
-                            }
-                            prev = w[i];
-                        }
-                    }
-                }
-                if (anyodd && par) blk_sts_b16(srow + 64 * nu, prev >> 16);  // my last element: low half of the next word
-            }
-            if (h == 0 && lane == 0) {
-                volatile UmPiece* d = pieces_desc + q * 2 + sb;
-                d->g0 = cbase + (int64_t)(q * 32) * N + c0;
-                d->N = N;
-                d->pcols = pcols;
-                d->rows = max(0, min(M - q * 32, 32));
-                d->halves = (anyodd || (pcols & 1)) ? 1 : 0;
-                d->stop = 0;
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(filled_bar);
-            ++pieces;
-            return true;
-        };
-        // the pieces of columns [c_lo, c_hi) of a chunk
-        auto store_cols = [&](int c_lo, int c_hi, auto tcol, auto pack, int64_t cbase, int M, int N, bool anyodd,
-                              auto loaded) -> bool {
-            for (int c0 = c_lo; c0 < c_hi; c0 += PC) {
-                const bool last = c0 + PC >= c_hi;
-                if (!store_piece(c0, min(PC, c_hi - c0), tcol, pack, cbase, M, N, anyodd, [&]() { if (last) loaded(); }))
-                    return false;
-            }
-            return true;
-        };
-        // pack(r, w) for an elementwise map of the accumulator values
-        auto pack_with = [](auto xform) {
-            return [xform](const uint32_t (&r)[32], auto& w) {
-                if constexpr (OUT32) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(xform(__uint_as_float(r[i])));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        w[i] = BlkCvt<Tag>::pack2(xform(__uint_as_float(r[2 * i])), xform(__uint_as_float(r[2 * i + 1])));
-                }
-            };
-        };
-        // First sweep of a row too long for tensor memory, one chunk: running (maximum, sum) over this warp's blocks.
-        float mx1 = -INFINITY, sum1 = 0.f;
-        auto first_sweep_chunk = [&](int N, int ch) {
-            uint32_t r[32];
-            const int buf = slot & 1;
-            if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 6, lim)) { ok = false; return; }
-            tc_fence_after();
-            const int ncols = min(N - ch * UM_BN, UM_BN);
-            for (int b0 = h * SH; b0 < ncols; b0 += PC) {
-                const int hi = min(b0 + SH, ncols);
-                for (int c = b0; c < hi; c += UM_PIECE) {
-                    tc_ld32(lane_addr + (uint32_t)(buf * UM_BN + c), r);
-                    const bool part = c + 32 > hi;
-                    if (part) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (c + i >= hi) r[i] = 0xff800000u;  // -inf
-                    }
-                    float pm = -INFINITY;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) pm = blk_max3(pm, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                    const float mnew = fmaxf(mx1, pm);  // finite: column c of the piece is inside the row
-                    const float nm = -mnew * sl;
-                    float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) s4[i & 3] += blk_exp2(fmaf(__uint_as_float(r[i]), sl, nm));
-                    sum1 = sum1 * blk_exp2((mx1 - mnew) * sl) + ((s4[0] + s4[1]) + (s4[2] + s4[3]));
-                    mx1 = mnew;
-                }
-            }
+        auto release = [&](uint32_t buf) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(buf));
-            ++slot;
         };
-        // The quarter's warps combine their (maximum, sum) of a finished first sweep; the result is the offset with which
-        // exp2(x * sl + off) = exp2((x - max) * sl) / sum: no multiply after the exponential in the second sweep.
-        float off_next = 0.f;
-        auto first_sweep_done = [&]() {
-            volatile float* xm = xch + (seq++ & 1) * (2 * UM_SPLIT * 128);  // [part][row] maxima, then [UM_SPLIT + part][row] sums
-            xm[h * 128 + myrow] = mx1;
-            xm[(UM_SPLIT + h) * 128 + myrow] = sum1;
-            if (!pair_sync()) { ok = false; return; }
-            // a warp whose share held no column of the row (a last chunk of at most 64 columns) has maximum -inf
-            // and sum 0: its term is skipped
-            float m = -INFINITY;
-#pragma unroll
-            for (int o = 0; o < UM_SPLIT; ++o) m = fmaxf(m, xm[o * 128 + myrow]);
-            float l = 0.f;
-#pragma unroll
-            for (int o = 0; o < UM_SPLIT; ++o) {
-                const float mo = xm[o * 128 + myrow];
-                if (mo != -INFINITY) l += xm[(UM_SPLIT + o) * 128 + myrow] * blk_exp2((mo - m) * sl);
-            }
-            off_next = -m * sl - __log2f(l);
-        };
-        Work nx;
-        bool pre = false;  // this item's first sweep ran alongside the previous item's second
-        for (uint32_t w = blockIdx.x; ok && next_work(p, w, wk); w += gridDim.x) {
-            const bool pair = pairs_with_next(p, w, wk, nx);
-            const bool had_first = pre;
-            pre = pair;
-            const int M = wk.it.M - wk.it.tm * UM_BM;  // rows of the segment from this block on
-            const int N = wk.it.N;
-            const int64_t cbase = (int64_t)wk.head * p.Dout + wk.it.offC + (int64_t)wk.it.tm * UM_BM * N;
-            // 16-bit rows that start on an odd element need the half-word shift while staging (chunks and pieces start
-            // on even columns, so a row's parity is the same for all of them); the quarter's warps hold the same rows
-            const bool anyodd = !OUT32 && __any_sync(0xffffffffu, (int)((cbase + (int64_t)myrow * N) & 1));
-            if (!softmax) {
-                for (int ch = wk.it.ch0; ok && ch < wk.it.ch0 + wk.nchunks; ++ch, ++slot) {
-                    const int buf = slot & 1;
-                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 4, lim)) { ok = false; break; }
-                    tc_fence_after();
-                    const int ncols = min(N - ch * UM_BN, UM_BN);
-                    auto release = [&]() {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(tempty_bar(buf));
-                    };
-                    ok = store_cols(ch * UM_BN, ch * UM_BN + ncols,
-                                    [&](int c) { return (uint32_t)(buf * UM_BN + (c - ch * UM_BN)); },
-                                    pack_with([sl](float x) { return x * sl; }), cbase, M, N, anyodd, release);
-                }
-            } else if (wk.sweeps == 1) {
-                // whole row resident: chunk k of the row sits in accumulator (slot + k) & 1
-                volatile float* xm = xch + (seq++ & 1) * (2 * UM_SPLIT * 128);  // [part][row] maxima, then [UM_SPLIT + part][row] sums
-                for (int ch = 0; ok && ch < wk.nchunks; ++ch)
-                    if (!mbar_wait(tfull_bar((slot + ch) & 1), ((slot + ch) >> 1) & 1u, abort_flag, 5, lim)) ok = false;
-                if (!ok) break;
-                tc_fence_after();
-                auto tcol = [&](int c) {  // tensor-memory column of row column c
-                    return (uint32_t)((((slot + (c >> 8)) & 1) * UM_BN) + (c & (UM_BN - 1)));
-                };
+        // f(values, unit) for the 32-column units of [col, col + 32 units) of the accumulators; loaded() after the last load.
+        // (Four warps per scheduler hide a load's latency; a second buffer of values would not fit their registers.)
+        auto each_unit = [&](uint32_t col, int units, auto f, auto loaded) {
+#pragma unroll 1
+            for (int u = 0; u < units; ++u) {
                 uint32_t r[32];
-                // pass 1: maximum over this warp's blocks
-                float mx = -INFINITY;
-                for (int b0 = h * SH; b0 < N; b0 += PC) {
-                    const int bend = min(b0 + SH, N);
-                    for (int c = b0; c < bend; c += UM_PIECE) {
-                        tc_ld32(lane_addr + tcol(c), r);
-                        if (c + 32 <= bend) {
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) mx = blk_max3(mx, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (c + i < bend) mx = fmaxf(mx, __uint_as_float(r[i]));
-                        }
-                    }
-                }
-                xm[h * 128 + myrow] = mx;
-                if (!pair_sync()) { ok = false; break; }
-#pragma unroll
-                for (int o = 0; o < UM_SPLIT; ++o) mx = fmaxf(mx, xm[o * 128 + myrow]);
-                const float nm = -mx * sl;
-                // pass 2: exponentials back into tensor memory, partial sum
-                float s4[4] = {0.f, 0.f, 0.f, 0.f};
-                for (int b0 = h * SH; b0 < N; b0 += PC) {
-                    const int bend = min(b0 + SH, N);
-                    for (int c = b0; c < bend; c += UM_PIECE) {
-                        tc_ld32(lane_addr + tcol(c), r);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            float e = blk_exp2(fmaf(__uint_as_float(r[i]), sl, nm));
-                            if (c + 32 > bend) e = (c + i < bend) ? e : 0.f;
-                            s4[i & 3] += e;
-                            r[i] = __float_as_uint(e);
-                        }
-                        tc_st32(lane_addr + tcol(c), r);
-                    }
-                }
-                tc_wait_st();
-                float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-                xm[(UM_SPLIT + h) * 128 + myrow] = sum;
-                if (!pair_sync()) { ok = false; break; }
-                sum = 0.f;
-#pragma unroll
-                for (int o = 0; o < UM_SPLIT; ++o) sum += xm[(UM_SPLIT + o) * 128 + myrow];
-                const float inv = __frcp_rn(sum);
-                // pass 3: normalise and stage (this warp reads back the columns it wrote in pass 2); an accumulator goes
-                // back to the MMA role as soon as this warp has read its share of it, so the next item's products overlap
-                // the rest of this item's epilogue
-                for (int ch = 0; ok && ch < wk.nchunks; ++ch) {
-                    auto release = [&]() {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(tempty_bar((slot + ch) & 1));
-                    };
-                    ok = store_cols(ch * UM_BN, min((ch + 1) * UM_BN, N), tcol, pack_with([inv](float x) { return x * inv; }),
-                                    cbase, M, N, anyodd, release);
-                }
-                slot += wk.nchunks;
-            } else {
-                // two sweeps: running (max, sum) over this warp's blocks, then recompute and stage; when the next item
-                // pairs with this one, each storing chunk is followed by a first-sweep chunk of the next item, whose
-                // exponentials run while this chunk's pieces drain
-                if (!had_first) {
-                    mx1 = -INFINITY; sum1 = 0.f;
-                    for (int ch = 0; ok && ch < wk.nchunks; ++ch) first_sweep_chunk(N, ch);
-                    if (ok) first_sweep_done();
-                    if (!ok) break;
-                }
-                const float off = off_next;
-                if (pair) { mx1 = -INFINITY; sum1 = 0.f; }
-                for (int ch = 0; ok && ch < wk.nchunks; ++ch) {
-                    const int buf = slot & 1;
-                    if (!mbar_wait(tfull_bar(buf), (slot >> 1) & 1u, abort_flag, 7, lim)) { ok = false; break; }
-                    tc_fence_after();
-                    const int ncols = min(N - ch * UM_BN, UM_BN);
-                    auto release = [&]() {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(tempty_bar(buf));
-                    };
-                    ok = store_cols(ch * UM_BN, ch * UM_BN + ncols,
-                                    [&](int c) { return (uint32_t)(buf * UM_BN + (c - ch * UM_BN)); },
-                                    pack_with([sl, off](float x) { return blk_exp2(fmaf(x, sl, off)); }), cbase, M, N, anyodd,
-                                    release);
-                    ++slot;
-                    if (ok && pair) first_sweep_chunk(nx.it.N, ch);
-                }
-                if (ok && pair) first_sweep_done();
+                tc_ld32_nowait(col + 32u * u, r);
+                tc_ld_wait(r);
+                if (u == units - 1) loaded();
+                f(r, u);
             }
-        }
-        // tell the quarter's store warp that nothing follows: one more "piece" that only says stop (posted on both strips;
-        // the store warp leaves at the first)
-        for (int t = 0; t < 2; ++t) {
-            const int sb = (int)(pieces & 1u);
-            const uint32_t filled_bar = bar0 + 8u * (20 + q * 2 + sb), drained_bar = bar0 + 8u * (28 + q * 2 + sb);
-            if (ok && !mbar_wait(drained_bar, ((pieces >> 1) & 1u) ^ 1u, abort_flag, 8, lim)) ok = false;
-            if (h == 0 && lane == 0) (pieces_desc + q * 2 + sb)->stop = 1;
+        };
+        // Columns [c0, c0 + cols) of this warp's rows (the first starts at element cbase), from accumulator columns col on,
+        // through xform (two values at a time) to the output; loaded() after the last load.
+        auto put = [&](uint32_t col, int c0, int cols, int64_t cbase, int rows, int N, bool anyodd, auto xform, auto loaded) {
+#pragma unroll 1
+            for (int pc = 0; pc < cols; pc += PC) {
+                const int pcols = min(PC, cols - pc);
+                const int64_t g0 = cbase + c0 + pc;
+                const uint32_t par = OUT32 ? 0u : (uint32_t)((g0 + (int64_t)lane * N) & 1);
+                uint32_t prev = 0;
+                each_unit(col + (uint32_t)pc, (pcols + 31) >> 5,
+                          [&](const uint32_t (&r)[32], int u) {
+                              if constexpr (OUT32) {
+#pragma unroll
+                                  for (int i = 0; i < 32; i += 2) {
+                                      const float2 v = xform(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])));
+                                      blk_sts_f32(srow + 128u * u + 4 * i, v.x);
+                                      blk_sts_f32(srow + 128u * u + 4 * i + 4, v.y);
+                                  }
+                              } else {
+                                  uint32_t w[16];
+#pragma unroll
+                                  for (int i = 0; i < 16; ++i) {
+                                      const float2 v = xform(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+                                      w[i] = BlkCvt<Tag>::pack2(v.x, v.y);
+                                  }
+                                  const uint32_t a = srow + 64u * u;
+                                  if (!anyodd) {
+#pragma unroll
+                                      for (int i = 0; i < 16; ++i) blk_sts_b32(a + 4 * i, w[i]);
+                                  } else {
+                                      // a row that starts on an odd element is shifted by half a word
+#pragma unroll
+                                      for (int i = 0; i < 16; ++i) {
+                                          blk_sts_b32(a + 4 * i, __funnelshift_l(prev, w[i], par * 16u));
+                                          prev = w[i];
+                                      }
+                                  }
+                              }
+                          },
+                          [&]() { if (pc + PC >= cols) loaded(); });
+                if (!OUT32 && anyodd) blk_sts_b32(srow + 64u * (uint32_t)((pcols + 31) >> 5), prev >> 16);
+                __syncwarp();
+                store_strip<OUT32>(strip, p.C, g0, N, pcols, rows, anyodd || (pcols & 1), lane);
+                __syncwarp();
+            }
+        };
+        auto mask_unit = [](uint32_t (&r)[32], int lim_) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (i >= lim_) r[i] = 0xff800000u;  // -inf
+        };
+        // Softmax, running over the units of a row that this warp has: reference and sum of exp2((x - reference) sl).
+        float ref = -INFINITY, sum = 0.f;
+        // Rendezvous with the warp of the other group that shares the item's rows: mbarrier, bounded like every wait.
+        auto meet = [&]() -> bool {
+            const uint32_t bar = bar0 + 8u * (44u + 4u * (grp >> 1) + (uint32_t)q);
             __syncwarp();
-            if (lane == 0) mbar_arrive(filled_bar);
-            ++pieces;
+            if (lane == 0) mbar_arrive(bar);
+            return mbar_wait(bar, meetings++ & 1u, abort_flag, 8, lim);
+        };
+        // Reference and sum of the whole row, through the strips (free at that time); false when the other gave up.
+        auto combine = [&](float& m, float& l) -> bool {
+            const uint32_t mine = strip + 8u * lane, other = strip + ((grp & 1u) ? -4 * UM_STRIP_BYTES : 4 * UM_STRIP_BYTES) + 8u * lane;
+            blk_sts_f32x2(mine, ref, sum);
+            if (!meet()) return false;
+            const float r2 = __uint_as_float(lds_b32(other)), s2 = __uint_as_float(lds_b32(other + 4));
+            m = fmaxf(ref, r2);
+            l = (ref == -INFINITY ? 0.f : sum * blk_exp2((ref - m) * sl)) + (r2 == -INFINITY ? 0.f : s2 * blk_exp2((r2 - m) * sl));
+            return meet();  // both have read: the strips may be written
+        };
+        // New reference for a unit; true when some row's has moved (f: what its earlier exponentials are to be multiplied by)
+        auto unit_ref = [&](const uint32_t (&r)[32], float& f) -> bool {
+            float m4[4] = {ref, __uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2])};
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m4[e] = blk_max3(m4[e], __uint_as_float(r[i + 2 * e]), __uint_as_float(r[i + 2 * e + 1]));
+            const float m = fmaxf(blk_max3(m4[0], m4[1], m4[2]), m4[3]);
+            const bool move = (m - ref) * sl > UM_LAZY;  // always at the first unit (ref = -inf)
+            if (!__any_sync(0xffffffffu, move)) return false;
+            f = move ? blk_exp2((ref - m) * sl) : 1.f;
+            if (move) ref = m;
+            return true;
+        };
+        // exponentials of a unit in place, added to the sum; sum_only: the values are not wanted, and half of the exponentials
+        // go to the multiply-add pipe (a two-sweep softmax takes two exponentials per element, which kept the
+        // special-function unit 57 % busy; 512 segments of 16..2048 rows 870 -> 834 us)
+        auto unit_exp = [&](uint32_t (&r)[32], auto sum_only) {
+            const float nm = ref == -INFINITY ? 0.f : -ref * sl;
+            const float2 nm2 = make_float2(nm, nm);
+            float2 s2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                float2 t = blk_fma2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2, nm2);
+                if (decltype(sum_only)::value && (i & 2)) {
+                    t = blk_exp2_fma2(t);
+                } else {
+                    t.x = blk_exp2(t.x);
+                    t.y = blk_exp2(t.y);
+                }
+                s2[(i >> 1) & 1] = blk_add2(s2[(i >> 1) & 1], t);
+                r[i] = __float_as_uint(t.x);
+                r[i + 1] = __float_as_uint(t.y);
+            }
+            sum += (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
+        };
+
+#pragma unroll 1
+        for (uint32_t n = 0; ok; ++n) {
+            if (!item_wait(n)) break;
+            const Work& wk = ring[n % UM_ITEMS];
+            const int rec_rows = wk.rows, N = wk.N, ch0 = wk.ch0, nchunks = wk.nchunks, sweeps = wk.sweeps, pair = wk.pair;
+            const int next_rows = wk.next_rows, next_N = wk.next_N, valid = wk.valid;
+            const int r0 = (q - (rec_rows >> 8)) * 32;  // row of the block that this warp's first lane holds
+            const int64_t cbase = wk.cbase + (int64_t)r0 * N;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(item_empty(n));
+            if (!valid) break;
+            const int rows = min((rec_rows & 255) - r0, 32);
+            const bool here = r0 >= 0 && rows > 0;  // some of this warp's rows exist
+            // 16-bit rows that start on an odd element need the half-word shift while staging (chunks and pieces start
+            // on even columns, so a row's parity is the same for all of them)
+            const bool anyodd = !OUT32 && __any_sync(0xffffffffu, (int)((cbase + (int64_t)lane * N) & 1));
+            if constexpr (SOFT) {
+                if (sweeps == 1) {
+                    if ((n & 1u) == grp >> 1) {
+                        // the whole row resident: chunk k in accumulator (slot + k) mod NBUF; this warp has every other one
+                        const int k0 = (int)((grp ^ (n >> 1)) & 1u);
+                        ref = -INFINITY;
+                        sum = 0.f;
+#pragma unroll 1
+                        for (int k = k0; k < nchunks; k += 2) {
+                            if (!chunk_wait()) { ok = false; break; }
+                            const uint32_t buf = (slot + (uint32_t)k) % NBUF;
+                            if (!here) { release(buf); continue; }
+                            const int cols = min(N - k * BN, BN);
+                            const uint32_t col = lane_addr + buf * (uint32_t)BN;
+                            each_unit(col, (cols + 31) >> 5,
+                                      [&](uint32_t (&r)[32], int u) {
+                                          if (32 * u + 32 > cols) mask_unit(r, cols - 32 * u);
+                                          float f;
+                                          if (unit_ref(r, f) && (k > k0 || u)) {
+                                              // a reference moved far: what this warp has written is rescaled
+                                              sum *= f;
+#pragma unroll 1
+                                              for (int c = k0 * BN; c < k * BN + 32 * u; c += 16) {
+                                                  if (((c / BN) ^ k0) & 1) continue;  // the other warp's chunk
+                                                  uint32_t o[16];
+                                                  const uint32_t at = lane_addr + ((slot + (uint32_t)(c / BN)) % NBUF) * (uint32_t)BN + (uint32_t)(c % BN);
+                                                  tc_wait_st();
+                                                  tc_ld16(at, o);
+#pragma unroll
+                                                  for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+                                                  tc_st16(at, o);
+                                              }
+                                          }
+                                          unit_exp(r, UmNo{});
+                                          tc_st32(col + 32u * u, r);
+                                      },
+                                      []() {});
+                        }
+                        if (!ok) break;
+                        if (here && nchunks > k0) {
+                            tc_wait_st();
+                            float m = ref, l = sum;
+                            if (nchunks > 1 && !combine(m, l)) { ok = false; break; }
+                            const float inv = __frcp_rn(l) * (nchunks > 1 ? blk_exp2((ref - m) * sl) : 1.f);
+                            const float2 inv2 = make_float2(inv, inv);
+#pragma unroll 1
+                            for (int k = k0; k < nchunks; k += 2) {
+                                const uint32_t buf = (slot + (uint32_t)k) % NBUF;
+                                put(lane_addr + buf * (uint32_t)BN, k * BN, min(N - k * BN, BN), cbase, rows, N, anyodd,
+                                    [&](float2 v) { return blk_mul2(v, inv2); }, [&]() { release(buf); });
+                            }
+                        }
+                    }
+                    slot += (uint32_t)nchunks;
+                } else {
+                    // (after `pre` the reference and sum are those of the first sweep that ran alongside the item before)
+                    bool begun = false, off_known = false;
+                    float off = 0.f;
+                    chunk_order(ch0, nchunks, sweeps, pair, pre, [&](bool next, int ch, bool first) -> bool {
+                        const uint32_t buf = slot % NBUF, owner = group_of(slot, next ? n + 1u : n, ch);
+                        ++slot;
+                        if (owner != grp) return true;
+                        if (!chunk_wait()) { ok = false; return false; }
+                        const int cols = min((next ? next_N : N) - ch * BN, BN);
+                        const uint32_t col = lane_addr + buf * (uint32_t)BN;
+                        const int nr0 = (q - (next_rows >> 8)) * 32;
+                        if (next ? nr0 < 0 || nr0 >= (next_rows & 255) : !here) { release(buf); return true; }
+                        if (first) {
+                            if (!begun) {
+                                begun = true;
+                                ref = -INFINITY;
+                                sum = 0.f;
+                            }
+                            each_unit(col, (cols + 31) >> 5,
+                                      [&](uint32_t (&r)[32], int u) {
+                                          if (32 * u + 32 > cols) mask_unit(r, cols - 32 * u);
+                                          float f;
+                                          if (unit_ref(r, f)) sum *= f;
+                                          unit_exp(r, UmYes{});
+                                      },
+                                      [&]() { release(buf); });
+                        } else {
+                            if (!off_known) {
+                                // exp2(x sl + off) = exp2((x - m) sl) / l: no multiply after the exponential
+                                float m, l;
+                                if (!combine(m, l)) { ok = false; return false; }
+                                off_known = true;
+                                off = -m * sl - __log2f(l);
+                            }
+                            const float2 off2 = make_float2(off, off);
+                            put(col, ch * BN, cols, cbase, rows, N, anyodd,
+                                [&](float2 v) {
+                                    const float2 t = blk_fma2(v, sl2, off2);
+                                    return make_float2(blk_exp2(t.x), blk_exp2(t.y));
+                                },
+                                [&]() { release(buf); });
+                        }
+                        return true;
+                    });
+                    pre = pair != 0;
+                }
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < nchunks; ++k, ++slot) {
+                    if (slot % GROUPS != grp) continue;
+                    const uint32_t buf = slot % NBUF;
+                    const int c0 = (ch0 + k) * BN;
+                    if (!chunk_wait()) { ok = false; break; }
+                    if (!here) { release(buf); continue; }
+                    put(lane_addr + buf * (uint32_t)BN, c0, min(N - c0, BN), cbase, rows, N, anyodd,
+                        [&](float2 v) { return blk_mul2(v, sl2); }, [&]() { release(buf); });
+                }
+            }
         }
     }
 
@@ -770,14 +721,14 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <typename Tag, bool OUT32, int SPLIT>
+template <typename Tag, bool OUT32, bool SOFT, bool WIDE>
 cudaError_t launch(const BlkUmmaParams& p, const UmMaps& maps, int sms, cudaStream_t st) {
-    auto kern = blk_gemm_umma_kernel<Tag, OUT32, SPLIT>;
-    cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), UM_SMEM_BYTES);
+    auto kern = blk_gemm_umma_kernel<Tag, OUT32, SOFT, WIDE>;
+    cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), UL<WIDE>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_items * p.H;
-    const dim3 grid((unsigned)(total < sms ? total : sms)), block(um_threads(SPLIT));
-    kern<<<grid, block, UM_SMEM_BYTES, st>>>(p, maps);
+    const dim3 grid((unsigned)(total < sms ? total : sms)), block(UL<WIDE>::THREADS);
+    kern<<<grid, block, UL<WIDE>::SMEM_BYTES, st>>>(p, maps);
     return cudaGetLastError();
 }
 
@@ -875,7 +826,7 @@ namespace {
 struct LaunchKey {
     const void *a, *b;
     int64_t Da, Db, H;
-    int na, nb, bf16, ga, gb;
+    int na, nb, bf16, ga, gb, wide;
     BlkOperandLayout layA, layB;
     BlkUmmaView va[BLK_UMMA_VIEWS], vb[BLK_UMMA_VIEWS];
 };
@@ -886,7 +837,7 @@ uint64_t g_launch_clock = 0;
 std::mutex g_launch_mu;
 bool same_key(const LaunchKey& x, const LaunchKey& y) {
     if (x.a != y.a || x.b != y.b || x.Da != y.Da || x.Db != y.Db || x.H != y.H || x.na != y.na || x.nb != y.nb ||
-        x.bf16 != y.bf16 || x.ga != y.ga || x.gb != y.gb)
+        x.bf16 != y.bf16 || x.wide != y.wide || x.ga != y.ga || x.gb != y.gb)
         return false;
     auto lay_eq = [](const BlkOperandLayout& p, const BlkOperandLayout& q) {
         return p.rows == q.rows && p.row_stride == q.row_stride && p.head_stride == q.head_stride;
@@ -909,6 +860,7 @@ cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand
     static thread_local UmMaps maps;
     key.a = A.base; key.b = B.base; key.Da = A.D; key.Db = B.D; key.H = p.H;
     key.na = A.num_views; key.nb = B.num_views; key.bf16 = p.bf16;
+    key.wide = p.wide;  // the box of the second operand
     key.ga = A.given != nullptr; key.gb = B.given != nullptr;
     if (A.given) key.layA = *A.given;
     if (B.given) key.layB = *B.given;
@@ -943,7 +895,7 @@ cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand
             }
             return true;
         };
-        if (!encode(A, maps.a, UM_BM, &p.head_firstA) || !encode(B, maps.b, UM_BN, &p.head_firstB)) return cudaErrorInvalidValue;
+        if (!encode(A, maps.a, UM_BM, &p.head_firstA) || !encode(B, maps.b, key.wide ? UL<true>::BN : UL<false>::BN, &p.head_firstB)) return cudaErrorInvalidValue;
         std::lock_guard<std::mutex> g(g_launch_mu);
         LaunchSlot* victim = &g_launch_slots[0];
         for (LaunchSlot& sl : g_launch_slots) {
@@ -957,10 +909,12 @@ cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand
         victim->stamp = ++g_launch_clock;
         victim->used = true;
     }
-    const bool four = !p.out_f32 && p.epi == BLK_EPI_SOFTMAX && p.long_rows;
-    if (p.bf16)
-        return p.out_f32 ? launch<BlkBf16Tag, true, 2>(p, maps, sms, st)
-                         : (four ? launch<BlkBf16Tag, false, 4>(p, maps, sms, st) : launch<BlkBf16Tag, false, 2>(p, maps, sms, st));
-    return p.out_f32 ? launch<BlkHalfTag, true, 2>(p, maps, sms, st)
-                     : (four ? launch<BlkHalfTag, false, 4>(p, maps, sms, st) : launch<BlkHalfTag, false, 2>(p, maps, sms, st));
+    auto run = [&](auto tag) {
+        typedef decltype(tag) Tag;
+        if (p.epi == BLK_EPI_SOFTMAX)
+            return p.out_f32 ? launch<Tag, true, true, false>(p, maps, sms, st) : launch<Tag, false, true, false>(p, maps, sms, st);
+        if (p.wide) return p.out_f32 ? launch<Tag, true, false, true>(p, maps, sms, st) : launch<Tag, false, false, true>(p, maps, sms, st);
+        return p.out_f32 ? launch<Tag, true, false, false>(p, maps, sms, st) : launch<Tag, false, false, false>(p, maps, sms, st);
+    };
+    return p.bf16 ? run(BlkBf16Tag{}) : run(BlkHalfTag{});
 }

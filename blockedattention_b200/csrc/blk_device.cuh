@@ -102,25 +102,6 @@ __device__ __forceinline__ float2 blk_add2(float2 a, float2 b) {
     return d;
 }
 
-// exp2 of two values on the multiply-add pipe: 2^t = 2^i 2^f with i = round(t), f in [-0.5, 0.5]; 2^f by a degree-5
-// polynomial fitted for the relative error (9e-8 in exact arithmetic, 1.7e-7 in fp32: as good as ex2.approx), 2^i added to
-// the exponent field.  For sums: arguments below -126 give 2^-126, not 0.  Twelve instructions for two values instead of two
-// of a pipe that takes eight cycles each; worth it only where that pipe is what a loop waits for.
-__device__ __forceinline__ float2 blk_exp2_fma2(float2 t) {
-    const float2 magic = make_float2(12582912.f, 12582912.f), unmagic = make_float2(-12582912.f, -12582912.f);  // 1.5 * 2^23
-    t.x = fmaxf(t.x, -126.f);
-    t.y = fmaxf(t.y, -126.f);
-    const float2 r = blk_add2(t, magic);  // i in the low bits
-    const float2 f = blk_fma2(blk_add2(r, unmagic), make_float2(-1.f, -1.f), t);
-    float2 p = make_float2(0.00132647f, 0.00132647f);
-    p = blk_fma2(p, f, make_float2(0.009671515f, 0.009671515f));
-    p = blk_fma2(p, f, make_float2(0.05550734f, 0.05550734f));
-    p = blk_fma2(p, f, make_float2(0.24022242f, 0.24022242f));
-    p = blk_fma2(p, f, make_float2(0.693147f, 0.693147f));
-    p = blk_fma2(p, f, make_float2(1.f, 1.f));
-    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(r.x) << 23)),
-                       __int_as_float(__float_as_int(p.y) + (__float_as_int(r.y) << 23)));
-}
 __device__ __forceinline__ float2 blk_mul2(float2 a, float2 b) {
     float2 d;
     asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mul.rn.f32x2 d, a, b;\n"

@@ -26,7 +26,7 @@
 // piece exceeds it by 2^32) and writes them back as fp32 while summing, pass 2 normalises and stores, so the exponential is
 // evaluated once per element and the scores never leave the SM.  Softmax with N > 512: the products are computed twice -- a
 // first sweep keeps only (reference, sum) per row, a second recomputes each chunk and stores normalised probabilities; the
-// second sweep of an item alternates chunk by chunk with the first sweep of the next, which the other two groups do.
+// second sweep of an item alternates chunk by chunk with the first sweep of the next, all four groups taking chunks of both.
 //
 // Measured against one item at a time with 8 arithmetic and 4 store warps: scores + softmax of 1024 segments of 64..512 rows,
 // 16 heads, K = 128: 2054 -> 1532 us; 2048 products of at most 256 x 256, fp32 out: 56.6 -> 54.3 us; 64 products of
@@ -74,12 +74,9 @@ struct UL {
     static constexpr int STAGE_BYTES = UM_A_BYTES + BN * UM_BK * 2;
     static constexpr int STRIP_OFF = STAGES * STAGE_BYTES;
     static constexpr int BAR_OFF = STRIP_OFF + 4 * GROUPS * UM_STRIP_BYTES;
-    static constexpr int SMEM_BYTES = BAR_OFF + 448 + (int)UM_ITEMS * 64;
+    static constexpr int SMEM_BYTES = BAR_OFF + 464 + (int)UM_ITEMS * 64;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
-
-struct UmYes { static constexpr bool value = true; };
-struct UmNo { static constexpr bool value = false; };
 
 // A work item as the roles see it, in shared memory.
 struct __align__(16) Work {
@@ -265,10 +262,11 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
     }
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
     // [0..] stage full, [4..] stage empty, [8..] accumulator free, [12 + 4 g + i] chunk i mod 4 of group g ready,
-    // [28..] item record written, [36..] read by all, [44 + 4 (g / 2) + q] rendezvous of quarter q's warps of two groups
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 52);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 53);
-    Work* const ring = reinterpret_cast<Work*>(bars + 56);
+    // [28..] item record written, [36..] read by all, [44 + 4 (g / 2) + q] rendezvous of quarter q's warps of two groups,
+    // [52 + q] of all groups
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 56);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 57);
+    Work* const ring = reinterpret_cast<Work*>(bars + 58);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_u32 = blk_smem_u32(smem);
@@ -279,9 +277,13 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
     auto ready_bar = [&](uint32_t g, uint32_t k) { return bar0 + 8u * (12u + 4u * g + (k & 3u)); };
     auto item_full = [&](uint32_t n) { return bar0 + 8u * (28u + n % UM_ITEMS); };
     auto item_empty = [&](uint32_t n) { return bar0 + 8u * (36u + n % UM_ITEMS); };
-    // the group that takes a chunk: scores in turn (by slot); softmax two groups per item, in turn within it
-    auto group_of = [&](uint32_t slot, uint32_t n, int ch) {
-        return SOFT ? 2u * (n & 1u) + (((uint32_t)ch + (n >> 1)) & 1u) : slot % GROUPS;
+    // The group that takes a chunk.  Scores: in turn.  Softmax of a resident row: two groups per item, in turn within it.
+    // Two sweeps: in turn, shifted by one every four chunks, so that a group gets first-sweep and storing chunks alternately
+    // (a storing chunk takes half as long again; two groups with the one kind and two with the other waited for each other
+    // a quarter of the time).
+    auto group_of = [&](uint32_t slot, uint32_t n, int ch, int sweeps) {
+        if (!SOFT) return slot % GROUPS;
+        return sweeps == 2 ? (slot + (slot >> 2)) & 3u : 2u * (n & 1u) + (((uint32_t)ch + (n >> 1)) & 1u);
     };
 
     if (threadIdx.x == 0) {
@@ -291,7 +293,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             mbar_init(tempty_bar(s), 4);  // the warps of the group that consumed the chunk
         }
         for (uint32_t i = 0; i < 16; ++i) mbar_init(ready_bar(i >> 2, i), 1);
-        for (uint32_t i = 0; i < 8; ++i) mbar_init(bar0 + 8u * (44u + i), 2);
+        for (uint32_t i = 0; i < 12; ++i) mbar_init(bar0 + 8u * (44u + i), i < 8 ? 2 : 4);
         for (uint32_t i = 0; i < UM_ITEMS; ++i) {
             mbar_init(item_full(i), 1);
             mbar_init(item_empty(i), 2 + 4 * GROUPS);  // producer, MMA, the groups
@@ -384,7 +386,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                 mbar_arrive(item_empty(n));
                 chunk_order(ch0, nchunks, sweeps, pair, pre, [&](bool next, int ch, bool) -> bool {
                     // the chunk's products into the next accumulator
-                    const uint32_t buf = slot % NBUF, grp = group_of(slot, next ? n + 1u : n, ch);
+                    const uint32_t buf = slot % NBUF, grp = group_of(slot, n, ch, sweeps);
                     const uint32_t ready = ready_bar(grp, counts >> (8u * grp));
                     const int ncols = min((next ? N2 : N) - ch * BN, BN);
                     const uint32_t idesc = idesc0 | ((uint32_t)((ncols + 15) >> 4) << 18);  // columns in units of 16
@@ -428,7 +430,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
         const float sl = SOFT ? fabsf(p.scale) * BLK_LOG2E : p.scale;  // a negative softmax scale is applied by the MMA (negated A)
         const float2 sl2 = make_float2(sl, sl);
         constexpr int PC = OUT32 ? UM_PW : 2 * UM_PW;  // columns of a staged piece
-        uint32_t slot = 0, mychunks = 0, meetings = 0;
+        uint32_t slot = 0, mychunks = 0, meetings = 0, assemblies = 0;
         bool ok = true, pre = false;
 
         auto chunk_wait = [&]() -> bool {
@@ -506,23 +508,34 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                 if (i >= lim_) r[i] = 0xff800000u;  // -inf
         };
         // Softmax, running over the units of a row that this warp has: reference and sum of exp2((x - reference) sl).
-        float ref = -INFINITY, sum = 0.f;
-        // Rendezvous with the warp of the other group that shares the item's rows: mbarrier, bounded like every wait.
-        auto meet = [&]() -> bool {
-            const uint32_t bar = bar0 + 8u * (44u + 4u * (grp >> 1) + (uint32_t)q);
+        float ref = -INFINITY, sum = 0.f, off = 0.f;
+        // Rendezvous with the warps of the other groups that share the item's rows (the other of a pair, or all four):
+        // mbarriers, bounded like every wait.
+        auto meet = [&](bool all) -> bool {
+            const uint32_t bar = bar0 + 8u * (all ? 52u + (uint32_t)q : 44u + 4u * (grp >> 1) + (uint32_t)q);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
-            return mbar_wait(bar, meetings++ & 1u, abort_flag, 8, lim);
+            return mbar_wait(bar, (all ? assemblies++ : meetings++) & 1u, abort_flag, 8, lim);
         };
-        // Reference and sum of the whole row, through the strips (free at that time); false when the other gave up.
-        auto combine = [&](float& m, float& l) -> bool {
-            const uint32_t mine = strip + 8u * lane, other = strip + ((grp & 1u) ? -4 * UM_STRIP_BYTES : 4 * UM_STRIP_BYTES) + 8u * lane;
-            blk_sts_f32x2(mine, ref, sum);
-            if (!meet()) return false;
-            const float r2 = __uint_as_float(lds_b32(other)), s2 = __uint_as_float(lds_b32(other + 4));
-            m = fmaxf(ref, r2);
-            l = (ref == -INFINITY ? 0.f : sum * blk_exp2((ref - m) * sl)) + (r2 == -INFINITY ? 0.f : s2 * blk_exp2((r2 - m) * sl));
-            return meet();  // both have read: the strips may be written
+        // Reference and sum of the whole row, through the strips (free at that time); false when another gave up.
+        auto combine = [&](bool all, float& m, float& l) -> bool {
+            const uint32_t base = strip - (all ? grp : grp & 1u) * (4u * UM_STRIP_BYTES) + 8u * lane;
+            blk_sts_f32x2(strip + 8u * lane, ref, sum);
+            if (!meet(all)) return false;
+            float r[4], t[4];
+            m = -INFINITY;
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g) {
+                const uint32_t at = base + (all || g < 2 ? g : 0u) * (4u * UM_STRIP_BYTES);
+                r[g] = __uint_as_float(lds_b32(at));
+                t[g] = __uint_as_float(lds_b32(at + 4));
+                m = fmaxf(m, r[g]);
+            }
+            l = 0.f;
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g)
+                if ((all || g < 2) && r[g] != -INFINITY) l += t[g] * blk_exp2((r[g] - m) * sl);
+            return meet(all);  // everybody has read: the strips may be written
         };
         // New reference for a unit; true when some row's has moved (f: what its earlier exponentials are to be multiplied by)
         auto unit_ref = [&](const uint32_t (&r)[32], float& f) -> bool {
@@ -538,22 +551,16 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
             if (move) ref = m;
             return true;
         };
-        // exponentials of a unit in place, added to the sum; sum_only: the values are not wanted, and half of the exponentials
-        // go to the multiply-add pipe (a two-sweep softmax takes two exponentials per element, which kept the
-        // special-function unit 57 % busy; 512 segments of 16..2048 rows 870 -> 834 us)
-        auto unit_exp = [&](uint32_t (&r)[32], auto sum_only) {
+        // exponentials of a unit in place, added to the sum
+        auto unit_exp = [&](uint32_t (&r)[32]) {
             const float nm = ref == -INFINITY ? 0.f : -ref * sl;
             const float2 nm2 = make_float2(nm, nm);
             float2 s2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
                 float2 t = blk_fma2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2, nm2);
-                if (decltype(sum_only)::value && (i & 2)) {
-                    t = blk_exp2_fma2(t);
-                } else {
-                    t.x = blk_exp2(t.x);
-                    t.y = blk_exp2(t.y);
-                }
+                t.x = blk_exp2(t.x);
+                t.y = blk_exp2(t.y);
                 s2[(i >> 1) & 1] = blk_add2(s2[(i >> 1) & 1], t);
                 r[i] = __float_as_uint(t.x);
                 r[i + 1] = __float_as_uint(t.y);
@@ -610,7 +617,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                                                   tc_st16(at, o);
                                               }
                                           }
-                                          unit_exp(r, UmNo{});
+                                          unit_exp(r);
                                           tc_st32(col + 32u * u, r);
                                       },
                                       []() {});
@@ -619,7 +626,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                         if (here && nchunks > k0) {
                             tc_wait_st();
                             float m = ref, l = sum;
-                            if (nchunks > 1 && !combine(m, l)) { ok = false; break; }
+                            if (nchunks > 1 && !combine(false, m, l)) { ok = false; break; }
                             const float inv = __frcp_rn(l) * (nchunks > 1 ? blk_exp2((ref - m) * sl) : 1.f);
                             const float2 inv2 = make_float2(inv, inv);
 #pragma unroll 1
@@ -632,41 +639,51 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                     }
                     slot += (uint32_t)nchunks;
                 } else {
-                    // (after `pre` the reference and sum are those of the first sweep that ran alongside the item before)
-                    bool begun = false, off_known = false;
-                    float off = 0.f;
+                    // first sweep of this item (unless it ran alongside the item before), then its storing chunks
+                    // alternating with the first sweep of the next item
+                    const int nr0 = (q - (next_rows >> 8)) * 32;
+                    const bool next_here = nr0 >= 0 && nr0 < (next_rows & 255);
+                    bool fresh = !pre;  // the first sweep of this item is still to be finished
+                    if (fresh) {
+                        ref = -INFINITY;
+                        sum = 0.f;
+                    }
+                    auto statistics = [&]() -> bool {
+                        // exp2(x sl + off) = exp2((x - m) sl) / l: no multiply after the exponential
+                        float m, l;
+                        if (!combine(true, m, l)) return false;
+                        off = -m * sl - __log2f(l);
+                        return true;
+                    };
+                    float off_now = off;
                     chunk_order(ch0, nchunks, sweeps, pair, pre, [&](bool next, int ch, bool first) -> bool {
-                        const uint32_t buf = slot % NBUF, owner = group_of(slot, next ? n + 1u : n, ch);
+                        if (fresh && !(first && !next)) {
+                            fresh = false;
+                            if (here && !statistics()) { ok = false; return false; }
+                            off_now = off;
+                        }
+                        if (!fresh && next && ch == 0) {
+                            ref = -INFINITY;
+                            sum = 0.f;
+                        }
+                        const uint32_t buf = slot % NBUF, owner = group_of(slot, n, ch, 2);
                         ++slot;
                         if (owner != grp) return true;
                         if (!chunk_wait()) { ok = false; return false; }
                         const int cols = min((next ? next_N : N) - ch * BN, BN);
                         const uint32_t col = lane_addr + buf * (uint32_t)BN;
-                        const int nr0 = (q - (next_rows >> 8)) * 32;
-                        if (next ? nr0 < 0 || nr0 >= (next_rows & 255) : !here) { release(buf); return true; }
+                        if (!(next ? next_here : here)) { release(buf); return true; }
                         if (first) {
-                            if (!begun) {
-                                begun = true;
-                                ref = -INFINITY;
-                                sum = 0.f;
-                            }
                             each_unit(col, (cols + 31) >> 5,
                                       [&](uint32_t (&r)[32], int u) {
                                           if (32 * u + 32 > cols) mask_unit(r, cols - 32 * u);
                                           float f;
                                           if (unit_ref(r, f)) sum *= f;
-                                          unit_exp(r, UmYes{});
+                                          unit_exp(r);
                                       },
                                       [&]() { release(buf); });
                         } else {
-                            if (!off_known) {
-                                // exp2(x sl + off) = exp2((x - m) sl) / l: no multiply after the exponential
-                                float m, l;
-                                if (!combine(m, l)) { ok = false; return false; }
-                                off_known = true;
-                                off = -m * sl - __log2f(l);
-                            }
-                            const float2 off2 = make_float2(off, off);
+                            const float2 off2 = make_float2(off_now, off_now);
                             put(col, ch * BN, cols, cbase, rows, N, anyodd,
                                 [&](float2 v) {
                                     const float2 t = blk_fma2(v, sl2, off2);
@@ -676,6 +693,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                         }
                         return true;
                     });
+                    if (ok && pair && next_here && !statistics()) ok = false;
                     pre = pair != 0;
                 }
             } else {

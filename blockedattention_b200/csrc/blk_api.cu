@@ -888,6 +888,7 @@ static int gemm_run_impl(const blk_plan* p, const void* mat1, const void* mat2, 
         vp.num_items = (int)p->pv_items.size();
         vp.H = (int)p->H;
         vp.D = p->pv_D;
+        vp.ta = p->ta;
         vp.bf16 = p->dtype_in == BLK_BF16;
         vp.scale = scale;
         vp.status = p->d_status;

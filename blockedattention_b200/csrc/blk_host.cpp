@@ -444,9 +444,10 @@ int blk_build_gemm_schedule(blk_plan* p) {
     // The tcgen05 kernel for a second operand stored (K, D) -- the product of a probability block with the values --
     // takes 16-bit segments whose second operand has D = 64 or 128 columns (one D per plan: the one carrying the
     // most work), whose value rows are rows of the (rows, D) view of the strip and whose result rows are 16-byte
-    // aligned.  The first operand may have any row length and alignment.
+    // aligned.  The first operand may have any row length and alignment, and may be stored transposed (the products of a
+    // backward pass with a gradient block).
     const bool allow_pv = !blk_env_flag("BLK_DISABLE_UMMA") && p->dtype_in != BLK_F32 && p->dtype_out == p->dtype_in &&
-                          !p->ta && p->tb && p->epi == BLK_EPI_SCORES && p->Dm2 % 8 == 0 && p->Dout % 8 == 0 && !p->attn;
+                          p->tb && p->epi == BLK_EPI_SCORES && p->Dm2 % 8 == 0 && p->Dout % 8 == 0 && !p->attn;
     auto pv_candidate = [&](int64_t s, int64_t D) {
         return allow_pv && p->N[s] == D && p->M[s] > 0 && p->K[s] > 0 && p->a2[s] % D == 0 && p->ao[s] % 8 == 0 &&
                p->Dm2 / D < INT32_MAX;
@@ -503,8 +504,9 @@ int blk_build_gemm_schedule(blk_plan* p) {
         }
         if (p->pv_D != 0 && pv_candidate(s, p->pv_D)) {
             for (int64_t tm = 0; tm * BLK_UMMA_BM < m; ++tm)
-                p->pv_items.push_back(BlkPvItem{sd.offA + tm * BLK_UMMA_BM * k, sd.offC + tm * BLK_UMMA_BM * n,
-                                                (int32_t)(sd.offB / n), (int32_t)(m - tm * BLK_UMMA_BM), (int32_t)k, 0});
+                p->pv_items.push_back(BlkPvItem{sd.offA + tm * BLK_UMMA_BM * (p->ta ? 1 : k), sd.offC + tm * BLK_UMMA_BM * n,
+                                                (int32_t)(sd.offB / n), (int32_t)(m - tm * BLK_UMMA_BM), (int32_t)k,
+                                                (int32_t)(p->ta ? m : 0)});
             continue;
         }
         if (allow_umma && umma_views[s] >= 0) {

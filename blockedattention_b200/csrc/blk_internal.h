@@ -119,8 +119,8 @@ struct BlkPvItem {
     int64_t offC;   // element offset of the block's first result row inside a head strip of the output
     int32_t rowB;   // first row of the segment in the (rows, D) view of the second operand
     int32_t M;      // rows of the segment from this block on (the block holds min(M, 128))
-    int32_t K;      // contraction length = row pitch of the first operand
-    int32_t pad;
+    int32_t K;      // contraction length; row pitch of the first operand unless it is stored transposed
+    int32_t pitch;  // of a first operand stored (K, M): its row pitch (0: stored (M, K))
 };
 static_assert(sizeof(BlkPvItem) == 32, "BlkPvItem layout");
 

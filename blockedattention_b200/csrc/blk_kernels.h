@@ -83,6 +83,7 @@ struct BlkPvParams {
     int num_items;
     int H;
     int D;  // columns of the second operand and of the result: 64 or 128
+    int ta; // the first operand is stored (K, M)
     int bf16;
     float scale;
     int* status;

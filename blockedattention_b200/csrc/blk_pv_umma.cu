@@ -5,26 +5,33 @@
 // N_s) and the second operand is stored (K, D) with D = 64 or 128 (the values V_s
 // of a segment: upstream's transpose2 = true).
 //
-// The rows of P cannot be fetched by TMA (a tensor map needs 16-byte aligned row
+// The rows of P cannot be fetched by tiled TMA (a tensor map needs 16-byte aligned row
 // pitches; a packed score block has whatever pitch its segment has), so they take
-// another road into the tensor core: loader warps read them with aligned 16-byte
-// loads, shift them into place in registers and store them into tensor memory,
-// from where tcgen05.mma takes them as its first operand ([tmem], 16-bit elements,
-// two per column, row = lane).  The values are fetched by tiled TMA exactly as
-// they lie (MN-major second operand, 128-byte swizzle).
+// another road into the tensor core: one bulk copy a row brings the aligned 16-byte
+// vectors that hold a tile's part of it to shared memory, loader warps shift the rows
+// into place in registers and store them into tensor memory, from where tcgen05.mma
+// takes them as its first operand ([tmem], 16-bit elements, two per column, row =
+// lane).  A first operand stored (K, M) -- a gradient block in a backward pass -- is
+// copied the same way and read across its rows.  The values are fetched by tiled TMA
+// exactly as they lie (MN-major second operand, 128-byte swizzle).
+// Bound by those copies and by memory: 1024 segments of 64..512 rows and columns, 16
+// heads, D = 128 take 1150-1180 us (1333 with vector loads by the lane that owns a
+// row, 32 cache lines an instruction; 1709 with 8-byte asynchronous copies); the
+// transposed product of a long-tailed batch, D = 64, that the staged mma.sync kernel
+// did in 350 us takes 127.
 //
 // A persistent CTA (one per SM, 22 warps) walks a static list of work items, an
 // item being a 128-row block of the first operand of one segment of one head; it
 // sweeps the contraction index in tiles of 128.  Roles:
 //   warp 0      producer: one lane issues the TMA loads of the value tiles into a ring;
-//   warp 1      MMA: one lane issues O += P V for each tile, P from one of two
+//   warp 1      MMA: one lane issues O += P V for each tile, P from one of four
 //               64-column buffers in tensor memory, O in one of two accumulators
 //               (items alternate); tcgen05.commit frees the value stage and the P
 //               buffer and, after an item's last tile, hands O to the output warps;
-//   warps 2-17  loaders, two groups of eight, one per P buffer (so a group takes every other
-//               tile and the global loads of two tiles are in flight at a time): thread
-//               (quarter q, lane) owns row 32 q + lane of the block; the two warps of a
-//               quarter in a group each bring 64 of the 128 columns of a tile;
+//   warps 2-17  loaders, four groups of four, one per P buffer (so a group takes every
+//               fourth tile, and the copies of up to four tiles are in flight): a lane
+//               issues the copy of one row of its warp's 32, the next tile's as soon as
+//               this one has left shared memory;
 //   warps 18-21 output: read O, scale, round and store the rows (a row of the result is
 //               D contiguous, 16-byte aligned elements).
 //
@@ -47,14 +54,11 @@ namespace {
 
 static_assert(BLK_UMMA_BM == 128, "a work item is a block of 128 rows: one accumulator lane per row");
 constexpr int PV_BK = 128;           // contraction elements per tile
-constexpr int PV_LOAD_WARPS = 8;     // loader warps of a group: four lane quarters x two halves of a tile's 128 columns
-#ifndef PV_GROUPS_N
-#define PV_GROUPS_N 2
-#endif
-constexpr int PV_GROUPS = PV_GROUPS_N;  // groups of loader warps, one per tensor-memory buffer: their loads are in flight together
-                                        // (two: 13 % faster than one; three measured the same as two)
-constexpr int PV_PBUFS = PV_GROUPS > 2 ? PV_GROUPS : 2;  // buffers of the first operand in tensor memory, 64 columns each
-static_assert(PV_PBUFS <= 4, "the first-operand buffers lie below the result accumulators (column 256)");
+constexpr int PV_LOAD_WARPS = 4;     // loader warps of a group: the four lane quarters
+constexpr int PV_GROUPS = 4;         // groups of loader warps, one per tensor-memory buffer of the first operand (64 columns each,
+                                     // below the result accumulators at column 256)
+constexpr int PV_ROW_BYTES = 272;    // a row of a tile in shared memory: 17 vectors of 16 bytes (an odd number: conflict-free by row)
+constexpr int PV_STRIP_BYTES = 128 * PV_ROW_BYTES;  // per group
 constexpr int PV_OUT_WARPS = 4;
 constexpr int PV_THREADS = 64 + 32 * (PV_LOAD_WARPS * PV_GROUPS + PV_OUT_WARPS);
 constexpr int PV_BLOCK_BYTES = 128 * 128;  // 128 value rows of one 64-column block: 16 KB
@@ -63,10 +67,11 @@ constexpr int PV_O_COL = 256;              // tensor-memory columns of the two r
 template <int D>
 struct PVL {
     static constexpr int NB = D / 64;                       // 64-column blocks of a value row
-    static constexpr int VS = D == 64 ? 6 : 4;              // value ring
+    static constexpr int VS = D == 64 ? 5 : 2;              // value ring
     static constexpr int OPER_BYTES = NB * PV_BLOCK_BYTES;  // a 128 x D tile
     static constexpr int V_OFF = 0;
-    static constexpr int BAR_OFF = VS * OPER_BYTES;
+    static constexpr int STRIP_OFF = VS * OPER_BYTES;
+    static constexpr int BAR_OFF = STRIP_OFF + PV_GROUPS * PV_STRIP_BYTES;
     static constexpr int SMEM_BYTES = BAR_OFF + 512;
     static_assert(VS <= 6, "barrier slots");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -88,13 +93,45 @@ __device__ __forceinline__ bool pv_work(const BlkPvParams& p, uint32_t w, PvWork
     return true;
 }
 
-__device__ __forceinline__ uint4 ldg_v4_if(const void* ptr, bool ok) {
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (ok) v = __ldg(reinterpret_cast<const uint4*>(ptr));
-    return v;
-}
+// The items of a CTA in order, the record of the next one always on its way.
+struct PvItems {
+    PvWork nx;
+    uint32_t w;
+    bool has;
+    __device__ __forceinline__ explicit PvItems(const BlkPvParams& p) : w(blockIdx.x) { has = pv_work(p, w, nx); }
+    __device__ __forceinline__ bool next(const BlkPvParams& p, PvWork& wk) {
+        if (!has) return false;
+        wk = nx;
+        w += gridDim.x;
+        has = pv_work(p, w, nx);
+        return true;
+    }
+};
 
-template <typename Tag, int D>
+// A walk over the tiles of one loader group: every PV_GROUPS-th tile of the CTA.
+struct PvTiles {
+    PvItems items;
+    PvWork wk;
+    int j;
+    uint32_t g;
+    bool valid;
+    __device__ __forceinline__ PvTiles(const BlkPvParams& p, uint32_t grp) : items(p), j(0), g(0) {
+        valid = items.next(p, wk);
+        seek(p, grp);
+    }
+    __device__ __forceinline__ void seek(const BlkPvParams& p, uint32_t to) {  // to tile number `to` of the CTA
+#pragma unroll 1
+        while (valid && g + (uint32_t)(wk.T - j) <= to) {
+            g += (uint32_t)(wk.T - j);
+            j = 0;
+            valid = items.next(p, wk);
+        }
+        j += (int)(to - g);
+        g = to;
+    }
+};
+
+template <typename Tag, int D, bool TA>
 __global__ void __launch_bounds__(PV_THREADS, 1)
 blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV) {
     using L = PVL<D>;
@@ -106,9 +143,10 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
         return;
     }
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-    // barriers: 0.. p_full[4], 4.. p_free[4], 8.. o_ready[2], 10.. o_free[2], 12.. v_full[VS], 18.. v_empty[VS]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 25);
+    // barriers: 0.. p_full[4], 4.. p_free[4], 8.. o_ready[2], 10.. o_free[2], 12.. v_full[VS], 18.. v_empty[VS],
+    // 24.. rows_in[16], 40.. rows_out[4]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 45);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_u32 = blk_smem_u32(smem);
@@ -119,12 +157,15 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
     auto o_free = [&](int b) { return bar0 + 8u * (10 + b); };
     auto v_full = [&](int s) { return bar0 + 8u * (12 + s); };
     auto v_empty = [&](int s) { return bar0 + 8u * (18 + s); };
+    auto rows_in = [&](int w) { return bar0 + 8u * (24 + w); };  // per loader warp; with a transposed operand, the first of its group's
+    auto rows_out = [&](int g) { return bar0 + 8u * (40 + g); };
     auto sV = [&](int s) { return smem_u32 + L::V_OFF + s * L::OPER_BYTES; };
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < PV_PBUFS; ++b) {
+        for (int b = 0; b < PV_GROUPS; ++b) {
             mbar_init(p_full(b), PV_LOAD_WARPS);
             mbar_init(p_free(b), 1);
+            mbar_init(rows_out(b), PV_LOAD_WARPS);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(o_ready(b), 1);
@@ -134,6 +175,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
             mbar_init(v_full(s), 1);
             mbar_init(v_empty(s), 1);
         }
+        for (int w = 0; w < PV_LOAD_WARPS * PV_GROUPS; ++w) mbar_init(rows_in(w), TA ? PV_LOAD_WARPS : 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -149,11 +191,14 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
 
     if (warp == 0) {
         // ---------------- producer: value tiles ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t g = 0;
+            PvItems items(p);
             PvWork wk;
             bool ok = true;
-            for (uint32_t w = blockIdx.x; ok && pv_work(p, w, wk); w += gridDim.x) {
+#pragma unroll 1
+            while (ok && items.next(p, wk)) {
+#pragma unroll 1
                 for (int j = 0; j < wk.T; ++j, ++g) {
                     const int vs = (int)(g % VS);
                     if (!mbar_wait(v_empty(vs), ((g / VS) & 1u) ^ 1u, abort_flag, 41)) { ok = false; break; }
@@ -167,17 +212,20 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
         }
     } else if (warp == 1) {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = instr_desc(p.bf16, D, 0, 1);  // second operand MN-major
             uint32_t g = 0, itc = 0;
+            PvItems items(p);
             PvWork wk;
             bool ok = true;
-            for (uint32_t w = blockIdx.x; ok && pv_work(p, w, wk); w += gridDim.x, ++itc) {
+#pragma unroll 1
+            for (; ok && items.next(p, wk); ++itc) {
                 const int ob = (int)(itc & 1u);
                 if (!mbar_wait(o_free(ob), ((itc >> 1) & 1u) ^ 1u, abort_flag, 42)) break;
+#pragma unroll 1
                 for (int j = 0; j < wk.T; ++j, ++g) {
-                    const int vs = (int)(g % VS), buf = (int)(g % PV_PBUFS);
-                    if (!mbar_wait(p_full(buf), (g / PV_PBUFS) & 1u, abort_flag, 43)) { ok = false; break; }
+                    const int vs = (int)(g % VS), buf = (int)(g % PV_GROUPS);
+                    if (!mbar_wait(p_full(buf), (g / PV_GROUPS) & 1u, abort_flag, 43)) { ok = false; break; }
                     if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, 44)) { ok = false; break; }
                     tc_fence_after();
                     const int ncols = min(wk.it.K - j * PV_BK, PV_BK);
@@ -195,57 +243,81 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
             }
         }
     } else if (warp < 2 + PV_LOAD_WARPS * PV_GROUPS) {
-        // ---------------- loaders: warps 2..17, group grp fills buffer grp (every other tile) ----------------
-        const int lw = (warp - 2) % PV_LOAD_WARPS, grp = (warp - 2) / PV_LOAD_WARPS;
-        const int q = warp & 3, h = lw >> 2;
-        const int row = q * 32 + lane;
+        // ---------------- loaders: warps 2..17, group grp fills buffer grp (every fourth tile) ----------------
+        const int grp = (warp - 2) / PV_LOAD_WARPS;
+        const int q = warp & 3;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const unsigned char* A = reinterpret_cast<const unsigned char*>(p.A);
-        uint32_t g = 0;
-        PvWork wk;
-        bool ok = true;
-        for (uint32_t w = blockIdx.x; ok && pv_work(p, w, wk); w += gridDim.x) {
-            const int K = wk.it.K;
-            const bool row_ok = row < wk.it.M;
-            // byte address of this lane's row of the block
-            const int64_t rowb = ((int64_t)wk.head * p.Dm1 + wk.it.offA + (int64_t)row * K) * 2;
-            for (int j = 0; ok && j < wk.T; ++j, ++g) {
-                if (PV_GROUPS > 1 && (int)(g % PV_GROUPS) != grp) continue;  // another group's tile
-                const int buf = (int)(g % PV_PBUFS), vs = (int)(g % VS);
-                const int ncols = min(K - j * PV_BK, PV_BK);
-                const int ksteps = (ncols + 15) >> 4;
-                const int nv = row_ok ? max(0, min(ncols - 64 * h, 64)) : 0;   // elements of this lane's 64 that exist
-                // 64 elements from byte address b: the aligned 16-byte vectors that hold at least one of them
-                const int64_t b = rowb + (int64_t)(j * PV_BK + 64 * h) * 2;
-                const int sh = (int)(b & 15);
-                const unsigned char* base = A + (b - sh);
-                const int need = sh + 2 * nv;  // bytes [sh, need) of the vectors are wanted
-                uint32_t v[36];
+        const uint32_t strip = smem_u32 + L::STRIP_OFF + (uint32_t)grp * PV_STRIP_BYTES;
+        const uint32_t bar_rows = rows_in(TA ? grp * PV_LOAD_WARPS : warp - 2);
+        // byte address, from the start of the operand, of the first element of row r of a tile as it lies in memory
+        auto addr_of = [&](const PvTiles& t, int r) {
+            const int64_t e = (int64_t)t.wk.head * p.Dm1 + t.wk.it.offA;
+            return TA ? 2 * (e + (int64_t)(t.j * PV_BK + r) * t.wk.it.pitch) : 2 * (e + (int64_t)r * t.wk.it.K + t.j * PV_BK);
+        };
+        // a lane copies one of its warp's 32 rows: the aligned 16-byte vectors that hold its elements
+        auto copy = [&](const PvTiles& t) {
+            const int r = q * 32 + lane;
+            const int kk = min(t.wk.it.K - t.j * PV_BK, PV_BK), mm = min(t.wk.it.M, 128);
+            const int64_t b = addr_of(t, r);
+            const int sh = (int)(b & 15);
+            const uint32_t bytes = r < (TA ? kk : mm) ? (uint32_t)((sh + 2 * (TA ? mm : kk) + 15) & ~15) : 0u;
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, bytes);
+            if (lane == 0) mbar_expect_tx(bar_rows, sum);
+            __syncwarp();
+            if (bytes)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                                 strip + (uint32_t)r * PV_ROW_BYTES),
+                             "l"(A + (b - sh)), "r"(bytes), "r"(bar_rows)
+                             : "memory");
+        };
+        uint32_t round = 0;
+        PvTiles cur(p, (uint32_t)grp);
+        if (cur.valid) copy(cur);
+#pragma unroll 1
+        while (cur.valid) {
+            const uint32_t g = cur.g;
+            const int vs = (int)(g % VS);
+            const int ncols = min(cur.wk.it.K - cur.j * PV_BK, PV_BK);
+            const bool row_ok = q * 32 + lane < cur.wk.it.M;
+            bool ok = mbar_wait(bar_rows, round & 1u, abort_flag, 48);
+            ++round;
 #pragma unroll
-                for (int i = 0; i < 9; ++i) {
-                    const uint4 t = ldg_v4_if(base + 16 * i, nv > 0 && 16 * i < need);
-                    v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
-                }
-                // shift by sh bytes: whole words by the case, the odd half word with a funnel shift
+            for (int h = 0; h < 2; ++h) {  // 64 elements of the row at a time, two per word
+                const int nv = row_ok ? max(0, min(ncols - 64 * h, 64)) : 0;  // of these that exist
                 uint32_t pk[32];
-                const uint32_t hs = (uint32_t)(sh & 2) * 8u;
-                switch (sh >> 2) {
-                    case 0:
+                if constexpr (TA) {
+                    // element (k, this lane's row): neighbouring lanes read neighbouring elements of row k
+                    // (the rows' first bytes repeat modulo 16 after eight rows)
+                    const uint32_t src = strip + (uint32_t)(64 * h) * PV_ROW_BYTES + 2u * (q * 32 + lane);
+                    const uint32_t b = (uint32_t)addr_of(cur, 0), step = 2u * (uint32_t)cur.wk.it.pitch;
+                    uint32_t at[8];
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) pk[i] = __funnelshift_r(v[i], v[i + 1], hs);
-                        break;
-                    case 1:
+                    for (int i = 0; i < 8; ++i) at[i] = src + ((b + i * step) & 15u);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) pk[i] = __funnelshift_r(v[i + 1], v[i + 2], hs);
-                        break;
-                    case 2:
+                    for (int i = 0; i < 64; i += 2) {
+                        uint32_t lo, hi;
+                        asm volatile("ld.shared.u16 %0, [%1];\n" : "=r"(lo) : "r"(at[i & 7] + i * PV_ROW_BYTES));
+                        asm volatile("ld.shared.u16 %0, [%1];\n" : "=r"(hi) : "r"(at[(i + 1) & 7] + (i + 1) * PV_ROW_BYTES));
+                        pk[i >> 1] = __byte_perm(lo, hi, 0x5410);
+                    }
+                } else {
+                    const uint32_t sh = (uint32_t)addr_of(cur, q * 32 + lane) & 15u;  // bytes before the row's first element
+                    uint32_t v[36];
+                    const uint32_t src = strip + (uint32_t)(q * 32 + lane) * PV_ROW_BYTES + 128u * h;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) pk[i] = __funnelshift_r(v[i + 2], v[i + 3], hs);
-                        break;
-                    default:
+                    for (int i = 0; i < 9; ++i)
+                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n"
+                                     : "=r"(v[4 * i]), "=r"(v[4 * i + 1]), "=r"(v[4 * i + 2]), "=r"(v[4 * i + 3])
+                                     : "r"(src + 16u * i));
+                    const bool up2 = (sh & 8u) != 0, up1 = (sh & 4u) != 0;
+                    const uint32_t hs = (sh & 2u) * 8u;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) pk[i] = __funnelshift_r(v[i + 3], v[i + 4], hs);
-                        break;
+                    for (int i = 0; i < 34; ++i) v[i] = up2 ? v[i + 2] : v[i];
+#pragma unroll
+                    for (int i = 0; i < 33; ++i) v[i] = up1 ? v[i + 1] : v[i];
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) pk[i] = __funnelshift_r(v[i], v[i + 1], hs);
                 }
                 if (nv < 64) {
                     // elements past the end of the row (or a row past the end of the block) count as zeros
@@ -255,29 +327,42 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
                         else if (2 * i + 1 >= nv) pk[i] &= 0xffffu;
                     }
                 }
-                if (!mbar_wait(p_free(buf), ((g / PV_PBUFS) & 1u) ^ 1u, abort_flag, 45)) { ok = false; break; }
-                tc_fence_after();
-                // this row's elements [64 h, 64 h + 64) of the tile: columns [32 h, 32 h + 32) of the buffer (only the
-                // columns the products of this tile read)
-                if (64 * h < 16 * ksteps) {
-                    tc_st32(lane_addr + (uint32_t)(buf * 64 + 32 * h), pk);
-                    tc_wait_st();
-                }
-                if (ncols & 15) {
-                    // last tile of the row: clear the value rows between its end and the next multiple of 16
-                    if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, 46)) { ok = false; break; }
-                    const int nz = (16 - (ncols & 15)) * L::NB * 8;  // 16-byte pieces to clear
-                    const int t = lw * 32 + lane;
-                    if (t < nz) {
-                        const int rr = t / (L::NB * 8), rem = t % (L::NB * 8);
-                        tc_sts_v4(sV(vs) + (rem >> 3) * PV_BLOCK_BYTES + (ncols + rr) * 128 + (rem & 7) * 16, 0u, 0u, 0u, 0u);
+                if (h == 0) {
+                    ok = ok && mbar_wait(p_free(grp), ((g / PV_GROUPS) & 1u) ^ 1u, abort_flag, 45);
+                    tc_fence_after();
+                } else {
+                    cur.seek(p, g + PV_GROUPS);
+                    // the strip has been read: by this warp, or (a transposed operand) by all of the group
+                    __syncwarp();
+                    if constexpr (TA) {
+                        if (lane == 0) mbar_arrive(rows_out(grp));
+                        ok = ok && mbar_wait(rows_out(grp), (round & 1u) ^ 1u, abort_flag, 39);
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic-proxy writes before the MMA's reads
+                    if (ok && cur.valid) copy(cur);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_full(buf));
+                if (64 * h < ncols) tc_st32(lane_addr + (uint32_t)(grp * 64 + 32 * h), pk);
             }
+            if (!ok) break;
+            tc_wait_st();
+            if (ncols & 15) {
+                // last tile of the row: clear the value rows between its end and the next multiple of 16
+                // (a ring shorter than the number of groups: tile g - VS must have been multiplied first, or the parity of
+                // tile g - 2 VS would pass for that of g)
+                if (VS < PV_GROUPS && g >= (uint32_t)VS &&
+                    !mbar_wait(p_free((grp + PV_GROUPS - VS) % PV_GROUPS), ((g - VS) / PV_GROUPS) & 1u, abort_flag, 40))
+                    break;
+                if (!mbar_wait(v_full(vs), (g / VS) & 1u, abort_flag, 46)) break;
+                const int nz = (16 - (ncols & 15)) * L::NB * 8;  // 16-byte pieces to clear
+#pragma unroll 1
+                for (int t = q * 32 + lane; t < nz; t += 128) {
+                    const int rr = t / (L::NB * 8), rem = t % (L::NB * 8);
+                    tc_sts_v4(sV(vs) + (rem >> 3) * PV_BLOCK_BYTES + (ncols + rr) * 128 + (rem & 7) * 16, 0u, 0u, 0u, 0u);
+                }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic-proxy writes before the MMA's reads
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full(grp));
         }
     } else {
         // ---------------- output: the last four warps ----------------
@@ -285,9 +370,11 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
         const int row = q * 32 + lane;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         uint32_t itc = 0;
+        PvItems items(p);
         PvWork wk;
         uint32_t r[32];
-        for (uint32_t w = blockIdx.x; pv_work(p, w, wk); w += gridDim.x, ++itc) {
+#pragma unroll 1
+        for (; items.next(p, wk); ++itc) {
             const int ob = (int)(itc & 1u);
             if (!mbar_wait(o_ready(ob), (itc >> 1) & 1u, abort_flag, 47)) break;
             tc_fence_after();
@@ -321,9 +408,9 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
     }
 }
 
-template <typename Tag, int D>
+template <typename Tag, int D, bool TA>
 cudaError_t launch(const BlkPvParams& p, const CUtensorMap& mv, int sms, cudaStream_t st) {
-    auto kern = blk_pv_umma_kernel<Tag, D>;
+    auto kern = blk_pv_umma_kernel<Tag, D, TA>;
     cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), PVL<D>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_items * p.H;
@@ -341,6 +428,10 @@ cudaError_t blk_launch_pv_umma(const BlkPvParams& p, const void* V, int sms, cud
     int head_first = 0;
     const BlkOperandLayout lay{p.Dm2 / p.D, p.D, p.Dm2};  // the values as a (rows, D) matrix per head strip
     if (!blk_make_row_map(&mv, V, p.bf16, p.D, p.H, lay, 64, PV_BK, &head_first) || head_first) return cudaErrorInvalidValue;
-    if (p.D == 64) return p.bf16 ? launch<BlkBf16Tag, 64>(p, mv, sms, st) : launch<BlkHalfTag, 64>(p, mv, sms, st);
-    return p.bf16 ? launch<BlkBf16Tag, 128>(p, mv, sms, st) : launch<BlkHalfTag, 128>(p, mv, sms, st);
+    auto run = [&](auto tag) {
+        typedef decltype(tag) Tag;
+        if (p.D == 64) return p.ta ? launch<Tag, 64, true>(p, mv, sms, st) : launch<Tag, 64, false>(p, mv, sms, st);
+        return p.ta ? launch<Tag, 128, true>(p, mv, sms, st) : launch<Tag, 128, false>(p, mv, sms, st);
+    };
+    return p.bf16 ? run(BlkBf16Tag{}) : run(BlkHalfTag{});
 }

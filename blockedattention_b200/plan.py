@@ -57,7 +57,7 @@ TABLES = {
     "small_items_64": (4, _SMALL_ITEM),
     "umma_items": (5, _rec(("views", "<i4"), ("tm", "<i4"), ("rowA", "<i4"), ("rowB", "<i4"), ("offC", "<i8"),
                            ("M", "<i4"), ("N", "<i4"), ("K", "<i4"), ("ch0", "<i4"), ("nch", "<i4"), ("pad", "<i4"))),
-    "pv_items": (6, _rec(("offA", "<i8"), ("offC", "<i8"), ("rowB", "<i4"), ("M", "<i4"), ("K", "<i4"), ("pad", "<i4"))),
+    "pv_items": (6, _rec(("offA", "<i8"), ("offC", "<i8"), ("rowB", "<i4"), ("M", "<i4"), ("K", "<i4"), ("pitch", "<i4"))),
     "packs": (7, _rec(("offA", "<i8"), ("offB", "<i8"), ("rowsA", "<i4"), ("rowsB", "<i4"), ("first_block", "<i4"),
                       ("nblocks", "<i4"))),
     "pack_blocks": (8, _rec(("offC", "<i8"), ("rowA", "<i4"), ("rowB", "<i4"), ("M", "<i4"), ("N", "<i4"),

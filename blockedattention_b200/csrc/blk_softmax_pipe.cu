@@ -2,18 +2,24 @@
 //
 // The host groups consecutive row pieces (blk_softmax.cu's chunks) whose bytes are contiguous in memory into
 // windows of at most 12 KB -- many small segments, or a few rows of a wide one.  A persistent CTA walks windows
-// w = blockIdx.x, + gridDim.x, ... of the (window, head) list with two shared-memory stages:
-//   * one thread fetches the next window with a bulk asynchronous copy (cp.async.bulk, completion on the
-//     stage's mbarrier) of the 16-byte aligned range that covers it -- no thread waits for a load it issued;
-//   * all threads do the row arithmetic of the current window out of shared memory (fp32, base-2 exponent,
-//     one rounding): one lane per short row (one warp per small segment); one warp per longer row, which reads and writes the row as
-//     16-byte vectors between its first and last 16-byte boundary (the few elements outside go one per lane)
-//     and keeps up to 1024 columns in registers between the maximum, the sum and the normalisation;
-//   * one thread writes the window back with a bulk asynchronous store of the aligned vectors that lie wholly
-//     inside it, a few lanes store the ragged edge elements, and the CTA moves on without waiting for either.
-// Loads, arithmetic and stores of neighbouring windows overlap inside one CTA, so the kernel streams at memory
-// speed with few resident CTAs.  A row longer than a window is streamed from global memory by the whole CTA.
+// w = blockIdx.x, + gridDim.x, ... of the (window, head) list through a ring of shared-memory stages:
+//   * one warp copies: it fetches windows ahead with bulk asynchronous copies (cp.async.bulk, completion on the
+//     stage's mbarrier) of the 16-byte aligned range that covers them, and when the computing warps are done with
+//     a window writes it back with a bulk store of the aligned vectors that lie wholly inside it, a few lanes
+//     storing the ragged edge elements;
+//   * the other warps do the row arithmetic out of shared memory (fp32, base-2 exponent, one rounding).  Work is
+//     dealt out in units -- a long row, four short ones to eight lanes each, 32 very short ones to a lane each --
+//     in turn through all windows of the CTA, so no warp waits for another inside a window.  A long row is read
+//     and written as 16-byte vectors between its first and last 16-byte boundary (the few elements outside go one
+//     per lane).
+// A row longer than a window is streamed from global memory by all computing warps.
 // Every barrier wait is bounded and reports through the status word.
+//
+// Bound by the instructions it issues and their latency, with memory close behind (the copies alone: 650 us where the
+// forward takes 800, and 187 where the backward takes 204).  A spilled register in a row loop costs more than any
+// parallelism: with 28 warps of 64 registers the loops over a row's vectors stay rolled, and rows of short segments are
+// functions of their own.  512 segments of 16..2048 rows and columns, 4 heads, bf16: 870 -> 800 us forward; a quarter of
+// it 200 -> 187 forward, 223 -> 204 backward (before: two stages, all warps of a CTA meeting twice a window).
 //
 // Forward: out = softmax_rows(scale * src); replaces upstream sparseBlockedSoftmax_warp / _block
 // (csrc/cuda/spBlkSoftmax.cu:88-138, :182-269).  Backward: grad_src = scale * (grad_out - rowsum(out *
@@ -23,8 +29,15 @@
 
 namespace {
 
-constexpr int SP_THREADS = 128;
-constexpr int SP_WARPS = SP_THREADS / 32;
+// Warps that compute in a CTA, CTAs on an SM and shared-memory stages of a CTA: 16 windows of an SM are in flight or in
+// work (backward, with two inputs a window: 8).
+template <bool BWD>
+struct SpShape {
+    static constexpr int NW = BWD ? 9 : 7;
+    static constexpr int CTAS = BWD ? 2 : 4;
+    static constexpr int STAGES = 4;
+    static constexpr int THREADS = 32 * (NW + 1);
+};
 constexpr int SP_WIN = BLK_SMX_WINDOW_BYTES;
 constexpr int SP_BUF = SP_WIN + 32;  // a window plus the slack of its 16-byte aligned cover
 constexpr uint32_t SP_SPIN_LIMIT = 1u << 22;
@@ -38,21 +51,20 @@ struct SpIO16<BlkHalfTag> {
     static constexpr int VE = 8;
     static __device__ __forceinline__ float ld(E v) { return BlkCvt<BlkHalfTag>::unpack1(v); }
     static __device__ __forceinline__ E st(float v) { return BlkCvt<BlkHalfTag>::pack1(v); }
-    static __device__ __forceinline__ void unpack(const uint4& q, float (&f)[8]) {
+    static __device__ __forceinline__ void unpack(const uint4& q, float2 (&f)[4]) {
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            f[2 * i] = t.x;
-            f[2 * i + 1] = t.y;
+            f[i] = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
         }
     }
-    static __device__ __forceinline__ uint4 pack(const float (&f)[8]) {
-        return make_uint4(BlkCvt<BlkHalfTag>::pack2(f[0], f[1]), BlkCvt<BlkHalfTag>::pack2(f[2], f[3]),
-                          BlkCvt<BlkHalfTag>::pack2(f[4], f[5]), BlkCvt<BlkHalfTag>::pack2(f[6], f[7]));
+    static __device__ __forceinline__ uint4 pack(const float2 (&f)[4]) {
+        return make_uint4(BlkCvt<BlkHalfTag>::pack2(f[0].x, f[0].y), BlkCvt<BlkHalfTag>::pack2(f[1].x, f[1].y),
+                          BlkCvt<BlkHalfTag>::pack2(f[2].x, f[2].y), BlkCvt<BlkHalfTag>::pack2(f[3].x, f[3].y));
     }
     // running extreme (maximum, or minimum for a negative scale) of a row, taken on the packed pairs as they lie in
     // memory: one instruction per two elements and no conversion
+    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7c007c00u : 0xfc00fc00u; }
     typedef uint32_t X;
     template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? 0x7c007c00u : 0xfc00fc00u; }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
@@ -72,18 +84,18 @@ struct SpIO16<BlkBf16Tag> {
     static constexpr int VE = 8;
     static __device__ __forceinline__ float ld(E v) { return BlkCvt<BlkBf16Tag>::unpack1(v); }
     static __device__ __forceinline__ E st(float v) { return BlkCvt<BlkBf16Tag>::pack1(v); }
-    static __device__ __forceinline__ void unpack(const uint4& q, float (&f)[8]) {
+    static __device__ __forceinline__ void unpack(const uint4& q, float2 (&f)[4]) {
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            f[2 * i] = __uint_as_float(w[i] << 16);
-            f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            f[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
         }
     }
-    static __device__ __forceinline__ uint4 pack(const float (&f)[8]) {
-        return make_uint4(BlkCvt<BlkBf16Tag>::pack2(f[0], f[1]), BlkCvt<BlkBf16Tag>::pack2(f[2], f[3]),
-                          BlkCvt<BlkBf16Tag>::pack2(f[4], f[5]), BlkCvt<BlkBf16Tag>::pack2(f[6], f[7]));
+    static __device__ __forceinline__ uint4 pack(const float2 (&f)[4]) {
+        return make_uint4(BlkCvt<BlkBf16Tag>::pack2(f[0].x, f[0].y), BlkCvt<BlkBf16Tag>::pack2(f[1].x, f[1].y),
+                          BlkCvt<BlkBf16Tag>::pack2(f[2].x, f[2].y), BlkCvt<BlkBf16Tag>::pack2(f[3].x, f[3].y));
     }
+    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7f807f80u : 0xff80ff80u; }
     typedef uint32_t X;
     template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? 0x7f807f80u : 0xff80ff80u; }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
@@ -102,12 +114,14 @@ struct SpIO32 {
     static constexpr int VE = 4;
     static __device__ __forceinline__ float ld(E v) { return v; }
     static __device__ __forceinline__ E st(float v) { return v; }
-    static __device__ __forceinline__ void unpack(const uint4& q, float (&f)[4]) {
-        f[0] = __uint_as_float(q.x); f[1] = __uint_as_float(q.y); f[2] = __uint_as_float(q.z); f[3] = __uint_as_float(q.w);
+    static __device__ __forceinline__ void unpack(const uint4& q, float2 (&f)[2]) {
+        f[0] = make_float2(__uint_as_float(q.x), __uint_as_float(q.y));
+        f[1] = make_float2(__uint_as_float(q.z), __uint_as_float(q.w));
     }
-    static __device__ __forceinline__ uint4 pack(const float (&f)[4]) {
-        return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+    static __device__ __forceinline__ uint4 pack(const float2 (&f)[2]) {
+        return make_uint4(__float_as_uint(f[0].x), __float_as_uint(f[0].y), __float_as_uint(f[1].x), __float_as_uint(f[1].y));
     }
+    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7f800000u : 0xff800000u; }
     typedef float X;
     template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? INFINITY : -INFINITY; }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
@@ -141,10 +155,20 @@ __device__ __forceinline__ bool sp_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool sp_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < SP_SPIN_LIMIT; ++i)
-        if (sp_try(bar, parity)) return true;
-    return false;
+__device__ __forceinline__ bool sp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+    for (uint32_t i = 0; !sp_try(bar, parity); ++i) {
+        if (*abort_flag) return false;
+        if (i >= SP_SPIN_LIMIT) {
+            *abort_flag = 1;
+            return false;
+        }
+        __nanosleep(40);
+    }
+    return true;
+}
+__device__ __forceinline__ void sp_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 // contiguous bulk copies (16-byte aligned addresses and size)
 __device__ __forceinline__ void sp_bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -156,8 +180,8 @@ __device__ __forceinline__ void sp_bulk_s2g(void* dst, uint32_t src, uint32_t by
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void sp_bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
-// all earlier bulk stores of this thread have finished reading shared memory
-__device__ __forceinline__ void sp_bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+// all bulk stores of this thread but the last have finished reading shared memory
+__device__ __forceinline__ void sp_bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory"); }
 // ... and have completed
 __device__ __forceinline__ void sp_bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
@@ -169,16 +193,15 @@ __device__ __forceinline__ void sp_bulk_wait_all() { asm volatile("cp.async.bulk
 // whole vector (one per lane 8..15).
 template <typename IO>
 struct RowSplit {
-    typename IO::E* row;
-    uint4* body;
-    int nv;  // whole vectors
-    int xi;  // this lane's extra element, or -1
-    __device__ __forceinline__ RowSplit(typename IO::E* r, int cols, int lane) : row(r) {
+    uint32_t row, body;  // shared-memory addresses
+    int nv;              // whole vectors
+    int xi;              // this lane's extra element, or -1
+    __device__ __forceinline__ RowSplit(uint32_t r, int cols, int lane) : row(r) {
         constexpr int ES = (int)sizeof(typename IO::E);
-        const int h = (int)((16u - (blk_smem_u32(r) & 15u)) & 15u) / ES;
+        const int h = (int)((16u - (r & 15u)) & 15u) / ES;
         nv = (cols - h) / IO::VE;
         const int tail = cols - h - nv * IO::VE;
-        body = reinterpret_cast<uint4*>(r + h);
+        body = r + (uint32_t)(h * ES);
         xi = -1;
         if (lane < 8) {
             if (lane < h) xi = lane;
@@ -187,327 +210,515 @@ struct RowSplit {
         }
     }
 };
+// elements and 16-byte vectors of a shared-memory buffer
+__device__ __forceinline__ void sp_lds(uint16_t& v, uint32_t a) { asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a)); }
+__device__ __forceinline__ void sp_lds(float& v, uint32_t a) { asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void sp_sts(uint32_t a, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(a), "h"(v) : "memory"); }
+__device__ __forceinline__ void sp_sts(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory"); }
+template <typename IO>
+__device__ __forceinline__ float sp_ld(uint32_t row, int i) {
+    typename IO::E v;
+    sp_lds(v, row + (uint32_t)(i * (int)sizeof(typename IO::E)));
+    return IO::ld(v);
+}
+template <typename IO>
+__device__ __forceinline__ void sp_st(uint32_t row, int i, float v) {
+    sp_sts(row + (uint32_t)(i * (int)sizeof(typename IO::E)), IO::st(v));
+}
+__device__ __forceinline__ uint4 sp_ldv(uint32_t body, int vi) {
+    uint4 q;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
+                 : "r"(body + 16u * (uint32_t)vi));
+    return q;
+}
+__device__ __forceinline__ void sp_stv(uint32_t body, int vi, const uint4& q) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(body + 16u * (uint32_t)vi), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w)
+                 : "memory");
+}
 
-// forward, at most 32 EPV whole vectors per row, values kept in registers (one exponential per element)
+// exp2(x * sl + off) of a vector's elements
+template <typename IO>
+__device__ __forceinline__ void sp_exp(const uint4& q, float2 sl, float2 off, float2 (&f)[IO::VE / 2]) {
+    IO::unpack(q, f);
+#pragma unroll
+    for (int e = 0; e < IO::VE / 2; ++e) {
+        f[e] = blk_fma2(f[e], sl, off);
+        f[e].x = blk_exp2(f[e].x);
+        f[e].y = blk_exp2(f[e].y);
+    }
+}
+// f(vi) for this lane's vectors; kept rolled, see the note on registers at the head of the file
+template <typename F>
+__device__ __forceinline__ void sp_each(int nv, int lane, F f) {
+#pragma unroll 1
+    for (int vi = lane; vi < nv; vi += 32) f(vi);
+}
+template <typename IO, bool NEG>
+__device__ __forceinline__ float sp_extreme(uint32_t body, int nv, int lane) {
+    typename IO::X ex = IO::template xinit<NEG>();
+    sp_each(nv, lane, [&](int vi) { ex = IO::template xacc<NEG>(ex, sp_ldv(body, vi)); });
+    return IO::template xfin<NEG>(ex);
+}
+
+// forward, at most 32 EPV whole vectors per row and a scale that is not zero: values kept in registers, one exponential
+// per element.  Lanes without a vector hold elements that scale to minus infinity.
 template <typename IO, int EPV, int NW>
-__device__ __forceinline__ void fwd_rows_vec(typename IO::E* piece, int rows, int cols, float sl, int warp, int lane) {
-    constexpr int VE = IO::VE;
-    for (int r = warp; r < rows; r += NW) {
-        RowSplit<IO> rs(piece + (size_t)r * cols, cols, lane);
-        float x = rs.xi >= 0 ? IO::ld(rs.row[rs.xi]) * sl : -INFINITY;
-        float v[EPV][VE];
+__device__ __forceinline__ void fwd_rows_vec(uint32_t piece, int rows, int cols, float sl, int r0, int lane) {
+    constexpr int VP = IO::VE / 2;
+    const float2 sl2 = make_float2(sl, sl);
+    const uint32_t none = IO::lowest(sl < 0.f);
+#pragma unroll 1
+    for (int r = r0; r < rows; r += NW) {
+        RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
+        float x = rs.xi >= 0 ? sp_ld<IO>(rs.row, rs.xi) * sl : -INFINITY;
+        float2 v[EPV][VP];
         float mx = x;
 #pragma unroll
         for (int i = 0; i < EPV; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < rs.nv) {
-                IO::unpack(rs.body[vi], v[i]);
+            uint4 q = make_uint4(none, none, none, none);
+            if (lane + 32 * i < rs.nv) q = sp_ldv(rs.body, lane + 32 * i);
+            IO::unpack(q, v[i]);
 #pragma unroll
-                for (int e = 0; e < VE; ++e) {
-                    v[i][e] *= sl;
-                    mx = fmaxf(mx, v[i][e]);
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < VE; ++e) v[i][e] = -INFINITY;
+            for (int e = 0; e < VP; ++e) {
+                v[i][e] = blk_mul2(v[i][e], sl2);
+                mx = blk_max3(mx, v[i][e].x, v[i][e].y);
             }
         }
         mx = sp_max(mx, 32);
         x = blk_exp2(x - mx);
-        float sum = x;
+        const float2 nmx = make_float2(-mx, -mx);
+        float2 sum = make_float2(x, 0.f);
 #pragma unroll
         for (int i = 0; i < EPV; ++i)
 #pragma unroll
-            for (int e = 0; e < VE; ++e) {
-                v[i][e] = blk_exp2(v[i][e] - mx);
-                sum += v[i][e];
+            for (int e = 0; e < VP; ++e) {
+                v[i][e] = blk_add2(v[i][e], nmx);
+                v[i][e].x = blk_exp2(v[i][e].x);
+                v[i][e].y = blk_exp2(v[i][e].y);
+                sum = blk_add2(sum, v[i][e]);
             }
-        sum = sp_sum(sum, 32);
-        const float inv = 1.f / sum;
+        const float inv = 1.f / sp_sum(sum.x + sum.y, 32);
+        const float2 inv2 = make_float2(inv, inv);
 #pragma unroll
         for (int i = 0; i < EPV; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < rs.nv) {
 #pragma unroll
-                for (int e = 0; e < VE; ++e) v[i][e] *= inv;
-                rs.body[vi] = IO::pack(v[i]);
-            }
+            for (int e = 0; e < VP; ++e) v[i][e] = blk_mul2(v[i][e], inv2);
+            if (lane + 32 * i < rs.nv) sp_stv(rs.body, lane + 32 * i, IO::pack(v[i]));
         }
-        if (rs.xi >= 0) rs.row[rs.xi] = IO::st(x * inv);
+        if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, x * inv);
     }
 }
 // forward, any column count that fits the window: three passes over the row, exponential evaluated twice.  The first
 // pass takes the extreme of the raw packed elements; the third folds the normalisation into the exponent.
-template <typename IO, int NW, bool NEG>
-__device__ __forceinline__ void fwd_rows_vec_streamed_impl(typename IO::E* piece, int rows, int cols, float sl, int warp,
-                                                           int lane) {
-    constexpr int VE = IO::VE;
-    for (int r = warp; r < rows; r += NW) {
-        RowSplit<IO> rs(piece + (size_t)r * cols, cols, lane);
-        const float x = rs.xi >= 0 ? IO::ld(rs.row[rs.xi]) * sl : -INFINITY;
-        float f[VE];
-        typename IO::X ex = IO::template xinit<NEG>();
-        for (int vi = lane; vi < rs.nv; vi += 32) ex = IO::template xacc<NEG>(ex, rs.body[vi]);
-        const float mx = sp_max(fmaxf(x, IO::template xfin<NEG>(ex) * sl), 32);
-        float sum = blk_exp2(x - mx);
-        for (int vi = lane; vi < rs.nv; vi += 32) {
-            IO::unpack(rs.body[vi], f);
-#pragma unroll
-            for (int e = 0; e < VE; ++e) sum += blk_exp2(fmaf(f[e], sl, -mx));
-        }
-        sum = sp_sum(sum, 32);
-        const float off = -mx - __log2f(sum);  // exp2(x * sl + off) = exp2(x * sl - max) / sum
-        for (int vi = lane; vi < rs.nv; vi += 32) {
-            IO::unpack(rs.body[vi], f);
-#pragma unroll
-            for (int e = 0; e < VE; ++e) f[e] = blk_exp2(fmaf(f[e], sl, off));
-            rs.body[vi] = IO::pack(f);
-        }
-        if (rs.xi >= 0) rs.row[rs.xi] = IO::st(blk_exp2(x + off));
-    }
-}
 template <typename IO, int NW>
-__device__ __forceinline__ void fwd_rows_vec_streamed(typename IO::E* piece, int rows, int cols, float sl, int warp,
-                                                      int lane) {
-    if (sl < 0.f) fwd_rows_vec_streamed_impl<IO, NW, true>(piece, rows, cols, sl, warp, lane);
-    else fwd_rows_vec_streamed_impl<IO, NW, false>(piece, rows, cols, sl, warp, lane);
+__device__ __forceinline__ void fwd_rows_vec_streamed(uint32_t piece, int rows, int cols, float sl, int r0, int lane) {
+    constexpr int VP = IO::VE / 2;
+    const float2 sl2 = make_float2(sl, sl);
+#pragma unroll 1
+    for (int r = r0; r < rows; r += NW) {
+        RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
+        const float x = rs.xi >= 0 ? sp_ld<IO>(rs.row, rs.xi) * sl : -INFINITY;
+        const float ex = sl < 0.f ? sp_extreme<IO, true>(rs.body, rs.nv, lane) : sp_extreme<IO, false>(rs.body, rs.nv, lane);
+        const float mx = sp_max(fmaxf(x, lane < rs.nv ? ex * sl : -INFINITY), 32);
+        float2 sum = make_float2(blk_exp2(x - mx), 0.f);
+        float2 off = make_float2(-mx, -mx);
+        sp_each(rs.nv, lane, [&](int vi) {
+            float2 f[VP];
+            sp_exp<IO>(sp_ldv(rs.body, vi), sl2, off, f);
+#pragma unroll
+            for (int e = 0; e < VP; ++e) sum = blk_add2(sum, f[e]);
+        });
+        off.x = off.y = -mx - __log2f(sp_sum(sum.x + sum.y, 32));  // exp2(x * sl + off) = exp2(x * sl - max) / sum
+        sp_each(rs.nv, lane, [&](int vi) {
+            float2 f[VP];
+            sp_exp<IO>(sp_ldv(rs.body, vi), sl2, off, f);
+            sp_stv(rs.body, vi, IO::pack(f));
+        });
+        if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, blk_exp2(x + off.x));
+    }
 }
 // backward over whole vectors, two passes (dot product, then the result over the gradient)
 template <typename IO, int NW>
-__device__ __forceinline__ void bwd_rows_vec(const typename IO::E* ppiece, typename IO::E* gpiece, int rows, int cols,
-                                             float scale, int warp, int lane) {
-    constexpr int VE = IO::VE;
-    for (int r = warp; r < rows; r += NW) {
-        RowSplit<IO> rs(gpiece + (size_t)r * cols, cols, lane);  // both rows sit at the same offset of their buffers
-        const typename IO::E* prow = ppiece + (size_t)r * cols;
-        const uint4* pbody = reinterpret_cast<const uint4*>(prow + (reinterpret_cast<typename IO::E*>(rs.body) - rs.row));
+__device__ __forceinline__ void bwd_rows_vec(uint32_t ppiece, uint32_t gpiece, int rows, int cols,
+                                             float scale, int r0, int lane) {
+    constexpr int VP = IO::VE / 2;
+    const float2 scale2 = make_float2(scale, scale);
+#pragma unroll 1
+    for (int r = r0; r < rows; r += NW) {
+        RowSplit<IO> rs(gpiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);  // both rows sit at the same offset of their buffers
+        const uint32_t prow = ppiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+        const uint32_t pbody = prow + (rs.body - rs.row);
         float px = 0.f, gx = 0.f;
         if (rs.xi >= 0) {
-            px = IO::ld(prow[rs.xi]);
-            gx = IO::ld(rs.row[rs.xi]);
+            px = sp_ld<IO>(prow, rs.xi);
+            gx = sp_ld<IO>(rs.row, rs.xi);
         }
-        float pf[VE], gf[VE];
-        float dot = px * gx;
-        for (int vi = lane; vi < rs.nv; vi += 32) {
-            IO::unpack(pbody[vi], pf);
-            IO::unpack(rs.body[vi], gf);
+        float2 dot2 = make_float2(px * gx, 0.f);
+        sp_each(rs.nv, lane, [&](int vi) {
+            float2 pf[VP], gf[VP];
+            IO::unpack(sp_ldv(pbody, vi), pf);
+            IO::unpack(sp_ldv(rs.body, vi), gf);
 #pragma unroll
-            for (int e = 0; e < VE; ++e) dot = fmaf(pf[e], gf[e], dot);
-        }
-        dot = sp_sum(dot, 32);
-        for (int vi = lane; vi < rs.nv; vi += 32) {
-            IO::unpack(pbody[vi], pf);
-            IO::unpack(rs.body[vi], gf);
+            for (int e = 0; e < VP; ++e) dot2 = blk_fma2(pf[e], gf[e], dot2);
+        });
+        const float dot = sp_sum(dot2.x + dot2.y, 32);
+        const float2 ndot = make_float2(-dot, -dot);
+        sp_each(rs.nv, lane, [&](int vi) {
+            float2 pf[VP], gf[VP];
+            IO::unpack(sp_ldv(pbody, vi), pf);
+            IO::unpack(sp_ldv(rs.body, vi), gf);
 #pragma unroll
-            for (int e = 0; e < VE; ++e) gf[e] = (gf[e] - dot) * pf[e] * scale;
-            rs.body[vi] = IO::pack(gf);
-        }
-        if (rs.xi >= 0) rs.row[rs.xi] = IO::st((gx - dot) * px * scale);
+            for (int e = 0; e < VP; ++e) gf[e] = blk_mul2(blk_mul2(blk_add2(gf[e], ndot), pf[e]), scale2);
+            sp_stv(rs.body, vi, IO::pack(gf));
+        });
+        if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, (gx - dot) * px * scale);
     }
 }
 
-// Short rows (fewer columns than eight vectors): one lane per row, one warp per piece, so a window of many
-// small segments keeps every warp busy and no shuffle is needed.  Up to 32 columns stay in registers.
+// Short rows (fewer columns than eight vectors).  Up to 16 columns: one lane per row, no shuffle.  More: eight lanes per
+// row, which keeps the row in registers and every warp busy when a window is one long piece of short rows.
+constexpr int SP_LANE_COLS = 16;
 template <typename IO>
-__device__ __forceinline__ void fwd_rows_lane(typename IO::E* piece, int rows, int cols, float sl, int lane) {
-    for (int r = lane; r < rows; r += 32) {
-        typename IO::E* row = piece + (size_t)r * cols;
-        if (cols <= 32) {
-            float v[32];
-            float mx = -INFINITY;
+__device__ __noinline__ void fwd_rows_lane(uint32_t piece, int rows, int cols, float sl, int r, int lane) {
+    r += lane;
+    if (r >= rows) return;
+    const uint32_t row = piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    float v[SP_LANE_COLS];
+    float mx = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                v[c] = c < cols ? IO::ld(row[c]) * sl : -INFINITY;
-                mx = fmaxf(mx, v[c]);
-            }
-            float sum = 0.f;
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                v[c] = blk_exp2(v[c] - mx);
-                sum += v[c];
-            }
-            const float inv = 1.f / sum;
-#pragma unroll
-            for (int c = 0; c < 32; ++c)
-                if (c < cols) row[c] = IO::st(v[c] * inv);
-        } else {
-            float mx = -INFINITY;
-            for (int c = 0; c < cols; ++c) mx = fmaxf(mx, IO::ld(row[c]) * sl);
-            float sum = 0.f;
-            for (int c = 0; c < cols; ++c) sum += blk_exp2(fmaf(IO::ld(row[c]), sl, -mx));
-            const float inv = 1.f / sum;
-            for (int c = 0; c < cols; ++c) row[c] = IO::st(blk_exp2(fmaf(IO::ld(row[c]), sl, -mx)) * inv);
-        }
+    for (int c = 0; c < SP_LANE_COLS; ++c) {
+        v[c] = c < cols ? sp_ld<IO>(row, c) * sl : -INFINITY;
+        mx = fmaxf(mx, v[c]);
     }
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < SP_LANE_COLS; ++c) {
+        v[c] = blk_exp2(v[c] - mx);
+        sum += v[c];
+    }
+    const float inv = 1.f / sum;
+#pragma unroll
+    for (int c = 0; c < SP_LANE_COLS; ++c)
+        if (c < cols) sp_st<IO>(row, c, v[c] * inv);
 }
 template <typename IO>
-__device__ __forceinline__ void bwd_rows_lane(const typename IO::E* ppiece, typename IO::E* gpiece, int rows, int cols,
-                                              float scale, int lane) {
-    for (int r = lane; r < rows; r += 32) {
-        const typename IO::E* prow = ppiece + (size_t)r * cols;
-        typename IO::E* grow = gpiece + (size_t)r * cols;
-        float dot = 0.f;
-        for (int c = 0; c < cols; ++c) dot = fmaf(IO::ld(prow[c]), IO::ld(grow[c]), dot);
-        for (int c = 0; c < cols; ++c) grow[c] = IO::st((IO::ld(grow[c]) - dot) * IO::ld(prow[c]) * scale);
+__device__ __noinline__ void fwd_rows_group(uint32_t piece, int rows, int cols, float sl, int r, int lane) {
+    r += lane >> 3;
+    const int l = lane & 7;
+    const uint32_t row = piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    float v[IO::VE];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < IO::VE; ++i) {
+        v[i] = r < rows && l + 8 * i < cols ? sp_ld<IO>(row, l + 8 * i) * sl : -INFINITY;
+        mx = fmaxf(mx, v[i]);
     }
+    mx = sp_max(mx, 8);
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < IO::VE; ++i) {
+        v[i] = blk_exp2(v[i] - mx);
+        sum += v[i];
+    }
+    const float inv = 1.f / sp_sum(sum, 8);
+#pragma unroll
+    for (int i = 0; i < IO::VE; ++i)
+        if (r < rows && l + 8 * i < cols) sp_st<IO>(row, l + 8 * i, v[i] * inv);
+}
+template <typename IO>
+__device__ __forceinline__ void bwd_rows_lane(uint32_t ppiece, uint32_t gpiece, int rows, int cols,
+                                              float scale, int r, int lane) {
+    r += lane;
+    if (r >= rows) return;
+    const uint32_t prow = ppiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    const uint32_t grow = gpiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    float dot = 0.f;
+    for (int c = 0; c < cols; ++c) dot = fmaf(sp_ld<IO>(prow, c), sp_ld<IO>(grow, c), dot);
+    for (int c = 0; c < cols; ++c) sp_st<IO>(grow, c, (sp_ld<IO>(grow, c) - dot) * sp_ld<IO>(prow, c) * scale);
+}
+template <typename IO>
+__device__ __forceinline__ void bwd_rows_group(uint32_t ppiece, uint32_t gpiece, int rows, int cols,
+                                               float scale, int r, int lane) {
+    r += lane >> 3;
+    const int l = lane & 7;
+    const uint32_t prow = ppiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    const uint32_t grow = gpiece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
+    float pv[IO::VE], gv[IO::VE];
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < IO::VE; ++i) {
+        const bool in = r < rows && l + 8 * i < cols;
+        pv[i] = in ? sp_ld<IO>(prow, l + 8 * i) : 0.f;
+        gv[i] = in ? sp_ld<IO>(grow, l + 8 * i) : 0.f;
+        dot = fmaf(pv[i], gv[i], dot);
+    }
+    dot = sp_sum(dot, 8);
+#pragma unroll
+    for (int i = 0; i < IO::VE; ++i)
+        if (r < rows && l + 8 * i < cols) sp_st<IO>(grow, l + 8 * i, (gv[i] - dot) * pv[i] * scale);
 }
 
-// One piece.  Pieces of short rows are dealt out to the warps one piece each (piece index pi); the warps share
-// the rows of a piece of longer rows.
-template <typename IO>
-__device__ __forceinline__ void fwd_piece(typename IO::E* srow, int rows, int cols, float sl, int pi, int warp, int lane) {
+// Rows of a unit of short rows, the amount of work that goes to one warp.
+__device__ __forceinline__ int sp_unit_rows(int cols) { return cols <= SP_LANE_COLS ? 32 : 4; }
+
+// One piece: this warp's units -- rows, or groups of short rows -- are u, u + NW, ...
+template <typename IO, int NW>
+__device__ __forceinline__ void fwd_piece(uint32_t srow, int rows, int cols, float sl, int u, int lane) {
     constexpr int VE = IO::VE;
     if (cols < 8 * VE) {
-        if (pi % SP_WARPS == warp) fwd_rows_lane<IO>(srow, rows, cols, sl, lane);
+        const int ur = sp_unit_rows(cols);
+#pragma unroll 1
+        for (int r = u * ur; r < rows; r += NW * ur) {
+            if (cols <= SP_LANE_COLS) fwd_rows_lane<IO>(srow, rows, cols, sl, r, lane);
+            else fwd_rows_group<IO>(srow, rows, cols, sl, r, lane);
+        }
         return;
     }
     const int nvmax = cols / VE;  // whole vectors of a row never exceed this
-    if (nvmax <= 32) fwd_rows_vec<IO, 1, SP_WARPS>(srow, rows, cols, sl, warp, lane);
-    else if (nvmax <= 64) fwd_rows_vec<IO, 2, SP_WARPS>(srow, rows, cols, sl, warp, lane);
-    else if (nvmax <= 128) fwd_rows_vec<IO, 4, SP_WARPS>(srow, rows, cols, sl, warp, lane);
-    else fwd_rows_vec_streamed<IO, SP_WARPS>(srow, rows, cols, sl, warp, lane);
+    if (nvmax > 64 || sl == 0.f) fwd_rows_vec_streamed<IO, NW>(srow, rows, cols, sl, u, lane);
+    else if (nvmax <= 32) fwd_rows_vec<IO, 1, NW>(srow, rows, cols, sl, u, lane);
+    else fwd_rows_vec<IO, 2, NW>(srow, rows, cols, sl, u, lane);
 }
-// backward: the result overwrites the gradient piece
-template <typename IO>
-__device__ __forceinline__ void bwd_piece(const typename IO::E* prow0, typename IO::E* grow0, int rows, int cols, float scale,
-                                          int pi, int warp, int lane) {
+template <typename IO, int NW>
+__device__ __forceinline__ void bwd_piece(uint32_t prow0, uint32_t grow0, int rows, int cols, float scale,
+                                          int u, int lane) {
     if (cols >= 8 * IO::VE) {
-        bwd_rows_vec<IO, SP_WARPS>(prow0, grow0, rows, cols, scale, warp, lane);
+        bwd_rows_vec<IO, NW>(prow0, grow0, rows, cols, scale, u, lane);
         return;
     }
-    if (pi % SP_WARPS == warp) bwd_rows_lane<IO>(prow0, grow0, rows, cols, scale, lane);
+    const int ur = sp_unit_rows(cols);
+#pragma unroll 1
+    for (int r = u * ur; r < rows; r += NW * ur) {
+        if (cols <= SP_LANE_COLS) bwd_rows_lane<IO>(prow0, grow0, rows, cols, scale, r, lane);
+        else bwd_rows_group<IO>(prow0, grow0, rows, cols, scale, r, lane);
+    }
 }
 
+template <int NW>
+__device__ __forceinline__ void sp_compute_sync() {  // among the computing warps
+    asm volatile("bar.sync 1, %0;\n" ::"n"(32 * NW) : "memory");
+}
+template <int NW>
 __device__ __forceinline__ float sp_cta_reduce(float v, bool is_max, float* red, int warp, int lane) {
     v = is_max ? sp_max(v, 32) : sp_sum(v, 32);
-    __syncthreads();  // red may still be read from the previous reduction
+    sp_compute_sync<NW>();  // red may still be read from the previous reduction
     if (lane == 0) red[warp] = v;
-    __syncthreads();
+    sp_compute_sync<NW>();
     float r = red[0];
 #pragma unroll
-    for (int w = 1; w < SP_WARPS; ++w) r = is_max ? fmaxf(r, red[w]) : r + red[w];
+    for (int w = 1; w < NW; ++w) r = is_max ? fmaxf(r, red[w]) : r + red[w];
     return r;
 }
 
+// A window in its stage.
+struct SpWin {
+    int64_t e0;   // its first element in the buffers
+    int64_t off;  // ... inside the head strip
+    int nbytes, npieces, first_piece, pad;
+};
+
+// The (window, head) list of a CTA: window index and head of entry blockIdx.x, + gridDim.x, ...
+struct SpWalk {
+    int idx, head, didx, dhead;
+    bool has;
+    __device__ __forceinline__ explicit SpWalk(const BlkSmxPipeParams& p) {
+        head = (int)(blockIdx.x / (unsigned)p.num_windows);
+        idx = (int)(blockIdx.x - (unsigned)head * (unsigned)p.num_windows);
+        dhead = (int)(gridDim.x / (unsigned)p.num_windows);
+        didx = (int)(gridDim.x - (unsigned)dhead * (unsigned)p.num_windows);
+        has = head < p.H;
+    }
+    __device__ __forceinline__ void step(const BlkSmxPipeParams& p) {
+        idx += didx;
+        head += dhead;
+        if (idx >= p.num_windows) {
+            idx -= p.num_windows;
+            ++head;
+        }
+        has = head < p.H;
+    }
+    __device__ __forceinline__ SpWin load(const BlkSmxPipeParams& p) const {
+        const BlkSmxWindow w = p.windows[idx];
+        return SpWin{(int64_t)head * p.D + w.off, w.off, w.nbytes, w.npieces, w.first_piece, 0};
+    }
+};
+
 // BWD = false: in0 = src, result = softmax; BWD = true: in0 = forward result, in1 = its gradient.
 template <typename IO, bool BWD>
-__global__ void __launch_bounds__(SP_THREADS, BWD ? 4 : 8) blk_softmax_pipe_kernel(const BlkSmxPipeParams p) {
+__global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk_softmax_pipe_kernel(const BlkSmxPipeParams p) {
     typedef typename IO::E E;
     constexpr int ES = (int)sizeof(E);
     constexpr int NIN = BWD ? 2 : 1;
-    extern __shared__ __align__(128) unsigned char sp_smem[];  // [2 stages][NIN][SP_BUF]
-    __shared__ __align__(8) uint64_t bars[2];
-    __shared__ float red[SP_WARPS];
-    __shared__ __align__(16) BlkSmxChunk recs[2][BLK_SMX_WINDOW_PIECES];  // the windows' piece records, per stage
+    constexpr int NW = SpShape<BWD>::NW, ST = SpShape<BWD>::STAGES;
+    extern __shared__ __align__(128) unsigned char sp_smem[];  // [stages][NIN][SP_BUF]
+    __shared__ __align__(8) uint64_t bars[2 * ST];             // full[stage], done[stage]
+    __shared__ float red[NW];
+    __shared__ SpWin wins[ST];
+    __shared__ __align__(16) BlkSmxChunk recs[ST][BLK_SMX_WINDOW_PIECES];  // the windows' piece records, per stage
+    __shared__ volatile int abort_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bar0 = blk_smem_u32(bars);
+    auto full = [&](int st) { return bar0 + 8u * st; };
+    auto done = [&](int st) { return bar0 + 8u * (ST + st); };
     auto buf = [&](int st, int in) { return sp_smem + (st * NIN + in) * SP_BUF; };
     if (tid == 0) {
-        sp_bar_init(bar0, 1);
-        sp_bar_init(bar0 + 8, 1);
+        for (int i = 0; i < ST; ++i) {
+            sp_bar_init(full(i), 1);
+            sp_bar_init(done(i), NW);
+        }
+        abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
 
-    const int64_t total = (int64_t)p.num_windows * p.H, G = gridDim.x;
     const E* g0 = reinterpret_cast<const E*>(p.in0);
     const E* g1 = reinterpret_cast<const E*>(p.in1);
     E* gd = reinterpret_cast<E*>(p.out);
-    const float sl = BWD ? p.scale : p.scale * BLK_LOG2E;
 
-    // thread 0: start the copies of window w into stage st (nothing for a row longer than a window)
-    auto issue = [&](int64_t w, int st) {
-        const BlkSmxWindow win = p.windows[w % p.num_windows];
-        if (win.nbytes > SP_WIN) return;
-        const int64_t a = ((w / p.num_windows) * p.D + win.off) * ES;  // byte offset of the window in each buffer
-        const int mis = (int)(a & 15);
-        const uint32_t bytes = (uint32_t)((mis + win.nbytes + 15) & ~15);
-        const uint32_t bar = bar0 + 8u * st;
-        const uint32_t rbytes = (uint32_t)win.npieces * (uint32_t)sizeof(BlkSmxChunk);
-        sp_expect_tx(bar, NIN * bytes + rbytes);
-        sp_bulk_g2s(blk_smem_u32(recs[st]), p.pieces + win.first_piece, rbytes, bar);
-        sp_bulk_g2s(blk_smem_u32(buf(st, 0)), reinterpret_cast<const unsigned char*>(g0) + (a - mis), bytes, bar);
-        if (BWD) sp_bulk_g2s(blk_smem_u32(buf(st, 1)), reinterpret_cast<const unsigned char*>(g1) + (a - mis), bytes, bar);
-    };
-
-    uint32_t phase0 = 0u, phase1 = 0u;  // parity of the next completion of each stage's barrier
-    int64_t w = blockIdx.x;
-    if (tid == 0 && w < total) issue(w, 0);
-    for (int k = 0; w < total; w += G, ++k) {
-        const int st = k & 1;
-        // the other stage is free once the bulk store that read it (previous window) is done with shared memory
-        if (tid == 0) sp_bulk_wait_read();
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // this thread's reads of that stage come first
-        __syncthreads();
-        if (tid == 0 && w + G < total) issue(w + G, st ^ 1);
-
-        const BlkSmxWindow win = p.windows[w % p.num_windows];
-        const int64_t e0 = (w / p.num_windows) * p.D + win.off;
-        if (win.nbytes > SP_WIN) {
-            // one row longer than a window: streamed from global memory by the whole CTA
-            const int cols = p.pieces[win.first_piece].cols;
-            if (!BWD) {
-                float mx = -INFINITY;
-                for (int c = tid; c < cols; c += SP_THREADS) mx = fmaxf(mx, IO::ld(g0[e0 + c]) * sl);
-                mx = sp_cta_reduce(mx, true, red, warp, lane);
-                float sum = 0.f;
-                for (int c = tid; c < cols; c += SP_THREADS) sum += blk_exp2(IO::ld(g0[e0 + c]) * sl - mx);
-                sum = sp_cta_reduce(sum, false, red, warp, lane);
-                const float inv = 1.f / sum;
-                for (int c = tid; c < cols; c += SP_THREADS) gd[e0 + c] = IO::st(blk_exp2(IO::ld(g0[e0 + c]) * sl - mx) * inv);
-            } else {
-                float dot = 0.f;
-                for (int c = tid; c < cols; c += SP_THREADS) dot += IO::ld(g0[e0 + c]) * IO::ld(g1[e0 + c]);
-                dot = sp_cta_reduce(dot, false, red, warp, lane);
-                for (int c = tid; c < cols; c += SP_THREADS)
-                    gd[e0 + c] = IO::st((IO::ld(g1[e0 + c]) - dot) * IO::ld(g0[e0 + c]) * sl);
+    if (warp == NW) {
+        // ---------------- the copying warp ----------------
+        SpWalk next(p);   // the next window to fetch
+        SpWin rec = {};
+        if (next.has) rec = next.load(p);
+        // lane 0: start the copies of the next window into stage st (none for a row longer than a window)
+        auto issue = [&](int st) {
+            wins[st] = rec;
+            const bool fits = rec.nbytes <= SP_WIN;
+            const int64_t a = rec.e0 * ES;  // byte offset of the window in each buffer
+            const int mis = (int)(a & 15);
+            const uint32_t bytes = fits ? (uint32_t)((mis + rec.nbytes + 15) & ~15) : 0u;
+            const uint32_t rbytes = fits ? (uint32_t)rec.npieces * (uint32_t)sizeof(BlkSmxChunk) : 0u;
+            sp_expect_tx(full(st), NIN * bytes + rbytes);
+            if (fits) {
+                sp_bulk_g2s(blk_smem_u32(recs[st]), p.pieces + rec.first_piece, rbytes, full(st));
+                sp_bulk_g2s(blk_smem_u32(buf(st, 0)), reinterpret_cast<const unsigned char*>(g0) + (a - mis), bytes, full(st));
+                if (BWD)
+                    sp_bulk_g2s(blk_smem_u32(buf(st, 1)), reinterpret_cast<const unsigned char*>(g1) + (a - mis), bytes, full(st));
             }
-            continue;
+            next.step(p);
+            if (next.has) rec = next.load(p);
+        };
+        if (lane == 0) {
+#pragma unroll 1
+            for (int i = 0; i < ST && next.has; ++i) issue(i);
         }
-        const int mis = (int)((e0 * ES) & 15);
-        bool arrived = true;
-        if (lane == 0) arrived = sp_wait(bar0 + 8u * st, st ? phase1 : phase0);  // one lane per warp polls
-        arrived = __shfl_sync(0xffffffffu, arrived, 0);
-        if (st) phase1 ^= 1u;
-        else phase0 ^= 1u;
-        unsigned char* res = buf(st, BWD ? 1 : 0);  // the buffer that ends up holding the result
-        if (arrived) {
-            E* r0 = reinterpret_cast<E*>(res + mis);
-            const E* p0 = reinterpret_cast<const E*>(buf(st, 0) + mis);
-            int eo = 0;
-            for (int pi = 0; pi < win.npieces; ++pi) {
-                const BlkSmxChunk pc = recs[st][pi];
-                if (!BWD) fwd_piece<IO>(r0 + eo, pc.rows, pc.cols, sl, pi, warp, lane);
-                else bwd_piece<IO>(p0 + eo, r0 + eo, pc.rows, pc.cols, sl, pi, warp, lane);
-                eo += pc.rows * pc.cols;
+        SpWalk cur(p);
+#pragma unroll 1
+        for (uint32_t k = 0; cur.has; cur.step(p), ++k) {
+            const int st = (int)(k % ST);
+            if (!__all_sync(0xffffffffu, sp_wait(done(st), (k / ST) & 1u, &abort_flag) && !abort_flag)) break;
+            const int64_t e0 = wins[st].e0;
+            const int nbytes = wins[st].nbytes;
+            if (nbytes <= SP_WIN) {
+                // aligned vectors wholly inside the window: one bulk store; ragged edges: single elements
+                const int mis = (int)((e0 * ES) & 15);
+                unsigned char* res = buf(st, BWD ? 1 : 0);  // the buffer that holds the result
+                const int span = mis + nbytes;
+                const int lo = mis ? 16 : 0, hi = span & ~15;
+                unsigned char* dst_al = reinterpret_cast<unsigned char*>(gd) + (e0 * ES - mis);
+                if (lane == 0 && hi > lo) sp_bulk_s2g(dst_al + lo, blk_smem_u32(res + lo), (uint32_t)(hi - lo));
+                // head edge: bytes [mis, min(lo, span)); tail edge: bytes [max(hi, lo), span)  (hi >= lo or the window is tiny)
+                const int h_end = lo < span ? lo : span;
+                const int b = mis + lane * ES;
+                if (lane < 16 / ES && b < h_end) *reinterpret_cast<E*>(dst_al + b) = *reinterpret_cast<const E*>(res + b);
+                const int t0 = hi > h_end ? hi : h_end;
+                const int bt = t0 + (lane - 16) * ES;
+                if (lane >= 16 && lane < 16 + 16 / ES && bt < span)
+                    *reinterpret_cast<E*>(dst_al + bt) = *reinterpret_cast<const E*>(res + bt);
+            }
+            __syncwarp();
+            if (lane == 0) {
+                sp_bulk_commit();
+                // the stage of the window before this one is free once its bulk store is done with shared memory
+                if (k > 0 && next.has) {
+                    sp_bulk_wait_read1();
+                    issue((int)((k - 1) % ST));
+                }
             }
         }
-        // results (generic-proxy writes) must be visible to the bulk store (async proxy)
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        if (__syncthreads_or(!arrived)) {
-            if (tid == 0) atomicCAS(p.status, 0, 21);
-            break;
-        }
-        // aligned vectors wholly inside the window: one bulk store; ragged edges: single elements
-        const int span = mis + win.nbytes;
-        const int lo = mis ? 16 : 0, hi = span & ~15;
-        unsigned char* dst_al = reinterpret_cast<unsigned char*>(gd) + (e0 * ES - mis);
-        if (tid == 0 && hi > lo) {
-            sp_bulk_s2g(dst_al + lo, blk_smem_u32(res + lo), (uint32_t)(hi - lo));
-            sp_bulk_commit();
-        }
-        if (warp == 1 % SP_WARPS) {
-            // head edge: bytes [mis, min(lo, span)); tail edge: bytes [max(hi, lo), span)  (hi >= lo or the window is tiny)
-            const int h_end = lo < span ? lo : span;
-            const int b = mis + lane * ES;
-            if (lane < 16 / ES && b < h_end) *reinterpret_cast<E*>(dst_al + b) = *reinterpret_cast<const E*>(res + b);
-            const int t0 = hi > h_end ? hi : h_end;
-            const int bt = t0 + (lane - 16) * ES;
-            if (lane >= 16 && lane < 16 + 16 / ES && bt < span) *reinterpret_cast<E*>(dst_al + bt) = *reinterpret_cast<const E*>(res + bt);
+        if (lane == 0) sp_bulk_wait_all();
+    } else {
+        // ---------------- computing warps ----------------
+        const float sl = BWD ? p.scale : p.scale * BLK_LOG2E;
+        constexpr int LONG = 8 * IO::VE;  // rows of at least this many columns take a warp each
+        int turn = warp;                  // the unit of the next window, counted from its first, that is this warp's
+        bool ok = true;
+        SpWalk cur(p);
+#pragma unroll 1
+        for (uint32_t k = 0; cur.has; cur.step(p), ++k) {
+            const int st = (int)(k % ST);
+            ok = __all_sync(0xffffffffu, ok && sp_wait(full(st), (k / ST) & 1u, &abort_flag));
+            const SpWin win = ok ? wins[st] : cur.load(p);
+            if (win.nbytes > SP_WIN) {
+                // one row longer than a window: streamed from global memory by all computing warps
+                const int cols = p.pieces[win.first_piece].cols;
+                const int64_t e0 = win.e0;
+                constexpr int NT = 32 * NW;
+                if (!BWD) {
+                    float mx = -INFINITY;
+                    for (int c = tid; c < cols; c += NT) mx = fmaxf(mx, IO::ld(g0[e0 + c]) * sl);
+                    mx = sp_cta_reduce<NW>(mx, true, red, warp, lane);
+                    float sum = 0.f;
+                    for (int c = tid; c < cols; c += NT) sum += blk_exp2(IO::ld(g0[e0 + c]) * sl - mx);
+                    sum = sp_cta_reduce<NW>(sum, false, red, warp, lane);
+                    const float inv = 1.f / sum;
+                    for (int c = tid; c < cols; c += NT) gd[e0 + c] = IO::st(blk_exp2(IO::ld(g0[e0 + c]) * sl - mx) * inv);
+                } else {
+                    float dot = 0.f;
+                    for (int c = tid; c < cols; c += NT) dot += IO::ld(g0[e0 + c]) * IO::ld(g1[e0 + c]);
+                    dot = sp_cta_reduce<NW>(dot, false, red, warp, lane);
+                    for (int c = tid; c < cols; c += NT)
+                        gd[e0 + c] = IO::st((IO::ld(g1[e0 + c]) - dot) * IO::ld(g0[e0 + c]) * sl);
+                }
+            } else if (ok) {
+                const int mis = (int)((win.e0 * ES) & 15);
+                const uint32_t r0 = blk_smem_u32(buf(st, BWD ? 1 : 0)) + mis, p0 = blk_smem_u32(buf(st, 0)) + mis;
+                // The window's units -- a row of a piece of long rows, a whole piece of short ones -- go to the warps in
+                // turn, from window to window.  A lane counts those of one piece; a warp then visits the pieces that
+                // hold one of its own.
+#pragma unroll 1
+                for (int base = 0; base < win.npieces; base += 32) {
+                    int units = 0;
+                    if (base + lane < win.npieces) {
+                        const BlkSmxChunk pc = recs[st][base + lane];
+                        units = pc.cols >= LONG ? pc.rows : (pc.rows + sp_unit_rows(pc.cols) - 1) / sp_unit_rows(pc.cols);
+                    }
+                    int incl = units;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    const int excl = incl - units;
+                    // this warp's first unit of the piece: the smallest turn + i NW >= excl
+                    const int first = turn + (excl > turn ? (excl - turn + NW - 1) / NW * NW : 0) - excl;
+                    uint32_t mine = __ballot_sync(0xffffffffu, first < units);
+                    while (mine) {
+                        const int src = __ffs(mine) - 1;
+                        mine &= mine - 1;
+                        const int r = __shfl_sync(0xffffffffu, first, src);
+                        const BlkSmxChunk pc = recs[st][base + src];
+                        const uint32_t eo = (uint32_t)(pc.off - win.off) * ES;
+                        if (BWD) bwd_piece<IO, NW>(p0 + eo, r0 + eo, pc.rows, pc.cols, sl, r, lane);
+                        else fwd_piece<IO, NW>(r0 + eo, pc.rows, pc.cols, sl, r, lane);
+                    }
+                    const int n = __shfl_sync(0xffffffffu, incl, 31);
+                    turn += (n > turn ? (n - turn + NW - 1) / NW * NW : 0) - n;
+                }
+            }
+            // results (generic-proxy writes) must be visible to the bulk store (async proxy)
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) sp_arrive(done(st));
         }
     }
-    if (tid == 0) sp_bulk_wait_all();
+    __syncthreads();
+    if (tid == 0 && abort_flag) {
+        atomicCAS(p.status, 0, 21);
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);  // copies in flight land before the CTA's memory is released
+    }
 }
 
 }  // namespace
@@ -515,21 +726,22 @@ __global__ void __launch_bounds__(SP_THREADS, BWD ? 4 : 8) blk_softmax_pipe_kern
 cudaError_t blk_launch_softmax_pipe(const BlkSmxPipeParams& p, int dtype, int backward, int sms, cudaStream_t st) {
     const int64_t total = (int64_t)p.num_windows * p.H;
     if (total == 0) return cudaSuccess;
-    auto go = [&](auto kern, int nin) -> cudaError_t {
-        const int smem = 2 * nin * SP_BUF;
+    auto go = [&](auto kern, int nin, auto shape) -> cudaError_t {
+        typedef decltype(shape) S;
+        const int smem = S::STAGES * nin * SP_BUF;
         cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
-        const int64_t resident = (int64_t)sms * (nin == 1 ? 8 : 4);
-        const dim3 grid((unsigned)(total < resident ? total : resident)), block(SP_THREADS);
+        const int64_t resident = (int64_t)sms * S::CTAS;
+        const dim3 grid((unsigned)(total < resident ? total : resident)), block(S::THREADS);
         kern<<<grid, block, smem, st>>>(p);
         return cudaGetLastError();
     };
     if (!backward) {
-        if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, false>, 1);
-        if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, false>, 1);
-        return go(blk_softmax_pipe_kernel<SpIO32, false>, 1);
+        if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, false>, 1, SpShape<false>{});
+        if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, false>, 1, SpShape<false>{});
+        return go(blk_softmax_pipe_kernel<SpIO32, false>, 1, SpShape<false>{});
     }
-    if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, true>, 2);
-    if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, true>, 2);
-    return go(blk_softmax_pipe_kernel<SpIO32, true>, 2);
+    if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, true>, 2, SpShape<true>{});
+    if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, true>, 2, SpShape<true>{});
+    return go(blk_softmax_pipe_kernel<SpIO32, true>, 2, SpShape<true>{});
 }

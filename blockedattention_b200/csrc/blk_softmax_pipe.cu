@@ -16,10 +16,11 @@
 // Every barrier wait is bounded and reports through the status word.
 //
 // Bound by the instructions it issues and their latency, with memory close behind (the copies alone: 650 us where the
-// forward takes 800, and 187 where the backward takes 204).  A spilled register in a row loop costs more than any
+// forward takes 711, and 187 where the backward takes 199).  A spilled register in a row loop costs more than any
 // parallelism: with 28 warps of 64 registers the loops over a row's vectors stay rolled, and rows of short segments are
-// functions of their own.  512 segments of 16..2048 rows and columns, 4 heads, bf16: 870 -> 800 us forward; a quarter of
-// it 200 -> 187 forward, 223 -> 204 backward (before: two stages, all warps of a CTA meeting twice a window).
+// functions of their own.  512 segments of 16..2048 rows and columns, 4 heads, bf16: 870 -> 711 us forward; a quarter of
+// it 200 -> 167 forward, 223 -> 199 backward (before: two stages, all warps of a CTA meeting twice a window; a fifth of the
+// instructions were the counting of units in windows of one piece until those were told apart: 783 -> 711).
 //
 // Forward: out = softmax_rows(scale * src); replaces upstream sparseBlockedSoftmax_warp / _block
 // (csrc/cuda/spBlkSoftmax.cu:88-138, :182-269).  Backward: grad_src = scale * (grad_out - rowsum(out *
@@ -675,37 +676,47 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
             } else if (ok) {
                 const int mis = (int)((win.e0 * ES) & 15);
                 const uint32_t r0 = blk_smem_u32(buf(st, BWD ? 1 : 0)) + mis, p0 = blk_smem_u32(buf(st, 0)) + mis;
-                // The window's units -- a row of a piece of long rows, a whole piece of short ones -- go to the warps in
-                // turn, from window to window.  A lane counts those of one piece; a warp then visits the pieces that
-                // hold one of its own.
-#pragma unroll 1
-                for (int base = 0; base < win.npieces; base += 32) {
-                    int units = 0;
-                    if (base + lane < win.npieces) {
-                        const BlkSmxChunk pc = recs[st][base + lane];
-                        units = pc.cols >= LONG ? pc.rows : (pc.rows + sp_unit_rows(pc.cols) - 1) / sp_unit_rows(pc.cols);
-                    }
-                    int incl = units;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += v;
-                    }
-                    const int excl = incl - units;
-                    // this warp's first unit of the piece: the smallest turn + i NW >= excl
-                    const int first = turn + (excl > turn ? (excl - turn + NW - 1) / NW * NW : 0) - excl;
-                    uint32_t mine = __ballot_sync(0xffffffffu, first < units);
-                    while (mine) {
-                        const int src = __ffs(mine) - 1;
-                        mine &= mine - 1;
-                        const int r = __shfl_sync(0xffffffffu, first, src);
-                        const BlkSmxChunk pc = recs[st][base + src];
-                        const uint32_t eo = (uint32_t)(pc.off - win.off) * ES;
-                        if (BWD) bwd_piece<IO, NW>(p0 + eo, r0 + eo, pc.rows, pc.cols, sl, r, lane);
-                        else fwd_piece<IO, NW>(r0 + eo, pc.rows, pc.cols, sl, r, lane);
-                    }
-                    const int n = __shfl_sync(0xffffffffu, incl, 31);
+                auto piece = [&](int pi, int first) {
+                    const BlkSmxChunk pc = recs[st][pi];
+                    const uint32_t eo = (uint32_t)(pc.off - win.off) * ES;
+                    if (BWD) bwd_piece<IO, NW>(p0 + eo, r0 + eo, pc.rows, pc.cols, sl, first, lane);
+                    else fwd_piece<IO, NW>(r0 + eo, pc.rows, pc.cols, sl, first, lane);
+                };
+                auto units_of = [&](int pi) {
+                    const BlkSmxChunk pc = recs[st][pi];
+                    if (pc.cols >= LONG) return (int)pc.rows;
+                    const int ur = sp_unit_rows(pc.cols);
+                    return (int)(pc.rows + ur - 1) / ur;
+                };
+                // The window's units -- a row of a piece of long rows, a group of short ones -- go to the warps in turn, from
+                // window to window.  A lane counts those of one piece; a warp then visits the pieces that hold one of its
+                // own.  (A window of one piece, the usual one of wide segments, needs no counting.)
+                if (win.npieces == 1) {
+                    const int n = units_of(0);
+                    if (turn < n) piece(0, turn);
                     turn += (n > turn ? (n - turn + NW - 1) / NW * NW : 0) - n;
+                } else {
+#pragma unroll 1
+                    for (int base = 0; base < win.npieces; base += 32) {
+                        const int units = base + lane < win.npieces ? units_of(base + lane) : 0;
+                        int incl = units;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                            if (lane >= o) incl += v;
+                        }
+                        const int excl = incl - units;
+                        // this warp's first unit of the piece: the smallest turn + i NW >= excl
+                        const int first = turn + (excl > turn ? (excl - turn + NW - 1) / NW * NW : 0) - excl;
+                        uint32_t mine = __ballot_sync(0xffffffffu, first < units);
+                        while (mine) {
+                            const int src = __ffs(mine) - 1;
+                            mine &= mine - 1;
+                            piece(base + src, __shfl_sync(0xffffffffu, first, src));
+                        }
+                        const int n = __shfl_sync(0xffffffffu, incl, 31);
+                        turn += (n > turn ? (n - turn + NW - 1) / NW * NW : 0) - n;
+                    }
                 }
             }
             // results (generic-proxy writes) must be visible to the bulk store (async proxy)

@@ -64,10 +64,11 @@ struct SpIO16<BlkHalfTag> {
                           BlkCvt<BlkHalfTag>::pack2(f[2].x, f[2].y), BlkCvt<BlkHalfTag>::pack2(f[3].x, f[3].y));
     }
     // running extreme (maximum, or minimum for a negative scale) of a row, taken on the packed pairs as they lie in
-    // memory: one instruction per two elements and no conversion
-    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7c007c00u : 0xfc00fc00u; }
+    // memory: one instruction per two elements and no conversion; none: elements that scale to minus infinity
+    template <bool NEG> static __device__ __forceinline__ uint32_t none() { return NEG ? 0x7c007c00u : 0xfc00fc00u; }
+    template <bool NEG> static __device__ __forceinline__ E none1() { return (E)none<NEG>(); }
     typedef uint32_t X;
-    template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? 0x7c007c00u : 0xfc00fc00u; }
+    template <bool NEG> static __device__ __forceinline__ X xinit() { return none<NEG>(); }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
         X r;
         if (NEG) asm("{\n .reg .b32 t, u;\n min.f16x2 t, %1, %2;\n min.f16x2 u, %3, %4;\n min.f16x2 t, t, u;\n min.f16x2 %0, t, %5;\n}\n" : "=r"(r) : "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w), "r"(a));
@@ -96,9 +97,10 @@ struct SpIO16<BlkBf16Tag> {
         return make_uint4(BlkCvt<BlkBf16Tag>::pack2(f[0].x, f[0].y), BlkCvt<BlkBf16Tag>::pack2(f[1].x, f[1].y),
                           BlkCvt<BlkBf16Tag>::pack2(f[2].x, f[2].y), BlkCvt<BlkBf16Tag>::pack2(f[3].x, f[3].y));
     }
-    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7f807f80u : 0xff80ff80u; }
+    template <bool NEG> static __device__ __forceinline__ uint32_t none() { return NEG ? 0x7f807f80u : 0xff80ff80u; }
+    template <bool NEG> static __device__ __forceinline__ E none1() { return (E)none<NEG>(); }
     typedef uint32_t X;
-    template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? 0x7f807f80u : 0xff80ff80u; }
+    template <bool NEG> static __device__ __forceinline__ X xinit() { return none<NEG>(); }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
         X r;
         if (NEG) asm("{\n .reg .b32 t, u;\n min.bf16x2 t, %1, %2;\n min.bf16x2 u, %3, %4;\n min.bf16x2 t, t, u;\n min.bf16x2 %0, t, %5;\n}\n" : "=r"(r) : "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w), "r"(a));
@@ -122,9 +124,10 @@ struct SpIO32 {
     static __device__ __forceinline__ uint4 pack(const float2 (&f)[2]) {
         return make_uint4(__float_as_uint(f[0].x), __float_as_uint(f[0].y), __float_as_uint(f[1].x), __float_as_uint(f[1].y));
     }
-    static __device__ __forceinline__ uint32_t lowest(bool neg) { return neg ? 0x7f800000u : 0xff800000u; }
+    template <bool NEG> static __device__ __forceinline__ uint32_t none() { return NEG ? 0x7f800000u : 0xff800000u; }
+    template <bool NEG> static __device__ __forceinline__ E none1() { return __uint_as_float(none<NEG>()); }
     typedef float X;
-    template <bool NEG> static __device__ __forceinline__ X xinit() { return NEG ? INFINITY : -INFINITY; }
+    template <bool NEG> static __device__ __forceinline__ X xinit() { return none1<NEG>(); }
     template <bool NEG> static __device__ __forceinline__ X xacc(X a, const uint4& q) {
         const float x = __uint_as_float(q.x), y = __uint_as_float(q.y), z = __uint_as_float(q.z), w = __uint_as_float(q.w);
         return NEG ? fminf(fminf(a, x), fminf(fminf(y, z), w)) : fmaxf(fmaxf(a, x), fmaxf(fmaxf(y, z), w));
@@ -222,6 +225,13 @@ __device__ __forceinline__ float sp_ld(uint32_t row, int i) {
     sp_lds(v, row + (uint32_t)(i * (int)sizeof(typename IO::E)));
     return IO::ld(v);
 }
+// ... or the value that stands for no element
+template <typename IO, bool NEG>
+__device__ __forceinline__ float sp_ld_if(bool there, uint32_t row, int i) {
+    typename IO::E v = IO::template none1<NEG>();
+    if (there) sp_lds(v, row + (uint32_t)(i * (int)sizeof(typename IO::E)));
+    return IO::ld(v);
+}
 template <typename IO>
 __device__ __forceinline__ void sp_st(uint32_t row, int i, float v) {
     sp_sts(row + (uint32_t)(i * (int)sizeof(typename IO::E)), IO::st(v));
@@ -238,16 +248,36 @@ __device__ __forceinline__ void sp_stv(uint32_t body, int vi, const uint4& q) {
                  : "memory");
 }
 
-// exp2(x * sl + off) of a vector's elements
-template <typename IO>
-__device__ __forceinline__ void sp_exp(const uint4& q, float2 sl, float2 off, float2 (&f)[IO::VE / 2]) {
-    IO::unpack(q, f);
+// Every forward row is exp2(y) over its sum with y = (x - m) * sl, m the largest x of the row, or the smallest (NEG: the
+// kernel for negative scales).  The difference is taken before the product, so that y is rounded relative to itself: with
+// x * sl rounded first it is off by half a unit of m * sl (fp32 rows, measured against 64 bits: 5e-6 of the result for scores
+// around 200, 4e-4 around 20000; this form: below 1e-7 for both), and rows masked throughout with a type's lowest value
+// stay finite.
+__device__ __forceinline__ void sp_exp2(float2& f) {
+    f.x = blk_exp2(f.x);
+    f.y = blk_exp2(f.y);
+}
+// the value that stands for no element, and the larger of two in the order of x * sl
+template <bool NEG> __device__ __forceinline__ float sp_none() { return NEG ? INFINITY : -INFINITY; }
+template <bool NEG> __device__ __forceinline__ float sp_top(float a, float b) { return NEG ? fminf(a, b) : fmaxf(a, b); }
+template <bool NEG> __device__ __forceinline__ float sp_top3(float a, float b, float c) {
+    return NEG ? -blk_max3(-a, -b, -c) : blk_max3(a, b, c);
+}
+template <bool NEG> __device__ __forceinline__ float sp_tops(float v, int G) {  // over G lanes
+    return NEG ? -sp_max(-v, G) : sp_max(v, G);
+}
+// exp2(y) of a row's elements in place, and their sum
+template <int N>
+__device__ __forceinline__ float sp_exps(float2 (&v)[N], float m, float sl) {
+    const float2 nm = make_float2(-m, -m), sl2 = make_float2(sl, sl);
+    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int e = 0; e < IO::VE / 2; ++e) {
-        f[e] = blk_fma2(f[e], sl, off);
-        f[e].x = blk_exp2(f[e].x);
-        f[e].y = blk_exp2(f[e].y);
+    for (int i = 0; i < N; ++i) {
+        v[i] = blk_mul2(blk_add2(v[i], nm), sl2);
+        sp_exp2(v[i]);
+        sum = blk_add2(sum, v[i]);
     }
+    return sum.x + sum.y;
 }
 // f(vi) for this lane's vectors; kept rolled, see the note on registers at the head of the file
 template <typename F>
@@ -264,39 +294,35 @@ __device__ __forceinline__ float sp_extreme(uint32_t body, int nv, int lane) {
 
 // forward, at most 32 EPV whole vectors per row and a scale that is not zero: values kept in registers, one exponential
 // per element.  Lanes without a vector hold elements that scale to minus infinity.
-template <typename IO, int EPV, int NW>
+template <typename IO, bool NEG, int EPV, int NW>
 __device__ __forceinline__ void fwd_rows_vec(uint32_t piece, int rows, int cols, float sl, int r0, int lane) {
     constexpr int VP = IO::VE / 2;
     const float2 sl2 = make_float2(sl, sl);
-    const uint32_t none = IO::lowest(sl < 0.f);
+    const uint32_t none = IO::template none<NEG>();
 #pragma unroll 1
     for (int r = r0; r < rows; r += NW) {
-        RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
-        float x = rs.xi >= 0 ? sp_ld<IO>(rs.row, rs.xi) * sl : -INFINITY;
+        const RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
+        float x = sp_ld_if<IO, NEG>(rs.xi >= 0, rs.row, rs.xi);
         float2 v[EPV][VP];
-        float mx = x;
+        float m = x;
 #pragma unroll
         for (int i = 0; i < EPV; ++i) {
             uint4 q = make_uint4(none, none, none, none);
             if (lane + 32 * i < rs.nv) q = sp_ldv(rs.body, lane + 32 * i);
             IO::unpack(q, v[i]);
 #pragma unroll
-            for (int e = 0; e < VP; ++e) {
-                v[i][e] = blk_mul2(v[i][e], sl2);
-                mx = blk_max3(mx, v[i][e].x, v[i][e].y);
-            }
+            for (int e = 0; e < VP; ++e) m = sp_top3<NEG>(m, v[i][e].x, v[i][e].y);
         }
-        mx = sp_max(mx, 32);
-        x = blk_exp2(x - mx);
-        const float2 nmx = make_float2(-mx, -mx);
+        m = sp_tops<NEG>(m, 32);
+        x = blk_exp2((x - m) * sl);
+        const float2 nm = make_float2(-m, -m);
         float2 sum = make_float2(x, 0.f);
 #pragma unroll
         for (int i = 0; i < EPV; ++i)
 #pragma unroll
             for (int e = 0; e < VP; ++e) {
-                v[i][e] = blk_add2(v[i][e], nmx);
-                v[i][e].x = blk_exp2(v[i][e].x);
-                v[i][e].y = blk_exp2(v[i][e].y);
+                v[i][e] = blk_mul2(blk_add2(v[i][e], nm), sl2);
+                sp_exp2(v[i][e]);
                 sum = blk_add2(sum, v[i][e]);
             }
         const float inv = 1.f / sp_sum(sum.x + sum.y, 32);
@@ -310,33 +336,62 @@ __device__ __forceinline__ void fwd_rows_vec(uint32_t piece, int rows, int cols,
         if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, x * inv);
     }
 }
-// forward, any column count that fits the window: three passes over the row, exponential evaluated twice.  The first
-// pass takes the extreme of the raw packed elements; the third folds the normalisation into the exponent.
-template <typename IO, int NW>
-__device__ __forceinline__ void fwd_rows_vec_streamed(uint32_t piece, int rows, int cols, float sl, int r0, int lane) {
+// forward, any column count that fits the window: three passes over the row, exponential evaluated twice.  NEAR, for rows
+// whose |m * sl| is at most sp_near: y = x * sl - m * sl in one fused operation.  The rounding of m * sl is then the same
+// for the whole row and cancels; for 16-bit elements, whose third pass takes the logarithm of the sum off as well instead
+// of multiplying by its inverse, it does not, but is at most 2^-18, a hundredth of the result's own.
+template <typename IO> __device__ __forceinline__ float sp_near() { return IO::VE == 8 ? 64.f : 1048576.f; }
+template <typename IO, bool NEAR>
+__device__ __forceinline__ void fwd_row_streamed(const RowSplit<IO>& rs, float x, float m, float sl, int lane) {
     constexpr int VP = IO::VE / 2;
+    constexpr bool FOLD = NEAR && IO::VE == 8;
     const float2 sl2 = make_float2(sl, sl);
+    float2 off = make_float2(NEAR ? -m * sl : -m, NEAR ? -m * sl : -m);
+    auto exps = [&](int vi, float2 (&f)[VP]) {
+        IO::unpack(sp_ldv(rs.body, vi), f);
+#pragma unroll
+        for (int e = 0; e < VP; ++e) {
+            f[e] = NEAR ? blk_fma2(f[e], sl2, off) : blk_mul2(blk_add2(f[e], off), sl2);
+            sp_exp2(f[e]);
+        }
+    };
+    auto extra = [&]() { return rs.xi >= 0 ? blk_exp2(NEAR ? fmaf(x, sl, off.x) : (x - m) * sl) : 0.f; };
+    float2 sum = make_float2(extra(), 0.f);
+    sp_each(rs.nv, lane, [&](int vi) {
+        float2 f[VP];
+        exps(vi, f);
+#pragma unroll
+        for (int e = 0; e < VP; ++e) sum = blk_add2(sum, f[e]);
+    });
+    const float total = sp_sum(sum.x + sum.y, 32);
+    float2 inv2 = make_float2(1.f, 1.f);
+    if (FOLD) off.x = off.y = off.x - __log2f(total);
+    else inv2.x = inv2.y = 1.f / total;
+    sp_each(rs.nv, lane, [&](int vi) {
+        float2 f[VP];
+        exps(vi, f);
+        if (!FOLD) {
+#pragma unroll
+            for (int e = 0; e < VP; ++e) f[e] = blk_mul2(f[e], inv2);
+        }
+        sp_stv(rs.body, vi, IO::pack(f));
+    });
+    if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, extra() * inv2.x);
+}
+// (out of line: the loops of the usual rows stay close together, 1.5 % of the 16-bit long rows)
+template <typename IO>
+__device__ __noinline__ void fwd_row_far(RowSplit<IO> rs, float x, float m, float sl, int lane) {
+    fwd_row_streamed<IO, false>(rs, x, m, sl, lane);
+}
+template <typename IO, bool NEG, int NW>
+__device__ __forceinline__ void fwd_rows_vec_streamed(uint32_t piece, int rows, int cols, float sl, int r0, int lane) {
 #pragma unroll 1
     for (int r = r0; r < rows; r += NW) {
-        RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
-        const float x = rs.xi >= 0 ? sp_ld<IO>(rs.row, rs.xi) * sl : -INFINITY;
-        const float ex = sl < 0.f ? sp_extreme<IO, true>(rs.body, rs.nv, lane) : sp_extreme<IO, false>(rs.body, rs.nv, lane);
-        const float mx = sp_max(fmaxf(x, lane < rs.nv ? ex * sl : -INFINITY), 32);
-        float2 sum = make_float2(blk_exp2(x - mx), 0.f);
-        float2 off = make_float2(-mx, -mx);
-        sp_each(rs.nv, lane, [&](int vi) {
-            float2 f[VP];
-            sp_exp<IO>(sp_ldv(rs.body, vi), sl2, off, f);
-#pragma unroll
-            for (int e = 0; e < VP; ++e) sum = blk_add2(sum, f[e]);
-        });
-        off.x = off.y = -mx - __log2f(sp_sum(sum.x + sum.y, 32));  // exp2(x * sl + off) = exp2(x * sl - max) / sum
-        sp_each(rs.nv, lane, [&](int vi) {
-            float2 f[VP];
-            sp_exp<IO>(sp_ldv(rs.body, vi), sl2, off, f);
-            sp_stv(rs.body, vi, IO::pack(f));
-        });
-        if (rs.xi >= 0) sp_st<IO>(rs.row, rs.xi, blk_exp2(x + off.x));
+        const RowSplit<IO> rs(piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E)), cols, lane);
+        const float x = sp_ld_if<IO, NEG>(rs.xi >= 0, rs.row, rs.xi);
+        const float m = sp_tops<NEG>(sp_top<NEG>(x, sp_extreme<IO, NEG>(rs.body, rs.nv, lane)), 32);
+        if (fabsf(m * sl) <= sp_near<IO>()) fwd_row_streamed<IO, true>(rs, x, m, sl, lane);
+        else fwd_row_far<IO>(rs, x, m, sl, lane);
     }
 }
 // backward over whole vectors, two passes (dot product, then the result over the gradient)
@@ -380,52 +435,55 @@ __device__ __forceinline__ void bwd_rows_vec(uint32_t ppiece, uint32_t gpiece, i
 // Short rows (fewer columns than eight vectors).  Up to 16 columns: one lane per row, no shuffle.  More: eight lanes per
 // row, which keeps the row in registers and every warp busy when a window is one long piece of short rows.
 constexpr int SP_LANE_COLS = 16;
-template <typename IO>
+template <typename IO, bool NEG>
 __device__ __noinline__ void fwd_rows_lane(uint32_t piece, int rows, int cols, float sl, int r, int lane) {
     r += lane;
     if (r >= rows) return;
     const uint32_t row = piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
-    float v[SP_LANE_COLS];
-    float mx = -INFINITY;
+    float2 v[SP_LANE_COLS / 2];
+    float m = sp_none<NEG>();
 #pragma unroll
-    for (int c = 0; c < SP_LANE_COLS; ++c) {
-        v[c] = c < cols ? sp_ld<IO>(row, c) * sl : -INFINITY;
-        mx = fmaxf(mx, v[c]);
+    for (int c = 0; c < SP_LANE_COLS / 2; ++c) {
+        v[c] = make_float2(sp_ld_if<IO, NEG>(2 * c < cols, row, 2 * c), sp_ld_if<IO, NEG>(2 * c + 1 < cols, row, 2 * c + 1));
+        m = sp_top3<NEG>(m, v[c].x, v[c].y);
     }
-    float sum = 0.f;
+    const float inv = 1.f / sp_exps(v, m, sl);
 #pragma unroll
-    for (int c = 0; c < SP_LANE_COLS; ++c) {
-        v[c] = blk_exp2(v[c] - mx);
-        sum += v[c];
+    for (int c = 0; c < SP_LANE_COLS / 2; ++c) {
+        if (2 * c < cols) sp_st<IO>(row, 2 * c, v[c].x * inv);
+        if (2 * c + 1 < cols) sp_st<IO>(row, 2 * c + 1, v[c].y * inv);
     }
-    const float inv = 1.f / sum;
-#pragma unroll
-    for (int c = 0; c < SP_LANE_COLS; ++c)
-        if (c < cols) sp_st<IO>(row, c, v[c] * inv);
 }
-template <typename IO>
+template <typename IO, bool NEG>
 __device__ __noinline__ void fwd_rows_group(uint32_t piece, int rows, int cols, float sl, int r, int lane) {
     r += lane >> 3;
     const int l = lane & 7;
     const uint32_t row = piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
-    float v[IO::VE];
-    float mx = -INFINITY;
+    const int have = r < rows ? cols - l : 0;  // this lane's elements are l, l + 8, ...
+    float2 v[IO::VE / 2];
+    float m = sp_none<NEG>();
 #pragma unroll
-    for (int i = 0; i < IO::VE; ++i) {
-        v[i] = r < rows && l + 8 * i < cols ? sp_ld<IO>(row, l + 8 * i) * sl : -INFINITY;
-        mx = fmaxf(mx, v[i]);
+    for (int i = 0; i < IO::VE / 2; ++i) {
+        v[i] = make_float2(sp_ld_if<IO, NEG>(16 * i < have, row, l + 16 * i), sp_ld_if<IO, NEG>(16 * i + 8 < have, row, l + 16 * i + 8));
+        m = sp_top3<NEG>(m, v[i].x, v[i].y);
     }
-    mx = sp_max(mx, 8);
+    m = sp_tops<NEG>(m, 8);
+    const float inv = 1.f / sp_sum(sp_exps(v, m, sl), 8);
+#pragma unroll
+    for (int i = 0; i < IO::VE / 2; ++i) {
+        if (16 * i < have) sp_st<IO>(row, l + 16 * i, v[i].x * inv);
+        if (16 * i + 8 < have) sp_st<IO>(row, l + 16 * i + 8, v[i].y * inv);
+    }
+}
+// row r by a lane, for a scale of zero: the above keep elements past a row's end out by an infinite y
+template <typename IO>
+__device__ __noinline__ void fwd_row_zero_scale(uint32_t piece, int cols, int r) {
+    const uint32_t row = piece + (uint32_t)(r * cols * (int)sizeof(typename IO::E));
     float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < IO::VE; ++i) {
-        v[i] = blk_exp2(v[i] - mx);
-        sum += v[i];
-    }
-    const float inv = 1.f / sp_sum(sum, 8);
-#pragma unroll
-    for (int i = 0; i < IO::VE; ++i)
-        if (r < rows && l + 8 * i < cols) sp_st<IO>(row, l + 8 * i, v[i] * inv);
+#pragma unroll 1
+    for (int c = 0; c < cols; ++c) sum += blk_exp2(sp_ld<IO>(row, c) * 0.f);
+#pragma unroll 1
+    for (int c = 0; c < cols; ++c) sp_st<IO>(row, c, blk_exp2(sp_ld<IO>(row, c) * 0.f) / sum);
 }
 template <typename IO>
 __device__ __forceinline__ void bwd_rows_lane(uint32_t ppiece, uint32_t gpiece, int rows, int cols,
@@ -464,22 +522,27 @@ __device__ __forceinline__ void bwd_rows_group(uint32_t ppiece, uint32_t gpiece,
 __device__ __forceinline__ int sp_unit_rows(int cols) { return cols <= SP_LANE_COLS ? 32 : 4; }
 
 // One piece: this warp's units -- rows, or groups of short rows -- are u, u + NW, ...
-template <typename IO, int NW>
+template <typename IO, bool NEG, int NW>
 __device__ __forceinline__ void fwd_piece(uint32_t srow, int rows, int cols, float sl, int u, int lane) {
     constexpr int VE = IO::VE;
     if (cols < 8 * VE) {
         const int ur = sp_unit_rows(cols);
 #pragma unroll 1
         for (int r = u * ur; r < rows; r += NW * ur) {
-            if (cols <= SP_LANE_COLS) fwd_rows_lane<IO>(srow, rows, cols, sl, r, lane);
-            else fwd_rows_group<IO>(srow, rows, cols, sl, r, lane);
+            if (!NEG && sl == 0.f) {
+                if (lane < ur && r + lane < rows) fwd_row_zero_scale<IO>(srow, cols, r + lane);
+            } else if (cols <= SP_LANE_COLS) {
+                fwd_rows_lane<IO, NEG>(srow, rows, cols, sl, r, lane);
+            } else {
+                fwd_rows_group<IO, NEG>(srow, rows, cols, sl, r, lane);
+            }
         }
         return;
     }
     const int nvmax = cols / VE;  // whole vectors of a row never exceed this
-    if (nvmax > 64 || sl == 0.f) fwd_rows_vec_streamed<IO, NW>(srow, rows, cols, sl, u, lane);
-    else if (nvmax <= 32) fwd_rows_vec<IO, 1, NW>(srow, rows, cols, sl, u, lane);
-    else fwd_rows_vec<IO, 2, NW>(srow, rows, cols, sl, u, lane);
+    if (nvmax > 64 || (!NEG && sl == 0.f)) fwd_rows_vec_streamed<IO, NEG, NW>(srow, rows, cols, sl, u, lane);
+    else if (nvmax <= 32) fwd_rows_vec<IO, NEG, 1, NW>(srow, rows, cols, sl, u, lane);
+    else fwd_rows_vec<IO, NEG, 2, NW>(srow, rows, cols, sl, u, lane);
 }
 template <typename IO, int NW>
 __device__ __forceinline__ void bwd_piece(uint32_t prow0, uint32_t grow0, int rows, int cols, float scale,
@@ -516,7 +579,7 @@ __device__ __forceinline__ float sp_cta_reduce(float v, bool is_max, float* red,
 struct SpWin {
     int64_t e0;   // its first element in the buffers
     int64_t off;  // ... inside the head strip
-    int nbytes, npieces, first_piece, pad;
+    int nbytes, npieces, first_piece;
 };
 
 // The (window, head) list of a CTA: window index and head of entry blockIdx.x, + gridDim.x, ...
@@ -541,12 +604,12 @@ struct SpWalk {
     }
     __device__ __forceinline__ SpWin load(const BlkSmxPipeParams& p) const {
         const BlkSmxWindow w = p.windows[idx];
-        return SpWin{(int64_t)head * p.D + w.off, w.off, w.nbytes, w.npieces, w.first_piece, 0};
+        return SpWin{(int64_t)head * p.D + w.off, w.off, w.nbytes, w.npieces, w.first_piece};
     }
 };
 
-// BWD = false: in0 = src, result = softmax; BWD = true: in0 = forward result, in1 = its gradient.
-template <typename IO, bool BWD>
+// BWD = false: in0 = src, result = softmax (NEG: of a negative scale); BWD = true: in0 = forward result, in1 = its gradient.
+template <typename IO, bool BWD, bool NEG>
 __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk_softmax_pipe_kernel(const BlkSmxPipeParams p) {
     typedef typename IO::E E;
     constexpr int ES = (int)sizeof(E);
@@ -658,14 +721,15 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
                 const int64_t e0 = win.e0;
                 constexpr int NT = 32 * NW;
                 if (!BWD) {
-                    float mx = -INFINITY;
-                    for (int c = tid; c < cols; c += NT) mx = fmaxf(mx, IO::ld(g0[e0 + c]) * sl);
-                    mx = sp_cta_reduce<NW>(mx, true, red, warp, lane);
+                    constexpr float SIGN = NEG ? -1.f : 1.f;
+                    float m = -INFINITY;
+                    for (int c = tid; c < cols; c += NT) m = fmaxf(m, SIGN * IO::ld(g0[e0 + c]));
+                    m = SIGN * sp_cta_reduce<NW>(m, true, red, warp, lane);
                     float sum = 0.f;
-                    for (int c = tid; c < cols; c += NT) sum += blk_exp2(IO::ld(g0[e0 + c]) * sl - mx);
+                    for (int c = tid; c < cols; c += NT) sum += blk_exp2((IO::ld(g0[e0 + c]) - m) * sl);
                     sum = sp_cta_reduce<NW>(sum, false, red, warp, lane);
                     const float inv = 1.f / sum;
-                    for (int c = tid; c < cols; c += NT) gd[e0 + c] = IO::st(blk_exp2(IO::ld(g0[e0 + c]) * sl - mx) * inv);
+                    for (int c = tid; c < cols; c += NT) gd[e0 + c] = IO::st(blk_exp2((IO::ld(g0[e0 + c]) - m) * sl) * inv);
                 } else {
                     float dot = 0.f;
                     for (int c = tid; c < cols; c += NT) dot += IO::ld(g0[e0 + c]) * IO::ld(g1[e0 + c]);
@@ -680,7 +744,7 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
                     const BlkSmxChunk pc = recs[st][pi];
                     const uint32_t eo = (uint32_t)(pc.off - win.off) * ES;
                     if (BWD) bwd_piece<IO, NW>(p0 + eo, r0 + eo, pc.rows, pc.cols, sl, first, lane);
-                    else fwd_piece<IO, NW>(r0 + eo, pc.rows, pc.cols, sl, first, lane);
+                    else fwd_piece<IO, NEG, NW>(r0 + eo, pc.rows, pc.cols, sl, first, lane);
                 };
                 auto units_of = [&](int pi) {
                     const BlkSmxChunk pc = recs[st][pi];
@@ -747,12 +811,14 @@ cudaError_t blk_launch_softmax_pipe(const BlkSmxPipeParams& p, int dtype, int ba
         kern<<<grid, block, smem, st>>>(p);
         return cudaGetLastError();
     };
-    if (!backward) {
-        if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, false>, 1, SpShape<false>{});
-        if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, false>, 1, SpShape<false>{});
-        return go(blk_softmax_pipe_kernel<SpIO32, false>, 1, SpShape<false>{});
-    }
-    if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, true>, 2, SpShape<true>{});
-    if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, true>, 2, SpShape<true>{});
-    return go(blk_softmax_pipe_kernel<SpIO32, true>, 2, SpShape<true>{});
+    auto forward = [&](auto io) {
+        typedef decltype(io) IO;
+        return p.scale < 0.f ? go(blk_softmax_pipe_kernel<IO, false, true>, 1, SpShape<false>{})
+                             : go(blk_softmax_pipe_kernel<IO, false, false>, 1, SpShape<false>{});
+    };
+    if (!backward)
+        return dtype == BLK_F16 ? forward(SpIO16<BlkHalfTag>{}) : dtype == BLK_BF16 ? forward(SpIO16<BlkBf16Tag>{}) : forward(SpIO32{});
+    if (dtype == BLK_F16) return go(blk_softmax_pipe_kernel<SpIO16<BlkHalfTag>, true, false>, 2, SpShape<true>{});
+    if (dtype == BLK_BF16) return go(blk_softmax_pipe_kernel<SpIO16<BlkBf16Tag>, true, false>, 2, SpShape<true>{});
+    return go(blk_softmax_pipe_kernel<SpIO32, true, false>, 2, SpShape<true>{});
 }

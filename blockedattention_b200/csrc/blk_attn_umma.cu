@@ -81,7 +81,7 @@ struct FL {
 struct FaItem {
     int4 side[2];  // per stream: keys N, tiles T (0: no such block), steps of the item = larger T, shared tiles
     int4 rows;     // rowQ, rowKV of stream A, of stream B
-    int4 misc;     // query rows M of A, of B, head, tiles of A | tiles of B << 16 (0: nothing follows)
+    int4 misc;     // query rows M of A (0: nothing follows), of B, head, tiles of B
 };
 constexpr int FA_ITEMS = 4;
 constexpr int FA_ITEM_READERS = 18;  // 2 producers, 4 MMA warps, 8 softmax warps, 4 output warps
@@ -118,7 +118,7 @@ struct FaWalk {
         ++item;
         __syncwarp();
         if ((threadIdx.x & 31) == 0) mbar_arrive(r.bar + 8u * (FA_ITEMS + s));
-        return m.w != 0;
+        return m.x != 0;
     }
     // To the next step (called before every step, the first one too).
     __device__ __forceinline__ bool step(const FaRing& r, int4* rows = nullptr, int4* misc = nullptr) {
@@ -338,7 +338,7 @@ blk_attn_umma_kernel(const BlkFlashParams p, const __grid_constant__ CUtensorMap
                 const uint32_t full = keys ? k_full(slot) : v_full(slot), dst = keys ? sK(slot) : sV(slot);
                 if (!(ok = mbar_wait(keys ? k_empty(slot) : v_empty(slot), ((n >> LOG_NS) & 1u) ^ 1u, abort_flag, 22))) break;
                 const int row = (i ? rows.w : rows.y) + wk.j * FA_BN;
-                const bool there = wk.j < (i ? misc.w >> 16 : misc.w & 0xffff);
+                const bool there = i ? wk.j < misc.w : wk.mine();
                 if (elect_one()) {
                     if (there) {
                         mbar_expect_tx(full, L::TILE_BYTES);
@@ -485,7 +485,7 @@ blk_attn_umma_kernel(const BlkFlashParams p, const __grid_constant__ CUtensorMap
                 it->side[0] = make_int4(a.w, Ta, steps, shared);
                 it->side[1] = make_int4(b.w, Tb, steps, shared);
                 it->rows = make_int4(a.x, a.y, b.x, b.y);
-                it->misc = make_int4(a.z, b.z, (int)(n - q * (uint32_t)p.H), more ? (Ta | Tb << 16) : 0);
+                it->misc = make_int4(a.z, b.z, (int)(n - q * (uint32_t)p.H), Tb);
                 mbar_arrive(ring.bar + 8u * s);  // release: the record is visible to whoever sees the phase end
             }
             __syncwarp();

@@ -149,3 +149,29 @@ def test_attention_very_long_key_sweep_and_single_query(cuda_device):
         plan.run(q.to(dev), k.to(dev), v.to(dev), out=out, scale=0.09)
         plan.check()
     close(out, oracle_attention(q, k, v, M, N, d, 0.09), BF16, "attention, very long key sweep")
+
+
+def test_attention_over_millions_of_keys(cuda_device):
+    # a pair of blocks whose key sweeps have more tiles of 64 than 15 and 16 bits hold: every tile must be loaded, the last
+    # ones above all -- each long segment's answer is the value of a key near its end that dwarfs the others
+    dev, d, scale = cuda_device, 64, 0.125
+    N = np.array([(1 << 22) + 70, (1 << 21) + 1] + [70] * 160)   # enough short segments for the blocks to be paired
+    M = np.array([1, 1] + [1] * 160)
+    g = torch.Generator(device=dev).manual_seed(2)
+    q, k, v = (torch.randn((1, int(n) * d), generator=g, device=dev, dtype=torch.float32).to(F16)
+               for n in (M.sum(), N.sum(), N.sum()))
+    first = 0
+    for s, late in ((0, (1 << 22) + 60), (1, 1 << 21)):
+        at = first + late
+        k[0, at * d:(at + 1) * d] = 3.0 * q[0, s * d:(s + 1) * d]
+        first += int(N[s])
+    plan = AttentionPlan(M, N, 1, F16, device=dev, d=d)
+    got = plan.run(q, k, v, scale=scale)
+    plan.check()
+    first = 0
+    for s in range(len(M)):
+        n = int(N[s])
+        K, V = (t[0, first * d:(first + n) * d].reshape(n, d).float() for t in (k, v))
+        p = torch.softmax(scale * (K @ q[0, s * d:(s + 1) * d].float()).double(), 0)
+        close(got[0, s * d:(s + 1) * d], (p.float() @ V).cpu(), F16, f"segment {s}")
+        first += n

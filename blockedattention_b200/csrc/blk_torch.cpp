@@ -9,6 +9,10 @@
 // read to the host once and remembered while it is alive (a bounded number of them; the memo holds the tensor, so its
 // address cannot come back with other values, and an in-place write moves its version).  Lists on the host (numpy
 // arrays, CPU tensors, sequences) are compared by value on every call.
+//
+// An operator holds the lock of Python while it looks at its arguments and lets go of it for everything after: reading a
+// list from the GPU, creating and releasing plans and a full launch queue all wait for the device, and the process's other
+// threads must not wait with them.
 #include <Python.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -50,6 +54,15 @@ inline void ok(int rc) {
     if (rc != BLK_OK) throw BlkFailure(rc, blk_last_error());
 }
 
+// The lock of Python, let go of for a scope.
+struct NoGil {
+    PyThreadState* state;
+    NoGil() : state(PyEval_SaveThread()) {}
+    ~NoGil() { PyEval_RestoreThread(state); }
+    NoGil(const NoGil&) = delete;
+    NoGil& operator=(const NoGil&) = delete;
+};
+
 int dtype_code(at::ScalarType t) {
     switch (t) {
         case at::kHalf: return BLK_F16;
@@ -80,7 +93,7 @@ uint64_t hash_values(const int64_t* p, size_t n) {
     return r ^ (r >> 31);
 }
 
-std::mutex g_mu;  // guards the tables below (calls from Python hold the GIL, backward passes do not)
+std::mutex g_mu;  // guards the tables below; no plan or tensor is released and nothing of Python called while it is held
 
 // Interned values.  Owners are plans and the memo of GPU list tensors; expired entries are swept as the table grows.
 struct Interned {
@@ -190,9 +203,16 @@ struct PyRef {
 PyObject* g_host_i64 = nullptr;  // plan._host_i64: any sequence -> contiguous int64 numpy array
 PyObject* g_error = nullptr;     // _lib.BlkError
 
-ListP list_of(PyObject* o) {
-    if (o == Py_None) return nullptr;
-    if (THPVariable_Check(o)) return list_of_tensor(THPVariable_Unpack(o));
+// A list argument: the values, or the tensor they are to be read from (both unset for None).
+struct ListArg {
+    ListP values;
+    Tensor tensor;
+    explicit operator bool() const { return values || tensor.defined(); }
+    ListP read() const { return tensor.defined() ? list_of_tensor(tensor) : values; }
+};
+ListArg list_of(PyObject* o) {
+    if (o == Py_None) return {};
+    if (THPVariable_Check(o)) return {nullptr, THPVariable_Unpack(o)};
     auto from_buffer = [](PyObject* x, ListP* out) -> bool {
         Py_buffer b;
         if (PyObject_GetBuffer(x, &b, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) != 0) {
@@ -208,11 +228,11 @@ ListP list_of(PyObject* o) {
         return is64;
     };
     ListP l;
-    if (PyObject_CheckBuffer(o) && from_buffer(o, &l)) return l;
+    if (PyObject_CheckBuffer(o) && from_buffer(o, &l)) return {l, {}};
     PyRef arr(PyObject_CallFunctionObjArgs(g_host_i64, o, nullptr));
     if (!arr.o) throw python_error();
     TORCH_CHECK(from_buffer(arr.o, &l), "a list or offset argument cannot be read as int64 values");
-    return l;
+    return {l, {}};
 }
 
 // ---- plans -------------------------------------------------------------------------------------------
@@ -227,7 +247,14 @@ struct Plan {
     // plans of the backward pass and of compositions, made when first needed; index: purpose, type
     std::shared_ptr<Plan> derived[5][3];
     ~Plan() {
-        if (h) blk_plan_destroy(h);
+        if (!h) return;
+        // (the last owner may be an autograd node that Python releases; freeing device memory waits for the device)
+        if (Py_IsInitialized() && PyGILState_Check()) {
+            NoGil free;
+            blk_plan_destroy(h);
+        } else {
+            blk_plan_destroy(h);
+        }
     }
     void extents() { ok(blk_plan_extents(h, &Dm1, &Dm2, &Dout)); }
     void check(cudaStream_t st) const {
@@ -568,6 +595,7 @@ Tensor attention_op(const PlanP& p, const Tensor& q, const Tensor& k, const Tens
 }
 
 // ---- the operators -----------------------------------------------------------------------------------
+// (the caller holds the argument, and with it the tensor, until the operator returns)
 const Tensor& operand(const char* name, PyObject* o) {
     TORCH_CHECK(THPVariable_Check(o), name, " must be CUDA Tensor");
     const Tensor& t = THPVariable_Unpack(o);
@@ -616,11 +644,14 @@ Tensor py_gemm(PyObject* const* a) {
     const bool ta = as_bool(a[8]), tb = as_bool(a[9]), softmax = as_bool(a[12]);
     const double scale = as_double(a[10]);
     const auto dt = mat1.scalar_type(), odt = as_dtype(a[11], mat1.scalar_type());
-    ListP l[6];
+    ListArg given[6];
     if (have_lists)
-        for (int i = 0; i < 3; ++i) l[i] = list_of(a[5 + i]);
+        for (int i = 0; i < 3; ++i) given[i] = list_of(a[5 + i]);
     if (have_acc)
-        for (int i = 0; i < 3; ++i) l[3 + i] = list_of(a[2 + i]);
+        for (int i = 0; i < 3; ++i) given[3 + i] = list_of(a[2 + i]);
+    const NoGil free;
+    ListP l[6];
+    for (int i = 0; i < 6; ++i) l[i] = given[i].read();
     PlanKey key{0, (int)dt, (int)odt, (int)ta | (int)tb << 1 | (int)softmax << 2, (int)mat1.get_device(), 0, mat1.numel(), {}};
     for (int i = 0; i < 6; ++i) key.l[i] = l[i].get();
     PlanP p = plan_for(key, [&]() {
@@ -654,8 +685,15 @@ Tensor py_gemm(PyObject* const* a) {
 Tensor py_softmax(PyObject* const* a) {
     const Tensor& src = operand("src", a[0]);
     TORCH_CHECK(a[1] != Py_None && a[2] != Py_None, "blockSoftmax needs rowList and colList");
-    ListP l[3] = {list_of(a[1]), list_of(a[2]), list_of(a[3])};
+    const ListArg given[3] = {list_of(a[1]), list_of(a[2]), list_of(a[3])};
     const double scale = as_double(a[4]);
+    Tensor out;
+    if (a[5] != Py_None) {
+        TORCH_CHECK(THPVariable_Check(a[5]), "out must be a contiguous CUDA tensor shaped like src");
+        out = THPVariable_Unpack(a[5]);
+    }
+    const NoGil free;
+    const ListP l[3] = {given[0].read(), given[1].read(), given[2].read()};
     const auto dt = src.scalar_type();
     PlanKey key{1, (int)dt, (int)dt, 0, (int)src.get_device(), 0, src.numel(), {l[0].get(), l[1].get(), l[2].get()}};
     PlanP p = plan_for(key, [&]() {
@@ -667,18 +705,14 @@ Tensor py_softmax(PyObject* const* a) {
         for (int i = 0; i < 3; ++i) made->lists[i] = l[i];
         return made;
     });
-    if (a[5] != Py_None) {
-        TORCH_CHECK(THPVariable_Check(a[5]), "out must be a contiguous CUDA tensor shaped like src");
-        const Tensor& out = THPVariable_Unpack(a[5]);
-        return run_softmax(*p, src.detach(), &out, scale);
-    }
+    if (out.defined()) return run_softmax(*p, src.detach(), &out, scale);
     if (!(at::GradMode::is_enabled() && src.requires_grad())) return run_softmax(*p, src, nullptr, scale);
     auto node = new_node<BlockSoftmaxBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(src));
     node->plan = p;
     node->scale = scale;
     node->shape = src.sizes().vec();
-    Tensor out = run_softmax(*p, src.detach(), nullptr, scale);
+    out = run_softmax(*p, src.detach(), nullptr, scale);
     torch::autograd::set_history(out, node);
     node->result_ = SavedVariable(out, true);
     return out;
@@ -718,17 +752,20 @@ PlanP attention_plan(const ListP& M, const ListP& N, int64_t numel_q, int64_t d,
 // attention(q, k, v, MList, NList, scale, d)
 Tensor py_attention(PyObject* const* a) {
     const Tensor &q = operand("q", a[0]), &k = operand("k", a[1]), &v = operand("v", a[2]);
-    const ListP M = list_of(a[3]), N = list_of(a[4]);
-    TORCH_CHECK(M && N, "blockAttention needs MList and NList");
+    const ListArg m_list = list_of(a[3]), n_list = list_of(a[4]);
+    TORCH_CHECK(m_list && n_list, "blockAttention needs MList and NList");
     const double scale = as_double(a[5]);
+    const bool have_d = a[6] != Py_None;
     int64_t d = 0;
-    if (a[6] != Py_None) {
+    if (have_d) {
         d = PyLong_AsLongLong(a[6]);
         if (d == -1 && PyErr_Occurred()) throw python_error();
     }
+    const NoGil free;
+    const ListP M = m_list.read(), N = n_list.read();
     const int64_t rows_q = sum(M->v), rows_kv = sum(N->v);
     TORCH_CHECK(rows_q > 0 && rows_kv > 0, "blockAttention needs at least one query row and one key row");
-    if (a[6] == Py_None) {
+    if (!have_d) {
         // a (H, sum m_s * d) tensor tells d by its last extent; a flat one cannot (d and H only appear as a product)
         TORCH_CHECK(q.dim() >= 2 && q.size(-1) % rows_q == 0,
                     "give the head dimension d (a flat tensor cannot tell it apart from the number of heads)");
@@ -757,9 +794,11 @@ Tensor py_attention_token_major(PyObject* const* a) {
     const Tensor &q = operand("q", a[0]), &k = operand("k", a[1]), &v = operand("v", a[2]);
     TORCH_CHECK(q.dim() == 3 && q.sizes() == k.sizes() && q.sizes() == v.sizes() && (q.size(2) == 64 || q.size(2) == 128),
                 "q, k and v must all have shape (sum n, H, d), d 64 or 128");
-    const ListP n = list_of(a[3]);
-    TORCH_CHECK(n, "blockAttentionTokenMajor needs nList");
+    const ListArg n_list = list_of(a[3]);
+    TORCH_CHECK(n_list, "blockAttentionTokenMajor needs nList");
     const double scale = as_double(a[4]);
+    const NoGil free;
+    const ListP n = n_list.read();
     const auto dt = q.scalar_type();
     // the number of heads comes from the shape, not from the element count: the plan is made for H * sum(n) * d elements
     const int64_t rows = sum(n->v);
@@ -774,11 +813,13 @@ Tensor py_attention_token_major(PyObject* const* a) {
 Tensor py_scores_token_major(PyObject* const* a) {
     const Tensor &q = operand("q", a[0]), &k = operand("k", a[1]);
     TORCH_CHECK(q.dim() == 3 && q.sizes() == k.sizes(), "q and k must both have shape (sum n, H, d)");
-    const ListP n = list_of(a[2]);
-    TORCH_CHECK(n, "blockAttnScoresTokenMajor needs nList");
+    const ListArg n_list = list_of(a[2]);
+    TORCH_CHECK(n_list, "blockAttnScoresTokenMajor needs nList");
     const double scale = as_double(a[3]);
     const auto dt = q.scalar_type(), odt = as_dtype(a[4], dt);
     const bool softmax = as_bool(a[5]);
+    const NoGil free;
+    const ListP n = n_list.read();
     const int64_t H = q.size(1), d = q.size(2);
     PlanKey key{3, (int)dt, (int)odt, (int)softmax, (int)q.get_device(), (int)d, H, {n.get()}};
     const PlanP p = plan_for(key, [&]() {
@@ -816,9 +857,10 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 PyObject* py_clear(PyObject*, PyObject*) {
-    std::vector<PlanP> p;
-    std::vector<Remembered> r;
     {
+        const NoGil free;
+        std::vector<PlanP> p;
+        std::vector<Remembered> r;
         std::lock_guard<std::mutex> g(g_mu);
         plans().clear(&p);
         device_lists().clear(&r);
@@ -840,6 +882,7 @@ PyObject* py_check(PyObject*, PyObject*) {
         }
     }
     try {
+        const NoGil free;
         for (const PlanP& p : all) {
             if (!p->h) continue;
             c10::cuda::CUDAGuard guard(p->device);

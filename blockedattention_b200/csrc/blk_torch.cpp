@@ -32,7 +32,6 @@
 #include <list>
 #include <memory>
 #include <mutex>
-#include <stdexcept>
 #include <string>
 #include <unordered_map>
 #include <utility>
@@ -44,16 +43,6 @@ namespace {
 
 using at::Tensor;
 
-// A failed library call; becomes blockedattention_b200._lib.BlkError at the Python boundary.
-struct BlkFailure : std::runtime_error {
-    int code;
-    BlkFailure(int c, const char* msg) : std::runtime_error("libblkattn error " + std::to_string(c) + ": " + msg), code(c), text(msg) {}
-    std::string text;
-};
-inline void ok(int rc) {
-    if (rc != BLK_OK) throw BlkFailure(rc, blk_last_error());
-}
-
 // The lock of Python, let go of for a scope.
 struct NoGil {
     PyThreadState* state;
@@ -62,6 +51,35 @@ struct NoGil {
     NoGil(const NoGil&) = delete;
     NoGil& operator=(const NoGil&) = delete;
 };
+
+struct PyRef {
+    PyObject* o;
+    explicit PyRef(PyObject* x) : o(x) {}
+    ~PyRef() { Py_XDECREF(o); }
+    PyRef(const PyRef&) = delete;
+    PyRef& operator=(const PyRef&) = delete;
+};
+
+PyObject* g_host_i64 = nullptr;  // plan._host_i64: any sequence -> contiguous int64 numpy array
+PyObject* g_error = nullptr;     // _lib.BlkError
+
+// A failed library call: blockedattention_b200._lib.BlkError, whatever thread it happens on -- the caller of an operator
+// gets it from the entry below, the caller of a backward pass from torch's engine.
+[[noreturn]] void fail(int code) {
+    const std::string text = blk_last_error();
+    const PyGILState_STATE held = PyGILState_Ensure();
+    {
+        PyRef err(PyObject_CallFunction(g_error, "is", code, text.c_str()));
+        if (err.o) PyErr_SetObject(g_error, err.o);
+    }
+    python_error e;
+    e.persist();
+    PyGILState_Release(held);
+    throw e;
+}
+inline void ok(int rc) {
+    if (rc != BLK_OK) fail(rc);
+}
 
 int dtype_code(at::ScalarType t) {
     switch (t) {
@@ -191,17 +209,6 @@ ListP list_of_tensor(const Tensor& t) {
     if (remember && !device_lists().find(key)) device_lists().put(key, Remembered{t, l}, &dropped);
     return l;
 }
-
-struct PyRef {
-    PyObject* o;
-    explicit PyRef(PyObject* x) : o(x) {}
-    ~PyRef() { Py_XDECREF(o); }
-    PyRef(const PyRef&) = delete;
-    PyRef& operator=(const PyRef&) = delete;
-};
-
-PyObject* g_host_i64 = nullptr;  // plan._host_i64: any sequence -> contiguous int64 numpy array
-PyObject* g_error = nullptr;     // _lib.BlkError
 
 // A list argument: the values, or the tensor they are to be read from (both unset for None).
 struct ListArg {
@@ -846,13 +853,7 @@ template <Tensor (*F)(PyObject* const*), int NARGS>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     TORCH_CHECK(n == NARGS, "expected ", NARGS, " arguments");
-    try {
-        return THPVariable_Wrap(F(args));
-    } catch (const BlkFailure& e) {
-        PyRef err(PyObject_CallFunction(g_error, "is", e.code, e.text.c_str()));
-        if (err.o) PyErr_SetObject(g_error, err.o);
-        return nullptr;
-    }
+    return THPVariable_Wrap(F(args));
     END_HANDLE_TH_ERRORS
 }
 
@@ -881,17 +882,13 @@ PyObject* py_check(PyObject*, PyObject*) {
                     if (q) all.push_back(q);
         }
     }
-    try {
+    {
         const NoGil free;
         for (const PlanP& p : all) {
             if (!p->h) continue;
             c10::cuda::CUDAGuard guard(p->device);
             p->check(stream_of(p->device));
         }
-    } catch (const BlkFailure& e) {
-        PyRef err(PyObject_CallFunction(g_error, "is", e.code, e.text.c_str()));
-        if (err.o) PyErr_SetObject(g_error, err.o);
-        return nullptr;
     }
     Py_RETURN_NONE;
     END_HANDLE_TH_ERRORS

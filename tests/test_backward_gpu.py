@@ -148,3 +148,24 @@ def test_fused_attention_backward(cuda_device, d, sizes):
         s = max(1.0, float(want.abs().max()))
         err = float((got.float().cpu() - want.float()).abs().max())
         assert err <= 1e-2 * s, f"{name}: max abs err {err} (scale {s})"
+
+
+def test_library_errors_of_a_backward_pass_keep_their_class(cuda_device, monkeypatch):
+    # the gradient's own launch gives up a bounded wait (see test_timeout_gpu.py): the caller of backward() must get the
+    # same BlkError with its code as the caller of an operator
+    from blockedattention_b200 import _lib as L
+    dev, n = cuda_device, np.array([200, 136])
+    k = np.array([64, 64])
+    a = torch.randn((1, int((n * k).sum())), device=dev).half().requires_grad_()
+    b = torch.randn((1, int((n * k).sum())), device=dev).half()          # stored (k, n): the gradient of a is a plain product
+    out = blockGEMM(a, b, None, None, None, n, n, k, False, True)
+    g = torch.randn_like(out)
+    monkeypatch.setenv("BLK_CHECK", "1")
+    monkeypatch.setenv("BLK_TEST_STALL_PRODUCER", "1")
+    with pytest.raises(L.BlkError) as e:
+        out.backward(g, retain_graph=True)
+    assert e.value.code == L.BLK_ERR_TIMEOUT
+    monkeypatch.delenv("BLK_TEST_STALL_PRODUCER")
+    out.backward(g)
+    want = O.block_gemm_backward(a.detach().cpu(), b.cpu(), g.cpu(), n, n, k, transpose2=True)[0]
+    close(a.grad, want, F16, "mat1 grad after a failed pass")

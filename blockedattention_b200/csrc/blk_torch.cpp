@@ -545,9 +545,12 @@ Tensor gemm_op(const PlanP& p, const Tensor& mat1, const Tensor& mat2, double sc
     return out;
 }
 
-// The backward kernels recompute the probabilities: segments beyond 64 x 64 from the saved row logarithms.
+// The backward kernels recompute the probabilities: segments beyond 64 x 64 from the saved row logarithms.  These want the
+// result as well, which the caller may have written to since (a residual added in place): it is then computed again.
 struct BlockAttentionBackward : public Node {
     SavedVariable q_, k_, v_, out_, lse_;
+    c10::VariableVersion out_version;
+    uint32_t out_saved = 0;
     PlanP plan;
     double scale = 1.0;
     std::string name() const override { return "BlockAttentionBackward"; }
@@ -562,7 +565,9 @@ struct BlockAttentionBackward : public Node {
         variable_list res(3);
         if (!grads[0].defined()) return res;
         const Plan& p = *plan;
-        const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), out = out_.unpack(shared_from_this()), lse = lse_.unpack();
+        const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), lse = lse_.unpack();
+        const Tensor out = out_version.current_version() == out_saved ? out_.unpack(shared_from_this())
+                                                                      : run_attention(p, q, k, v, scale, false);
         const Tensor go = to_type(grads[0].contiguous(), q.scalar_type());
         TORCH_CHECK(go.numel() == q.numel(), "the gradient does not match the attention result");
         c10::cuda::CUDAGuard guard(p.device);
@@ -597,6 +602,8 @@ Tensor attention_op(const PlanP& p, const Tensor& q, const Tensor& k, const Tens
     Tensor out = run_attention(*p, q.detach(), k.detach(), v.detach(), scale, false, &lse);
     torch::autograd::set_history(out, node);
     node->out_ = SavedVariable(out, true);
+    node->out_version = torch::autograd::impl::version_counter(out);
+    node->out_saved = node->out_version.current_version();
     node->lse_ = SavedVariable(lse, false);
     return out;
 }

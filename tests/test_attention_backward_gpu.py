@@ -52,3 +52,18 @@ def test_attention_backward_edges(cuda_device, dtype, d, m, n, scale):
         rel = float((a.double() - b).norm() / b.norm())
         worst = float((a.double() - b).abs().max() / b.abs().max())
         assert rel <= tol and worst <= tol, f"{name}: rel {rel}, max {worst}"
+
+
+@pytest.mark.parametrize("m,n", [([20, 64], [33, 7]), ([200, 30], [70, 300])])
+def test_attention_result_changed_in_place_before_backward(cuda_device, m, n):
+    # a residual added to the result in place: the gradients are those of the same sum made out of place
+    d, H = 64, 2
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    q, k, v, r = (torch.randn((H, sum(t) * d), generator=g, device=cuda_device).to(F16) for t in (m, n, n, m))
+    grads = []
+    for inplace in (False, True):
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        out = blockAttention(*leaves, np.array(m), np.array(n), scale=0.1, d=d)
+        out = out.mul_(2.0).add_(r) if inplace else out * 2.0 + r
+        grads.append(torch.autograd.grad(out, leaves, r))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))

@@ -373,9 +373,17 @@ inline void after_run(const Plan& p, cudaStream_t st) {
     if (e && e[0] && std::strcmp(e, "0") != 0) p.check(st);
 }
 
+// What a kernel is about to read through a raw pointer: looked at before every run, since an operand of a backward pass may
+// come from a saved-tensor hook of the caller's.
+void check_input(const char* name, const Tensor& t, at::ScalarType dt, int64_t H, int64_t D) {
+    check_operand(name, t);
+    TORCH_CHECK(t.scalar_type() == dt, name, " has dtype ", t.scalar_type(), ", the plan was built for ", dt);
+    TORCH_CHECK(t.numel() == H * D, name, " has ", t.numel(), " elements, expected H*D = ", H, "*", D);
+}
+
 Tensor run_gemm(const Plan& p, const Tensor& m1, const Tensor& m2, double scale) {
-    TORCH_CHECK(m1.numel() == p.H * p.Dm1, "mat1 has ", m1.numel(), " elements, expected H*D = ", p.H, "*", p.Dm1);
-    TORCH_CHECK(m2.numel() == p.H * p.Dm2, "mat2 has ", m2.numel(), " elements, expected H*D = ", p.H, "*", p.Dm2);
+    check_input("mat1", m1, p.dt, p.H, p.Dm1);
+    check_input("mat2", m2, p.dt, p.H, p.Dm2);
     c10::cuda::CUDAGuard guard(p.device);
     const Tensor a = aligned(m1), b = aligned(m2);
     Tensor out = empty2(p.H, p.Dout, p.odt, p.device);
@@ -386,7 +394,7 @@ Tensor run_gemm(const Plan& p, const Tensor& m1, const Tensor& m2, double scale)
 }
 
 Tensor run_softmax(const Plan& p, const Tensor& src, const Tensor* into, double scale) {
-    TORCH_CHECK(src.numel() == p.H * p.Dm1, "src has ", src.numel(), " elements, expected H*D = ", p.H, "*", p.Dm1);
+    check_input("src", src, p.dt, p.H, p.Dm1);
     Tensor out;
     c10::cuda::CUDAGuard guard(p.device);
     if (into) {
@@ -405,8 +413,8 @@ Tensor run_softmax(const Plan& p, const Tensor& src, const Tensor* into, double 
 }
 
 Tensor run_softmax_backward(const Plan& p, const Tensor& result, const Tensor& grad, double scale) {
-    TORCH_CHECK(result.numel() == p.H * p.Dm1 && grad.numel() == p.H * p.Dm1,
-                "the gradient must have the softmax result's number of elements");
+    check_input("the softmax result", result, p.dt, p.H, p.Dm1);
+    check_input("the gradient", grad, p.dt, p.H, p.Dm1);
     c10::cuda::CUDAGuard guard(p.device);
     const Tensor r = aligned(result), g = aligned(grad);
     Tensor out = empty2(p.H, p.Dm1, p.dt, p.device);
@@ -418,6 +426,9 @@ Tensor run_softmax_backward(const Plan& p, const Tensor& result, const Tensor& g
 
 Tensor run_attention(const Plan& p, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool tokens,
                      Tensor* lse = nullptr) {
+    check_input("q", q, p.dt, p.H, p.rows_q * p.d);
+    check_input("k", k, p.dt, p.H, p.rows_kv * p.d);
+    check_input("v", v, p.dt, p.H, p.rows_kv * p.d);
     c10::cuda::CUDAGuard guard(p.device);
     const Tensor a = aligned(q), b = aligned(k), c = aligned(v);
     cudaStream_t st = stream_of(p.device);
@@ -565,19 +576,24 @@ struct BlockAttentionBackward : public Node {
         variable_list res(3);
         if (!grads[0].defined()) return res;
         const Plan& p = *plan;
-        const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), lse = lse_.unpack();
-        const Tensor out = out_version.current_version() == out_saved ? out_.unpack(shared_from_this())
+        const Tensor q = to_type(q_.unpack(), p.dt), k = to_type(k_.unpack(), p.dt), v = to_type(v_.unpack(), p.dt);
+        const Tensor out = out_version.current_version() == out_saved ? to_type(out_.unpack(shared_from_this()), p.dt)
                                                                       : run_attention(p, q, k, v, scale, false);
-        const Tensor go = to_type(grads[0].contiguous(), q.scalar_type());
-        TORCH_CHECK(go.numel() == q.numel(), "the gradient does not match the attention result");
-        c10::cuda::CUDAGuard guard(p.device);
-        const Tensor a = aligned(q), b = aligned(k), c = aligned(v), g = aligned(go);
+        const Tensor lse = lse_.unpack(), go = to_type(grads[0].contiguous(), p.dt);
         const int64_t nq = p.rows_q * p.d, nkv = p.rows_kv * p.d;
+        check_input("q", q, p.dt, p.H, nq);
+        check_input("k", k, p.dt, p.H, nkv);
+        check_input("v", v, p.dt, p.H, nkv);
+        check_input("the attention result", out, p.dt, p.H, nq);
+        check_input("the row statistics", lse, at::kFloat, p.H, p.rows_q);
+        check_input("the gradient", go, p.dt, p.H, nq);
+        c10::cuda::CUDAGuard guard(p.device);
+        const Tensor a = aligned(q), b = aligned(k), c = aligned(v), o = aligned(out), l = aligned(lse), g = aligned(go);
         Tensor work = empty2(p.H, p.rows_q, at::kFloat, p.device);
         Tensor dq = empty2(p.H, nq, p.dt, p.device), dk = empty2(p.H, nkv, p.dt, p.device), dv = empty2(p.H, nkv, p.dt, p.device);
         cudaStream_t st = stream_of(p.device);
-        ok(blk_attention_backward_run(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), out.data_ptr(),
-                                      static_cast<const float*>(lse.data_ptr()), g.data_ptr(), static_cast<float*>(work.data_ptr()),
+        ok(blk_attention_backward_run(p.h, a.data_ptr(), b.data_ptr(), c.data_ptr(), o.data_ptr(),
+                                      static_cast<const float*>(l.data_ptr()), g.data_ptr(), static_cast<float*>(work.data_ptr()),
                                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (float)scale, st));
         after_run(p, st);
         res[0] = dq.reshape(q.sizes());

@@ -169,3 +169,43 @@ def test_library_errors_of_a_backward_pass_keep_their_class(cuda_device, monkeyp
     out.backward(g)
     want = O.block_gemm_backward(a.detach().cpu(), b.cpu(), g.cpu(), n, n, k, transpose2=True)[0]
     close(a.grad, want, F16, "mat1 grad after a failed pass")
+
+
+def _attention(q, k, v, n, d):
+    return blockAttention(q, k, v, n, n, scale=0.1, d=d)
+
+
+@pytest.mark.parametrize("op", ["gemm", "scores", "softmax", "attention"])
+def test_saved_tensor_hooks(cuda_device, op):
+    # what a hook hands back is checked before a kernel reads it: another type is converted, a tensor on the host, of
+    # another size or not contiguous is refused (all of these on purpose do not reach a launch)
+    dev, d, n = cuda_device, 64, np.array([40, 100])
+    D, kl = int((n * 64).sum()), np.array([64, 64])
+    S = int((n * n).sum())
+    call, sizes = {"gemm": (lambda a, b: blockGEMM(a, b, None, None, None, n, n, kl), (D, D)),
+                   "scores": (lambda a, b: blockAttnScores(a, b, n, n, kl), (D, D)),
+                   "softmax": (lambda a: blockSoftmax(a, n, n), (S,)),
+                   "attention": (lambda a, b, c: _attention(a, b, c, n, d), (D, D, D))}[op]
+    g = torch.Generator(device=dev).manual_seed(4)
+    base = [(torch.randn((2, s), generator=g, device=dev) * 0.3).half() for s in sizes]
+    go = None
+
+    def grads(pack, unpack):
+        nonlocal go
+        leaves = [t.clone().requires_grad_(True) for t in base]
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = call(*leaves)
+        if go is None:
+            go = (torch.randn(out.shape, generator=g, device=dev)).half()
+        return torch.autograd.grad(out, leaves, go)
+
+    same = lambda x: x
+    want = grads(same, same)
+    for pack, unpack in ((lambda x: x.cpu(), lambda x: x.to(dev)), (same, lambda x: x.double().to(x.dtype)),
+                         (same, lambda x: x.float() if x.dtype == F16 else x)):
+        assert all(torch.equal(a, b) for a, b in zip(grads(pack, unpack), want))
+    for unpack in (lambda x: x.cpu(), lambda x: x[:, :-8], lambda x: x[:1], lambda x: torch.cat([x, x], 1)[:, ::2],
+                   lambda x: torch.stack([x, x], -1)[..., 0]):
+        with pytest.raises(RuntimeError):
+            grads(same, unpack)
+    assert all(torch.equal(a, b) for a, b in zip(grads(same, same), want))

@@ -29,6 +29,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <list>
 #include <memory>
 #include <mutex>
@@ -458,6 +459,18 @@ std::shared_ptr<N> new_node() {
     return std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
 }
 
+// Whether a call records a node for its backward pass.  The nodes have no forward-mode derivative: a tangent is refused, as
+// torch.autograd.Function refuses it, not dropped.
+bool recorded(std::initializer_list<const Tensor*> operands) {
+    bool any = false;
+    if (at::GradMode::is_enabled())
+        for (const Tensor* t : operands) any = any || t->requires_grad();
+    if (any)
+        for (const Tensor* t : operands)
+            TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(0).defined(), "the blocked operators have no forward-mode derivative");
+    return any;
+}
+
 Tensor to_type(const Tensor& t, at::ScalarType s) { return t.scalar_type() == s ? t : t.to(s); }
 
 // The two launches of upstream sparseBlockedGEMM::backward (csrc/sparseBlockedAttention.cpp:52-72):
@@ -543,7 +556,7 @@ struct BlockSoftmaxBackward : public Node {
 };
 
 Tensor gemm_op(const PlanP& p, const Tensor& mat1, const Tensor& mat2, double scale) {
-    if (!(at::GradMode::is_enabled() && (mat1.requires_grad() || mat2.requires_grad()))) return run_gemm(*p, mat1, mat2, scale);
+    if (!recorded({&mat1, &mat2})) return run_gemm(*p, mat1, mat2, scale);
     auto node = new_node<BlockGEMMBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(mat1, mat2));
     node->plan = p;
@@ -604,8 +617,7 @@ struct BlockAttentionBackward : public Node {
 };
 
 Tensor attention_op(const PlanP& p, const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
-    if (!(at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())))
-        return run_attention(*p, q, k, v, scale, false);
+    if (!recorded({&q, &k, &v})) return run_attention(*p, q, k, v, scale, false);
     auto node = new_node<BlockAttentionBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
     node->plan = p;
@@ -736,7 +748,7 @@ Tensor py_softmax(PyObject* const* a) {
         return made;
     });
     if (out.defined()) return run_softmax(*p, src.detach(), &out, scale);
-    if (!(at::GradMode::is_enabled() && src.requires_grad())) return run_softmax(*p, src, nullptr, scale);
+    if (!recorded({&src})) return run_softmax(*p, src, nullptr, scale);
     auto node = new_node<BlockSoftmaxBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(src));
     node->plan = p;

@@ -209,3 +209,19 @@ def test_saved_tensor_hooks(cuda_device, op):
         with pytest.raises(RuntimeError):
             grads(same, unpack)
     assert all(torch.equal(a, b) for a, b in zip(grads(same, same), want))
+
+
+@pytest.mark.parametrize("op", ["gemm", "scores", "softmax", "attention"])
+def test_forward_mode_is_refused_not_dropped(cuda_device, op):
+    import torch.autograd.forward_ad as fwAD
+    dev, n, kl = cuda_device, np.array([20, 70]), np.array([64, 64])
+    x, s = (torch.randn((2, int((n * t).sum())), device=dev).half() for t in (kl, n))
+    with fwAD.dual_level():
+        dual = lambda t: fwAD.make_dual(t.clone().requires_grad_(True), torch.ones_like(t))
+        with pytest.raises(NotImplementedError):
+            if op == "softmax":
+                blockSoftmax(dual(s), n, n)
+            elif op == "attention":
+                blockAttention(x, dual(x), x, n, n, d=64)
+            else:
+                (blockGEMM if op == "gemm" else blockAttnScores)(*((x, dual(x)) + ((None,) * 3 if op == "gemm" else ())), n, n, kl)

@@ -24,6 +24,7 @@ Differences from upstream, all at the boundary:
 from __future__ import annotations
 
 from collections import OrderedDict
+from contextlib import contextmanager
 from typing import Optional
 
 import numpy as np
@@ -33,7 +34,45 @@ from . import _lib as L
 from . import _ops
 from .plan import GemmPlan, _host_i64
 
-_ops.setup(_host_i64, L.BlkError)
+
+
+@contextmanager
+def _untraced():
+    state = torch._C._get_tracing_state()
+    torch._C._set_tracing_state(None)
+    try:
+        yield
+    finally:
+        torch._C._set_tracing_state(state)
+
+
+class _Traced(torch.autograd.Function):
+    """An operator call as ``torch.jit.trace`` records it: one node with the call's operands as inputs, whose forward runs
+    on every replay.  Lists, offsets and options are constants of the trace."""
+
+    @staticmethod
+    def forward(ctx, name, rest, *operands):
+        with _untraced(), torch.enable_grad():
+            ctx.operands = [t.detach().requires_grad_(t.requires_grad) for t in operands]
+            ctx.result = getattr(_ops, name)(*ctx.operands, *rest)
+            return ctx.result.detach()
+
+    @staticmethod
+    def backward(ctx, grad):
+        wanted = [t for t in ctx.operands if t.requires_grad]
+        grads = iter(torch.autograd.grad(ctx.result, wanted, grad))
+        return (None, None) + tuple(next(grads) if t.requires_grad else None for t in ctx.operands)
+
+
+def _traced(name, operands, args):
+    """Called by the native operators instead of running when the tracer is on."""
+    if name == "softmax" and args[-1] is not None:   # in place or into a given tensor: nothing to record
+        with _untraced():
+            return _ops.softmax(*args)
+    return _Traced.apply(name, args[operands:], *args[:operands])
+
+
+_ops.setup(_host_i64, L.BlkError, _traced)
 
 _CACHE: "OrderedDict[tuple, object]" = OrderedDict()
 _CACHE_MAX = 32

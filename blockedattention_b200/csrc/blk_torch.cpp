@@ -21,6 +21,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -63,6 +64,7 @@ struct PyRef {
 
 PyObject* g_host_i64 = nullptr;  // plan._host_i64: any sequence -> contiguous int64 numpy array
 PyObject* g_error = nullptr;     // _lib.BlkError
+PyObject* g_traced = nullptr;    // apply._traced(operator, number of operands, arguments)
 
 // A failed library call: blockedattention_b200._lib.BlkError, whatever thread it happens on -- the caller of an operator
 // gets it from the entry below, the caller of a backward pass from torch's engine.
@@ -884,10 +886,20 @@ Tensor py_scores_token_major(PyObject* const* a) {
 }
 
 // ---- the module --------------------------------------------------------------------------------------
-template <Tensor (*F)(PyObject* const*), int NARGS>
+// F takes NARGS arguments, the first NTENSORS of them its operands.  torch.jit.trace sees nothing of what happens here: a
+// call that it is to record goes to apply.py and comes back, with the tracer paused, from a torch.autograd.Function.
+template <Tensor (*F)(PyObject* const*), const char* NAME, int NARGS, int NTENSORS>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     TORCH_CHECK(n == NARGS, "expected ", NARGS, " arguments");
+    if (torch::jit::tracer::isTracing()) {
+        PyRef rest(PyTuple_New(NARGS));
+        for (int i = 0; rest.o && i < NARGS; ++i) {
+            Py_INCREF(args[i]);
+            PyTuple_SET_ITEM(rest.o, i, args[i]);
+        }
+        return rest.o ? PyObject_CallFunction(g_traced, "siO", NAME, NTENSORS, rest.o) : nullptr;
+    }
     return THPVariable_Wrap(F(args));
     END_HANDLE_TH_ERRORS
 }
@@ -929,26 +941,29 @@ PyObject* py_check(PyObject*, PyObject*) {
     END_HANDLE_TH_ERRORS
 }
 
-// setup(_host_i64, BlkError)
+// setup(_host_i64, BlkError, _traced)
 PyObject* py_setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 2) {
-        PyErr_SetString(PyExc_TypeError, "setup(host_i64, error_class)");
+    if (n != 3) {
+        PyErr_SetString(PyExc_TypeError, "setup(host_i64, error_class, traced)");
         return nullptr;
     }
-    Py_INCREF(args[0]);
-    Py_INCREF(args[1]);
+    for (Py_ssize_t i = 0; i < n; ++i) Py_INCREF(args[i]);
     g_host_i64 = args[0];
     g_error = args[1];
+    g_traced = args[2];
     Py_RETURN_NONE;
 }
 
-#define BLK_ENTRY(f, n) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<f, n>)), METH_FASTCALL
+#define BLK_ENTRY(name, nargs, ntensors) \
+    {g_##name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<py_##name, g_##name, nargs, ntensors>)), METH_FASTCALL, nullptr}
+constexpr char g_gemm[] = "gemm", g_softmax[] = "softmax", g_attention[] = "attention",
+               g_attention_token_major[] = "attention_token_major", g_scores_token_major[] = "scores_token_major";
 PyMethodDef g_methods[] = {
-    {"gemm", BLK_ENTRY(py_gemm, 13), nullptr},
-    {"softmax", BLK_ENTRY(py_softmax, 6), nullptr},
-    {"attention", BLK_ENTRY(py_attention, 7), nullptr},
-    {"attention_token_major", BLK_ENTRY(py_attention_token_major, 5), nullptr},
-    {"scores_token_major", BLK_ENTRY(py_scores_token_major, 6), nullptr},
+    BLK_ENTRY(gemm, 13, 2),
+    BLK_ENTRY(softmax, 6, 1),
+    BLK_ENTRY(attention, 7, 3),
+    BLK_ENTRY(attention_token_major, 5, 3),
+    BLK_ENTRY(scores_token_major, 6, 2),
     {"clear", py_clear, METH_NOARGS, nullptr},
     {"check", py_check, METH_NOARGS, nullptr},
     {"setup", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&py_setup)), METH_FASTCALL, nullptr},

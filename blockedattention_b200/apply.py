@@ -55,7 +55,13 @@ class _Traced(torch.autograd.Function):
         with _untraced(), torch.enable_grad():
             ctx.operands = [t.detach().requires_grad_(t.requires_grad) for t in operands]
             ctx.result = getattr(_ops, name)(*ctx.operands, *rest)
-            return ctx.result.detach()
+            result = ctx.result.detach()
+        if torch.jit.is_tracing():   # the tracer must have seen the result being made
+            seen = torch.empty(0, dtype=result.dtype, device=result.device)
+            with _untraced():
+                seen.data = result
+            result = seen
+        return result
 
     @staticmethod
     def backward(ctx, grad):

@@ -11,6 +11,7 @@ N, KL, D = np.array([20, 70]), np.array([64, 64]), 64
 ROWS, CELLS = int(N.sum()), int((N * N).sum())
 TOKENS = (ROWS, 2, D)
 OPS = {"gemm": (lambda a, b: blockGEMM(a, b, None, None, None, N, N, KL, scale=0.5), [(2, ROWS * D)] * 2),
+       "gemm, fp32 result": (lambda a, b: blockGEMM(a, b, None, None, None, N, N, KL, out_dtype=torch.float32), [(2, ROWS * D)] * 2),
        "scores": (lambda a, b: blockAttnScores(a, b, N, N, KL, scale=0.1), [(2, ROWS * D)] * 2),
        "softmax": (lambda a: blockSoftmax(a, N, N), [(2, CELLS)]),
        "chain": (lambda a, b: blockSoftmax(blockGEMM(a, b, None, None, None, N, N, KL, scale=0.1) * 1.0, N, N), [(2, ROWS * D)] * 2),
@@ -32,5 +33,5 @@ def test_trace_and_replay(cuda_device, name, grad):
         want, got = call(*ins), traced(*ins)
         assert torch.equal(got, want)
         if grad:
-            go = torch.randn(want.shape, generator=g, device=cuda_device).half()
+            go = torch.randn(want.shape, generator=g, device=cuda_device).to(want.dtype)
             assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(got, ins, go), torch.autograd.grad(want, ins, go)))

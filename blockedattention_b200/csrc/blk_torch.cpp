@@ -762,8 +762,8 @@ Tensor py_softmax(PyObject* const* a) {
     return out;
 }
 
-PlanP attention_plan(const ListP& M, const ListP& N, int64_t numel_q, int64_t d, at::ScalarType dt, c10::Device dev, bool may_compose) {
-    PlanKey key{2, (int)dt, (int)dt, may_compose, (int)dev.index(), (int)d, numel_q, {M.get(), N.get()}};
+PlanP attention_plan(const ListP& M, const ListP& N, int64_t H, int64_t d, at::ScalarType dt, c10::Device dev, bool may_compose) {
+    PlanKey key{2, (int)dt, (int)dt, may_compose, (int)dev.index(), (int)d, H, {M.get(), N.get()}};
     return plan_for(key, [&]() {
         const auto &m = M->v, &n = N->v;
         TORCH_CHECK(m.size() == n.size(), "MList and NList must have the same length");
@@ -776,7 +776,7 @@ PlanP attention_plan(const ListP& M, const ListP& N, int64_t numel_q, int64_t d,
         p->rows_kv = sum(n);
         TORCH_CHECK(!may_compose || (p->rows_q > 0 && p->rows_kv > 0), "blockAttention needs at least one query row and one key row");
         p->d = d;
-        p->H = p->rows_q > 0 ? numel_q / (p->rows_q * d) : 0;
+        p->H = H;
         p->dt = p->odt = dt;
         p->device = dev;
         p->lists[0] = M;
@@ -819,7 +819,7 @@ Tensor py_attention(PyObject* const* a) {
                 "q / k / v do not match the packed extents of the lists");
     const auto dt = q.scalar_type();
     const bool one_type = k.scalar_type() == dt && v.scalar_type() == dt;
-    const PlanP p = attention_plan(M, N, q.numel(), d, dt, q.device(), true);
+    const PlanP p = attention_plan(M, N, q.numel() / (rows_q * d), d, dt, q.device(), true);
     if (!p->compose && one_type) return attention_op(p, q, k, v, scale);
     // the composition of the two operators
     TORCH_CHECK(k.scalar_type() == dt && v.scalar_type() == dt, "mat1 and mat2 must have the same dtype");
@@ -844,12 +844,11 @@ Tensor py_attention_token_major(PyObject* const* a) {
     const NoGil free;
     const ListP n = n_list.read();
     const auto dt = q.scalar_type();
-    // the number of heads comes from the shape, not from the element count: the plan is made for H * sum(n) * d elements
     const int64_t rows = sum(n->v);
     TORCH_CHECK(q.size(0) == rows && k.scalar_type() == dt && v.scalar_type() == dt && !unaligned(q) && !unaligned(k) && !unaligned(v),
                 "q, k and v must be contiguous, 16-byte aligned CUDA tensors of one type and shape (", rows, ", ", q.size(1), ", ",
                 q.size(2), ")");
-    const PlanP p = attention_plan(n, n, q.numel(), q.size(2), dt, q.device(), false);
+    const PlanP p = attention_plan(n, n, q.size(1), q.size(2), dt, q.device(), false);
     return run_attention(*p, q.detach(), k.detach(), v.detach(), scale, true);
 }
 
@@ -864,6 +863,7 @@ Tensor py_scores_token_major(PyObject* const* a) {
     const bool softmax = as_bool(a[5]);
     const NoGil free;
     const ListP n = n_list.read();
+    TORCH_CHECK(!n->v.empty(), "blockAttnScoresTokenMajor needs at least one segment");
     const int64_t H = q.size(1), d = q.size(2);
     PlanKey key{3, (int)dt, (int)odt, (int)softmax, (int)q.get_device(), (int)d, H, {n.get()}};
     const PlanP p = plan_for(key, [&]() {

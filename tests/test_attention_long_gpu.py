@@ -175,3 +175,18 @@ def test_attention_over_millions_of_keys(cuda_device):
         p = torch.softmax(scale * (K @ q[0, s * d:(s + 1) * d].float()).double(), 0)
         close(got[0, s * d:(s + 1) * d], (p.float() @ V).cpu(), F16, f"segment {s}")
         first += n
+
+
+@pytest.mark.parametrize("sizes", [[0, 0], []])
+def test_token_major_batches_without_tokens(cuda_device, sizes):
+    # an empty batch of a data loader has an empty result with the heads and the head dimension of its operands
+    from blockedattention_b200 import blockAttnScoresTokenMajor
+    x = torch.empty((0, 4, 64), device=cuda_device, dtype=F16)
+    assert blockAttentionTokenMajor(x, x, x, np.array(sizes, np.int64)).shape == (0, 4, 64)
+    y = torch.empty((0, 8, 64), device=cuda_device, dtype=F16)
+    assert blockAttentionTokenMajor(y, y, y, np.array(sizes, np.int64)).shape == (0, 8, 64)
+    if sizes:
+        assert blockAttnScoresTokenMajor(x, x, np.array(sizes, np.int64)).shape == (4, 0)
+    else:
+        with pytest.raises(RuntimeError):
+            blockAttnScoresTokenMajor(x, x, np.array(sizes, np.int64))

@@ -97,7 +97,6 @@ int dtype_code(at::ScalarType t) {
 // ---- lists -------------------------------------------------------------------------------------------
 struct List {
     std::vector<int64_t> v;
-    uint64_t hash;
 };
 typedef std::shared_ptr<const List> ListP;
 
@@ -132,7 +131,6 @@ struct Interned {
         }
         auto l = std::make_shared<List>();
         l->v.assign(p, p + n);
-        l->hash = h;
         table.emplace(h, l);
         return l;
     }
@@ -941,6 +939,27 @@ PyObject* py_check(PyObject*, PyObject*) {
     END_HANDLE_TH_ERRORS
 }
 
+// same_list(a, b): whether the plan cache takes two list arguments for the same list.  For tests and debugging.
+PyObject* py_same_list(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK(n == 2, "expected 2 arguments");
+    const ListArg a = list_of(args[0]), b = list_of(args[1]);
+    ListP la, lb;
+    {
+        const NoGil free;
+        la = a.read();
+        lb = b.read();
+    }
+    return PyBool_FromLong(la == lb);
+    END_HANDLE_TH_ERRORS
+}
+
+// cached(): the numbers of plans and of GPU lists that are remembered.  For tests and debugging.
+PyObject* py_cached(PyObject*, PyObject*) {
+    std::lock_guard<std::mutex> g(g_mu);
+    return Py_BuildValue("nn", (Py_ssize_t)plans().order.size(), (Py_ssize_t)device_lists().order.size());
+}
+
 // setup(_host_i64, BlkError, _traced)
 PyObject* py_setup(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 3) {
@@ -966,6 +985,8 @@ PyMethodDef g_methods[] = {
     BLK_ENTRY(scores_token_major, 6, 2),
     {"clear", py_clear, METH_NOARGS, nullptr},
     {"check", py_check, METH_NOARGS, nullptr},
+    {"cached", py_cached, METH_NOARGS, nullptr},
+    {"same_list", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&py_same_list)), METH_FASTCALL, nullptr},
     {"setup", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&py_setup)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_ops", "native host path of the operators", -1, g_methods, nullptr, nullptr, nullptr, nullptr};

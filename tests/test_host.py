@@ -279,31 +279,32 @@ def test_partition_edge_cases():
 
 
 def test_plan_cache_is_keyed_on_list_values_not_addresses():
-    # a freed list tensor's address comes back with other values: the key must follow the values
-    from blockedattention_b200 import apply as A
-    A.clear_plan_cache()
-    keys, ptrs = set(), set()
+    # a freed list tensor's address comes back with other values: the operators' key must follow the values
+    from blockedattention_b200 import _ops
+    ptrs = set()
     for i in range(40):
         t = torch.tensor([10 + i, 50 - i])
         ptrs.add(t.data_ptr())
-        keys.add(A._key_of(t))
-        A._LISTS.clear()          # the memo would keep t alive; without it the allocator reuses the block
+        assert _ops.same_list(t, [10 + i, 50 - i]) and not _ops.same_list(t, [9 + i, 51 - i])
         del t
-    assert len(keys) == 40, "two lists with different values shared a key"
-    # a remembered tensor is not read again, and an in-place write is seen
+    # host sequences, arrays and tensors with equal values are one list, whatever their type and strides
     t = torch.tensor([3, 4, 5])
-    k1 = A._key_of(t)
-    assert A._key_of(t) == k1 and len(A._LISTS) == 1
+    for x in ([3, 4, 5], (3, 4, 5), np.array([3, 4, 5]), np.array([3, 4, 5], np.int32), np.array([3.0, 4.0, 5.0]),
+              np.array([3, 0, 4, 0, 5])[::2], t.int(), torch.tensor([3, 0, 4, 0, 5])[::2], t.reshape(3, 1)):
+        assert _ops.same_list(t, x) and not _ops.same_list(x, [3, 4]) and not _ops.same_list(x, [3, 4, 5, 0])
+    # a write is seen, also one that goes round the tensor
+    a = np.array([3, 4, 5])
+    u = torch.from_numpy(a)
+    assert _ops.same_list(t, u)
     t[1] = 9
-    assert A._key_of(t) != k1
-    # host sequences, arrays and tensors with equal values share one key
-    assert A._key_of([3, 9, 5]) == A._key_of(np.array([3, 9, 5])) == A._key_of(t)
-    A.clear_plan_cache()
+    assert not _ops.same_list(t, u)
+    a[1] = 9
+    assert _ops.same_list(t, u) and _ops.same_list([], np.empty(0, np.int64)) and not _ops.same_list([], [0])
 
 
 def test_evicted_plans_stay_usable_for_their_holders():
-    # the cache drops an evicted plan without closing it: whoever still holds it (an autograd context between
-    # forward and backward, a queued host-pipe step) keeps a live handle
+    # the table of host pipes drops an evicted one without closing it: whoever still holds it (a queued step) keeps a live
+    # handle.  (The operators' plans: test_plan_cache_gpu.py)
     from blockedattention_b200 import apply as A
     A.clear_plan_cache()
     first = A._cached(("t", 0), lambda: SoftmaxPlan([3], [4], 1, torch.float16))

@@ -80,32 +80,10 @@ def _traced(name, operands, args):
 
 _ops.setup(_host_i64, L.BlkError, _traced)
 
+# The host pipes of blockAttnScoresHost, least recently used first, under the values of their lists.  (Plans and GPU lists
+# of the operators are remembered by the native code.)
 _CACHE: "OrderedDict[tuple, object]" = OrderedDict()
 _CACHE_MAX = 32
-# List tensors already read to the host: (data_ptr, _version, numel, dtype, device) -> (the tensor, its values as
-# bytes).  The entry keeps the tensor alive, so its storage cannot be freed and handed to a tensor with other
-# values while the entry exists; an in-place write moves _version.  A hit therefore costs no device->host copy,
-# and the plan cache below is keyed on the values themselves, never on addresses.
-_LISTS: "OrderedDict[tuple, tuple]" = OrderedDict()
-_LISTS_MAX = 256
-
-
-def _key_of(x):
-    """Cache key of a list / offset argument: its int64 values."""
-    if x is None:
-        return None
-    if isinstance(x, torch.Tensor):
-        fast = (x.data_ptr(), x._version, x.numel(), x.dtype, str(x.device))
-        hit = _LISTS.get(fast)
-        if hit is not None:
-            _LISTS.move_to_end(fast)
-            return ("v", hit[1])
-        data = _host_i64(x).tobytes()
-        _LISTS[fast] = (x, data)
-        while len(_LISTS) > _LISTS_MAX:
-            _LISTS.popitem(last=False)
-        return ("v", data)
-    return ("v", np.ascontiguousarray(np.asarray(x, dtype=np.int64)).tobytes())
 
 
 def _cached(key, build):
@@ -113,8 +91,8 @@ def _cached(key, build):
     if plan is None:
         plan = build()
         _CACHE[key] = plan
-        # An evicted plan is only dropped from the table: an autograd context or a queued host-pipe step may
-        # still hold it, and the library handle is released when the last reference goes away.
+        # An evicted one is only dropped from the table: a queued step may still hold it, and the library handle
+        # is released when the last reference goes away.
         while len(_CACHE) > _CACHE_MAX:
             _CACHE.popitem(last=False)
     else:
@@ -126,7 +104,6 @@ def clear_plan_cache() -> None:
     """Forgets every cached plan and list (plans still referenced elsewhere stay usable)."""
     _ops.clear()
     _CACHE.clear()
-    _LISTS.clear()
 
 
 def check_plans() -> None:
@@ -258,7 +235,7 @@ def blockAttnScoresHost(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, s
         out = torch.empty((H, Dout), dtype=odt).pin_memory()
     elif out.is_cuda or not out.is_contiguous() or out.dtype != odt or out.numel() != H * Dout:
         raise RuntimeError("out must be a contiguous host tensor of the output dtype with H*Dout elements")
-    key = ("hostpipe", _key_of(MList), _key_of(NList), _key_of(KList), H, groups, q.dtype, odt, bool(softmax), str(dev))
+    key = ("hostpipe", M.tobytes(), N.tobytes(), K.tobytes(), H, groups, q.dtype, odt, bool(softmax), str(dev))
     pipe = _cached(key, lambda: _HostPipe(M, N, K, H, groups, q.dtype, odt, bool(softmax), dev))
     Hg = pipe.Hg
     qv, kv, ov = q.reshape(H, Dm1), k.reshape(H, Dm2), out.reshape(H, Dout)

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from helpers import O
-from blockedattention_b200 import _ops, blockAttention, blockAttnScores, blockGEMM, blockSoftmax, clear_plan_cache
+from blockedattention_b200 import _ops, blockAttention, blockAttnScores, blockAttnScoresHost, blockGEMM, blockSoftmax, clear_plan_cache
 
 pytestmark = pytest.mark.gpu
 PLANS, LISTS = 32, 256   # the bounds
@@ -98,3 +98,25 @@ def test_eviction_between_forward_and_backward(cuda_device):
             clear_plan_cache()
         grads.append(torch.autograd.grad(sum(o.float().square().sum() for o in outs), leaves))
     assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_host_pipe_follows_the_values_of_its_lists(cuda_device):
+    # lists of one storage, and a numpy array written to behind its tensor's back
+    g = torch.Generator().manual_seed(3)
+    base = torch.tensor([30, 50, 10])
+    a = np.array([30, 50])
+    alias = torch.from_numpy(a)
+
+    def check(n, lists):
+        n = np.array(n)
+        kl = np.full(len(n), 64)
+        q, k = (torch.randn((2, int(n.sum()) * 64), generator=g).half() for _ in range(2))
+        got = blockAttnScoresHost(q, k, lists, lists, kl, scale=0.125, device=cuda_device)
+        torch.cuda.synchronize()
+        assert (got.float() - O.block_scores(q, k, n, n, kl, scale=0.125)).abs().max() < 2e-3
+
+    check([30, 50], base[:2])
+    check([30, 10], base[::2])
+    check([30, 50], alias)
+    a[:] = 70, 20
+    check([70, 20], alias)

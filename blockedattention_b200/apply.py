@@ -23,11 +23,11 @@ Differences from upstream, all at the boundary:
 """
 from __future__ import annotations
 
+import threading
 from collections import OrderedDict
 from contextlib import contextmanager
 from typing import Optional
 
-import numpy as np
 import torch
 
 from . import _lib as L
@@ -84,26 +84,32 @@ _ops.setup(_host_i64, L.BlkError, _traced)
 # of the operators are remembered by the native code.)
 _CACHE: "OrderedDict[tuple, object]" = OrderedDict()
 _CACHE_MAX = 32
+_CACHE_LOCK = threading.Lock()
 
 
 def _cached(key, build):
-    plan = _CACHE.get(key)
-    if plan is None:
-        plan = build()
-        _CACHE[key] = plan
-        # An evicted one is only dropped from the table: a queued step may still hold it, and the library handle
-        # is released when the last reference goes away.
-        while len(_CACHE) > _CACHE_MAX:
-            _CACHE.popitem(last=False)
-    else:
+    with _CACHE_LOCK:
+        found = _CACHE.get(key)
+        if found is not None:
+            _CACHE.move_to_end(key)
+            return found
+    made = build()
+    dropped = []   # released after the lock, and only for the table: a queued step may still hold one
+    with _CACHE_LOCK:
+        found = _CACHE.setdefault(key, made)
         _CACHE.move_to_end(key)
-    return plan
+        while len(_CACHE) > _CACHE_MAX:
+            dropped.append(_CACHE.popitem(last=False))
+    return found
 
 
 def clear_plan_cache() -> None:
     """Forgets every cached plan and list (plans still referenced elsewhere stay usable)."""
     _ops.clear()
-    _CACHE.clear()
+    with _CACHE_LOCK:
+        dropped = list(_CACHE.values())
+        _CACHE.clear()
+    del dropped
 
 
 def check_plans() -> None:
@@ -111,7 +117,9 @@ def check_plans() -> None:
     (``BLK_ERR_TIMEOUT``) if a kernel of one of them gave up a bounded device-side wait since the last check --
     the result of that call is then incomplete.  ``BLK_CHECK=1`` in the environment does this after every run."""
     _ops.check()
-    for plan in list(_CACHE.values()):
+    with _CACHE_LOCK:
+        pipes = list(_CACHE.values())
+    for plan in pipes:
         inner = getattr(plan, "plan", plan)   # a host pipe wraps its plan
         if getattr(inner, "device", None) is not None:
             inner.check()
@@ -200,6 +208,11 @@ class _HostPipe:
                       torch.empty((self.Hg, p.Dm2), dtype=dtype, device=device),
                       torch.empty((self.Hg, p.Dout), dtype=odt, device=device)) for _ in range(2)]
         self.s_in, self.s_run, self.s_out = (torch.cuda.Stream(device=device) for _ in range(3))
+        for t in (t for buffers in self.bufs for t in buffers):
+            for s in (self.s_in, self.s_run, self.s_out):
+                t.record_stream(s)     # allocated on the stream of the first call
+        self.lock = threading.Lock()   # one call's steps are queued at a time
+        self.idle = None               # event: the last call is through with the buffers
 
 
 def blockAttnScoresHost(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, scale: float = 1.0,
@@ -242,33 +255,37 @@ def blockAttnScoresHost(q: torch.Tensor, k: torch.Tensor, MList, NList, KList, s
     cur = torch.cuda.current_stream(dev)
     start = torch.cuda.Event()
     start.record(cur)
-    for s in (pipe.s_in, pipe.s_run, pipe.s_out):
-        s.wait_event(start)
-    ran = [None, None]     # per buffer set: event after the kernels that read its operands
-    drained = [None, None]  # per buffer set: event after the copy that read its result
-    for g in range(groups):
-        b = g & 1
-        dq, dk, do = pipe.bufs[b]
-        rows = slice(g * Hg, (g + 1) * Hg)
-        with torch.cuda.stream(pipe.s_in):
-            if ran[b] is not None:
-                pipe.s_in.wait_event(ran[b])
-            dq.copy_(qv[rows], non_blocking=True)
-            dk.copy_(kv[rows], non_blocking=True)
-            loaded = torch.cuda.Event()
-            loaded.record(pipe.s_in)
-        with torch.cuda.stream(pipe.s_run):
-            pipe.s_run.wait_event(loaded)
-            if drained[b] is not None:
-                pipe.s_run.wait_event(drained[b])
-            pipe.plan.run(dq, dk, out=do, scale=scale)
-            ran[b] = torch.cuda.Event()
-            ran[b].record(pipe.s_run)
-        with torch.cuda.stream(pipe.s_out):
-            pipe.s_out.wait_event(ran[b])
-            ov[rows].copy_(do, non_blocking=True)
-            drained[b] = torch.cuda.Event()
-            drained[b].record(pipe.s_out)
+    with pipe.lock:
+        for s in (pipe.s_in, pipe.s_run, pipe.s_out):
+            s.wait_event(start)
+            if pipe.idle is not None:   # (the call before may have come from another stream)
+                s.wait_event(pipe.idle)
+        ran = [None, None]     # per buffer set: event after the kernels that read its operands
+        drained = [None, None]  # per buffer set: event after the copy that read its result
+        for g in range(groups):
+            b = g & 1
+            dq, dk, do = pipe.bufs[b]
+            rows = slice(g * Hg, (g + 1) * Hg)
+            with torch.cuda.stream(pipe.s_in):
+                if ran[b] is not None:
+                    pipe.s_in.wait_event(ran[b])
+                dq.copy_(qv[rows], non_blocking=True)
+                dk.copy_(kv[rows], non_blocking=True)
+                loaded = torch.cuda.Event()
+                loaded.record(pipe.s_in)
+            with torch.cuda.stream(pipe.s_run):
+                pipe.s_run.wait_event(loaded)
+                if drained[b] is not None:
+                    pipe.s_run.wait_event(drained[b])
+                pipe.plan.run(dq, dk, out=do, scale=scale)
+                ran[b] = torch.cuda.Event()
+                ran[b].record(pipe.s_run)
+            with torch.cuda.stream(pipe.s_out):
+                pipe.s_out.wait_event(ran[b])
+                ov[rows].copy_(do, non_blocking=True)
+                drained[b] = torch.cuda.Event()
+                drained[b].record(pipe.s_out)
+        pipe.idle = drained[(groups - 1) & 1]
     for ev in drained:
         if ev is not None:
             cur.wait_event(ev)

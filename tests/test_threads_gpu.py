@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 import torch
 
-from blockedattention_b200 import blockAttention, blockGEMM, blockSoftmax, check_plans, clear_plan_cache
+from blockedattention_b200 import (blockAttention, blockAttnScoresHost, blockGEMM, blockSoftmax, check_plans,
+                                   clear_plan_cache)
 
 pytestmark = pytest.mark.gpu
 BUSY = 0.3  # seconds of queued work that a call has to wait for
@@ -106,3 +107,39 @@ def test_threads_and_streams_share_the_caches(cuda_device):
     for t in threads:
         t.join()
     assert not failures, failures[:5]
+
+
+def test_host_pipe_from_several_streams_and_threads(cuda_device):
+    # calls on one batch share its device buffers: a call from another stream must not overtake the one before
+    n, kl, H = np.array([300, 200, 40]), np.full(3, 64), 8
+    g = torch.Generator().manual_seed(0)
+    ins = [[torch.randn((H, int(n.sum()) * 64), generator=g).half().pin_memory() for _ in range(2)] for _ in range(4)]
+
+    def call(i):
+        return blockAttnScoresHost(*ins[i], n, n, kl, scale=0.125, device=cuda_device)
+
+    want = []
+    for i in range(4):
+        want.append(call(i))
+        torch.cuda.synchronize()
+    wrong = []
+
+    def run(t):
+        streams = [torch.cuda.Stream(cuda_device) for _ in range(4)]
+        for _ in range(5):
+            got = []
+            for i, s in enumerate(streams):
+                with torch.cuda.stream(s):
+                    got.append(call(i))
+            for i, s in enumerate(streams):
+                s.synchronize()
+                if not torch.equal(got[i], want[i]):
+                    wrong.append((t, i))
+
+    run("alone")
+    threads = [threading.Thread(target=run, args=(t,)) for t in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:5]

@@ -173,7 +173,8 @@ def blockAttention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, MList, NLi
     that never stores the probabilities (the pack kernel when every segment has at most 64 rows and columns and
     ``d = 64``, the tcgen05 attention kernel otherwise); any other batch is the composition
     ``blockGEMM(blockAttnScores(q, k), v, transpose2=True)`` of the two operators.  Carries autograd history: the
-    backward pass recomputes the probabilities with the two-operator path."""
+    fused batches have backward kernels of their own, which recompute the probabilities (from saved row logarithms for
+    segments beyond 64 x 64); the composition differentiates through its operators."""
     return _ops.attention(q, k, v, MList, NList, scale, d)
 
 

@@ -21,8 +21,16 @@
 //   warps 4-11  softmax: warps 4-7 take the even tiles, 8-11 the odd ones; a thread owns one row of 64 columns and meets
 //               nobody;
 //   warps 12-15 output; <QUERIES>: also rowsum(dO O) of the next item, kept for the <KEYS> launch.
-// Bound by the tensor pipe (at d = 128 and 64-column tiles 1280 cycles a tile for <KEYS>, 1024 for <QUERIES>: the S and dP
-// products run at two thirds of the rate with 64 columns, but 128-column tiles would leave room for one pair of buffers).
+// Bound by the chain of a tile through the roles -- scores, exponentials, dP, dS, product -- with two pairs of buffers to
+// overlap it: at d = 128 the products of a tile are 1280 cycles of the tensor pipe for <KEYS> and 1024 for <QUERIES> (S and
+// dP run at two thirds of the rate with 64 columns, but 128-column tiles would leave room for one pair), and the pipe is
+// active 38 % and 28 % of the time, the special-function unit 20 %, the issue slots 30 % (48 segments of 64..512 rows, 16
+// heads: 126 and 124 us).
+//
+// rowsum(dO O) takes O as the forward pass rounded it, where a chain of operators has rowsum(P dP) of its own rounded P.
+// 2-norm errors of dQ against 64 bits, 300 rows, d = 64, bf16: 2.4e-3 (the chain: 3.3e-3) for scores of deviation 1, 5.4e-3
+// (4.2e-3) for 8 and 7.1e-3 (5.0e-3) for 32, where a row's probability sits on one key and dS is what is left of a
+// difference.
 //
 // Rows past the end of a segment belong to its neighbour: as resident rows they are computed and not stored, as passing
 // rows they get P = dS = 0.  Every wait is bounded, as in the forward kernel.

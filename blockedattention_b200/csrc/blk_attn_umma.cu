@@ -2,7 +2,7 @@
 // out_s = softmax(scale * Q_s K_s^T) V_s per segment and head, head dimension 64 or
 // 128, without the probabilities ever leaving the SM.
 //
-// A persistent CTA (one per SM, 16 warps) walks a static list of work items.  An item is
+// A persistent CTA (one per SM, 20 warps) walks a static list of work items.  An item is
 // up to two 128-row query blocks of one head, stream A and stream B: two blocks of one
 // segment, which share every key and value tile, or the odd last blocks of two segments
 // with tiles of their own.  A stream sweeps its keys and values in tiles of 64 rows with
@@ -10,13 +10,15 @@
 // whenever they are done with a tile, and two streams put two independent warps on every
 // scheduler: neither the chain Q K^T -> softmax -> P V of a tile nor a warp's own latencies
 // are waited for.  Roles:
-//   warps 0, 2   producers: a lane each issues tiled TMA loads (128-byte swizzle) of the query
+//   warps 0, 1   producers: a lane each issues tiled TMA loads (128-byte swizzle) of the query
 //                blocks and key tiles, of the value tiles, into rings;
-//   warps 1, 3   MMA of stream A, of stream B.  Per tile: O += P V of this tile, then
-//                S = Q K^T of the tile after the next.  P is read from tensor memory (first
-//                operand [tmem], two 16-bit elements per column, row = lane), V as loaded,
-//                i.e. MN-major.  Both warps see every tile of the rings: a tile is free when
-//                both have let go of it, and each sees all phases of the rings' barriers;
+//   warps 2, 3   scores of stream A, of stream B: S = Q K^T of a tile into the buffer whose
+//                probabilities (two tiles back) P V has read;
+//   warps 16, 17 products with the values of stream A, of stream B: O += P V.  P is read from
+//                tensor memory (first operand [tmem], two 16-bit elements per column, row =
+//                lane), V as loaded, i.e. MN-major.  The warps of a pair see every tile of their
+//                ring: a tile is free when both have let go of it, and each sees all phases of
+//                the ring's barriers;
 //   warps 4-7, 8-11  softmax of stream A, of stream B: a thread owns one row of 64 scores, so
 //                no row statistics are exchanged.  Online softmax with a lazy reference: the
 //                running maximum is only moved (and O rescaled in tensor memory) when the new
@@ -24,11 +26,18 @@
 //                rare.  P, rounded to the input type, overwrites the scores;
 //   warps 12-15  output: wait for a block's last P V and its row sums, read O, divide, store
 //                the rows (and the logarithm of the row sums when a backward pass will want
-//                them), hand the accumulator back.
+//                them), hand the accumulator back;
+//   warp 18      planner: the items' records, a ring of them in shared memory (warp 19 only
+//                completes the warpgroup for the trade of registers).
 //
 // Tensor memory at d = 128 is full: 2 streams x (2 x 64 columns of scores + 128 of result).
 // Tiles of 128 rows would leave room for one score buffer per stream only; measured, that
 // left the softmax warps waiting 2400 of every 5600 cycles.
+//
+// Bound by no single pipe in short runs (208 segments of 64..512 rows, 16 heads, d = 128: tensor
+// pipe active 44 %, special-function unit 48 %, issue slots 43 %, DRAM 52 %; the softmax warps
+// wait for their loads from tensor memory and for products), and by the power limit in long
+// ones: 1088 such segments take 1220 us alone and 1390-1490 us sustained at 1.35-1.4 GHz.
 //
 // Rows of the tiles past the end of a segment belong to its neighbour (or are zero
 // past the end of the buffer): extra query rows are never stored, extra key columns

@@ -29,9 +29,12 @@
 // second sweep of an item alternates chunk by chunk with the first sweep of the next, all four groups taking chunks of both.
 //
 // Measured against one item at a time with 8 arithmetic and 4 store warps: scores + softmax of 1024 segments of 64..512 rows,
-// 16 heads, K = 128: 2054 -> 1532 us; 2048 products of at most 256 x 256, fp32 out: 56.6 -> 54.3 us; 64 products of
-// 1024..2048 rows and columns, K 1024..4096: 850 -> 729 us (1.04 PFLOP/s).  Without its stores the first takes 1230 us: what
-// is left is the latency of a chunk through loads, products and registers, then the write rate of misaligned rows.
+// 16 heads, K = 128: 2054 -> 1532 us; of 512 segments of 16..2048 rows, 4 heads, K = 64 (two sweeps): 872 -> 897 us
+// sustained; 2048 products of at most 256 x 256, fp32 out: 57.3 -> 55.5 us; 64 products of 1024..2048 rows and columns,
+// K 1024..4096: 845 -> 835 us sustained.  Without its stores the first takes 1230 us, and one sweep and two run at the same
+// 2.1-2.3 TB/s: what bounds the softmax is the latency of a chunk through loads, products and registers, then the write rate
+// of misaligned rows (4 TB/s alone).  The long contractions (tensor pipe active 66 % in a single launch) move 48 KB from L2
+// per 128 x 256 x 64 step, 11 TB/s, half of what that path can do.
 //
 // Rows of the operand views past the end of a segment belong to its neighbour (or are zero-filled past the end of the
 // buffer); they only reach accumulator rows/columns the epilogue never stores, and columns >= N are masked before any row

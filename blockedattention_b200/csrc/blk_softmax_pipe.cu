@@ -15,12 +15,13 @@
 // A row longer than a window is streamed from global memory by all computing warps.
 // Every barrier wait is bounded and reports through the status word.
 //
-// Bound by the instructions it issues and their latency, with memory close behind (the copies alone: 650 us where the
-// forward takes 711, and 187 where the backward takes 199).  A spilled register in a row loop costs more than any
+// Bound by the instructions it issues and their latency, with memory close behind (in the profiler, 512 segments of 16..2048
+// rows and columns, 4 heads, bf16: 734 us, issue slots 63 %, special-function unit 64 %, DRAM 62 %; the copies alone 650; the
+// backward of a quarter of it 197, DRAM 76 %, its copies alone 187).  A spilled register in a row loop costs more than any
 // parallelism: with 28 warps of 64 registers the loops over a row's vectors stay rolled, and rows of short segments are
-// functions of their own.  512 segments of 16..2048 rows and columns, 4 heads, bf16: 870 -> 711 us forward; a quarter of
-// it 200 -> 167 forward, 223 -> 199 backward (before: two stages, all warps of a CTA meeting twice a window; a fifth of the
-// instructions were the counting of units in windows of one piece until those were told apart: 783 -> 711).
+// functions of their own.  Against the form with two stages, all warps of a CTA meeting twice a window, the call takes
+// 856 -> 771 us sustained, a quarter of it 200 -> 167 forward and 223 -> 199 backward (a fifth of the instructions were the
+// counting of units in windows of one piece until those were told apart).
 //
 // Forward: out = softmax_rows(scale * src); replaces upstream sparseBlockedSoftmax_warp / _block
 // (csrc/cuda/spBlkSoftmax.cu:88-138, :182-269).  Backward: grad_src = scale * (grad_out - rowsum(out *

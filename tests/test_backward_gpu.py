@@ -117,7 +117,7 @@ def test_fused_scores_backward(cuda_device, dtype):
                                      (64, [5, 200, 64, 130]),        # packs and the tcgen05 attention kernel
                                      (128, [150, 7, 260])])          # the tcgen05 attention kernel
 def test_fused_attention_backward(cuda_device, d, sizes):
-    # forward on the fused kernels; backward recomputes the probabilities with the two-operator path.  Checked against
+    # forward on the fused kernels, backward on kernels of its own that recompute the probabilities.  Checked against
     # torch autograd of the per-segment formula in float64.
     dev = cuda_device
     n = np.array(sizes, np.int64)

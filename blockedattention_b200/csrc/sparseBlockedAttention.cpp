@@ -8,6 +8,7 @@
 #include <c10/cuda/CUDAGuard.h>
 
 #include <list>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -79,35 +80,46 @@ struct ListMemo {
 } g_lists;
 
 // ---- plans, cached under the list values ------------------------------------------------------------
+// A plan lives as long as somebody runs it: another thread's call may push it out of the table meanwhile.  (Kernels
+// already queued only read the plan's device tables; cudaFree waits for them.)
+typedef std::shared_ptr<blk_plan_t> PlanP;
 struct PlanCache {
     std::mutex mu;
-    std::list<std::pair<std::string, blk_plan_t*>> lru;
-    std::unordered_map<std::string, std::list<std::pair<std::string, blk_plan_t*>>::iterator> index;
+    std::list<std::pair<std::string, PlanP>> lru;
+    std::unordered_map<std::string, std::list<std::pair<std::string, PlanP>>::iterator> index;
     static constexpr size_t kMax = 64;
 
-    template <typename Make>
-    blk_plan_t* get(const std::string& key, Make make) {
-        std::lock_guard<std::mutex> g(mu);
+    // with mu held
+    PlanP find(const std::string& key) {
         auto it = index.find(key);
-        if (it != index.end()) {
-            lru.splice(lru.begin(), lru, it->second);
-            return it->second->second;
+        if (it == index.end()) return nullptr;
+        lru.splice(lru.begin(), lru, it->second);
+        return it->second->second;
+    }
+    template <typename Make>
+    PlanP get(const std::string& key, Make make) {
+        {
+            std::lock_guard<std::mutex> g(mu);
+            if (PlanP p = find(key)) return p;
         }
-        blk_plan_t* p = make();
-        lru.emplace_front(key, p);
+        PlanP made(make(), blk_plan_destroy);  // created and released outside the lock: both wait for the device
+        std::vector<PlanP> dropped;
+        std::lock_guard<std::mutex> g(mu);
+        if (PlanP p = find(key)) return p;
+        lru.emplace_front(key, made);
         index[key] = lru.begin();
         while (lru.size() > kMax) {
-            // kernels already queued only read the plan's device tables; cudaFree waits for them
-            blk_plan_destroy(lru.back().second);
+            dropped.push_back(std::move(lru.back().second));
             index.erase(lru.back().first);
             lru.pop_back();
         }
-        return p;
+        return made;
     }
-    ~PlanCache() {
-        // process exit: the CUDA context may already be gone, so the device tables are left to it
-    }
-} g_plans;
+};
+PlanCache& plan_cache() {
+    static PlanCache* cache = new PlanCache();  // at process exit the CUDA context may already be gone: the tables are left to it
+    return *cache;
+}
 
 void append(std::string& key, const I64& v) {
     key.append(reinterpret_cast<const char*>(v.data()), v.size() * sizeof(int64_t));
@@ -139,7 +151,7 @@ Tensor gemm_launch_host(const Tensor& mat1, const Tensor& mat2, const I64& a1, c
     std::string key = "g" + std::to_string(dt) + (t1 ? "T" : "n") + (t2 ? "T" : "n") + std::to_string(dev) + ":" +
                       std::to_string(H) + "|";
     append(key, M); append(key, N); append(key, K); append(key, a1); append(key, a2); append(key, ao);
-    blk_plan_t* plan = g_plans.get(key, [&]() {
+    const PlanP plan = plan_cache().get(key, [&]() {
         blk_plan_t* p = nullptr;
         ok(blk_gemm_plan_create(&p, M.data(), N.data(), K.data(), a1.data(), a2.data(), ao.data(), S, H, dt, dt, t1, t2,
                                 BLK_EPI_SCORES, dev));
@@ -148,11 +160,11 @@ Tensor gemm_launch_host(const Tensor& mat1, const Tensor& mat2, const I64& a1, c
     Tensor out = torch::empty({H, ao[S]}, mat1.options());      // 2-D, dtype of the inputs (upstream spBlkGEMM.cu:1008)
     Tensor m1 = reinterpret_cast<uintptr_t>(mat1.data_ptr()) % 16 ? mat1.clone() : mat1;
     Tensor m2 = reinterpret_cast<uintptr_t>(mat2.data_ptr()) % 16 ? mat2.clone() : mat2;
-    ok(blk_gemm_run(plan, m1.data_ptr(), m2.data_ptr(), out.data_ptr(), 1.0f, at::cuda::getCurrentCUDAStream().stream()));
+    ok(blk_gemm_run(plan.get(), m1.data_ptr(), m2.data_ptr(), out.data_ptr(), 1.0f, at::cuda::getCurrentCUDAStream().stream()));
     return out;
 }
 
-blk_plan_t* softmax_plan(const Tensor& src, const I64& acc, const I64& rows, const I64& cols, int64_t* H_out) {
+PlanP softmax_plan(const Tensor& src, const I64& acc, const I64& rows, const I64& cols, int64_t* H_out) {
     const int64_t S = (int64_t)rows.size();
     TORCH_CHECK((int64_t)cols.size() == S && (int64_t)acc.size() == S + 1, "srcAccum must have one more entry than the lists");
     const int64_t H = heads_of(src, acc[S], "src");
@@ -160,7 +172,7 @@ blk_plan_t* softmax_plan(const Tensor& src, const I64& acc, const I64& rows, con
     std::string key = "s" + std::to_string(dt) + std::to_string(dev) + ":" + std::to_string(H) + "|";
     append(key, rows); append(key, cols); append(key, acc);
     *H_out = H;
-    return g_plans.get(key, [&]() {
+    return plan_cache().get(key, [&]() {
         blk_plan_t* p = nullptr;
         ok(blk_softmax_plan_create(&p, rows.data(), cols.data(), acc.data(), S, H, dt, dev));
         return p;
@@ -224,10 +236,10 @@ Tensor sparseBlockedSoftmaxLaunch(const Tensor& src, const Tensor& accumSrc, con
     c10::cuda::CUDAGuard guard(src.device());
     int64_t H = 0;
     const I64 acc = g_lists.get(accumSrc);
-    blk_plan_t* plan = softmax_plan(src, acc, g_lists.get(rowList), g_lists.get(colList), &H);
+    const PlanP plan = softmax_plan(src, acc, g_lists.get(rowList), g_lists.get(colList), &H);
     Tensor out = torch::empty({H, acc.back()}, src.options());   // upstream csrc/cuda/spBlkSoftmax.cu:398
     Tensor s = aligned(src);
-    ok(blk_softmax_run(plan, s.data_ptr(), out.data_ptr(), 1.0f, at::cuda::getCurrentCUDAStream().stream()));
+    ok(blk_softmax_run(plan.get(), s.data_ptr(), out.data_ptr(), 1.0f, at::cuda::getCurrentCUDAStream().stream()));
     return out;
 }
 
@@ -239,10 +251,10 @@ Tensor sparseBlockedSoftmaxBackwardLaunch(const Tensor& out, const Tensor& dout,
     c10::cuda::CUDAGuard guard(out.device());
     int64_t H = 0;
     const I64 acc = g_lists.get(accumSrc);
-    blk_plan_t* plan = softmax_plan(out, acc, g_lists.get(rowList), g_lists.get(colList), &H);
+    const PlanP plan = softmax_plan(out, acc, g_lists.get(rowList), g_lists.get(colList), &H);
     Tensor gs = torch::empty({H, acc.back()}, out.options());
     Tensor o = aligned(out), g = aligned(dout);
-    ok(blk_softmax_backward_run(plan, o.data_ptr(), g.data_ptr(), gs.data_ptr(), 1.0f,
+    ok(blk_softmax_backward_run(plan.get(), o.data_ptr(), g.data_ptr(), gs.data_ptr(), 1.0f,
                                 at::cuda::getCurrentCUDAStream().stream()));
     return gs;
 }

@@ -104,3 +104,26 @@ def test_fresh_list_tensors_with_other_values_get_their_own_plan(cuda_device):
             got = mod_gemm(A.to(dev), B.to(dev), None, None, None, tM, tM, tK)
             assert_scores_close(got, O.block_gemm(A, B, M, M, K), f"lists {M}")
             del tM, tK
+
+
+def test_plans_outlive_their_place_in_the_table(cuda_device):
+    # two threads, each with more batches than the table holds, push out each other's plans between look-up and run
+    import threading
+    dev, wrong = cuda_device, []
+
+    def run(t):
+        for i in range(150):
+            rows, cols = [3 + t, 1 + i % 50], [1 + (i * 7) % 90, 2 + i]
+            x = torch.randn((2, int(np.dot(rows, cols))), device=dev)
+            got = blockAttention.sparseBlockedSoftmax(x.requires_grad_(True), *lists(dev, rows, cols))
+            got.sum().backward()     # on torch's own thread
+            want = O.block_softmax(x.detach().cpu(), np.array(rows), np.array(cols))
+            if float((got.detach().cpu() - want).abs().max()) > 1e-6 or not torch.isfinite(x.grad).all():
+                wrong.append((t, i))
+
+    threads = [threading.Thread(target=run, args=(t,)) for t in range(3)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not wrong, wrong[:5]

@@ -142,15 +142,15 @@ Interned& interned() {
 
 struct TensorKey {
     const void* ptr;
-    int64_t version, numel;
+    int64_t version, numel, stride;
     int dtype, device;
     bool operator==(const TensorKey& o) const {
-        return ptr == o.ptr && version == o.version && numel == o.numel && dtype == o.dtype && device == o.device;
+        return ptr == o.ptr && version == o.version && numel == o.numel && stride == o.stride && dtype == o.dtype && device == o.device;
     }
 };
 struct TensorKeyHash {
     size_t operator()(const TensorKey& k) const {
-        return (size_t)(((uintptr_t)k.ptr >> 4) * 0x9E3779B97F4A7C15ull) ^ (size_t)(k.version * 1000003 + k.numel * 31 + k.device);
+        return (size_t)(((uintptr_t)k.ptr >> 4) * 0x9E3779B97F4A7C15ull) ^ (size_t)(k.version * 1000003 + k.numel * 31 + k.stride * 7 + k.device);
     }
 };
 
@@ -198,7 +198,7 @@ ListP list_of_tensor(const Tensor& t) {
     const bool remember = t.is_cuda() && !t.is_inference();
     TensorKey key{};
     if (remember) {
-        key = TensorKey{t.data_ptr(), (int64_t)t._version(), t.numel(), (int)t.scalar_type(), (int)t.get_device()};
+        key = TensorKey{t.data_ptr(), (int64_t)t._version(), t.numel(), t.dim() ? t.stride(-1) : 1, (int)t.scalar_type(), (int)t.get_device()};
         std::lock_guard<std::mutex> g(g_mu);
         if (Remembered* r = device_lists().find(key))
             if (r->keep.strides() == t.strides() && r->keep.sizes() == t.sizes()) return r->list;

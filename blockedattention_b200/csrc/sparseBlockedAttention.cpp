@@ -57,7 +57,7 @@ struct ListMemo {
         }
         const std::string key = std::to_string(reinterpret_cast<uintptr_t>(t.data_ptr())) + ":" + std::to_string(t._version()) +
                                 ":" + std::to_string(t.numel()) + ":" + std::to_string((int)t.scalar_type()) + ":" +
-                                std::to_string(t.get_device());
+                                std::to_string(t.get_device()) + ":" + std::to_string(t.dim() ? t.stride(-1) : 1);
         {
             std::lock_guard<std::mutex> g(mu);
             auto it = index.find(key);
@@ -68,10 +68,13 @@ struct ListMemo {
         }
         Tensor h = t.to(at::kCPU, at::kLong).contiguous();   // the one device->host copy of this list
         I64 v(h.data_ptr<int64_t>(), h.data_ptr<int64_t>() + h.numel());
+        std::vector<Tensor> dropped;  // released outside the lock
         std::lock_guard<std::mutex> g(mu);
+        if (index.count(key)) return v;  // another thread was faster
         lru.emplace_front(key, Entry{t, v});
         index[key] = lru.begin();
         while (lru.size() > kMax) {
+            dropped.push_back(std::move(lru.back().second.keep));
             index.erase(lru.back().first);
             lru.pop_back();
         }

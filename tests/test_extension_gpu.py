@@ -127,3 +127,14 @@ def test_plans_outlive_their_place_in_the_table(cuda_device):
     for th in threads:
         th.join()
     assert not wrong, wrong[:5]
+
+
+def test_list_views_of_one_storage(cuda_device):
+    # the same address, version, size and type, other strides: other lists
+    dev = cuda_device
+    rows, cols = lists(dev, [2, 4, 3], [6, 3, 4])
+    x = torch.randn((2, 24), device=dev)
+    for _ in range(2):
+        for r, c, want in ((rows[::2], cols[::2], ([2, 3], [6, 4])), (rows[:2], cols[:2], ([2, 4], [6, 3]))):
+            got = blockAttention.sparseBlockedSoftmax(x, r, c).cpu()
+            assert (got - O.block_softmax(x.cpu(), *map(np.array, want))).abs().max() < 1e-6

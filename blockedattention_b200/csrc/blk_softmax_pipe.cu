@@ -252,8 +252,9 @@ __device__ __forceinline__ void sp_stv(uint32_t body, int vi, const uint4& q) {
 // Every forward row is exp2(y) over its sum with y = (x - m) * sl, m the largest x of the row, or the smallest (NEG: the
 // kernel for negative scales).  The difference is taken before the product, so that y is rounded relative to itself: with
 // x * sl rounded first it is off by half a unit of m * sl (fp32 rows, measured against 64 bits: 5e-6 of the result for scores
-// around 200, 4e-4 around 20000; this form: below 1e-7 for both), and rows masked throughout with a type's lowest value
-// stay finite.
+// around 200, 4e-4 around 20000; this form: below 1.3e-7 for both), and rows masked throughout with a type's lowest value
+// stay finite.  (x - m overflows only where a row spans more than the largest number; y is then minus infinity, which is
+// right for any scale above 1e-37.)
 __device__ __forceinline__ void sp_exp2(float2& f) {
     f.x = blk_exp2(f.x);
     f.y = blk_exp2(f.y);
@@ -576,6 +577,27 @@ __device__ __forceinline__ float sp_cta_reduce(float v, bool is_max, float* red,
     return r;
 }
 
+// forward, one row longer than a window, from and to global memory by all computing warps (out of line, like fwd_row_far)
+template <typename IO, bool NEG, int NW>
+__device__ __noinline__ void fwd_wide_row(const typename IO::E* src, typename IO::E* dst, int cols, float sl, float* red, int tid) {
+    constexpr int NT = 32 * NW;
+    constexpr float SIGN = NEG ? -1.f : 1.f;
+    const int warp = tid >> 5, lane = tid & 31;
+    float m = -INFINITY;
+    for (int c = tid; c < cols; c += NT) m = fmaxf(m, SIGN * IO::ld(src[c]));
+    m = SIGN * sp_cta_reduce<NW>(m, true, red, warp, lane);
+    auto normalise = [&](auto y) {
+        float sum = 0.f;
+        for (int c = tid; c < cols; c += NT) sum += blk_exp2(y(IO::ld(src[c])));
+        sum = sp_cta_reduce<NW>(sum, false, red, warp, lane);
+        const float inv = 1.f / sum;
+        for (int c = tid; c < cols; c += NT) dst[c] = IO::st(blk_exp2(y(IO::ld(src[c]))) * inv);
+    };
+    const float mx = m * sl;
+    if (fabsf(mx) <= sp_near<SpIO32>()) normalise([&](float x) { return fmaf(x, sl, -mx); });
+    else normalise([&](float x) { return (x - m) * sl; });
+}
+
 // A window in its stage.
 struct SpWin {
     int64_t e0;   // its first element in the buffers
@@ -722,15 +744,7 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
                 const int64_t e0 = win.e0;
                 constexpr int NT = 32 * NW;
                 if (!BWD) {
-                    constexpr float SIGN = NEG ? -1.f : 1.f;
-                    float m = -INFINITY;
-                    for (int c = tid; c < cols; c += NT) m = fmaxf(m, SIGN * IO::ld(g0[e0 + c]));
-                    m = SIGN * sp_cta_reduce<NW>(m, true, red, warp, lane);
-                    float sum = 0.f;
-                    for (int c = tid; c < cols; c += NT) sum += blk_exp2((IO::ld(g0[e0 + c]) - m) * sl);
-                    sum = sp_cta_reduce<NW>(sum, false, red, warp, lane);
-                    const float inv = 1.f / sum;
-                    for (int c = tid; c < cols; c += NT) gd[e0 + c] = IO::st(blk_exp2((IO::ld(g0[e0 + c]) - m) * sl) * inv);
+                    fwd_wide_row<IO, NEG, NW>(g0 + e0, gd + e0, cols, sl, red, tid);
                 } else {
                     float dot = 0.f;
                     for (int c = tid; c < cols; c += NT) dot += IO::ld(g0[e0 + c]) * IO::ld(g1[e0 + c]);

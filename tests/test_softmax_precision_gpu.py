@@ -47,6 +47,7 @@ def test_rows_masked_with_the_lowest_value(cuda_device, dtype, scale):
     for t in x:
         t[0] = low              # a row masked throughout: uniform, as torch.softmax has it
         t[1, ::2] = low         # every other column masked (all of a single column)
+        t[2, 0], t[2, -1] = -low, low   # the whole range of the type in one row
     for a, t, c in zip(softmax(x, rows, COLS, scale, cuda_device), x, COLS):
         want = torch.softmax(t.double() * scale, -1)
         assert torch.isfinite(a).all(), c

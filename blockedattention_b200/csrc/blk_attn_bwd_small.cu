@@ -68,6 +68,8 @@ blk_attn_bwd_small_kernel(const BlkAttnBwdSmallParams p) {
     const uint32_t unit = blockIdx.x, item = unit / (uint32_t)p.H;
     const int head = (int)(unit - item * (uint32_t)p.H);
     const BlkFlashItem it = p.items[item];
+    blk_grid_ready();
+    blk_grid_wait();
     const int M = it.M, N = it.N, Mb = (M + 15) >> 4, Nb = (N + 15) >> 4;
     const int64_t offQ = ((int64_t)head * p.rows_q + it.rowQ) * D, offK = ((int64_t)head * p.rows_kv + it.rowKV) * D;
 
@@ -216,8 +218,7 @@ cudaError_t launch(const BlkAttnBwdSmallParams& p, cudaStream_t st) {
     auto kern = blk_attn_bwd_small_kernel<Tag, D, R>;
     cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), SB<D, R>::SMEM);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)((int64_t)p.num_items * p.H), SB<D, R>::WARPS * 32, SB<D, R>::SMEM, st>>>(p);
-    return cudaGetLastError();
+    return blk_launch(true, kern, (unsigned)((int64_t)p.num_items * p.H), SB<D, R>::WARPS * 32, SB<D, R>::SMEM, st, p);
 }
 
 }  // namespace

@@ -152,6 +152,8 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    blk_grid_ready();
+    blk_grid_wait();
 
     uint32_t item = 0;  // items begun by this warp
     int4 ia, ib;
@@ -569,8 +571,7 @@ cudaError_t launch(const BlkFlashBwdParams& p, const CUtensorMap* maps, int sms,
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_items * p.H;
     const dim3 grid((unsigned)(total < sms ? total : sms)), block(BW_THREADS);
-    kern<<<grid, block, BL<D>::SMEM_BYTES, st>>>(p, maps[0], maps[1], maps[2], maps[3]);
-    return cudaGetLastError();
+    return blk_launch(total <= 12 * (int64_t)sms, kern, grid, block, BL<D>::SMEM_BYTES, st, p, maps[0], maps[1], maps[2], maps[3]);
 }
 
 }  // namespace

@@ -220,6 +220,8 @@ blk_attn_umma_kernel(const BlkFlashParams p, const __grid_constant__ CUtensorMap
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    blk_grid_ready();
+    blk_grid_wait();
 
     // (the trade of registers is between whole warpgroups)
     if (warp >= 4 && warp < 12) {
@@ -564,8 +566,7 @@ cudaError_t launch(const BlkFlashParams& p, const CUtensorMap& mq, const CUtenso
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_pairs * p.H;
     const dim3 grid((unsigned)(total < sms ? total : sms)), block(FA_THREADS);
-    kern<<<grid, block, FL<D>::SMEM_BYTES, st>>>(p, mq, mk, mv);
-    return cudaGetLastError();
+    return blk_launch(total <= 12 * (int64_t)sms, kern, grid, block, FL<D>::SMEM_BYTES, st, p, mq, mk, mv);
 }
 
 }  // namespace

@@ -63,6 +63,13 @@ __device__ __forceinline__ void blk_mma16816<BlkBf16Tag>(float (&d)[4], uint32_t
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// A kernel may be resident before the one in front of it in the stream has finished (blk_launch).  Before its first access to
+// memory that another kernel writes or reads it waits for that one (and, as every kernel does, for all before it); work tables of
+// a plan are there before any launch and may be read earlier.  blk_grid_ready lets the next kernel of the stream come: to be called
+// when the block holds all it will ever need of its SM (tensor memory), or the next one's blocks could take what it waits for.
+__device__ __forceinline__ void blk_grid_ready() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void blk_grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t blk_smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }

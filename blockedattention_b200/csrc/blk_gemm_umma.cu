@@ -313,6 +313,8 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    blk_grid_ready();
+    blk_grid_wait();
     const uint32_t lim = p.spin_limit ? p.spin_limit : BLK_UMMA_SPIN_LIMIT;
     auto item_wait = [&](uint32_t n) { return mbar_wait(item_full(n), (n / UM_ITEMS) & 1u, abort_flag, 11, lim); };
 
@@ -749,8 +751,7 @@ cudaError_t launch(const BlkUmmaParams& p, const UmMaps& maps, int sms, cudaStre
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_items * p.H;
     const dim3 grid((unsigned)(total < sms ? total : sms)), block(UL<WIDE>::THREADS);
-    kern<<<grid, block, UL<WIDE>::SMEM_BYTES, st>>>(p, maps);
-    return cudaGetLastError();
+    return blk_launch(total <= (WIDE ? 4 : 24) * (int64_t)sms, kern, grid, block, UL<WIDE>::SMEM_BYTES, st, p, maps);
 }
 
 }  // namespace

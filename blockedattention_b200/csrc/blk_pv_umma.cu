@@ -188,6 +188,8 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    blk_grid_ready();
+    blk_grid_wait();
 
     if (warp == 0) {
         // ---------------- producer: value tiles ----------------
@@ -415,8 +417,7 @@ cudaError_t launch(const BlkPvParams& p, const CUtensorMap& mv, int sms, cudaStr
     if (e != cudaSuccess) return e;
     const int64_t total = (int64_t)p.num_items * p.H;
     const dim3 grid((unsigned)(total < sms ? total : sms)), block(PV_THREADS);
-    kern<<<grid, block, PVL<D>::SMEM_BYTES, st>>>(p, mv);
-    return cudaGetLastError();
+    return blk_launch(total <= 12 * (int64_t)sms, kern, grid, block, PVL<D>::SMEM_BYTES, st, p, mv);
 }
 
 }  // namespace

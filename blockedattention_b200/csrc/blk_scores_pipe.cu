@@ -444,6 +444,8 @@ blk_scores_pipe_kernel(const BlkPackParams p, const __grid_constant__ PackMaps m
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // before the first tensor-map copy lands there
     }
     __syncthreads();
+    blk_grid_ready();
+    blk_grid_wait();
 
     // The CTA's u-th unit is (pack, head) number w = blockIdx.x + u * G, pack = w / H, head = w % H; it uses ring
     // slot u % P_SLOTS and belongs to consumer group u % P_GROUPS (so each group owns P_SLOTS / P_GROUPS slots).
@@ -549,8 +551,7 @@ cudaError_t launch_pipe(const BlkPackParams& p_in, int sms, cudaStream_t st) {
     auto go = [&](auto kern, int smem) -> cudaError_t {
         cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
-        kern<<<grid, block, smem, st>>>(p, mA, mB, mV);
-        return cudaGetLastError();
+        return blk_launch(true, kern, grid, block, smem, st, p, mA, mB, mV);
     };
     if (attn)
         return p.scale < 0.f ? go(blk_scores_pipe_kernel<Tag, true, true, true>, PL<true>::SMEM_BYTES)

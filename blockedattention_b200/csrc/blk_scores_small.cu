@@ -203,6 +203,8 @@ __global__ void __launch_bounds__(SW * 32, MinBlocks<NTMAX>::value) blk_scores_s
     const bool flip = p.scale < 0.f;
     const float sl = SOFTMAX ? fabsf(p.scale) * BLK_LOG2E : p.scale;
     unsigned char* strip = strips + warp * STRIP;
+    blk_grid_ready();
+    blk_grid_wait();
 
     for (uint32_t w = blockIdx.x * SW + warp; w < total; w += stride) {
         const uint32_t item = w / H, head = w - item * H;
@@ -230,8 +232,7 @@ cudaError_t launch_variant(const BlkSmallParams& p, int sms, cudaStream_t st) {
             cudaError_t e = blk_func_smem(reinterpret_cast<const void*>(kern), (int)smem);
             if (e != cudaSuccess) return e;
         }
-        kern<<<grid, block, smem, st>>>(p);
-        return cudaGetLastError();
+        return blk_launch(true, kern, grid, block, smem, st, p);
     };
     if (sm && !o32) return go(blk_scores_small_kernel<Tag, KC, NTMAX, true, false>);
     if (sm && o32) return go(blk_scores_small_kernel<Tag, KC, NTMAX, true, true>);

@@ -659,6 +659,8 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    blk_grid_ready();
+    blk_grid_wait();
 
     const E* g0 = reinterpret_cast<const E*>(p.in0);
     const E* g1 = reinterpret_cast<const E*>(p.in1);
@@ -823,8 +825,7 @@ cudaError_t blk_launch_softmax_pipe(const BlkSmxPipeParams& p, int dtype, int ba
         if (e != cudaSuccess) return e;
         const int64_t resident = (int64_t)sms * S::CTAS;
         const dim3 grid((unsigned)(total < resident ? total : resident)), block(S::THREADS);
-        kern<<<grid, block, smem, st>>>(p);
-        return cudaGetLastError();
+        return blk_launch(true, kern, grid, block, smem, st, p);
     };
     auto forward = [&](auto io) {
         typedef decltype(io) IO;

@@ -1,0 +1,86 @@
+"""Kernels that start before the one in front of them has ended: every launch that reads what the last one wrote, or writes what
+it read, gives what it gives with the device idle in between, bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _lists(rs, S, lo, hi):
+    return rs.randint(lo, hi + 1, S).astype(np.int64)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("S,lo,hi,H,d", [(1, 1, 1, 1, 64), (32, 4, 32, 1, 32), (24, 1, 64, 4, 64), (6, 65, 300, 2, 64), (3, 100, 700, 2, 128)])
+def test_chains_without_waiting(dtype, S, lo, hi, H, d):
+    from blockedattention_b200 import blockGEMM, blockSoftmax
+
+    rs = np.random.RandomState(S + hi)
+    n = _lists(rs, S, lo, hi)
+    dl = np.full_like(n, d)
+    g = torch.Generator("cuda").manual_seed(7)
+    xs = [torch.randn((H, int(n.sum()) * d), device="cuda", generator=g).to(dtype) for _ in range(6)]
+
+    def step(x, y, wait):
+        # scores, their softmax, the product with y, which is the next step's operand
+        s = blockGEMM(x, y, None, None, None, n, n, dl, scale=d ** -0.5)
+        if wait:
+            torch.cuda.synchronize()
+        p = blockSoftmax(s, n, n)
+        if wait:
+            torch.cuda.synchronize()
+        o = blockGEMM(p, y, None, None, None, n, dl, n, False, True)
+        if wait:
+            torch.cuda.synchronize()
+        return s, p, o
+
+    def run(wait):
+        out, x = [], xs[0]
+        for y in xs[1:]:
+            r = step(x, y, wait)
+            out += r
+            x = r[2]
+        return out
+
+    expect = run(True)
+    for _ in range(3):
+        for a, b in zip(expect, run(False)):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("hi,d", [(40, 64), (300, 64), (300, 128)])
+def test_training_steps_without_waiting_and_captured(hi, d):
+    from blockedattention_b200 import blockAttention
+
+    rs = np.random.RandomState(hi)
+    n = _lists(rs, 12, 1, hi)
+    H, scale = 2, d ** -0.5
+    g = torch.Generator("cuda").manual_seed(3)
+    q, k, v, go = (torch.randn((H, int(n.sum()) * d), device="cuda", generator=g).half() for _ in range(4))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+
+    def step():
+        o = blockAttention(q, k, v, n, n, scale=scale, d=d)
+        return (o.detach(),) + torch.autograd.grad(o, (q, k, v), go)
+
+    expect = [x.clone() for x in step()]
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for a, b in zip(expect, step()):
+            assert torch.equal(a, b)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = step()
+    for _ in range(3):
+        for t in got:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(expect, got):
+            assert torch.equal(a, b)

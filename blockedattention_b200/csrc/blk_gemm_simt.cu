@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(SNT) blk_gemm_simt_kernel(const BlkSimtParams 
     const int head = (int)(bid / p.num_items);
     const BlkTileItem it = p.items[bid % p.num_items];
     const BlkSeg sd = p.segs[it.seg];
-    blk_grid_ready();
+    blk_grid_ready_if_few();
     blk_grid_wait();
     const float* gA = p.A + (int64_t)head * p.Dm1 + sd.offA;
     const float* gB = p.B + (int64_t)head * p.Dm2 + sd.offB;
@@ -93,8 +93,8 @@ cudaError_t blk_launch_gemm_simt(const BlkSimtParams& p, cudaStream_t st) {
     const int64_t blocks = (int64_t)p.num_items * p.H;
     if (blocks == 0) return cudaSuccess;
     const dim3 grid((unsigned)blocks), block(SNT);
-    if (!p.ta && !p.tb) return blk_launch(true, blk_gemm_simt_kernel<false, false>, grid, block, 0, st, p);
-    if (!p.ta && p.tb) return blk_launch(true, blk_gemm_simt_kernel<false, true>, grid, block, 0, st, p);
-    if (p.ta && !p.tb) return blk_launch(true, blk_gemm_simt_kernel<true, false>, grid, block, 0, st, p);
-    return blk_launch(true, blk_gemm_simt_kernel<true, true>, grid, block, 0, st, p);
+    if (!p.ta && !p.tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_simt_kernel<false, false>, grid, block, 0, st, p);
+    if (!p.ta && p.tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_simt_kernel<false, true>, grid, block, 0, st, p);
+    if (p.ta && !p.tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_simt_kernel<true, false>, grid, block, 0, st, p);
+    return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_simt_kernel<true, true>, grid, block, 0, st, p);
 }

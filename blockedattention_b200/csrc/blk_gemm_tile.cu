@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(SOFTMAX ? NT : NT_SC, (SOFTMAX || TA || TB) ? 
     const BlkTileRec rec = p.recs[bid % p.num_items];
     const BlkTileItem it = rec.it;
     const BlkSeg sd = rec.sd;
-    blk_grid_ready();
+    blk_grid_ready_if_few();
     blk_grid_wait();
     const int64_t baseA = (int64_t)head * p.Dm1 + sd.offA, baseB = (int64_t)head * p.Dm2 + sd.offB;
     const int64_t cbase = (int64_t)head * p.Dout + sd.offC;
@@ -366,10 +366,10 @@ template <typename Tag, bool SOFTMAX>
 cudaError_t launch_epi(const BlkGemmParams& p, int ta, int tb, cudaStream_t st) {
     const int64_t blocks = (int64_t)p.num_items * p.H;
     const dim3 grid((unsigned)blocks), block(SOFTMAX ? NT : NT_SC);
-    if (!ta && !tb) return blk_launch(true, blk_gemm_tile_kernel<Tag, false, false, SOFTMAX>, grid, block, 0, st, p);
-    if (!ta && tb) return blk_launch(true, blk_gemm_tile_kernel<Tag, false, true, SOFTMAX>, grid, block, 0, st, p);
-    if (ta && !tb) return blk_launch(true, blk_gemm_tile_kernel<Tag, true, false, SOFTMAX>, grid, block, 0, st, p);
-    return blk_launch(true, blk_gemm_tile_kernel<Tag, true, true, SOFTMAX>, grid, block, 0, st, p);
+    if (!ta && !tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_tile_kernel<Tag, false, false, SOFTMAX>, grid, block, 0, st, p);
+    if (!ta && tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_tile_kernel<Tag, false, true, SOFTMAX>, grid, block, 0, st, p);
+    if (ta && !tb) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_tile_kernel<Tag, true, false, SOFTMAX>, grid, block, 0, st, p);
+    return blk_launch(grid.x <= BLK_EARLY_GRID, blk_gemm_tile_kernel<Tag, true, true, SOFTMAX>, grid, block, 0, st, p);
 }
 
 template <typename Tag>

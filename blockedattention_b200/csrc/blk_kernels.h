@@ -166,6 +166,10 @@ struct BlkSmxParams {
     float scale;
 };
 
+// Grids of one-shot blocks up to which blk_launch is asked for an early start: several waves of them run up to an eighth slower
+// when launched that way (385 products of 256..1216 rows on the staged kernel 5238 -> 5880 us).
+constexpr unsigned BLK_EARLY_GRID = 296;
+
 // Launches a kernel that waits by itself for the one in front of it (blk_grid_wait): its start -- the launch, barriers, tensor
 // memory -- overlaps the end of that one.  Passes one after the other, us: 32 fp32 products and softmaxes of at most 32 x 32 x 32 (two
 // launches) 12.3 -> 8.7, attention of 16 graphs 8.2 -> 6.0, forward and backward of 1024 graphs (three launches) 84.5 -> 79.1.

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(SMX_THREADS) blk_softmax_kernel(const BlkSmxPa
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t bid = blockIdx.x;
     const int head = (int)(bid / p.num_chunks);
-    blk_grid_ready();
+    blk_grid_ready_if_few();
     blk_grid_wait();  // (the table of a call without plan memory goes up in the stream)
     const BlkSmxChunk ch = p.chunks[bid % p.num_chunks];
     const int64_t e0 = (int64_t)head * p.D + ch.off;
@@ -197,9 +197,9 @@ cudaError_t blk_launch_softmax(const BlkSmxParams& p, int dtype, cudaStream_t st
     const int64_t blocks = (int64_t)p.num_chunks * p.H;
     if (blocks == 0) return cudaSuccess;
     const dim3 grid((unsigned)blocks), block(SMX_THREADS);
-    if (dtype == BLK_F16) return blk_launch(true, blk_softmax_kernel<SmxIO16<BlkHalfTag>>, grid, block, 0, st, p);
-    if (dtype == BLK_BF16) return blk_launch(true, blk_softmax_kernel<SmxIO16<BlkBf16Tag>>, grid, block, 0, st, p);
-    return blk_launch(true, blk_softmax_kernel<SmxIO32>, grid, block, 0, st, p);
+    if (dtype == BLK_F16) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_softmax_kernel<SmxIO16<BlkHalfTag>>, grid, block, 0, st, p);
+    if (dtype == BLK_BF16) return blk_launch(grid.x <= BLK_EARLY_GRID, blk_softmax_kernel<SmxIO16<BlkBf16Tag>>, grid, block, 0, st, p);
+    return blk_launch(grid.x <= BLK_EARLY_GRID, blk_softmax_kernel<SmxIO32>, grid, block, 0, st, p);
 }
 
 // ---------------------------------------------------------------------------

@@ -95,7 +95,8 @@ int upload_plan(blk_plan* p) {
     add(nullptr, nrecs * sizeof(BlkTileRec), reinterpret_cast<void**>(&p->d_tile_recs));
     add_vec(p->simt_items, &p->d_simt_items);
     for (int b = 0; b < BLK_SMALL_BUCKETS; ++b) add_vec(p->small_items[b], &p->d_small_items[b]);
-    add_vec(p->umma_items, &p->d_umma_items);
+    if (p->stream_items.empty()) add_vec(p->umma_items, &p->d_umma_items);
+    add_vec(p->stream_items, &p->d_stream_items);
     add_vec(p->pv_items, &p->d_pv_items);
     add_vec(p->flash_pairs, &p->d_flash_pairs);
     add_vec(p->packs, &p->d_packs);
@@ -501,6 +502,7 @@ static int attention_plan_impl(blk_plan_t** plan, const int64_t* M, const int64_
         packs = rc == BLK_OK && p->small_pipe && !p->packs.empty();
         p->tile_items.clear();
         p->umma_items.clear();
+        p->stream_items.clear();
         p->simt_items.clear();
         if (!packs) {
             p->packs.clear(); p->pack_blocks.clear(); p->small_pipe = 0; p->small_segments = 0;
@@ -860,7 +862,8 @@ static int gemm_run_impl(const blk_plan* p, const void* mat1, const void* mat2, 
     if (!p->umma_items.empty()) {
         BlkUmmaParams up{};
         up.C = out;
-        up.items = p->d_umma_items;
+        const bool streams = !p->stream_items.empty();
+        up.items = streams ? p->d_stream_items : p->d_umma_items;
         up.Dout = p->Dout;
         up.num_items = (int)p->umma_items.size();
         up.H = (int)p->H;
@@ -876,7 +879,7 @@ static int gemm_run_impl(const blk_plan* p, const void* mat1, const void* mat2, 
         }
         const BlkUmmaOperand opA{mat1, p->Dm1, p->umma_viewsA.data(), (int)p->umma_viewsA.size(), layA};
         const BlkUmmaOperand opB{mat2, p->Dm2, p->umma_viewsB.data(), (int)p->umma_viewsB.size(), layB};
-        if ((e = blk_launch_gemm_umma(up, opA, opB, p->num_sms, st)) != cudaSuccess)
+        if ((e = (streams ? blk_launch_scores_umma : blk_launch_gemm_umma)(up, opA, opB, p->num_sms, st)) != cudaSuccess)
             return cuda_fail("tcgen05 GEMM launch", e);
     }
     if (!p->pv_items.empty()) {

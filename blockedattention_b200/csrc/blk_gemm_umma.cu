@@ -52,6 +52,7 @@
 
 #include "blk_device.cuh"
 #include "blk_kernels.h"
+#include "blk_umma_items.cuh"
 #include "blk_umma_ptx.cuh"
 
 namespace {
@@ -95,33 +96,6 @@ struct __align__(16) Work {
 };
 static_assert(sizeof(Work) == 64, "Work is written as four 16-byte vectors");
 
-// The tensor maps of the operands' views (BlkUmmaView), passed as one kernel parameter.
-struct UmMaps {
-    CUtensorMap a[BLK_UMMA_VIEWS];
-    CUtensorMap b[BLK_UMMA_VIEWS];
-};
-
-// Item n of a CTA's walk, from global memory.  Odd rounds run through the CTAs backwards, so that with the items sorted by
-// cost no CTA always gets the heaviest of a round.  Only the last round can point past the end, so a CTA that gets nothing
-// there has nothing left either.
-__device__ __forceinline__ bool fetch_item(const BlkUmmaParams& p, uint32_t n, BlkUmmaItem& it, int& head) {
-    const uint32_t w = n * gridDim.x + ((n & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
-    if (w >= (uint32_t)p.num_items * (uint32_t)p.H) return false;
-    const uint32_t item = w / (uint32_t)p.H;
-    head = (int)(w - item * (uint32_t)p.H);
-    const int4* src = reinterpret_cast<const int4*>(p.items + item);
-    int4* dst = reinterpret_cast<int4*>(&it);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
-    return true;
-}
-// Rows of an item's block.  A block that fills less than four quarters of the accumulator lanes is put into other
-// quarters from item to item (its operand rows are loaded that much earlier): a quarter is one scheduler's warps.
-__device__ __forceinline__ int item_rows(const BlkUmmaItem& it, uint32_t n) {
-    const int rows = min(it.M - it.tm * UM_BM, UM_BM);
-    const uint32_t slack = 4u - (uint32_t)((rows + 31) >> 5);
-    return rows | (int)((n % (slack + 1u)) << 8);
-}
 template <bool SOFT, bool WIDE>
 __device__ __forceinline__ void publish(const BlkUmmaParams& p, Work* dst, const BlkUmmaItem& it, int head, uint32_t n,
                                         bool valid, const BlkUmmaItem& nx, bool nx_valid) {
@@ -356,7 +330,8 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
         if (elect_one() && !p.stall) {
             BlkUmmaItem it{}, nx{};  // records n and n + 1
             int head = 0, nhead = 0;
-            bool have = fetch_item(p, 0, it, head), nhave = have && fetch_item(p, 1, nx, nhead);
+            bool have = fetch_item(p, 0, gridDim.x, blockIdx.x, it, head),
+                 nhave = have && fetch_item(p, 1, gridDim.x, blockIdx.x, nx, nhead);
 #pragma unroll 1
             for (uint32_t n = 0;; ++n) {
                 if (!mbar_wait(item_empty(n), ((n / UM_ITEMS) & 1u) ^ 1u, abort_flag, 12, lim)) break;
@@ -366,7 +341,7 @@ blk_gemm_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps maps)
                 it = nx;
                 head = nhead;
                 have = nhave;
-                if (nhave) nhave = fetch_item(p, n + 2u, nx, nhead);
+                if (nhave) nhave = fetch_item(p, n + 2u, gridDim.x, blockIdx.x, nx, nhead);
             }
         }
     } else if (warp == 1) {
@@ -848,7 +823,7 @@ namespace {
 struct LaunchKey {
     const void *a, *b;
     int64_t Da, Db, H;
-    int na, nb, bf16, ga, gb, wide;
+    int na, nb, bf16, ga, gb, box_a, box_b;
     BlkOperandLayout layA, layB;
     BlkUmmaView va[BLK_UMMA_VIEWS], vb[BLK_UMMA_VIEWS];
 };
@@ -859,7 +834,7 @@ uint64_t g_launch_clock = 0;
 std::mutex g_launch_mu;
 bool same_key(const LaunchKey& x, const LaunchKey& y) {
     if (x.a != y.a || x.b != y.b || x.Da != y.Da || x.Db != y.Db || x.H != y.H || x.na != y.na || x.nb != y.nb ||
-        x.bf16 != y.bf16 || x.wide != y.wide || x.ga != y.ga || x.gb != y.gb)
+        x.bf16 != y.bf16 || x.box_a != y.box_a || x.box_b != y.box_b || x.ga != y.ga || x.gb != y.gb)
         return false;
     auto lay_eq = [](const BlkOperandLayout& p, const BlkOperandLayout& q) {
         return p.rows == q.rows && p.row_stride == q.row_stride && p.head_stride == q.head_stride;
@@ -873,22 +848,17 @@ bool same_key(const LaunchKey& x, const LaunchKey& y) {
 }
 }  // namespace
 
-cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand& A, const BlkUmmaOperand& B, int sms,
-                                 cudaStream_t st) {
-    if ((int64_t)p_in.num_items * p_in.H == 0) return cudaSuccess;
-    if (A.num_views < 1 || B.num_views < 1 || A.num_views > BLK_UMMA_VIEWS || B.num_views > BLK_UMMA_VIEWS) return cudaErrorInvalidValue;
-    BlkUmmaParams p = p_in;
-    static thread_local LaunchKey key;   // these are kilobytes: not on the stack of a caller's thread
-    static thread_local UmMaps maps;
+bool blk_umma_maps(BlkUmmaParams& p, const BlkUmmaOperand& A, const BlkUmmaOperand& B, int box_a, int box_b, UmMaps& maps) {
+    if (A.num_views < 1 || B.num_views < 1 || A.num_views > BLK_UMMA_VIEWS || B.num_views > BLK_UMMA_VIEWS) return false;
+    static thread_local LaunchKey key;   // kilobytes: not on the stack of a caller's thread
     key.a = A.base; key.b = B.base; key.Da = A.D; key.Db = B.D; key.H = p.H;
     key.na = A.num_views; key.nb = B.num_views; key.bf16 = p.bf16;
-    key.wide = p.wide;  // the box of the second operand
+    key.box_a = box_a; key.box_b = box_b;
     key.ga = A.given != nullptr; key.gb = B.given != nullptr;
     if (A.given) key.layA = *A.given;
     if (B.given) key.layB = *B.given;
     for (int i = 0; i < A.num_views; ++i) key.va[i] = A.views[i];
     for (int i = 0; i < B.num_views; ++i) key.vb[i] = B.views[i];
-    bool hit = false;
     {
         std::lock_guard<std::mutex> g(g_launch_mu);
         for (LaunchSlot& sl : g_launch_slots)
@@ -897,40 +867,46 @@ cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand
                 maps = sl.maps;
                 p.head_firstA = sl.hfA;
                 p.head_firstB = sl.hfB;
-                hit = true;
-                break;
+                return true;
             }
     }
-    if (!hit) {
-        // every view of an operand has the same order of its strides, so the same order of coordinates
-        auto encode = [&](const BlkUmmaOperand& op, CUtensorMap* out, int box_rows, int* head_first) {
-            if (op.given && (op.num_views != 1 || op.views[0].residue != 0)) return false;
-            for (int v = 0; v < op.num_views; ++v) {
-                const BlkUmmaView& vw = op.views[v];
-                const BlkOperandLayout lay = op.given ? *op.given : BlkOperandLayout{(op.D - vw.residue) / vw.K, vw.K, op.D};
-                int hf = 0;
-                if (!blk_make_row_map(&out[v], static_cast<const unsigned char*>(op.base) + 2 * vw.residue, p.bf16, vw.K, p.H, lay,
-                                      UM_BK, box_rows, &hf))
-                    return false;
-                if (v > 0 && hf != *head_first) return false;
-                *head_first = hf;
-            }
-            return true;
-        };
-        if (!encode(A, maps.a, UM_BM, &p.head_firstA) || !encode(B, maps.b, key.wide ? UL<true>::BN : UL<false>::BN, &p.head_firstB)) return cudaErrorInvalidValue;
-        std::lock_guard<std::mutex> g(g_launch_mu);
-        LaunchSlot* victim = &g_launch_slots[0];
-        for (LaunchSlot& sl : g_launch_slots) {
-            if (!sl.used) { victim = &sl; break; }
-            if (sl.stamp < victim->stamp) victim = &sl;
+    // every view of an operand has the same order of its strides, so the same order of coordinates
+    auto encode = [&](const BlkUmmaOperand& op, CUtensorMap* out, int box_rows, int* head_first) {
+        if (op.given && (op.num_views != 1 || op.views[0].residue != 0)) return false;
+        for (int v = 0; v < op.num_views; ++v) {
+            const BlkUmmaView& vw = op.views[v];
+            const BlkOperandLayout lay = op.given ? *op.given : BlkOperandLayout{(op.D - vw.residue) / vw.K, vw.K, op.D};
+            int hf = 0;
+            if (!blk_make_row_map(&out[v], static_cast<const unsigned char*>(op.base) + 2 * vw.residue, p.bf16, vw.K, p.H, lay,
+                                  64, box_rows, &hf))
+                return false;
+            if (v > 0 && hf != *head_first) return false;
+            *head_first = hf;
         }
-        victim->key = key;
-        victim->maps = maps;
-        victim->hfA = p.head_firstA;
-        victim->hfB = p.head_firstB;
-        victim->stamp = ++g_launch_clock;
-        victim->used = true;
+        return true;
+    };
+    if (!encode(A, maps.a, box_a, &p.head_firstA) || !encode(B, maps.b, box_b, &p.head_firstB)) return false;
+    std::lock_guard<std::mutex> g(g_launch_mu);
+    LaunchSlot* victim = &g_launch_slots[0];
+    for (LaunchSlot& sl : g_launch_slots) {
+        if (!sl.used) { victim = &sl; break; }
+        if (sl.stamp < victim->stamp) victim = &sl;
     }
+    victim->key = key;
+    victim->maps = maps;
+    victim->hfA = p.head_firstA;
+    victim->hfB = p.head_firstB;
+    victim->stamp = ++g_launch_clock;
+    victim->used = true;
+    return true;
+}
+
+cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p_in, const BlkUmmaOperand& A, const BlkUmmaOperand& B, int sms,
+                                 cudaStream_t st) {
+    if ((int64_t)p_in.num_items * p_in.H == 0) return cudaSuccess;
+    BlkUmmaParams p = p_in;
+    static thread_local UmMaps maps;
+    if (!blk_umma_maps(p, A, B, UM_BM, p.wide ? UL<true>::BN : UL<false>::BN, maps)) return cudaErrorInvalidValue;
     auto run = [&](auto tag) {
         typedef decltype(tag) Tag;
         if (p.epi == BLK_EPI_SOFTMAX)

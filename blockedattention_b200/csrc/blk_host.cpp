@@ -571,6 +571,38 @@ int blk_build_gemm_schedule(blk_plan* p) {
     p->umma_wide = 0;
     for (const BlkUmmaItem& it : p->umma_items)
         if (it.nch) p->umma_wide = 1;
+    // Short contractions go to the kernel of independent streams (blk_scores_umma.cu) where there are tiles enough for all
+    // streams to be busy and in different phases; below that the other kernel, whose warps share an item, is done sooner.
+    // With a softmax it is the better one only for rows that the other kernel computes twice as well (beyond 512 columns), which
+    // have to carry most of the work, and for K up to 64 (four streams; three are slower).  us, other kernel -> streams:
+    // plain bf16 scores, K = 64: 3 600 tiles 20.7 -> 24.8, 7 700 49.4 -> 47.7, 17 000 75 -> 65, 43 000 211 -> 150; fp32 of
+    // mixed K up to 128: 3 900 38.5 -> 43.3, 7 700 71.2 -> 70.5, 29 000 271 -> 233; softmax, K = 64: rows up to 512
+    // 170 -> 184, up to 2048 242 -> 222 (and 898 -> 755 for four times as many), K = 128 267 -> 288.
+    p->stream_items.clear();
+    if (!p->umma_items.empty() && !p->umma_wide) {
+        int64_t K = 0, tiles = 0, tiles_long = 0;
+        for (const BlkUmmaView& v : p->umma_viewsA) K = std::max<int64_t>(K, v.K);
+        for (const BlkUmmaItem& it : p->umma_items) {
+            const int64_t t = ((int64_t)it.N + 63) / 64 * p->H;
+            tiles += t;
+            if (it.N > 512) tiles_long += t;
+        }
+        const char* e = std::getenv("BLK_UMMA_STREAMS");  // 0 or 1: the choice, for comparisons
+        const bool softmax = p->epi == BLK_EPI_SOFTMAX;
+        const bool use = K <= (softmax ? BLK_STREAM_MAXK / 2 : BLK_STREAM_MAXK) &&
+                         (e && e[0] ? e[0] != '0' : tiles >= BLK_STREAM_MIN_TILES && (!softmax || 2 * tiles_long >= tiles));
+        if (use) {
+            std::vector<std::pair<uint64_t, int32_t>> order(p->umma_items.size());
+            for (size_t i = 0; i < order.size(); ++i) {
+                const BlkUmmaItem& it = p->umma_items[i];
+                const uint64_t cost = (uint64_t)(it.N + 63) / 64 * 2 + 2 + (it.K > 64);  // tiles, and about one more to get started
+                order[i] = std::make_pair(~cost, (int32_t)i);
+            }
+            sort_by_key(order);
+            p->stream_items.reserve(order.size());
+            for (const auto& o : order) p->stream_items.push_back(p->umma_items[o.second]);
+        }
+    }
     // longest contractions first for the same reason
     std::stable_sort(p->pv_items.begin(), p->pv_items.end(), [](const BlkPvItem& a, const BlkPvItem& b) { return a.K > b.K; });
     // K = 64 with 16-bit output: the small segments run on the pipelined kernel, grouped into packs of

@@ -112,6 +112,9 @@ struct BlkUmmaItem {
 };
 static_assert(sizeof(BlkUmmaItem) == 48, "BlkUmmaItem layout");
 
+constexpr int64_t BLK_STREAM_MAXK = 128;      // longest contraction of the kernel of independent streams
+constexpr int64_t BLK_STREAM_MIN_TILES = 8000; // 128 x 64 tiles of a batch from which on it is used
+
 // One work item of the tcgen05 kernel for the product with a (K, D) second operand (P V): a 128-row block of the
 // first operand of one segment.
 struct BlkPvItem {
@@ -183,6 +186,8 @@ struct blk_plan {
     int64_t max_chunks = 0;                 // > 0: the softmax scheduler refuses batches that need more chunks
     int umma_K = 0;                         // K of the tcgen05 bin when it has one view per operand that starts at the
                                             // strip (the only case the strided entry takes); 0: no such bin; -1: several views
+    std::vector<BlkUmmaItem> stream_items;  // the tcgen05 items in the order of the kernel of independent streams, where that one runs
+    BlkUmmaItem* d_stream_items = nullptr;
     int umma_wide = 0;                      // tcgen05 items are single 256-column chunks (of the segments with long contractions)
     std::vector<BlkUmmaView> umma_viewsA, umma_viewsB;  // views of the operands the tcgen05 items refer to
     int small_K = 0;                        // uniform K of the small bin

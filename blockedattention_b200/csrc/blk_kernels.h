@@ -234,6 +234,9 @@ struct BlkUmmaOperand {
 };
 cudaError_t blk_launch_gemm_umma(const BlkUmmaParams& p, const BlkUmmaOperand& A, const BlkUmmaOperand& B, int sms,
                                  cudaStream_t st);
+// The same for contractions of at most BLK_STREAM_MAXK: independent streams of items (blk_scores_umma.cu).
+cudaError_t blk_launch_scores_umma(const BlkUmmaParams& p, const BlkUmmaOperand& A, const BlkUmmaOperand& B, int sms,
+                                   cudaStream_t st);
 cudaError_t blk_launch_pv_umma(const BlkPvParams& p, const void* V, int sms, cudaStream_t st);
 cudaError_t blk_launch_attn_umma(const BlkFlashParams& p, const void* q, const void* k, const void* v, int sms,
                                  cudaStream_t st);

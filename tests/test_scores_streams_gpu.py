@@ -1,0 +1,68 @@
+"""GPU: the kernel of independent streams (blk_scores_umma.cu) at the edges of its work split -- 64-column tiles, rows that begin and
+end anywhere in a 32-byte sector or share one, row blocks that fill one to four lane quarters, rows swept twice, contractions of
+one and two blocks -- against the oracle, with canaries around the result."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import O, assert_probs_close, assert_scores_close, packed_inputs
+from blockedattention_b200.plan import GemmPlan
+
+pytestmark = pytest.mark.gpu
+F16, BF16, F32 = torch.float16, torch.bfloat16, torch.float32
+M = [1, 31, 32, 33, 64, 65, 96, 97, 128, 129, 200, 5, 70, 300, 2, 16, 127, 40]
+N = [1, 5, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 191, 192, 200, 320, 511, 513]
+
+
+@pytest.fixture
+def streams(monkeypatch):
+    monkeypatch.setenv("BLK_UMMA_STREAMS", "1")
+    monkeypatch.setenv("BLK_DISABLE_SMALL", "1")
+    monkeypatch.setenv("BLK_FORCE_UMMA", "1")
+
+
+def run(dev, m, n, K, H, dtype, out_dtype, softmax, scale, shift):
+    A, B = packed_inputs(m, n, K, H, dtype, 11)
+    plan = GemmPlan(m, n, K, H, dtype, out_dtype, softmax=softmax, device=dev)
+    assert plan.summary["umma_items"] > 0 and plan.summary["tile_items"] == 0
+    buf = torch.full((H * plan.Dout + 64,), float("nan"), dtype=out_dtype, device=dev)
+    out = buf[shift:shift + H * plan.Dout].view(H, plan.Dout)
+    plan.run(A.to(dev), B.to(dev), out=out, scale=scale)
+    plan.check()
+    assert torch.isnan(buf[:shift]).all() and torch.isnan(buf[shift + H * plan.Dout:]).all()
+    if softmax:
+        assert_probs_close(out, O.block_scores(A, B, m, n, K, scale=scale), "softmax")
+    else:
+        assert_scores_close(out, O.block_gemm(A, B, m, n, K, scale=scale), "scores")
+
+
+@pytest.mark.parametrize("dtype,out_dtype", [(F16, F16), (BF16, BF16), (F16, F32)])
+@pytest.mark.parametrize("softmax,scale,k", [(True, 0.125, 64), (True, -0.11, 40), (False, 0.5, 16), (False, 1.0, 64), (False, -0.5, 72), (False, 0.3, 128)])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_tiles_sectors_and_quarters(cuda_device, streams, dtype, out_dtype, softmax, scale, k, shift):
+    n = N + N
+    m = [M[i % len(M)] for i in range(len(n))]
+    run(cuda_device, m, n, [k] * len(n), 3, dtype, out_dtype, softmax, scale, shift)
+
+
+@pytest.mark.parametrize("softmax", [False, True])
+def test_more_items_than_streams_and_mixed_contractions(cuda_device, streams, softmax):
+    rs = np.random.RandomState(5)
+    n = rs.randint(1, 300, 400).tolist()
+    m = rs.randint(1, 200, 400).tolist()
+    K = rs.choice([16, 32, 48, 64] if softmax else [16, 48, 64, 96, 128], 400).tolist()
+    run(cuda_device, m, n, K, 2, F16, F32, softmax, 0.2, 0)
+
+
+def test_masked_rows_and_far_scores(cuda_device, streams):
+    """References that move from tile to tile, and scores beyond what one reference covers."""
+    n, d, H = [700, 129], 64, 2
+    K = [d, d]
+    A, B = packed_inputs(n, n, K, H, BF16, 3)
+    plan = GemmPlan(n, n, K, H, BF16, softmax=True, device=cuda_device)
+    for scale in (3.0, -8.0):
+        out = plan.run(A.to(cuda_device), B.to(cuda_device), scale=scale)
+        plan.check()
+        assert_probs_close(out, O.block_scores(A, B, n, n, K, scale=scale), "softmax")
+    out = plan.run(A.to(cuda_device), B.to(cuda_device), scale=0.0).float()
+    assert torch.allclose(out[:, :700], torch.full_like(out[:, :700], 1 / 700), rtol=8e-3)

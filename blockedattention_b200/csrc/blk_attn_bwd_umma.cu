@@ -483,11 +483,7 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
 #pragma unroll
                 for (int i = 0; i < 32; i += 2)
                     v[i >> 1] = BlkCvt<Tag>::pack2(__uint_as_float(v[i]) * f, __uint_as_float(v[i + 1]) * f);
-                if (mine) {
-                    uint4* dst = reinterpret_cast<uint4*>(orow + c);
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) dst[cc] = make_uint4(v[4 * cc], v[4 * cc + 1], v[4 * cc + 2], v[4 * cc + 3]);
-                }
+                if (mine) blk_stg64(orow + c, v);
             }
             tc_fence_before();
             __syncwarp();

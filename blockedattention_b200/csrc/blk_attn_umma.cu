@@ -534,11 +534,7 @@ blk_attn_umma_kernel(const BlkFlashParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
                     for (int i = 0; i < 32; i += 2)
                         r[i >> 1] = BlkCvt<Tag>::pack2(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                    if (mine) {
-                        uint4* dst = reinterpret_cast<uint4*>(orow + c);
-#pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) dst[cc] = make_uint4(r[4 * cc], r[4 * cc + 1], r[4 * cc + 2], r[4 * cc + 3]);
-                    }
+                    if (mine) blk_stg64(orow + c, r);
                 }
                 tc_fence_before();
                 __syncwarp();

@@ -153,6 +153,23 @@ __device__ __forceinline__ void blk_sts_f32x2(uint32_t addr, float x, float y) {
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(x), "f"(y));
 }
 
+// 64 contiguous bytes of a lane, to 16-byte aligned memory.  As whole 32-byte sectors where it lies on them: two 16-byte stores
+// to a sector, each of them 16 bytes for every row of a warp, pass through the memory system as two partial writes, at half
+// the rate.
+__device__ __forceinline__ void blk_stg64(void* p, const uint32_t* w) {
+    if (!(reinterpret_cast<uintptr_t>(p) & 31u)) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(static_cast<char*>(p) + 32 * i), "r"(w[8 * i]),
+                         "r"(w[8 * i + 1]), "r"(w[8 * i + 2]), "r"(w[8 * i + 3]), "r"(w[8 * i + 4]), "r"(w[8 * i + 5]), "r"(w[8 * i + 6]),
+                         "r"(w[8 * i + 7])
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) static_cast<uint4*>(p)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    }
+}
+
 __device__ __forceinline__ uint4 blk_ldg16(const void* p) {
     return __ldg(reinterpret_cast<const uint4*>(p));
 }

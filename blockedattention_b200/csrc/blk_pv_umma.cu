@@ -388,11 +388,7 @@ blk_pv_umma_kernel(const BlkPvParams p, const __grid_constant__ CUtensorMap mapV
 #pragma unroll
                 for (int i = 0; i < 32; i += 2)
                     r[i >> 1] = BlkCvt<Tag>::pack2(__uint_as_float(r[i]) * p.scale, __uint_as_float(r[i + 1]) * p.scale);
-                if (row < wk.it.M) {
-                    uint4* dst = reinterpret_cast<uint4*>(orow + c);
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) dst[cc] = make_uint4(r[4 * cc], r[4 * cc + 1], r[4 * cc + 2], r[4 * cc + 3]);
-                }
+                if (row < wk.it.M) blk_stg64(orow + c, r);
             }
             tc_fence_before();
             __syncwarp();

@@ -93,7 +93,9 @@ int upload_plan(blk_plan* p) {
     // the staged kernel reads an item and its segment as one record: built straight into the staging block
     const size_t nrecs = p->dtype_in != BLK_F32 ? p->tile_items.size() : 0;
     add(nullptr, nrecs * sizeof(BlkTileRec), reinterpret_cast<void**>(&p->d_tile_recs));
-    add_vec(p->simt_items, &p->d_simt_items);
+    if (p->simt_big.empty()) add_vec(p->simt_items, &p->d_simt_items);
+    add_vec(p->simt_big, &p->d_simt_big);
+    add_vec(p->simt_rest, &p->d_simt_rest);
     for (int b = 0; b < BLK_SMALL_BUCKETS; ++b) add_vec(p->small_items[b], &p->d_small_items[b]);
     if (p->stream_items.empty()) add_vec(p->umma_items, &p->d_umma_items);
     add_vec(p->stream_items, &p->d_stream_items);
@@ -297,7 +299,7 @@ extern "C" int blk_plan_offsets(const blk_plan_t* p, int64_t* a1, int64_t* a2, i
 static int launches_per_run(const blk_plan* p) {
     if (p->attn) return (p->flash_items.empty() ? 0 : 1) + (p->packs.empty() ? 0 : 1);
     int n = (!p->tile_items.empty()) + (!p->simt_items.empty()) + (!p->umma_items.empty()) + (!p->smx_chunks.empty()) +
-            (!p->pv_items.empty());
+            (!p->pv_items.empty()) + (!p->simt_big.empty() && !p->simt_rest.empty());
     if (p->small_pipe) return n + 1;
     for (const auto& v : p->small_items) n += !v.empty();
     return n;
@@ -504,6 +506,8 @@ static int attention_plan_impl(blk_plan_t** plan, const int64_t* M, const int64_
         p->umma_items.clear();
         p->stream_items.clear();
         p->simt_items.clear();
+        p->simt_big.clear();
+        p->simt_rest.clear();
         if (!packs) {
             p->packs.clear(); p->pack_blocks.clear(); p->small_pipe = 0; p->small_segments = 0;
             for (auto& v : p->small_items) v.clear();
@@ -807,13 +811,22 @@ static int gemm_run_impl(const blk_plan* p, const void* mat1, const void* mat2, 
         sp.B = reinterpret_cast<const float*>(mat2);
         sp.C = reinterpret_cast<float*>(out);
         sp.segs = p->d_segs;
-        sp.items = p->d_simt_items;
         sp.Dm1 = p->Dm1; sp.Dm2 = p->Dm2; sp.Dout = p->Dout;
-        sp.num_items = (int)p->simt_items.size();
         sp.H = (int)p->H;
         sp.ta = p->ta; sp.tb = p->tb;
         sp.scale = scale;
-        if ((e = blk_launch_gemm_simt(sp, st)) != cudaSuccess) return cuda_fail("fp32 GEMM launch", e);
+        auto tiles = [&](const BlkTileItem* items, size_t n, int big) {
+            sp.items = items;
+            sp.num_items = (int)n;
+            return blk_launch_gemm_simt(sp, big, st);
+        };
+        if (p->simt_big.empty()) {
+            e = tiles(p->d_simt_items, p->simt_items.size(), 0);
+        } else {
+            e = tiles(p->d_simt_big, p->simt_big.size(), 1);
+            if (e == cudaSuccess) e = tiles(p->d_simt_rest, p->simt_rest.size(), 0);
+        }
+        if (e != cudaSuccess) return cuda_fail("fp32 GEMM launch", e);
         if (!p->smx_chunks.empty()) {
             BlkSmxParams xp{};
             xp.src = out; xp.dst = out;

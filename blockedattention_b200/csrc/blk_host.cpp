@@ -571,6 +571,31 @@ int blk_build_gemm_schedule(blk_plan* p) {
     p->umma_wide = 0;
     for (const BlkUmmaItem& it : p->umma_items)
         if (it.nch) p->umma_wide = 1;
+    // fp32 on the CUDA cores: tiles of 128 x 128 (a load from shared memory per 6.4 multiply-adds of a thread; 64 x 64: per 3.2)
+    // for the segments that fill them nearly as well as tiles of 64 x 64, if these make a block for every SM.
+    p->simt_big.clear();
+    p->simt_rest.clear();
+    if (!p->simt_items.empty()) {
+        auto up = [](int64_t x, int64_t t) { return (x + t - 1) / t; };
+        auto is_big = [&](int32_t s) {
+            const int64_t m = p->segs[s].M, n = p->segs[s].N;
+            return 8 * up(m, 128) * up(n, 128) <= 3 * up(m, 64) * up(n, 64);
+        };
+        int64_t tiles = 0;
+        for (const BlkTileItem& it : p->simt_items) {
+            if (it.tm || it.tn || !is_big(it.seg)) continue;
+            tiles += up(p->segs[it.seg].M, 128) * up(p->segs[it.seg].N, 128);
+        }
+        if (tiles * p->H >= 148) {
+            p->simt_big.reserve(tiles);
+            for (const BlkTileItem& it : p->simt_items) {
+                if (!is_big(it.seg)) { p->simt_rest.push_back(it); continue; }
+                if (it.tm || it.tn) continue;
+                for (int32_t tm = 0; tm * 128 < p->segs[it.seg].M; ++tm)
+                    for (int32_t tn = 0; tn * 128 < p->segs[it.seg].N; ++tn) p->simt_big.push_back(BlkTileItem{it.seg, tm, tn, 1});
+            }
+        }
+    }
     // Short contractions go to the kernel of independent streams (blk_scores_umma.cu) where there are tiles enough for all
     // streams to be busy and in different phases; below that the other kernel, whose warps share an item, is done sooner.
     // With a softmax it is the better one only for rows that the other kernel computes twice as well (beyond 512 columns), which

@@ -176,7 +176,9 @@ struct blk_plan {
 
     std::vector<BlkSeg> segs;
     std::vector<BlkTileItem> tile_items;    // staged mma.sync kernel (16-bit inputs)
-    std::vector<BlkTileItem> simt_items;    // fp32 SIMT kernel
+    std::vector<BlkTileItem> simt_items;    // fp32 SIMT kernel, as 64 x 64 tiles
+    std::vector<BlkTileItem> simt_big, simt_rest;  // the same as it runs, where some segments have 128 x 128 tiles: those, and the others' 64 x 64
+    BlkTileItem *d_simt_big = nullptr, *d_simt_rest = nullptr;
     std::vector<BlkSmallItem> small_items[BLK_SMALL_BUCKETS];  // packed small-segment kernel, by column count (empty when small_pipe)
     std::vector<BlkUmmaItem> umma_items;    // tcgen05 kernel
     std::vector<BlkPvItem> pv_items;        // tcgen05 kernel for transposed second operands of 64 or 128 columns

@@ -219,7 +219,8 @@ struct BlkSmxPipeParams {
     int* status;
 };
 cudaError_t blk_launch_softmax_pipe(const BlkSmxPipeParams& p, int dtype, int backward, int sms, cudaStream_t st);
-cudaError_t blk_launch_gemm_simt(const BlkSimtParams& p, cudaStream_t st);
+// big: the items are tiles of 128 x 128, not 64 x 64.
+cudaError_t blk_launch_gemm_simt(const BlkSimtParams& p, int big, cudaStream_t st);
 cudaError_t blk_launch_scores_small(const BlkSmallParams& p, int dtype_in, int K, int bucket, int sms,
                                     cudaStream_t st);
 // An operand of the tcgen05 GEMM kernel: the buffer, the length of a head strip, and the views the plan's items refer

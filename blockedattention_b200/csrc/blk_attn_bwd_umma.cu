@@ -21,11 +21,12 @@
 //   warps 4-11  softmax: warps 4-7 take the even tiles, 8-11 the odd ones; a thread owns one row of 64 columns and meets
 //               nobody;
 //   warps 12-15 output; <QUERIES>: also rowsum(dO O) of the next item, kept for the <KEYS> launch.
-// Bound by the chain of a tile through the roles -- scores, exponentials, dP, dS, product -- with two pairs of buffers to
-// overlap it: at d = 128 the products of a tile are 1280 cycles of the tensor pipe for <KEYS> and 1024 for <QUERIES> (S and
-// dP run at two thirds of the rate with 64 columns, but 128-column tiles would leave room for one pair), and the pipe is
-// active 38 % and 28 % of the time, the special-function unit 20 %, the issue slots 30 % (48 segments of 64..512 rows, 16
-// heads: 126 and 124 us).
+// Bound by the products and the chain of a tile through the roles -- scores, exponentials, dP, dS, product -- with two pairs
+// of buffers to overlap it: at d = 128 the products of a tile occupy the tensor pipe for 1280 cycles (<KEYS>) and 1024
+// (<QUERIES>; S and dP run at two thirds of the rate with 64 columns, but 128-column tiles would leave room for one pair) of
+// the 2120 and 1740 that it takes, and softmax warps wait for scores two fifths and a third of their time.  256 segments of
+// 64..512 rows, 16 heads: 620 and 484 us.  (<QUERIES> 609 with rowsum(dO O) made by the lane that owns a row, dO from the
+// resident block, four loads of O at a time: softmax warps waited two fifths of their time for it.)
 //
 // rowsum(dO O) takes O as the forward pass rounded it, where a chain of operators has rowsum(P dP) of its own rounded P.
 // 2-norm errors of dQ against 64 bits, 300 rows, d = 64, bf16: 2.4e-3 (the chain: 3.3e-3) for scores of deviation 1, 5.4e-3
@@ -120,7 +121,7 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < 2; ++i) {
             mbar_init(r_full(i), 1);
-            mbar_init(r_empty(i), MODE == QUERIES ? 5 : 1);  // the products; <QUERIES>: the output warps read dO too
+            mbar_init(r_empty(i), 1);
             mbar_init(s_full(i), 1);
             mbar_init(dp_full(i), 1);
             mbar_init(p_full(i), 4);
@@ -499,36 +500,57 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
             const int64_t r = more ? (int64_t)ib.y * p.rows_r + ia.x + row : 0;
             const bool mine = more && row < ib.x;
             if (MODE == QUERIES && more) {
-                // row values of the item: saved logarithm, rowsum(dO O) with dO from shared memory
+                // Row values of the item: saved logarithm, rowsum(dO O).  Both from global memory, so that they need not wait for
+                // the item's operands; eight lanes a row, everything of 16 rows on its way at a time.
                 const uint32_t i = item - 1u, slot = i & 1u;
-                if (!mbar_wait(r_full(slot), (i >> 1) & 1u, abort_flag, 68)) break;
-                float l = 0.f, d0 = 0.f, d1 = 0.f;
-                if (mine) {
-                    l = __ldg(p.lse + r);
-                    const uint4* orow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.o) + r * D);
-#pragma unroll 4
-                    for (int c = 0; c < D / 8; ++c) {
-                        const uint4 o = __ldg(orow + c);
-                        uint4 d;
-                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(d.x), "=r"(d.y), "=r"(d.z), "=r"(d.w)
-                                     : "r"(sR(slot, 1) + (c >> 3) * BW_RB_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4)));
-                        const uint32_t ow[4] = {o.x, o.y, o.z, o.w}, dw[4] = {d.x, d.y, d.z, d.w};
+                const float l = mine ? __ldg(p.lse + r) : 0.f;
+                const int64_t r0 = r - lane + (lane >> 3);  // row lane / 8 of this warp's; then every fourth
+                const int left = ib.x - q * 32 - (lane >> 3);
+                const uint4* o0 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.o) + r0 * D) + (lane & 7);
+                const uint4* g0 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.g) + r0 * D) + (lane & 7);
+                float d[8];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            d0 = fmaf(BlkCvt<Tag>::unpack1((uint16_t)ow[e]), BlkCvt<Tag>::unpack1((uint16_t)dw[e]), d0);
-                            d1 = fmaf(BlkCvt<Tag>::unpack1((uint16_t)(ow[e] >> 16)), BlkCvt<Tag>::unpack1((uint16_t)(dw[e] >> 16)), d1);
+                for (int half = 0; half < 2; ++half) {
+                    uint4 ov[4][NB], gv[4][NB];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) {
+                            const int row4 = 4 * (4 * half + k);
+                            ov[k][c] = gv[k][c] = make_uint4(0u, 0u, 0u, 0u);
+                            if (row4 < left) {
+                                ov[k][c] = __ldg(o0 + (row4 * D / 8 + 8 * c));
+                                gv[k][c] = __ldg(g0 + (row4 * D / 8 + 8 * c));
+                            }
                         }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+                        for (int c = 0; c < NB; ++c) {
+                            const uint32_t ow[4] = {ov[k][c].x, ov[k][c].y, ov[k][c].z, ov[k][c].w}, gw[4] = {gv[k][c].x, gv[k][c].y, gv[k][c].z, gv[k][c].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                d0 = fmaf(BlkCvt<Tag>::unpack1((uint16_t)ow[e]), BlkCvt<Tag>::unpack1((uint16_t)gw[e]), d0);
+                                d1 = fmaf(BlkCvt<Tag>::unpack1((uint16_t)(ow[e] >> 16)), BlkCvt<Tag>::unpack1((uint16_t)(gw[e] >> 16)), d1);
+                            }
+                        }
+                        d[4 * half + k] = d0 + d1;
                     }
-                    p.delta[r] = d0 + d1;
                 }
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+#pragma unroll
+                    for (int x = 4; x; x >>= 1) d[k] += __shfl_xor_sync(0xffffffffu, d[k], x);
                 if (!mbar_wait(rowv_empty(slot), ((i >> 1) & 1u) ^ 1u, abort_flag, 69)) break;
                 aux[256 * slot + row] = -l;
-                aux[256 * slot + 128 + row] = -(d0 + d1);
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(rowv_full(slot));
-                    mbar_arrive(r_empty(slot));
+                if (!(lane & 7)) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) aux[256 * slot + 128 + q * 32 + 4 * k + (lane >> 3)] = -d[k];
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(rowv_full(slot));
+                if (mine) p.delta[r] = -aux[256 * slot + 128 + row];
             }
             if (have) {
                 if constexpr (MODE == QUERIES) {
@@ -577,6 +599,7 @@ cudaError_t blk_launch_attn_bwd_umma(const BlkFlashBwdParams& p_in, int keys, co
     if ((int64_t)p_in.num_items * p_in.H == 0) return cudaSuccess;
     if (p_in.D != 64 && p_in.D != 128) return cudaErrorInvalidValue;
     BlkFlashBwdParams p = p_in;
+    p.g = tensors[1];
     CUtensorMap maps[4];
     for (int i = 0; i < 4; ++i)
         if (!blk_make_row_map(&maps[i], tensors[i], p.bf16, p.D, p.H, i < 2 ? layR : layT, 64, i < 2 ? 128 : BW_BN,

@@ -136,6 +136,7 @@ struct BlkFlashBwdParams {
     float scale;
     int* status;
     const void* o;     // forward result (query launch)
+    const void* g;     // its gradient (query launch; filled by the launcher)
     const float* lse;  // [head][query row] as the forward kernel leaves it
     float* delta;      // [head][query row] rowsum(dO O): written by the query launch, read by the key launch
     void* out0;        // dV (key launch)

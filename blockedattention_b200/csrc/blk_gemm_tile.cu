@@ -146,33 +146,37 @@ __device__ __forceinline__ void compute_tile(float (&acc)[NJ * 128 / NTHR][4], c
     const int ncols = min(N - n0, BN);
     const bool active = m0 + wrow * 16 < M && wcol0 < ncols;
 
-    TileStage<TA ? BK : BM, TA ? BM : BK, AA, NTHR> stA;
-    TileStage<TB ? BK : BN, TB ? BN : BK, AB, NTHR> stB;
-    auto loadA = [&](int k0) {
-        if constexpr (!TA) stA.load(gA, K, m0, k0, M, K, tid); else stA.load(gA, M, k0, m0, K, M, tid);
-    };
-    auto loadB = [&](int k0) {
-        if constexpr (!TB) stB.load(gB, K, n0, k0, N, K, tid); else stB.load(gB, N, k0, n0, K, N, tid);
-    };
+    // Two steps of registers: the operands of the next two steps are on their way while one is multiplied.
+    TileStage<TA ? BK : BM, TA ? BM : BK, AA, NTHR> stA[2];
+    TileStage<TB ? BK : BN, TB ? BN : BK, AB, NTHR> stB[2];
     constexpr int pA = TA ? A_PITCH_T : A_PITCH_N, pB = TB ? B_PITCH_T : B_PITCH_N;
-
-    loadA(0);
-    loadB(0);
-    stA.store(sA[0], pA, tid);
-    stB.store(sB[0], pB, tid);
+    auto fetch = [&](auto x, int kt) {  // step kt to registers x
+        if (kt >= nk) return;
+        const int k0 = kt * BK;
+        if constexpr (!TA) stA[x].load(gA, K, m0, k0, M, K, tid); else stA[x].load(gA, M, k0, m0, K, M, tid);
+        if constexpr (!TB) stB[x].load(gB, K, n0, k0, N, K, tid); else stB[x].load(gB, N, k0, n0, K, N, tid);
+    };
+    auto put = [&](auto x, int kt) {    // and on to shared memory
+        if (kt >= nk) return;
+        stA[x].store(sA[x], pA, tid);
+        stB[x].store(sB[x], pB, tid);
+    };
+    constexpr std::integral_constant<int, 0> zero{};
+    constexpr std::integral_constant<int, 1> one{};
+    fetch(zero, 0);
+    fetch(one, 1);
+    put(zero, 0);
     __syncthreads();
-    for (int kt = 0; kt < nk; ++kt) {
-        const int cur = kt & 1;
-        const bool more = kt + 1 < nk;
-        if (more) {
-            loadA((kt + 1) * BK);
-            loadB((kt + 1) * BK);
-        }
-        if (active) mma_stage<Tag, TA, TB, NJW>(acc, sA[cur], sB[cur], wrow, wcol0, lane, ncols);
-        if (more) {
-            stA.store(sA[cur ^ 1], pA, tid);
-            stB.store(sB[cur ^ 1], pB, tid);
-        }
+#pragma unroll 1
+    for (int kt = 0; kt < nk; kt += 2) {
+        fetch(zero, kt + 2);
+        if (active) mma_stage<Tag, TA, TB, NJW>(acc, sA[0], sB[0], wrow, wcol0, lane, ncols);
+        put(one, kt + 1);
+        __syncthreads();
+        if (kt + 1 >= nk) break;
+        fetch(one, kt + 3);
+        if (active) mma_stage<Tag, TA, TB, NJW>(acc, sA[1], sB[1], wrow, wcol0, lane, ncols);
+        put(zero, kt + 2);
         __syncthreads();
     }
 }
@@ -327,12 +331,12 @@ __device__ __forceinline__ void scores_body(const BlkGemmParams& p, const BlkSeg
     store_frag<Tag, NJW>(p.C, p.out_f32, cbase, acc, r0, M, N, n0 + (warp >> 2) * (8 * NJW), t, pair_ok);
 }
 
-// SOFTMAX: the fused two-sweep kernel (four warps); otherwise the scores kernel (eight warps).  The scores kernel
-// without transposed operands is held to 64 registers (a few spills) for a fourth resident CTA: its tiles are bound
-// by the latency of their load chain, and one more tile in flight measured 8 % faster; the transposed variants
-// measured slower that way.
+// SOFTMAX: the fused two-sweep kernel (four warps); otherwise the scores kernel (eight warps).  Bound by the latency of its load
+// chain.  Two steps of operands on their way and three CTAs an SM without a spill, against one step and four CTAs of 64 registers
+// (with spills), us: 1510 products of 1..164 rows and columns over any K up to 128 65.0 -> 60.4, 113 of 1..242, 4 heads, 34.4 -> 30.9,
+// 74 of 1..44 9.6 -> 6.0, 357 of 256..1195 over up to 2328 5820 -> 5307 (two steps and four CTAs: 64.4, 34.1, 9.9, 6128).
 template <typename Tag, bool TA, bool TB, bool SOFTMAX>
-__global__ void __launch_bounds__(SOFTMAX ? NT : NT_SC, (SOFTMAX || TA || TB) ? 3 : 4) blk_gemm_tile_kernel(const BlkGemmParams p) {
+__global__ void __launch_bounds__(SOFTMAX ? NT : NT_SC, 3) blk_gemm_tile_kernel(const BlkGemmParams p) {
     __shared__ __align__(16) uint16_t sA[2][A_STAGE];
     __shared__ __align__(16) uint16_t sB[2][B_STAGE];
     const int64_t bid = blockIdx.x;

@@ -129,7 +129,8 @@ __device__ __forceinline__ void store_sectors(uint32_t strip, uint64_t r0, uint3
         }
     }
 }
-// The same for the whole piece of 32 rows: goes[i] past origin is where the lane's part of row lane / 8 + 4 i goes.
+// The same for the whole piece of 32 rows: the lane's part of row lane / 8 + 4 i goes `goes[i]` sectors past origin.  (Counted in
+// sectors, since 31 rows of up to 2^32 bytes are beyond 32 bits of bytes.)
 __device__ __forceinline__ void store_sectors_all(uint32_t from, uint32_t o1, uint32_t o2, uint64_t origin, const uint32_t (&goes)[8]) {
 #pragma unroll
     for (int t = 0; t < 8; t += 4) {
@@ -140,7 +141,7 @@ __device__ __forceinline__ void store_sectors_all(uint32_t from, uint32_t o1, ui
         w[2] = lds_v4(at + o2);
         w[3] = lds_v4(at + o1 + o2);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) stg_v4(origin + goes[t + i], w[i]);
+        for (int i = 0; i < 4; ++i) stg_v4(origin + 32ull * goes[t + i], w[i]);
     }
 }
 // Element i of a strip row (32-byte aligned base `from`), to p.
@@ -449,12 +450,11 @@ blk_scores_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps map
             const uint64_t pitch = (uint64_t)N * E;
             uint64_t own = base + (uint64_t)lane * pitch;                  // this lane's row ...
             uint64_t quarter = base + (uint64_t)(lane >> 3) * pitch;       // ... and row lane / 8, at the piece's first column
-            // where this lane's halves of sectors go, less the start of the first row's sector: rows lane / 8 + 4 i
-            uint64_t origin = base & ~31ull;
+            // where this lane's halves of sectors go: in the first row, and the sectors from there to rows lane / 8 + 4 i
+            uint64_t origin = (base & ~31ull) + 16u * ((uint32_t)lane & 7u);
             uint32_t goes[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 8; ++i)
-                goes[i] = (((uint32_t)base & 31u) + ((uint32_t)(lane >> 3) + 4u * i) * (uint32_t)pitch & ~31u) + 16u * ((uint32_t)lane & 7u);
+            for (uint32_t i = 0; i < 8; ++i) goes[i] = (uint32_t)((quarter - (base & ~31ull) + 4ull * i * pitch) >> 5);
             const uint32_t phase = (uint32_t)own & 31u;                    // how far into a sector the row starts
             const bool odd16 = !OUT32 && (N & 1);
             const bool anyodd = !OUT32 && __any_sync(0xffffffffu, (int)(phase & 2u));

@@ -66,3 +66,20 @@ def test_masked_rows_and_far_scores(cuda_device, streams):
         assert_probs_close(out, O.block_scores(A, B, n, n, K, scale=scale), "softmax")
     out = plan.run(A.to(cuda_device), B.to(cuda_device), scale=0.0).float()
     assert torch.allclose(out[:, :700], torch.full_like(out[:, :700], 1 / 700), rtol=8e-3)
+
+
+@pytest.mark.parametrize("out_dtype,n", [(F32, 34_700_003), (F16, 69_300_003)])
+def test_rows_whose_offsets_exceed_32_bits_of_bytes(cuda_device, out_dtype, n):
+    """31 rows of such a segment are more than 2^32 bytes.  Small whole numbers: every product is exact in either result type."""
+    m, k = 32, 16
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    A = torch.randint(-2, 3, (1, m * k), generator=g, device=cuda_device).half()
+    B = torch.randint(-2, 3, (1, n * k), generator=g, device=cuda_device, dtype=torch.int8).half()
+    plan = GemmPlan([m], [n], [k], 1, F16, out_dtype, device=cuda_device)
+    out = torch.full((1, plan.Dout), float("nan"), dtype=out_dtype, device=cuda_device)
+    plan.run(A, B, out=out)
+    plan.check()
+    got, a, b = out.view(m, n), A.view(m, k), B.view(n, k)
+    for c in range(0, n, 1 << 22):
+        want = (a.double() @ b[c:c + (1 << 22)].double().T).to(out_dtype)
+        assert torch.equal(got[:, c:c + (1 << 22)], want), f"columns from {c}"

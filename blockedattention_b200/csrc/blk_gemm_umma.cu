@@ -174,22 +174,25 @@ __device__ __forceinline__ void store_strip(uint32_t strip, void* out, int64_t g
             for (int i = 0; i < 2; ++i) v[k][i] = lds_b32(rbase + (uint32_t)(kb + k) * (UM_STRIP_PITCHW * 4) + 128u * i);
     };
     if (rows == 32 && pcols == (OUT32 ? UM_PW : 2 * UM_PW)) {
-        // A whole piece (the common case), with as few instructions per row as it takes.  Row k starts at element g0 + k N:
-        // of 16-bit elements, at word (t >> 1) past the word of g0 with t = (g0 & 1) + k N, on its odd half when t is odd.
-        // Words 1..63 of the row are whole; word 0 is whole when the row starts on an even element (its upper half goes out
-        // below otherwise, and so does the lower half of word 64).
-        uint32_t* const w0 = static_cast<uint32_t*>(out) + (OUT32 ? g0 : g0 >> 1) + lane;
-        uint32_t t = OUT32 ? 0u : (uint32_t)(g0 & 1);
+        // A whole piece (the common case), with as few instructions per row as it takes.  Rows go by twos: row 2 j starts j * two
+        // words past the word of g0, as far into its first word as g0 (`even`), and row 2 j + 1 starts `one` words further and is
+        // `odd` elements into its word.  (A row may have 2^30 columns: nothing but a row's own length fits 32 bits.)  Words 1..63
+        // of a row are whole; word 0 is whole when the row starts on an even element (its upper half goes out below
+        // otherwise, and so does the lower half of word 64).
+        const uint32_t even = OUT32 ? 0u : (uint32_t)(g0 & 1), one = OUT32 ? (uint32_t)N : (even + (uint32_t)N) >> 1;
+        const uint32_t odd = OUT32 ? 0u : (even + (uint32_t)N) & 1u;
+        const int64_t two = OUT32 ? 2 * (int64_t)N : N;
+        uint32_t* w0 = static_cast<uint32_t*>(out) + (OUT32 ? g0 : g0 >> 1) + lane;
 #pragma unroll 1
         for (int kb = 0; kb < 32; kb += BATCH) {
             fetch(kb);
 #pragma unroll
             for (int k = 0; k < BATCH; ++k) {
-                uint32_t* wp = w0 + (OUT32 ? t : t >> 1);
+                uint32_t* wp = w0 + (k & 1 ? one : 0u);
                 if (OUT32) asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp), "r"(v[k][0]) : "memory");
-                else stg_b32_if(wp, v[k][0], lane >= (int)(t & 1u));
+                else stg_b32_if(wp, v[k][0], lane >= (int)(k & 1 ? odd : even));
                 asm volatile("st.global.b32 [%0], %1;\n" ::"l"(wp + 32), "r"(v[k][1]) : "memory");
-                t += (uint32_t)N;
+                if (k & 1) w0 += two;
             }
         }
     } else {

@@ -56,3 +56,18 @@ def test_long_contractions_take_single_wide_chunks(cuda_device, out_dtype):
     items = plan.table("umma_items")
     assert (items["nch"] == 1).any() and (items["nch"] == 0).any()
     assert_scores_close(out, O.block_gemm(A, B, m, n, K), "wide chunks")
+
+
+@pytest.mark.parametrize("out_dtype", [F16, F32])
+def test_rows_whose_offsets_exceed_32_bits(cuda_device, monkeypatch, out_dtype):
+    """31 rows of such a segment are more than 2^32 elements.  Small whole numbers: every product is exact in either result type."""
+    monkeypatch.setenv("BLK_UMMA_STREAMS", "0")   # (plain scores of so many tiles run on the kernel of streams otherwise)
+    m, n, k = 32, 138_600_003, 16
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    A = torch.randint(-2, 3, (1, m * k), generator=g, device=cuda_device).half()
+    B = torch.randint(-2, 3, (1, n * k), generator=g, device=cuda_device, dtype=torch.int8).half()
+    plan, out = run(cuda_device, [m], [n], [k], 1, F16, out_dtype, False, 1.0, A, B)
+    got, a, b = out.view(m, n), A.view(m, k), B.view(n, k)
+    for c in range(0, n, 1 << 23):
+        want = (a.double() @ b[c:c + (1 << 23)].double().T).to(out_dtype)
+        assert torch.equal(got[:, c:c + (1 << 23)], want), f"columns from {c}"

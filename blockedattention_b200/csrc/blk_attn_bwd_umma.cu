@@ -438,7 +438,7 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
                 uint32_t q = 0;
                 if (more) {
                     q = n / (uint32_t)p.H;
-                    f = __ldg(reinterpret_cast<const int4*>(p.items + q));
+                    f = blk_ld_table(reinterpret_cast<const int4*>(p.items + q));
                 }
                 if (!mbar_wait(item_empty(s), ((pub / BW_ITEMS) & 1u) ^ 1u, abort_flag, 66)) { ok = false; break; }
                 if (lane == 0) {
@@ -460,8 +460,8 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
 #pragma unroll
                     for (int r = lane; r < BW_BN; r += 32) {
                         const int at = j * BW_BN + r;
-                        aux[128 * s + r] = at < ia.z ? -__ldg(p.lse + base + at) : 0.f;
-                        aux[128 * s + 64 + r] = at < ia.z ? -__ldg(p.delta + base + at) : 0.f;
+                        aux[128 * s + r] = at < ia.z ? -p.lse[base + at] : 0.f;
+                        aux[128 * s + 64 + r] = at < ia.z ? -p.delta[base + at] : 0.f;
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(aux_full(s));
@@ -503,7 +503,7 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
                 // Row values of the item: saved logarithm, rowsum(dO O).  Both from global memory, so that they need not wait for
                 // the item's operands; eight lanes a row, everything of 16 rows on its way at a time.
                 const uint32_t i = item - 1u, slot = i & 1u;
-                const float l = mine ? __ldg(p.lse + r) : 0.f;
+                const float l = mine ? p.lse[r] : 0.f;
                 const int64_t r0 = r - lane + (lane >> 3);  // row lane / 8 of this warp's; then every fourth
                 const int left = ib.x - q * 32 - (lane >> 3);
                 const uint4* o0 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.o) + r0 * D) + (lane & 7);
@@ -519,8 +519,8 @@ blk_attn_bwd_umma_kernel(const BlkFlashBwdParams p, const __grid_constant__ CUte
                             const int row4 = 4 * (4 * half + k);
                             ov[k][c] = gv[k][c] = make_uint4(0u, 0u, 0u, 0u);
                             if (row4 < left) {
-                                ov[k][c] = __ldg(o0 + (row4 * D / 8 + 8 * c));
-                                gv[k][c] = __ldg(g0 + (row4 * D / 8 + 8 * c));
+                                ov[k][c] = o0[row4 * D / 8 + 8 * c];
+                                gv[k][c] = g0[row4 * D / 8 + 8 * c];
                             }
                         }
 #pragma unroll

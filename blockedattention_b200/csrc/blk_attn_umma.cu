@@ -485,8 +485,8 @@ blk_attn_umma_kernel(const BlkFlashParams p, const __grid_constant__ CUtensorMap
             if (more) {
                 q = n / (uint32_t)p.H;
                 const int4* src = reinterpret_cast<const int4*>(p.pairs + q);
-                a = __ldg(src);
-                b = __ldg(src + 1);
+                a = blk_ld_table(src);
+                b = blk_ld_table(src + 1);
             }
             if (!mbar_wait(ring.bar + 8u * (FA_ITEMS + s), ((i / FA_ITEMS) & 1u) ^ 1u, abort_flag, 17)) break;
             if (lane == 0) {

@@ -170,9 +170,10 @@ __device__ __forceinline__ void blk_stg64(void* p, const uint32_t* w) {
     }
 }
 
-__device__ __forceinline__ uint4 blk_ldg16(const void* p) {
-    return __ldg(reinterpret_cast<const uint4*>(p));
-}
+// Loads of what another kernel may have written are plain ones.  Loads through the read-only path (__ldg) ask for memory that
+// nobody writes as long as the kernel runs, and a kernel runs from before the one in front of it has finished (blk_launch); the
+// compiler may also move them ahead of blk_grid_wait.  They are for the work tables of a plan alone, here:
+__device__ __forceinline__ int4 blk_ld_table(const int4* p) { return __ldg(p); }
 
 __device__ __forceinline__ float blk_quad_max(float v) {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));

@@ -27,20 +27,20 @@ struct Share {
     static constexpr int B = 16 * TM, PITCH = B + 4;
     float v[TM];
     // vec: rows (TR: columns of the stored operand) are a multiple of four elements and start on 16 bytes
-    __device__ __forceinline__ void load(const float* __restrict__ g, int R, int K, int r0, int k0, int tid, bool vec) {
+    __device__ __forceinline__ void load(const float* g, int R, int K, int r0, int k0, int tid, bool vec) {
         if (vec) {
 #pragma unroll
             for (int i = 0; i < TM / 4; ++i) {
                 const int r = r0 + (TR ? tid % (B / 4) * 4 : tid / 4 + 64 * i), k = k0 + (TR ? tid / (B / 4) + 1024 / B * i : tid % 4 * 4);
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (r < R && k < K) x = __ldg(reinterpret_cast<const float4*>(g + (TR ? (int64_t)k * R + r : (int64_t)r * K + k)));
+                if (r < R && k < K) x = *reinterpret_cast<const float4*>(g + (TR ? (int64_t)k * R + r : (int64_t)r * K + k));
                 v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
             }
         } else {
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
                 const int r = r0 + (TR ? tid % B : tid / 16 + 16 * i), k = k0 + (TR ? tid / B + SNT / B * i : tid % 16);
-                v[i] = r < R && k < K ? __ldg(g + (TR ? (int64_t)k * R + r : (int64_t)r * K + k)) : 0.f;
+                v[i] = r < R && k < K ? g[TR ? (int64_t)k * R + r : (int64_t)r * K + k] : 0.f;
             }
         }
     }

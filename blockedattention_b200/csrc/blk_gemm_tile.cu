@@ -39,9 +39,9 @@ __device__ __forceinline__ uint4 ldg8_any(const uint16_t* src, int nvalid) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(src);
     const uint4* base = reinterpret_cast<const uint4*>(a & ~static_cast<uintptr_t>(15));
     const uint32_t m = static_cast<uint32_t>(a) & 15u;  // even
-    const uint4 v0 = __ldg(base);
+    const uint4 v0 = *base;
     uint4 v1 = make_uint4(0u, 0u, 0u, 0u);
-    if ((int)m + 2 * nvalid > 16) v1 = __ldg(base + 1);
+    if ((int)m + 2 * nvalid > 16) v1 = base[1];
     uint32_t w0 = v0.x, w1 = v0.y, w2 = v0.z, w3 = v0.w, w4 = v1.x, w5 = v1.y;
     if (m & 8u) {
         w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = v1.z; w5 = v1.w;
@@ -73,7 +73,7 @@ struct TileStage {
     static_assert(UNITS % NTHR == 0, "tile must divide among the threads");
     uint4 r[PT];
 
-    __device__ __forceinline__ void load(const uint16_t* __restrict__ g, int64_t ld, int o0, int i0, int o_lim,
+    __device__ __forceinline__ void load(const uint16_t* g, int64_t ld, int o0, int i0, int o_lim,
                                          int i_lim, int tid) {
 #pragma unroll
         for (int j = 0; j < PT; ++j) {
@@ -82,7 +82,7 @@ struct TileStage {
             const uint16_t* src = g + (int64_t)o * ld + i;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (o < o_lim && i < i_lim) {
-                if constexpr (ALIGNED) v = blk_ldg16(src);
+                if constexpr (ALIGNED) v = *reinterpret_cast<const uint4*>(src);
                 else v = ldg8_any(src, min(8, i_lim - i));
             }
             r[j] = v;
@@ -133,8 +133,8 @@ __device__ __forceinline__ void mma_stage(float (&acc)[NJW][4], const uint16_t* 
 // acc = A[m0.., :] * B[n0.., :]^T for the CTA's 64 x 128 tile.
 // NTHR threads: NTHR / 128 warp columns, each warp 16 rows x (BN / warp columns) columns.
 template <typename Tag, bool TA, bool TB, bool AA, bool AB, int NTHR>
-__device__ __forceinline__ void compute_tile(float (&acc)[NJ * 128 / NTHR][4], const uint16_t* __restrict__ gA,
-                                             const uint16_t* __restrict__ gB, int M, int N, int K, int m0, int n0,
+__device__ __forceinline__ void compute_tile(float (&acc)[NJ * 128 / NTHR][4], const uint16_t* gA,
+                                             const uint16_t* gB, int M, int N, int K, int m0, int n0,
                                              uint16_t (*sA)[A_STAGE], uint16_t (*sB)[B_STAGE], int tid) {
     constexpr int NJW = NJ * 128 / NTHR;
 #pragma unroll

@@ -26,7 +26,7 @@ __device__ __forceinline__ bool fetch_item(const BlkUmmaParams& p, uint32_t n, u
     const int4* src = reinterpret_cast<const int4*>(p.items + item);
     int4* dst = reinterpret_cast<int4*>(&it);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) dst[i] = __ldg(src + i);
+    for (int i = 0; i < 3; ++i) dst[i] = blk_ld_table(src + i);
     return true;
 }
 // Rows of an item's block.  A block that fills less than four quarters of the accumulator lanes is put into other

@@ -345,6 +345,9 @@ extern "C" int blk_plan_table(const blk_plan_t* p, int table, void* dst, int64_t
         case BLK_TABLE_FLASH_ITEMS: take(p->flash_items); break;
         case BLK_TABLE_UMMA_VIEWS_A: take(p->umma_viewsA); break;
         case BLK_TABLE_UMMA_VIEWS_B: take(p->umma_viewsB); break;
+        case BLK_TABLE_SIMT_BIG: take(p->simt_big); break;
+        case BLK_TABLE_SIMT_REST: take(p->simt_rest); break;
+        case BLK_TABLE_STREAM_ITEMS: take(p->stream_items); break;
         default:
             blk_set_error("blk_plan_table: no table " + std::to_string(table));
             return BLK_ERR_INVALID;

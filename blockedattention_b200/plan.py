@@ -46,6 +46,8 @@ def _rec(*fields):
 
 _TILE_ITEM = _rec(("seg", "<i4"), ("tm", "<i4"), ("tn", "<i4"), ("ntn", "<i4"))
 _SMALL_ITEM = _rec(("offA", "<i8"), ("offB", "<i8"), ("offC", "<i8"), ("M", "<i4"), ("N", "<i4"))
+_UMMA_ITEM = _rec(("views", "<i4"), ("tm", "<i4"), ("rowA", "<i4"), ("rowB", "<i4"), ("offC", "<i8"),
+                  ("M", "<i4"), ("N", "<i4"), ("K", "<i4"), ("ch0", "<i4"), ("nch", "<i4"), ("pad", "<i4"))
 _VIEW = _rec(("K", "<i8"), ("residue", "<i8"))
 # name -> (blk_table_t value, record layout): mirrors of the schedule records of csrc/blk_internal.h
 TABLES = {
@@ -55,8 +57,7 @@ TABLES = {
     "simt_items": (2, _TILE_ITEM),
     "small_items_32": (3, _SMALL_ITEM),
     "small_items_64": (4, _SMALL_ITEM),
-    "umma_items": (5, _rec(("views", "<i4"), ("tm", "<i4"), ("rowA", "<i4"), ("rowB", "<i4"), ("offC", "<i8"),
-                           ("M", "<i4"), ("N", "<i4"), ("K", "<i4"), ("ch0", "<i4"), ("nch", "<i4"), ("pad", "<i4"))),
+    "umma_items": (5, _UMMA_ITEM),
     "pv_items": (6, _rec(("offA", "<i8"), ("offC", "<i8"), ("rowB", "<i4"), ("M", "<i4"), ("K", "<i4"), ("pitch", "<i4"))),
     "packs": (7, _rec(("offA", "<i8"), ("offB", "<i8"), ("rowsA", "<i4"), ("rowsB", "<i4"), ("first_block", "<i4"),
                       ("nblocks", "<i4"))),
@@ -68,6 +69,9 @@ TABLES = {
     "flash_items": (11, _rec(("rowQ", "<i4"), ("rowKV", "<i4"), ("M", "<i4"), ("N", "<i4"))),
     "umma_views_a": (12, _VIEW),
     "umma_views_b": (13, _VIEW),
+    "simt_big": (14, _TILE_ITEM),
+    "simt_rest": (15, _TILE_ITEM),
+    "stream_items": (16, _UMMA_ITEM),
 }
 
 

@@ -265,10 +265,10 @@ BLK_API int blk_plan_summary(const blk_plan_t* plan, int64_t counts[8]);
 typedef enum {
     BLK_TABLE_SEGMENTS = 0,      /* BlkSeg: one per segment, batch order */
     BLK_TABLE_TILE_ITEMS = 1,    /* BlkTileItem: staged mma.sync kernel */
-    BLK_TABLE_SIMT_ITEMS = 2,    /* BlkTileItem: fp32 SIMT kernel */
+    BLK_TABLE_SIMT_ITEMS = 2,    /* BlkTileItem: fp32 SIMT kernel, as 64 x 64 tiles; run as they are unless 14 has any */
     BLK_TABLE_SMALL_ITEMS_32 = 3,/* BlkSmallItem: per-warp small-segment kernel, at most 32 columns */
     BLK_TABLE_SMALL_ITEMS_64 = 4,/* BlkSmallItem: ... 33 to 64 columns */
-    BLK_TABLE_UMMA_ITEMS = 5,    /* BlkUmmaItem: tcgen05 kernel, in the order the CTAs take them */
+    BLK_TABLE_UMMA_ITEMS = 5,    /* BlkUmmaItem: tcgen05 kernels, in the order the CTAs take them unless 16 has any */
     BLK_TABLE_PV_ITEMS = 6,      /* BlkPvItem: tcgen05 kernel for (K, D) second operands */
     BLK_TABLE_PACKS = 7,         /* BlkPack: pipelined small-segment kernel */
     BLK_TABLE_PACK_BLOCKS = 8,   /* BlkPackBlock */
@@ -276,7 +276,10 @@ typedef enum {
     BLK_TABLE_SMX_WINDOWS = 10,  /* BlkSmxWindow */
     BLK_TABLE_FLASH_ITEMS = 11,  /* BlkFlashItem: tcgen05 attention kernel */
     BLK_TABLE_UMMA_VIEWS_A = 12, /* BlkUmmaView: views of the first operand the tcgen05 items refer to */
-    BLK_TABLE_UMMA_VIEWS_B = 13  /* BlkUmmaView: ... of the second operand */
+    BLK_TABLE_UMMA_VIEWS_B = 13, /* BlkUmmaView: ... of the second operand */
+    BLK_TABLE_SIMT_BIG = 14,     /* BlkTileItem: the fp32 SIMT kernel as it runs where some segments have 128 x 128 tiles: those ... */
+    BLK_TABLE_SIMT_REST = 15,    /* BlkTileItem: ... and the 64 x 64 tiles of the others */
+    BLK_TABLE_STREAM_ITEMS = 16  /* BlkUmmaItem: the tcgen05 items in the order the streams take them, where they run as streams */
 } blk_table_t;
 BLK_API int blk_plan_table(const blk_plan_t* plan, int table, void* dst, int64_t capacity, int64_t* bytes,
                            int64_t* record_bytes);

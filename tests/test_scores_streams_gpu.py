@@ -83,3 +83,30 @@ def test_rows_whose_offsets_exceed_32_bits_of_bytes(cuda_device, out_dtype, n):
     for c in range(0, n, 1 << 22):
         want = (a.double() @ b[c:c + (1 << 22)].double().T).to(out_dtype)
         assert torch.equal(got[:, c:c + (1 << 22)], want), f"columns from {c}"
+
+
+@pytest.mark.parametrize("out_dtype", [F16, F32])
+@pytest.mark.parametrize("scale", [1.0, -1.0])
+@pytest.mark.parametrize("size", [1.0, 300.0, 3000.0, 20000.0])
+def test_error_is_relative_to_the_differences(cuda_device, streams, out_dtype, scale, size):
+    """Probabilities of large scores that differ little.  The scores are exact: one product of `size`, the others of multiples of 1/4."""
+    cols = [1, 40, 64, 65, 128, 129, 300, 512, 513, 700]
+    rows, k = [37] * len(cols), [64] * len(cols)
+    g = torch.Generator().manual_seed(7)
+    A, B = ((torch.randint(-2, 3, (sum(x) * 64,), generator=g).float() / 4).view(-1, 64) for x in (rows, cols))
+    A[:, 0], B[:, 0] = 100.0, size / 100
+    A, B = A.half(), B.half()
+    plan = GemmPlan(rows, cols, k, 1, F16, out_dtype, softmax=True, device=cuda_device)
+    assert plan.table("stream_items").size == len(cols)
+    out = plan.run(A.view(1, -1).to(cuda_device), B.view(1, -1).to(cuda_device), scale=scale).cpu().double()
+    plan.check()
+    # scale * log2(e) is one 32-bit factor, rounded twice (2^-23); the exponent is rounded relative to itself and the exponential
+    # to 2^-22.  For results above 2^-10 of their row's largest, with exponents down to -10, (10 (2^-23 + 2^-24) ln 2 + 2^-22)
+    # for the element and as much again for the sum: 3e-6.  The inverse and its product: 2^-23.  16 bits: half a unit in the last
+    # place besides
+    tol = 3.2e-6 + (2.0 ** -11 if out_dtype == F16 else 0.0)
+    for got, a, b, n in zip(out[0].split([37 * c for c in cols]), A.double().split(rows), B.double().split(cols), cols):
+        want = torch.softmax(a @ b.T * scale, -1)
+        sure = (want >= want.amax(-1, keepdim=True) / 1024) & (want >= 2.0 ** -14)  # (below that a half is denormal)
+        err = ((got.view(37, n) - want).abs() / want)[sure].max().item()
+        assert err <= tol, f"{n} columns: relative error {err}"

@@ -68,7 +68,6 @@ blk_attn_bwd_small_kernel(const BlkAttnBwdSmallParams p) {
     const uint32_t unit = blockIdx.x, item = unit / (uint32_t)p.H;
     const int head = (int)(unit - item * (uint32_t)p.H);
     const BlkFlashItem it = p.items[item];
-    blk_grid_ready_if_few();
     blk_grid_wait();
     const int M = it.M, N = it.N, Mb = (M + 15) >> 4, Nb = (N + 15) >> 4;
     const int64_t offQ = ((int64_t)head * p.rows_q + it.rowQ) * D, offK = ((int64_t)head * p.rows_kv + it.rowKV) * D;

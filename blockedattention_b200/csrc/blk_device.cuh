@@ -68,12 +68,11 @@ __device__ __forceinline__ void blk_mma16816<BlkBf16Tag>(float (&d)[4], uint32_t
 // a plan are there before any launch and may be read earlier.  blk_grid_ready lets the next kernel of the stream come: to be called
 // when the block holds all it will ever need of its SM (tensor memory), or the next one's blocks could take what it waits for.
 __device__ __forceinline__ void blk_grid_ready() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-// For kernels with several blocks on an SM: only a grid of at most one block per SM.  Blocks of the next kernel that come while
-// those of a larger one are still there settle where there happens to be room, several on one SM (36 products of up to 369 rows
-// and columns on the staged kernel, 14.3 us one after the other: 17.1, without this 11.7).
-__device__ __forceinline__ void blk_grid_ready_if_few() {
-    if (gridDim.x <= 148u) blk_grid_ready();
-}
+// Kernels with several blocks on an SM never call it: their blocks let the next kernel come by ending.  Blocks of the next one that
+// come while these are still there settle where there happens to be room, several on one SM.  Announced from the start by grids
+// of at most a block per SM, us against this: 148 products of 60 rows and columns over 2001 on the staged kernel 90.5 -> 63.2
+// (one after the other 65.5), its fused softmax for 9 segments of 1000 123.7 -> 97.3 (99.6); nothing gained over 33 to 1001
+// either (3.6 to 33 us, both the same within 0.3).
 __device__ __forceinline__ void blk_grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t blk_smem_u32(const void* p) {

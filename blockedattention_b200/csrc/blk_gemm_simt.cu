@@ -74,7 +74,6 @@ __global__ void __launch_bounds__(SNT, TM == 8 ? 2 : 4) blk_gemm_simt_kernel(con
     const int head = (int)(bid / p.num_items);
     const BlkTileItem it = p.items[bid % p.num_items];
     const BlkSeg sd = p.segs[it.seg];
-    blk_grid_ready_if_few();
     blk_grid_wait();
     const int64_t baseA = (int64_t)head * p.Dm1 + sd.offA, baseB = (int64_t)head * p.Dm2 + sd.offB;
     const float* gA = p.A + baseA;

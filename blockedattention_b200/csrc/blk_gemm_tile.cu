@@ -344,7 +344,6 @@ __global__ void __launch_bounds__(SOFTMAX ? NT : NT_SC, 3) blk_gemm_tile_kernel(
     const BlkTileRec rec = p.recs[bid % p.num_items];
     const BlkTileItem it = rec.it;
     const BlkSeg sd = rec.sd;
-    blk_grid_ready_if_few();
     blk_grid_wait();
     const int64_t baseA = (int64_t)head * p.Dm1 + sd.offA, baseB = (int64_t)head * p.Dm2 + sd.offB;
     const int64_t cbase = (int64_t)head * p.Dout + sd.offC;

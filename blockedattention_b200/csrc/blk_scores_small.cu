@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(SW * 32, MinBlocks<NTMAX>::value) blk_scores_s
     const bool flip = p.scale < 0.f;
     const float sl = SOFTMAX ? fabsf(p.scale) * BLK_LOG2E : p.scale;
     unsigned char* strip = strips + warp * STRIP;
-    blk_grid_ready_if_few();
     blk_grid_wait();
 
     for (uint32_t w = blockIdx.x * SW + warp; w < total; w += stride) {

@@ -136,7 +136,6 @@ __global__ void __launch_bounds__(SMX_THREADS) blk_softmax_kernel(const BlkSmxPa
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t bid = blockIdx.x;
     const int head = (int)(bid / p.num_chunks);
-    blk_grid_ready_if_few();
     blk_grid_wait();  // (the table of a call without plan memory goes up in the stream)
     const BlkSmxChunk ch = p.chunks[bid % p.num_chunks];
     const int64_t e0 = (int64_t)head * p.D + ch.off;

@@ -659,7 +659,6 @@ __global__ void __launch_bounds__(SpShape<BWD>::THREADS, SpShape<BWD>::CTAS) blk
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    blk_grid_ready_if_few();
     blk_grid_wait();
 
     const E* g0 = reinterpret_cast<const E*>(p.in0);

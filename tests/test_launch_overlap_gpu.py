@@ -101,3 +101,36 @@ def test_training_steps_without_waiting_and_captured(hi, d):
         torch.cuda.synchronize()
         for a, b in zip(expect, got):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("S,n,k,softmax", [(148, 60, 2001, False), (9, 1000, 65, True), (148, 60, 65, False)])
+def test_an_early_start_costs_no_time(S, n, k, softmax):
+    """Launches of one block per SM: blocks of the next kernel that settle unevenly, several on one SM, would take up to half as long
+    again.  Compared with launches that a kernel of torch's, which announces nothing, keeps apart."""
+    from blockedattention_b200.plan import GemmPlan
+
+    g = torch.Generator("cuda").manual_seed(1)
+    plan = GemmPlan([n] * S, [n] * S, [k] * S, 1, torch.float16, softmax=softmax, device="cuda")
+    assert plan.summary["tile_items"] > 0 and plan.summary["launches"] == 1
+    a, b = (torch.randn((1, d), device="cuda", generator=g).half() for d in (plan.Dm1, plan.Dm2))
+    out = torch.empty((1, plan.Dout), dtype=torch.float16, device="cuda")
+    small = torch.empty(1, device="cuda")
+
+    def measure(apart):
+        t = []
+        for _ in range(9):
+            x, y = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            torch.cuda._sleep(2000000)  # the launches are queued before the first one runs
+            x.record()
+            for _ in range(50):
+                plan.run(a, b, out=out)
+                if apart:
+                    small.zero_()
+            y.record()
+            torch.cuda.synchronize()
+            t.append(x.elapsed_time(y))
+        return sorted(t)[4]
+
+    measure(False)
+    assert measure(False) <= 1.1 * measure(True)

@@ -339,8 +339,9 @@ class Runner:
         if self.fused_attn:
             return "blk_attn_umma_kernel" if s["umma_items"] else "blk_scores_pipe_kernel"
         small = "blk_scores_pipe_kernel" if s["packs"] else "blk_scores_small_kernel"
+        umma = "blk_scores_umma_kernel" if self.plan.table("stream_items").size else "blk_gemm_umma_kernel"
         return max(((small, s["small_items"]), ("blk_gemm_tile_kernel", s["tile_items"]),
-                    ("blk_gemm_umma_kernel", s["umma_items"]), ("blk_gemm_simt_kernel", s["simt_items"])),
+                    (umma, s["umma_items"]), ("blk_gemm_simt_kernel", s["simt_items"])),
                    key=lambda kv: kv[1])[0]
 
     def check(self):

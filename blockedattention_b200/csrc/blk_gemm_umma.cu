@@ -29,7 +29,7 @@
 // second sweep of an item alternates chunk by chunk with the first sweep of the next, all four groups taking chunks of both.
 //
 // Large batches of short contractions, plain or with rows beyond 512 columns, run on the kernel of independent streams instead
-// (blk_scores_umma.cu; the second of the following then takes 755).
+// (blk_scores_umma.cu; the second of the following then takes 757).
 //
 // Measured against one item at a time with 8 arithmetic and 4 store warps: scores + softmax of 1024 segments of 64..512 rows,
 // 16 heads, K = 128: 2054 -> 1532 us; of 512 segments of 16..2048 rows, 4 heads, K = 64 (two sweeps): 872 -> 897 us

@@ -586,7 +586,7 @@ int blk_build_gemm_schedule(blk_plan* p) {
             if (it.tm || it.tn || !is_big(it.seg)) continue;
             tiles += up(p->segs[it.seg].M, 128) * up(p->segs[it.seg].N, 128);
         }
-        if (tiles * p->H >= 148) {
+        if (tiles * p->H >= p->num_sms) {
             p->simt_big.reserve(tiles);
             for (const BlkTileItem& it : p->simt_items) {
                 if (!is_big(it.seg)) { p->simt_rest.push_back(it); continue; }
@@ -600,9 +600,10 @@ int blk_build_gemm_schedule(blk_plan* p) {
     // streams to be busy and in different phases; below that the other kernel, whose warps share an item, is done sooner.
     // With a softmax it is the better one only for rows that the other kernel computes twice as well (beyond 512 columns), which
     // have to carry most of the work, and for K up to 64 (four streams; three are slower).  us, other kernel -> streams:
-    // plain bf16 scores, K = 64: 3 600 tiles 20.7 -> 24.8, 7 700 49.4 -> 47.7, 17 000 75 -> 65, 43 000 211 -> 150; fp32 of
-    // mixed K up to 128: 3 900 38.5 -> 43.3, 7 700 71.2 -> 70.5, 29 000 271 -> 233; softmax, K = 64: rows up to 512
-    // 170 -> 184, up to 2048 242 -> 222 (and 898 -> 755 for four times as many), K = 128 267 -> 288.
+    // plain bf16 scores, K = 64: 3 600 tiles 20.7 -> 24.8, 7 700 49.4 -> 47.7, 17 000 75 -> 65, 43 000 211 -> 150; fp32 results of
+    // mixed K up to 128: 3 900 38.5 -> 43.3, 7 700 71.2 -> 70.5, 29 000 271 -> 233 (even, within what
+    // boards differ by, at the line); softmax, K = 64: rows up to 512 170 -> 184, up to 2048 190 -> 170 (and 820 -> 737 for four
+    // times as many), K = 128 267 -> 288.
     p->stream_items.clear();
     if (!p->umma_items.empty() && !p->umma_wide) {
         int64_t K = 0, tiles = 0, tiles_long = 0;

@@ -167,16 +167,25 @@ struct BlkSmxParams {
     float scale;
 };
 
-// Grids of one-shot blocks up to which blk_launch is asked for an early start: several waves of them run up to an eighth slower
-// when launched that way (385 products of 256..1216 rows on the staged kernel 5238 -> 5880 us).
+// Grids of one-shot blocks up to which blk_launch is asked for an early start.  What it saves is the same 2 us a launch on both sides
+// of the line as long as blocks are alike: products of 60 rows and columns over 100 on the staged kernel 8.2 -> 6.4 us for 296 blocks,
+// 10.3 -> 7.5 for 444, 22.4 -> 19.6 for 1184, 39.1 -> 37.4 for 2368; fp32 ones of 64 over 64 9.9 -> 7.2, 12.2 -> 9.3, 24.6 -> 21.8,
+// 47.4 -> 45.3.  Several waves of unlike blocks lose up to an eighth (385 products of 256..1216 rows on the staged kernel
+// 5238 -> 5880 us): the line is low for their sake.
 constexpr unsigned BLK_EARLY_GRID = 296;
 
 // Launches a kernel that waits by itself for the one in front of it (blk_grid_wait): its start -- the launch, barriers, tensor
 // memory -- overlaps the end of that one.  Passes one after the other, us: 32 fp32 products and softmaxes of at most 32 x 32 x 32 (two
 // launches) 12.3 -> 8.7, attention of 16 graphs 8.2 -> 6.0, forward and backward of 1024 graphs (three launches) 84.5 -> 79.1.
-// early = false: an ordinary launch.  Persistent kernels of the tensor cores ask for it from about 100 us on, where nothing is
-// gained: blocks that come one by one where an SM is free lie on the chip in no order, and neighbours in the list of items, which
-// read the same operands, no longer share a part of the L2 (64 products of 1024..2048 rows and columns 839 -> 850 and 865 us).
+// early = false: an ordinary launch.  Persistent kernels of the tensor cores ask for that beyond a number of items per SM that is a
+// launch of 45 us for short items and 200 to 450 for long ones: the 2 us that are saved are below 2 % there, and blocks that come
+// one by one where an SM is free lie on the chip in no order, so that neighbours in the list of items, which read the same
+// operands, may no longer share a part of the L2 (64 products of 1024..2048 rows and columns, long contractions: 839 -> 850 and
+// 865 us).  Ordinary -> early at the lines, items of segments of 256 and of 1024 rows: attention, 12 items an SM, 95.0 -> 93.5 us and
+// 234 -> 230; with its backward 231 -> 230 and 564 -> 559; P V, 12, 46.4 -> 45.8 and 126 -> 122; plain scores, 24, streams 90.8 -> 88.9
+// and 332 -> 330, grouped 82.3 -> 80.4 and 279 -> 274; softmax, 24, streams 123.5 -> 121.5 and 462 -> 460, grouped 92.5 -> 89.1 and
+// 439 -> 435; long contractions of 1024 and 4096, 4, 51.8 -> 51.4 and 181 -> 179.  Four times as many items: all within 1.8 % either
+// way, less than their runs differ by.
 template <typename... P>
 inline cudaError_t blk_launch(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
     cudaLaunchAttribute attr[1];

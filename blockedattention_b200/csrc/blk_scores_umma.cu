@@ -25,9 +25,10 @@
 // between the sweeps), so the other kernel keeps those.
 //
 // Measured, us, the other kernel -> this one: plain bf16 scores of 128 segments of 16..2048 rows, 4 heads, K = 64: 168 -> 121 (3.7
-// of the 4.8 TB/s that such rows can be written at); their softmax for 512 segments: 898 -> 755.  What bounds the softmax: exponentials
-// (two per element, the unit 57 % busy), 53 % of the issue slots, the shared-memory path; without exponentials 676, without
-// stores 674.  Bulk copies from the strips in place of the stores: 917, they queue in front of the operands' copies.
+// of the 4.8 TB/s that such rows can be written at); their softmax for 512 segments: 898 -> 757 (743 with the logarithm of
+// a row's sum in the exponent instead of a division, see below).  What bounds the softmax: exponentials (two per element, the unit
+// 65 % busy in a single launch), 58 % of the issue slots, the shared-memory path; of 810 us, when that was its time, 676 were left without
+// exponentials and 674 without stores.  Bulk copies from the strips in place of the stores: 917, they queue in front of the operands' copies.
 //
 // Every wait on an mbarrier is bounded: when the bound is hit the kernel records a status code, all roles leave their
 // loops, tensor memory is released and the kernel returns.  Rows past the end of a segment belong to its neighbour (or are
@@ -437,7 +438,8 @@ blk_scores_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps map
                 if (!stay) acc += (uint32_t)tiles;
                 // exp2(x sl + off) / sum with the offset that the sum was made with: its rounding, which is that of the scores' own
                 // size, is the same for both and cancels.  (With the sum's logarithm in the offset it does not: up to 7e-4 of a
-                // probability for scores of 20000, more than the rounding of a half.)
+                // probability for scores of 20000, more than the rounding of a half.  A choice between the two by the size of the
+                // offset took as long as the division always.)
                 const float off = ref == -INFINITY ? 0.f : -ref * sl, inv = __frcp_rn(sum);
                 inv2 = make_float2(inv, inv);
                 off2 = make_float2(off, off);

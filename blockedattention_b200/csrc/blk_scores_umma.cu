@@ -55,6 +55,7 @@ constexpr float SS_LAZY = 32.f;         // exponent slack before a softmax refer
 // Strip of an epilogue warp: 32 row pieces of 128 bytes and the sector that a first element inside a sector pushes past the
 // end, and for each row the sector that it begins in.
 constexpr int SS_PITCH = 160;
+constexpr uint64_t SS_NEAR = 0xffffffffull / 32;  // rows of so many bytes: 31 of them and a sector are within 32 bits
 constexpr int SS_HEADS = 32 * SS_PITCH;
 constexpr int SS_STRIP_BYTES = SS_HEADS + 32 * 32;
 
@@ -130,8 +131,8 @@ __device__ __forceinline__ void store_sectors(uint32_t strip, uint64_t r0, uint3
         }
     }
 }
-// The same for the whole piece of 32 rows: the lane's part of row lane / 8 + 4 i goes `goes[i]` sectors past origin.  (Counted in
-// sectors, since 31 rows of up to 2^32 bytes are beyond 32 bits of bytes.)
+// The same for the whole piece of 32 rows of at most SS_NEAR bytes: the lane's part of row lane / 8 + 4 i goes `goes[i]` bytes past
+// origin.
 __device__ __forceinline__ void store_sectors_all(uint32_t from, uint32_t o1, uint32_t o2, uint64_t origin, const uint32_t (&goes)[8]) {
 #pragma unroll
     for (int t = 0; t < 8; t += 4) {
@@ -142,7 +143,7 @@ __device__ __forceinline__ void store_sectors_all(uint32_t from, uint32_t o1, ui
         w[2] = lds_v4(at + o2);
         w[3] = lds_v4(at + o1 + o2);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) stg_v4(origin + 32ull * goes[t + i], w[i]);
+        for (int i = 0; i < 4; ++i) stg_v4(origin + goes[t + i], w[i]);
     }
 }
 // Element i of a strip row (32-byte aligned base `from`), to p.
@@ -448,11 +449,14 @@ blk_scores_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps map
             const uint64_t pitch = (uint64_t)N * E;
             uint64_t own = base + (uint64_t)lane * pitch;                  // this lane's row ...
             uint64_t quarter = base + (uint64_t)(lane >> 3) * pitch;       // ... and row lane / 8, at the piece's first column
-            // where this lane's halves of sectors go: in the first row, and the sectors from there to rows lane / 8 + 4 i
+            // where this lane's halves of sectors go: in the first row, and the bytes from there to rows lane / 8 + 4 i, which fit 32
+            // bits for rows that are not longer than SS_NEAR (others take the general way out; offsets counted in sectors, for rows
+            // of any length, took 714.5 us for the softmax of 512 segments of 16..2048 rows where this takes 710.5)
+            const bool near = pitch <= SS_NEAR;
             uint64_t origin = (base & ~31ull) + 16u * ((uint32_t)lane & 7u);
             uint32_t goes[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) goes[i] = (uint32_t)((quarter - (base & ~31ull) + 4ull * i * pitch) >> 5);
+            for (uint32_t i = 0; i < 8; ++i) goes[i] = ((uint32_t)base & 31u) + ((uint32_t)(lane >> 3) + 4u * i) * (uint32_t)pitch & ~31u;
             const uint32_t phase = (uint32_t)own & 31u;                    // how far into a sector the row starts
             const bool odd16 = !OUT32 && (N & 1);
             const bool anyodd = !OUT32 && __any_sync(0xffffffffu, (int)(phase & 2u));
@@ -516,7 +520,7 @@ blk_scores_umma_kernel(const BlkUmmaParams p, const __grid_constant__ UmMaps map
                     __syncwarp();
                     return;
                 }
-                if (rows == 32 && cols >= PC && !(first && shifted))
+                if (near && rows == 32 && cols >= PC && !(first && shifted))
                     store_sectors_all(from, o1, o2, origin, goes);
                 else
                     store_sectors<E>(strip, quarter, (uint32_t)pitch, first ? 0 : -SE, cols, rows, odd16, lane);
